@@ -431,6 +431,86 @@ int b200pf_add_bf16(float* z, const b200pf_bf16* upd, long long n_elems, void* s
 int b200pf_peer_barrier(const unsigned long long* pad_ptrs, unsigned int generation, int rank, int world,
                         long long timeout_ns, void* stream);
 
+/* ------------------------------------------------------------------------------------------
+ * fp32-accurate tensor-core path: every fp32 factor is multiplied as a sum of 16-bit parts (two fp16 parts of a scaled
+ * value for linear layers, three bf16 parts for attention, the triangle contraction and unbounded inputs), fp32
+ * accumulation.  Widths that are multiples of 64 (64, 128, 256; 384 without head projections).  It carries the single
+ * track of every tier and the pair track of the fp32 tier.
+ * ---------------------------------------------------------------------------------------- */
+
+/* A linear layer's weights w[n][k]: two fp16 parts [2][n][k] of w * scale_w; alpha = 1 / (scale_w * scale of the operand). */
+typedef struct b200pf_split_weight {
+    const void* w;
+    float       alpha;
+} b200pf_split_weight;
+
+/* LayerNorm gains and offsets below are given times the scale of the planes they produce. */
+typedef struct b200pf_single_track_weights {
+    const float *ln_gamma, *ln_beta;
+    b200pf_split_weight qkvg;       /* rows q (times log2 e / sqrt(head width)) | k | v | g: [4 c_s][c_s] */
+    const float* qkvg_bias;         /* [4 c_s], q part scaled like its rows */
+    b200pf_split_weight o;          /* [c_s][c_s] */
+    float o_scale;                  /* scale of the gated attention output's parts */
+    const float *ln2_gamma, *ln2_beta;
+    b200pf_split_weight fc12;       /* 32 rows of fc1, then 32 of fc2, in turn: [2 hidden][c_s] */
+    float hidden_scale;             /* scale of the hidden activations' parts */
+    b200pf_split_weight fc3;        /* [c_s][hidden] */
+    int cs, heads, hidden;
+} b200pf_single_track_weights;
+
+/* Bytes of workspace for n tokens. */
+long long b200pf_single_track_workspace(int n, int cs, int hidden);
+/* Parts [2][nq][c_s] of sigmoid(g) * softmax(q k^T + bias + mask) v for the query rows q0 .. q0 + nq - 1
+ * (AttentionPairBias without its output projection, tt_bio/boltz2.py:351-366); bias[h][q - q0][key] times log2 e;
+ * mask[n] (NULL: none masked). */
+int b200pf_single_track_attention(const float* s, const b200pf_single_track_weights* w, const float* bias, const uint8_t* mask, void* og,
+                                  int n, int q0, int nq, void* workspace, void* stream);
+/* s[rows] += og W_o^T; s += Transition(s)  (tt_bio/reference.py:906-912). */
+int b200pf_single_track_finish(float* s, const b200pf_single_track_weights* w, const void* og, int rows, void* workspace, void* stream);
+
+typedef struct b200pf_split_trimul_weights {
+    const float *ln_in_gamma, *ln_in_beta;
+    b200pf_split_weight in;         /* p_in rows, then g_in rows: [4 c][c] */
+    const float *ln_out_gamma, *ln_out_beta;
+    b200pf_split_weight p_out, g_out;
+    int c;
+} b200pf_split_trimul_weights;
+typedef struct b200pf_split_triatt_weights {
+    const float *ln_gamma, *ln_beta;
+    const float* head_w;            /* [heads][c] times log2 e over the planes' scale */
+    b200pf_split_weight qkvg;       /* as in the single track: [4 heads hd][c] */
+    b200pf_split_weight o;          /* [c][heads hd] */
+    float o_scale;
+    int c, heads, hd;
+} b200pf_split_triatt_weights;
+typedef struct b200pf_split_transition_weights {
+    const float *ln_gamma, *ln_beta;
+    b200pf_split_weight fc12, fc3;
+    float hidden_scale;
+    int c, hidden;
+} b200pf_split_transition_weights;
+
+/* Bytes of workspace for a pair tensor [n][n][c]; heads = 0: no attention. */
+long long b200pf_split_pair_workspace(int n, int c, int heads, int hd, int hidden);
+/* z += TriangleMultiplication(z) (tt_bio/reference.py:456-470, 545-559); mask [n][n]. */
+int b200pf_split_tri_mul(float* z, const uint8_t* mask, const b200pf_split_trimul_weights* w, int n, int incoming, void* workspace, void* stream);
+/* z += TriangleAttention(z) (tt_bio/reference.py:326-363); mask [n][n]. */
+int b200pf_split_tri_att(float* z, const uint8_t* mask, const b200pf_split_triatt_weights* w, int n, int ending, void* workspace, void* stream);
+/* x[rows] += Transition(x) (tt_bio/boltz2.py:1241-1246). */
+int b200pf_split_transition(float* x, long long rows, const b200pf_split_transition_weights* w, void* workspace, void* stream);
+
+/* out[h * head_stride + row] = <LN(x[row]), w[h]> in fp32, 4, 8 or 16 heads (tt_bio/boltz2.py:326-330). */
+int b200pf_ln_heads(const float* x, const float* gamma, const float* beta, const float* w, float* out, long long head_stride, long long rows,
+                    int c, int heads, void* stream);
+/* y[rows][n] (+)= x[rows][k] w[n][k]^T (+ bias) for any finite fp32 x; w as three bf16 parts [3][n][k]; k % 8 == 0, n % 4 == 0. */
+long long b200pf_split_linear_workspace(long long rows, int k);
+int b200pf_split_linear(const float* x, const void* w, const float* bias, float* y, long long rows, int k, int n, int accumulate,
+                        void* workspace, void* stream);
+/* y[rows][n] += LN(x)[rows][c] w[n][c]^T (the recycling projections, tt_bio/boltz2.py:5207-5208). */
+long long b200pf_split_ln_linear_workspace(long long rows, int c);
+int b200pf_split_ln_linear_add(const float* x, const float* gamma, const float* beta, const b200pf_split_weight* w, float* y, long long rows,
+                               int c, int n, void* workspace, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -34,6 +34,35 @@ class PlaneOut(C.Structure):
     _fields_ = [("ptr", _vp), ("plane_stride", _ll), ("group_stride", _ll), ("row_group", _i)]
 
 
+class SplitWeight(C.Structure):
+    """Mirror of ``b200pf_split_weight``."""
+    _fields_ = [("w", _vp), ("alpha", _f)]
+
+
+class SingleTrackWeights(C.Structure):
+    """Mirror of ``b200pf_single_track_weights``."""
+    _fields_ = [("ln_gamma", _vp), ("ln_beta", _vp), ("qkvg", SplitWeight), ("qkvg_bias", _vp), ("o", SplitWeight), ("o_scale", _f),
+                ("ln2_gamma", _vp), ("ln2_beta", _vp), ("fc12", SplitWeight), ("hidden_scale", _f), ("fc3", SplitWeight),
+                ("cs", _i), ("heads", _i), ("hidden", _i)]
+
+
+class SplitTriMulWeights(C.Structure):
+    """Mirror of ``b200pf_split_trimul_weights``."""
+    _fields_ = [("ln_in_gamma", _vp), ("ln_in_beta", _vp), ("inp", SplitWeight), ("ln_out_gamma", _vp), ("ln_out_beta", _vp),
+                ("p_out", SplitWeight), ("g_out", SplitWeight), ("c", _i)]
+
+
+class SplitTriAttWeights(C.Structure):
+    """Mirror of ``b200pf_split_triatt_weights``."""
+    _fields_ = [("ln_gamma", _vp), ("ln_beta", _vp), ("head_w", _vp), ("qkvg", SplitWeight), ("o", SplitWeight), ("o_scale", _f),
+                ("c", _i), ("heads", _i), ("hd", _i)]
+
+
+class SplitTransitionWeights(C.Structure):
+    """Mirror of ``b200pf_split_transition_weights``."""
+    _fields_ = [("ln_gamma", _vp), ("ln_beta", _vp), ("fc12", SplitWeight), ("fc3", SplitWeight), ("hidden_scale", _f), ("c", _i), ("hidden", _i)]
+
+
 # name -> argtypes (all return int unless listed in _RESTYPES)
 SIGNATURES = {
     "b200pf_version": [],
@@ -84,8 +113,22 @@ SIGNATURES = {
     "b200pf_peer_broadcast_sync": [_vp, C.POINTER(C.c_ulonglong), _ll, _i, _i, C.POINTER(PeerSync), _vp],
     "b200pf_peer_scatter_strided_sync": [_vp, C.POINTER(C.c_ulonglong), _ll, _i, _ll, _ll, _ll, _ll, _i, _i, C.POINTER(PeerSync), _vp],
     "b200pf_tri_mul_noalloc": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp],
+    "b200pf_single_track_workspace": [_i, _i, _i],
+    "b200pf_single_track_attention": [_vp, C.POINTER(SingleTrackWeights), _vp, _vp, _vp, _i, _i, _i, _vp, _vp],
+    "b200pf_single_track_finish": [_vp, C.POINTER(SingleTrackWeights), _vp, _i, _vp, _vp],
+    "b200pf_split_pair_workspace": [_i, _i, _i, _i, _i],
+    "b200pf_split_tri_mul": [_vp, _vp, C.POINTER(SplitTriMulWeights), _i, _i, _vp, _vp],
+    "b200pf_split_tri_att": [_vp, _vp, C.POINTER(SplitTriAttWeights), _i, _i, _vp, _vp],
+    "b200pf_split_transition": [_vp, _ll, C.POINTER(SplitTransitionWeights), _vp, _vp],
+    "b200pf_ln_heads": [_vp, _vp, _vp, _vp, _vp, _ll, _ll, _i, _i, _vp],
+    "b200pf_split_linear_workspace": [_ll, _i],
+    "b200pf_split_linear": [_vp, _vp, _vp, _vp, _ll, _i, _i, _i, _vp, _vp],
+    "b200pf_split_ln_linear_workspace": [_ll, _i],
+    "b200pf_split_ln_linear_add": [_vp, _vp, _vp, C.POINTER(SplitWeight), _vp, _ll, _i, _i, _vp, _vp],
 }
-_RESTYPES = {"b200pf_last_error": C.c_char_p, "b200pf_launch_count": _ll, "b200pf_mx_scale_bytes": _ll}
+_RESTYPES = {"b200pf_single_track_workspace": _ll, "b200pf_split_pair_workspace": _ll, "b200pf_split_linear_workspace": _ll,
+             "b200pf_split_ln_linear_workspace": _ll,
+             "b200pf_last_error": C.c_char_p, "b200pf_launch_count": _ll, "b200pf_mx_scale_bytes": _ll}
 
 _lib: Optional[C.CDLL] = None
 

@@ -1,0 +1,102 @@
+// Operands of the fp32-accurate tensor-core path: an fp32 value kept as a sum of 16-bit parts.
+//
+//   F16X2   v * scale = hi + lo, two fp16 parts (22 bits: what a 3xTF32 product keeps).  `scale` is a power of two chosen
+//           when the weights are packed from a bound of |v| (a LayerNorm output is at most sqrt(C) * gain + offset, a
+//           projection of it at most that times the row norm), so neither part can overflow and `lo` keeps its 11 bits
+//           down to 2^-17 of the bound.  Products: hi*hi + hi*lo + lo*hi, three MMAs.
+//   BF16X3  v = h + m + l, three bf16 parts (24 bits, the whole fp32 mantissa, and fp32's own range: no scale).
+//           Products of total order <= 2: six MMAs.
+// Both accumulate in fp32.  A plane stack is [parts][rows][cols] of 16-bit values.
+#pragma once
+
+#include <cuda_fp16.h>
+
+#include "sm100.cuh"
+
+namespace b200pf {
+namespace split {
+
+// ---- programmatic dependent launch ---------------------------------------------------------------
+// A kernel launched with launch_pdl may start while its predecessor on the stream drains: everything before
+// grid_dependency_wait() (barriers, tensor memory, descriptors) overlaps the predecessor's tail; nothing the
+// predecessor wrote, or reads, may be touched before it.  Kernels launched this way read global memory with plain loads only:
+// an ld.global.nc (__ldg, const __restrict__) may be moved above the wait.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
+    __half2 t = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&t);
+}
+// Two values into fp16 part words {hi, lo}.
+__device__ __forceinline__ void split_f16x2(float a, float b, uint32_t& hi, uint32_t& lo) {
+    hi = pack_f16x2(a, b);
+    const float2 f = __half22float2(*reinterpret_cast<__half2*>(&hi));
+    lo = pack_f16x2(a - f.x, b - f.y);
+}
+// Two values into bf16 part words {h, m, l}.
+__device__ __forceinline__ void split_bf16x3(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
+    h = pack_bf16x2(a, b);
+    const float ra = a - bf16_lo(h), rb = b - bf16_hi(h);
+    m = pack_bf16x2(ra, rb);
+    l = pack_bf16x2(ra - bf16_lo(m), rb - bf16_hi(m));
+}
+
+// ---- host side -----------------------------------------------------------------------------------
+template <class... KArgs, class... Args>
+static inline int launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    B200PF_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+    count_launch();
+    return B200PF_OK;
+}
+
+// Two-part (fp16) or three-part (bf16) operand of a GEMM: element (part, batch, row, col) at
+// ptr + part * part_stride + batch * batch_stride + row * row_stride + col (16-bit elements; strides multiples of 8).
+struct Operand {
+    const void* ptr;
+    int rows, cols, batches;
+    long long row_stride, batch_stride, part_stride;
+};
+// Output of a GEMM: element (part, batch, row, col), strides in elements of its type; `rows_outer` swaps the roles of row and
+// batch in memory order only (the operand planes of a triangle multiplication, [channel][line][position], with
+// row = channel and batch = line).
+struct Output {
+    void* ptr;
+    int rows, cols, batches, parts;
+    long long row_stride, batch_stride, part_stride;
+    bool rows_outer;
+};
+
+enum Epilogue { EPI_STORE, EPI_ADD, EPI_SWIGLU, EPI_QKVG, EPI_GATE_PLANES, EPI_GATE_ADD };
+
+struct Gemm {
+    int parts = 2;                  // 2: F16X2, 3: BF16X3
+    Epilogue epi = EPI_STORE;
+    Operand a[2], b[2];             // second pair: EPI_GATE_ADD (its own K loop and accumulator)
+    bool a_batched = false, b_batched = false;
+    int a_second_row = 0;           // EPI_GATE_PLANES: row offset of the gate rows in A
+    int m_rows = 0, n_rows = 0, batches = 1;
+    int k[2] = {0, 0};
+    int k_splits = 1;               // > 1: batch index = K split, partial sums stored per batch (EPI_STORE only)
+    float alpha[2] = {1.f, 1.f};
+    float out_scale = 1.f;          // EPI_SWIGLU: scale of the stored parts
+    const float* bias = nullptr;    // [n_rows]
+    const uint8_t* mask = nullptr;  // EPI_GATE_PLANES: position (batch, col) at mask + batch * mask_bs + col * mask_cs
+    long long mask_bs = 0, mask_cs = 0;
+    int n_split = 0;                // EPI_QKVG: columns below it go out as three bf16 parts, the others as sigmoid, fp32
+    Output out[2];
+};
+int launch_gemm(const Gemm& g, cudaStream_t st);
+
+}  // namespace split
+}  // namespace b200pf

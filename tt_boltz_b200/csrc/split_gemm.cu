@@ -1,0 +1,407 @@
+// GEMM at fp32 accuracy on the 5th-generation tensor cores: D[m][n] = sum_k A[m][k] B[n][k] with A and B given as 16-bit
+// part planes (split.cuh) and fp32 accumulation in tensor memory.
+//
+// One k-block of 64 brings every part of both operands into shared memory once and multiplies them three (fp16 parts) or
+// six (bf16 parts) times, so the kernel asks L2 for a half / a third of the bytes per MMA of a plain bf16 GEMM and is bound
+// by the tensor pipe for large K, by its epilogue for K = 64, and by latency for the single track's few hundred rows.
+// Persistent, warp-specialised: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 epilogue (two warps per TMEM lane quarter,
+// each half of the columns).  Two accumulator sets let the epilogue of a tile run under the next tile's MMAs.  Every result
+// leaves through a swizzled staging slot per warp and a TMA store (or reduce-add), which also clips ragged edges.
+#include "split.cuh"
+#include "tmap.cuh"
+
+namespace b200pf {
+namespace split {
+
+constexpr int THREADS = 320, EPI_WARPS = 8, STG_BYTES = 4096;
+constexpr int SMEM_MAX = 232448, SMEM_FIXED = 1024 + 256 + EPI_WARPS * STG_BYTES;
+
+struct Dev {
+    int m_rows, n_rows, batches, bn;
+    int a_batched, b_batched, a_second_row;
+    int k[2], k_splits, kb_per_split;
+    float alpha[2], out_scale;
+    const float* bias;
+    const uint8_t* mask;
+    long long mask_bs, mask_cs;
+    int n_split, rows_outer, n_out;      // n_out: output columns
+};
+
+// Products of the parts, smallest first: (lo, hi), (hi, lo), (hi, hi) and (l, h), (m, m), (h, l), (m, h), (h, m), (h, h).
+constexpr int n_products(int pl) { return pl == 2 ? 3 : 6; }
+__host__ __device__ constexpr int product_a(int pl, int q) { return pl == 2 ? (q == 0 ? 1 : 0) : (q == 0 ? 2 : q == 1 || q == 3 ? 1 : 0); }
+__host__ __device__ constexpr int product_b(int pl, int q) { return pl == 2 ? (q == 1 ? 1 : 0) : (q == 2 ? 2 : q == 1 || q == 4 ? 1 : 0); }
+
+template <int PL> __host__ __device__ constexpr uint32_t make_idesc(int n) {
+    // fp32 accumulator; fp16 (0) or bf16 (1) operands, both K-major; M = 128
+    return (1u << 4) | (PL == 3 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+}
+constexpr int stage_bytes(int pl, int bn, int na) { return pl * (na * 128 + bn) * 128; }
+constexpr int stages_of(int pl, int bn, int na) {
+    int s = (SMEM_MAX - SMEM_FIXED) / stage_bytes(pl, bn, na);
+    return s > 4 ? 4 : s;
+}
+
+template <int PL, int BN, int NA, int NK, int EPI>
+__global__ void __launch_bounds__(THREADS, 1)
+split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CUtensorMap map_a1,
+                  const __grid_constant__ CUtensorMap map_b0, const __grid_constant__ CUtensorMap map_b1,
+                  const __grid_constant__ CUtensorMap map_o0, const __grid_constant__ CUtensorMap map_o1, Dev p, unsigned int* status) {
+    using namespace sm100;
+    // PL == 3: the leading product and the five small ones have an accumulator each.  The tensor core truncates when it
+    // aligns an addend, so every MMA into a running sum costs up to an ulp of that sum, all in one direction: with 6 K / 16
+    // of them in one accumulator a 300-long contraction was biased by 7e-7; the small products' sums have no ulps to lose.
+    constexpr bool SMALL = PL == 3;
+    constexpr int NACC = SMALL ? 2 : NA * NK, ACC_COLS = NACC * BN, TMEM_COLS = 2 * ACC_COLS;
+    constexpr int STAGES = stages_of(PL, BN, NA), A_PART = 128 * 128;
+    static_assert(STAGES >= 2 && TMEM_COLS <= 512, "tile too large");
+    constexpr int STAGE = stage_bytes(PL, BN, NA);
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* stg_base = smem + STAGES * STAGE;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(stg_base + EPI_WARPS * STG_BYTES);
+    uint64_t* full = bars;
+    uint64_t* empty = bars + STAGES;
+    uint64_t* acc_full = bars + 2 * STAGES;
+    uint64_t* acc_empty = acc_full + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int bn = p.bn;                                   // columns of a tile: a multiple of 32, at most BN
+    const int mt = (p.m_rows + 127) / 128, nt = (p.n_rows + bn - 1) / bn;
+    const long long tiles = (long long)p.batches * mt * nt;
+    const uint32_t b_part = (uint32_t)bn * 128;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], EPI_WARPS); }
+        *abort_flag = 0;
+        fence_barrier_init();
+        fence_proxy_async();
+    }
+    if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
+    if (warp == 0 && lane == 0) {
+        tma_prefetch_desc(&map_a0); tma_prefetch_desc(&map_b0); tma_prefetch_desc(&map_o0);
+        if (NK == 2) { tma_prefetch_desc(&map_a1); tma_prefetch_desc(&map_b1); }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    grid_dependency_wait();
+    grid_launch_dependents();
+
+    // k range of phase `ph` for batch `bt` in 64-wide blocks
+    auto kb_range = [&](int ph, int bt, int& kb0, int& kb1) {
+        const int total = (p.k[ph] + 63) / 64;
+        if (p.k_splits > 1) { kb0 = bt * p.kb_per_split; kb1 = min(total, kb0 + p.kb_per_split); }
+        else { kb0 = 0; kb1 = total; }
+    };
+
+    if (warp == 0 && lane == 0) {
+        uint32_t stage = 0, phase = 0;
+        bool ok = true;
+        for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+            const int bt = (int)(t / (mt * nt)), rem = (int)(t % (mt * nt));
+            const int m0 = (rem / nt) * 128, n0 = (rem % nt) * bn;
+            const int ba = p.a_batched ? bt : 0, bb = p.b_batched ? bt : 0;
+#pragma unroll
+            for (int ph = 0; ph < NK; ++ph) {
+                const CUtensorMap* ma = ph == 0 ? &map_a0 : &map_a1;
+                const CUtensorMap* mb = ph == 0 ? &map_b0 : &map_b1;
+                int kb0, kb1;
+                kb_range(ph, bt, kb0, kb1);
+                for (int kb = kb0; kb < kb1 && ok; ++kb) {
+                    ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag);
+                    if (!ok) break;
+                    uint8_t* sa = smem + stage * STAGE;
+                    uint8_t* sb = sa + NA * PL * A_PART;
+                    mbar_arrive_expect_tx(&full[stage], (uint32_t)(PL * (NA * A_PART)) + PL * b_part);
+#pragma unroll
+                    for (int pl = 0; pl < PL; ++pl) {
+#pragma unroll
+                        for (int na = 0; na < NA; ++na)
+                            tma_load_4d(sa + (na * PL + pl) * A_PART, ma, &full[stage], kb * 64, m0 + na * p.a_second_row, ba, pl);
+                        tma_load_4d(sb + pl * b_part, mb, &full[stage], kb * 64, n0, bb, pl);
+                    }
+                    if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                }
+            }
+        }
+        if (!ok) {   // give copies in flight time to land before the CTA's shared memory goes away
+            atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
+            uint64_t t0 = global_timer_ns();
+            while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = make_idesc<PL>(bn);
+        const uint64_t d0 = make_desc_k_sw128(smem_u32(smem));
+        uint32_t stage = 0, phase = 0, it = 0;
+        bool ok = true;
+        for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
+            const int bt = (int)(t / (mt * nt));
+            const uint32_t ab = it & 1;
+            ok = mbar_wait_warp(&acc_empty[ab], ((it >> 1) & 1) ^ 1, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int ph = 0; ph < NK; ++ph) {
+                int kb0, kb1;
+                kb_range(ph, bt, kb0, kb1);
+                for (int kb = kb0; kb < kb1 && ok; ++kb) {
+                    ok = mbar_wait_warp(&full[stage], phase, abort_flag);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const int ksteps = min(4, (p.k[ph] - kb * 64 + 15) >> 4);         // a short last block is zero-filled
+                    if (elect_one()) {
+                        const uint64_t da = d0 + stage * (uint64_t)(STAGE >> 4), db = da + ((NA * PL * A_PART) >> 4);
+#pragma unroll
+                        for (int q = 0; q < n_products(PL); ++q) {
+#pragma unroll
+                            for (int na = 0; na < NA; ++na) {
+                                const bool lead = q == n_products(PL) - 1;
+                                const uint32_t d = tmem_base + ab * ACC_COLS + (SMALL ? (lead ? 0 : BN) : (na + ph) * BN);
+                                const uint64_t xa = da + (na * PL + product_a(PL, q)) * (A_PART >> 4), xb = db + product_b(PL, q) * (b_part >> 4);
+#pragma unroll
+                                for (int kk = 0; kk < 4; ++kk)
+                                    if (kk < ksteps) umma_bf16(d, xa + kk * 2, xb + kk * 2, idesc, (kb > kb0 || kk > 0 || (q > 0 && !(SMALL && lead))) ? 1u : 0u);
+                            }
+                        }
+                        umma_commit(&empty[stage]);
+                        if (ph == NK - 1 && kb + 1 == kb1) umma_commit(&acc_full[ab]);
+                    }
+                    __syncwarp();
+                    if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                }
+            }
+        }
+        if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
+    } else if (warp >= 2) {
+        const int quarter = warp & 3, chalf = (warp - 2) >> 2;
+        uint8_t* stg = stg_base + (warp - 2) * STG_BYTES;
+        uint32_t it = 0, slot = 0;
+        bool ok = true;
+        // 32 rows x 32 fp32 values, 128-byte swizzle
+        auto put_f32 = [&](const float (&v)[32], const CUtensorMap* map, bool add, int c0, int c1, int c2) {
+            if (lane == 0) bulk_wait_read0();
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                *reinterpret_cast<float4*>(stg + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+                if (add) tma_reduce_add_4d(map, stg, c0, c1, c2, 0);
+                else tma_store_4d(map, stg, c0, c1, c2, 0);
+                bulk_commit();
+            }
+        };
+        // 32 rows x 32 16-bit values of one part, 64-byte swizzle, two slots in turn
+        auto put_part = [&](const uint32_t (&w)[16], const CUtensorMap* map, int c0, int c1, int c2, int part) {
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            __syncwarp();
+            uint8_t* s = stg + slot * 2048;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<uint4*>(s + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) { tma_store_4d(map, s, c0, c1, c2, part); bulk_commit(); }
+            slot ^= 1;
+        };
+        auto put_bf16x3 = [&](const float (&v)[32], const CUtensorMap* map, int c0, int c1, int c2) {
+            uint32_t w[3][16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) split_bf16x3(v[2 * e], v[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) put_part(w[q], map, c0, c1, c2, q);
+        };
+        for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
+            const int bt = (int)(t / (mt * nt)), rem = (int)(t % (mt * nt));
+            const int m0 = (rem / nt) * 128 + quarter * 32, n0 = (rem % nt) * bn;
+            const uint32_t ab = it & 1;
+            ok = mbar_wait(&acc_full[ab], (it >> 1) & 1, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t tb = tmem_base + ((uint32_t)(quarter * 32) << 16) + ab * ACC_COLS;
+            const int per = EPI == EPI_SWIGLU ? 64 : 32;                    // accumulator columns per round
+            const int rounds = bn / per, r0 = chalf ? (rounds + 1) / 2 : 0, r1 = chalf ? rounds : (rounds + 1) / 2;
+            if (m0 < p.m_rows) {
+#pragma unroll 1
+                for (int r = r0; r < r1; ++r) {
+                    const int col = n0 + r * per;
+                    if (col >= p.n_rows) break;
+                    uint32_t x[32], y[32];
+                    tmem_ld_32x32(tb + r * per, x);
+                    if (EPI == EPI_SWIGLU) tmem_ld_32x32(tb + r * per + 32, y);
+                    if (NACC == 2) tmem_ld_32x32(tb + BN + r * per, y);
+                    tmem_ld_wait();
+                    float v[32];
+                    if (EPI == EPI_STORE || EPI == EPI_ADD || EPI == EPI_QKVG) {
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) v[e] = (SMALL ? __uint_as_float(x[e]) + __uint_as_float(y[e]) : __uint_as_float(x[e])) * p.alpha[0];
+                        if (p.bias) {
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) v[e] += col + e < p.n_rows ? *(p.bias + col + e) : 0.f;
+                        }
+                        if (EPI == EPI_STORE) put_f32(v, &map_o0, false, col, m0, bt);
+                        else if (EPI == EPI_ADD) put_f32(v, &map_o0, true, col, m0, bt);
+                        else if (col < p.n_split) put_bf16x3(v, &map_o0, col, m0, bt);
+                        else {
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) v[e] = sigmoid_precise(v[e]);
+                            put_f32(v, &map_o1, false, col - p.n_split, m0, bt);
+                        }
+                    } else if (EPI == EPI_SWIGLU) {
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) {
+                            const float f1 = __uint_as_float(x[e]) * p.alpha[0], f2 = __uint_as_float(y[e]) * p.alpha[0];
+                            v[e] = f1 * sigmoid_precise(f1) * f2 * p.out_scale;
+                        }
+                        uint32_t w[2][16];
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) split_f16x2(v[2 * e], v[2 * e + 1], w[0][e], w[1][e]);
+                        put_part(w[0], &map_o0, col >> 1, m0, bt, 0);
+                        put_part(w[1], &map_o0, col >> 1, m0, bt, 1);
+                    } else if (EPI == EPI_GATE_PLANES) {
+                        const bool keep = col + lane < p.n_rows && *(p.mask + bt * p.mask_bs + (long long)(col + lane) * p.mask_cs) != 0;
+                        const uint32_t bits = __ballot_sync(0xffffffffu, keep);
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) {
+                            const float u = __uint_as_float(x[e]) * p.alpha[0] * sigmoid_precise(__uint_as_float(y[e]) * p.alpha[0]);
+                            v[e] = (bits >> e) & 1u ? u : 0.f;
+                        }
+                        put_bf16x3(v, &map_o0, col, bt, m0);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 32; ++e)
+                            v[e] = __uint_as_float(x[e]) * p.alpha[0] * sigmoid_precise(__uint_as_float(y[e]) * p.alpha[1]);
+                        put_f32(v, &map_o0, true, col, m0, bt);
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[ab]);
+        }
+        if (lane == 0) bulk_wait0();
+        if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
+}
+
+static int operand_map(CUtensorMap* m, const Operand& o, int parts, int box_rows, const char* what) {
+    B200PF_REQUIRE(o.ptr && aligned16(o.ptr) && o.row_stride % 8 == 0 && o.batch_stride % 8 == 0 && o.part_stride % 8 == 0, B200PF_ERR_INVALID,
+                   "split_gemm: operand %s is null, misaligned or has strides that are not multiples of 8", what);
+    cuuint64_t dims[4] = {(cuuint64_t)o.cols, (cuuint64_t)o.rows, (cuuint64_t)o.batches, (cuuint64_t)parts};
+    cuuint64_t str[3] = {(cuuint64_t)o.row_stride * 2, (cuuint64_t)(o.batches > 1 ? o.batch_stride : o.part_stride) * 2, (cuuint64_t)o.part_stride * 2};
+    cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 1};
+    return tmap_encode(m, parts == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, o.ptr, 4, dims, str, box,
+                       CU_TENSOR_MAP_SWIZZLE_128B, what);
+}
+
+static int output_map(CUtensorMap* m, const Output& o) {
+    const int es = o.parts == 1 ? 4 : 2;
+    B200PF_REQUIRE(o.ptr && aligned16(o.ptr) && o.row_stride * es % 16 == 0 && o.batch_stride * es % 16 == 0 && o.part_stride * es % 16 == 0,
+                   B200PF_ERR_INVALID, "split_gemm: output is null, misaligned or has strides that are not multiples of 16 bytes");
+    const CUtensorMapDataType dt = o.parts == 1 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : o.parts == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    const long long any = o.row_stride * o.rows;       // stride of a dimension of extent 1: anything valid
+    const long long bs = o.batches > 1 ? o.batch_stride : any, ps = o.parts > 1 ? o.part_stride : any;
+    cuuint64_t dims[4] = {(cuuint64_t)o.cols, (cuuint64_t)(o.rows_outer ? o.batches : o.rows), (cuuint64_t)(o.rows_outer ? o.rows : o.batches), (cuuint64_t)o.parts};
+    cuuint64_t str[3] = {(cuuint64_t)(o.rows_outer ? bs : o.row_stride) * es, (cuuint64_t)(o.rows_outer ? o.row_stride : bs) * es, (cuuint64_t)ps * es};
+    cuuint32_t box[4] = {32, o.rows_outer ? 1u : 32u, o.rows_outer ? 32u : 1u, 1};
+    return tmap_encode(m, dt, o.ptr, 4, dims, str, box, o.parts == 1 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, "split output");
+}
+
+template <int PL, int BN, int NA, int NK, int EPI>
+static int launch_one(const Gemm& g, int bn, int sms, cudaStream_t st) {
+    unsigned int* status = device_status_word();
+    B200PF_REQUIRE(status, B200PF_ERR_CUDA, "split_gemm: no device status word");
+    CUtensorMap a[2], b[2], o[2];
+    int rc;
+    for (int i = 0; i < NK; ++i) {
+        if ((rc = operand_map(&a[i], g.a[i], PL, 128, "A")) != B200PF_OK) return rc;
+        if ((rc = operand_map(&b[i], g.b[i], PL, bn, "B")) != B200PF_OK) return rc;
+    }
+    if (NK == 1) { a[1] = a[0]; b[1] = b[0]; }
+    if ((rc = output_map(&o[0], g.out[0])) != B200PF_OK) return rc;
+    if (EPI == EPI_QKVG) { if ((rc = output_map(&o[1], g.out[1])) != B200PF_OK) return rc; }
+    else o[1] = o[0];
+    constexpr int smem = stages_of(PL, BN, NA) * stage_bytes(PL, BN, NA) + SMEM_FIXED;
+    auto kern = split_gemm_kernel<PL, BN, NA, NK, EPI>;
+    B200PF_SMEM_ATTR_ONCE(kern, smem);
+    Dev d;
+    d.m_rows = g.m_rows; d.n_rows = g.n_rows; d.bn = bn;
+    d.batches = g.k_splits > 1 ? g.k_splits : g.batches;
+    d.a_batched = g.a_batched; d.b_batched = g.b_batched; d.a_second_row = g.a_second_row;
+    d.k[0] = g.k[0]; d.k[1] = g.k[1]; d.k_splits = g.k_splits;
+    d.kb_per_split = ((g.k[0] + 63) / 64 + g.k_splits - 1) / g.k_splits;
+    d.alpha[0] = g.alpha[0]; d.alpha[1] = g.alpha[1]; d.out_scale = g.out_scale;
+    d.bias = g.bias; d.mask = g.mask; d.mask_bs = g.mask_bs; d.mask_cs = g.mask_cs;
+    d.n_split = g.n_split; d.rows_outer = g.out[0].rows_outer; d.n_out = g.out[0].cols;
+    const long long tiles = (long long)d.batches * ((g.m_rows + 127) / 128) * ((g.n_rows + bn - 1) / bn);
+    return launch_pdl(kern, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(THREADS), smem, st, a[0], a[1], b[0], b[1], o[0], o[1], d, status);
+}
+
+// Tile width for `n` columns: the widest tile (at most `most`, a multiple of `step`) whose waves of CTAs, times the bytes a tile
+// stages per k-block, come to the least: narrow tiles only where wide ones leave SMs without work.
+static int pick_bn(long long row_tiles, int n, int most, int step, int sms) {
+    int best = step;
+    double best_cost = 1e30;
+    for (int bn = most; bn >= step; bn -= step) {
+        if (bn > step && bn - step >= n) continue;
+        const long long tiles = row_tiles * ((n + bn - 1) / bn);
+        const long long waves = (tiles + sms - 1) / sms;
+        const double cost = (double)waves * (128 + bn + 64);
+        if (cost < best_cost - 1e-9) { best_cost = cost; best = bn; }
+    }
+    return best;
+}
+
+int launch_gemm(const Gemm& g, cudaStream_t st) {
+    B200PF_REQUIRE(g.m_rows > 0 && g.n_rows > 0 && g.batches > 0 && g.k[0] > 0, B200PF_ERR_INVALID, "split_gemm: empty problem");
+    const int kb_total = (g.k[0] + 63) / 64;
+    B200PF_REQUIRE(g.k_splits == 1 || (g.epi == EPI_STORE && g.batches == 1 && g.k_splits > 1 &&
+                                       (g.k_splits - 1) * ((kb_total + g.k_splits - 1) / g.k_splits) < kb_total),
+                   B200PF_ERR_INVALID, "split_gemm: every K split needs a k-block of its own");
+    int dev = 0, sms = 148;
+    B200PF_CUDA(cudaGetDevice(&dev));
+    B200PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const long long row_tiles = (long long)(g.k_splits > 1 ? g.k_splits : g.batches) * ((g.m_rows + 127) / 128);
+#define SG(PL, BN, NA, NK, EPI) return launch_one<PL, BN, NA, NK, EPI>(g, bn, sms, st)
+    switch (g.epi) {
+        case EPI_STORE: {
+            if (g.parts == 3) { const int bn = pick_bn(row_tiles, g.n_rows, 128, 32, sms); SG(3, 128, 1, 1, EPI_STORE); }
+            const int bn = pick_bn(row_tiles, g.n_rows, 256, 32, sms);
+            if (bn > 128) SG(2, 256, 1, 1, EPI_STORE);
+            SG(2, 128, 1, 1, EPI_STORE);
+        }
+        case EPI_ADD: {
+            if (g.parts == 3) { const int bn = pick_bn(row_tiles, g.n_rows, 128, 32, sms); SG(3, 128, 1, 1, EPI_ADD); }
+            const int bn = pick_bn(row_tiles, g.n_rows, 256, 32, sms);
+            if (bn > 128) SG(2, 256, 1, 1, EPI_ADD);
+            SG(2, 128, 1, 1, EPI_ADD);
+        }
+        case EPI_SWIGLU: {
+            const int bn = pick_bn(row_tiles, g.n_rows, 256, 64, sms);
+            if (bn > 128) SG(2, 256, 1, 1, EPI_SWIGLU);
+            SG(2, 128, 1, 1, EPI_SWIGLU);
+        }
+        case EPI_QKVG: {
+            const int bn = pick_bn(row_tiles, g.n_rows, 256, 32, sms);
+            if (bn > 128) SG(2, 256, 1, 1, EPI_QKVG);
+            SG(2, 128, 1, 1, EPI_QKVG);
+        }
+        case EPI_GATE_PLANES: { const int bn = pick_bn(row_tiles, g.n_rows, 128, 32, sms); SG(2, 128, 2, 1, EPI_GATE_PLANES); }
+        case EPI_GATE_ADD: { const int bn = pick_bn(row_tiles, g.n_rows, 128, 32, sms); SG(2, 128, 1, 2, EPI_GATE_ADD); }
+    }
+#undef SG
+    B200PF_REQUIRE(false, B200PF_ERR_UNSUPPORTED, "split_gemm: unknown epilogue");
+}
+
+}  // namespace split
+}  // namespace b200pf

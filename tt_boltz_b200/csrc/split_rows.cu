@@ -1,0 +1,342 @@
+// LayerNorm and conversion kernels in front of the split GEMM (split_gemm.cu): one pass over the fp32 rows, 16-bit part planes
+// out.  Bound by HBM (or by launch latency for the single track's few hundred rows): a warp owns R rows at a time so that
+// R rows' loads are in flight per warp, every access is a contiguous run of a row.
+#include "split_rows.cuh"
+
+namespace b200pf {
+namespace split {
+
+// Reduces V values per lane over the 32 lanes of a warp; lane l ends up with the totals of max(1, V / 32) values from index
+// reduced_base<V>(l) on (V a power of two; for V < 32 neighbouring lanes hold the same value).
+template <int V> __device__ __forceinline__ void lane_reduce(float (&v)[V], int lane) {
+    int cnt = V;
+#pragma unroll
+    for (int bit = 16; bit >= 1; bit >>= 1) {
+        if (cnt > 1) {
+            const int half = cnt / 2;
+            const bool upper = (lane & bit) != 0;
+#pragma unroll
+            for (int i = 0; i < V / 2; ++i)
+                if (i < half) {
+                    const float keep = upper ? v[i + half] : v[i], send = upper ? v[i] : v[i + half];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+                }
+            cnt = half;
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], bit);
+        }
+    }
+}
+template <int V> __device__ __forceinline__ int reduced_base(int lane) {
+    int base = 0, half = V / 2;
+#pragma unroll
+    for (int bit = 16; bit >= 1; bit >>= 1)
+        if (half >= 1) { base += (lane & bit) ? half : 0; half /= 2; }
+    return base;
+}
+
+template <int C, int NH, int R>
+__global__ void __launch_bounds__(256) ln_split_kernel(LnArgs p) {
+    constexpr int V = C >= 128 ? 4 : 2, J = C / (32 * V);            // V consecutive channels per lane and step
+    static_assert(J * 32 * V == C, "width must be 64 or a multiple of 128");
+    extern __shared__ __align__(16) float head_s[];                  // [NH][C]
+    const int lane = threadIdx.x & 31;
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (NH > 0) {
+        for (int i = threadIdx.x; i < NH * C; i += blockDim.x) head_s[i] = *(p.head_w + i);
+        __syncthreads();
+    }
+    float gam[J][V], bet[J][V];
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int e = 0; e < V; ++e) { gam[j][e] = *(p.gamma + (j * 32 + lane) * V + e); bet[j][e] = *(p.beta + (j * 32 + lane) * V + e); }
+    const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+    for (long long base = warp * R; base < p.rows; base += nwarps * R) {
+        float x[R][J][V];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const long long row = base + r < p.rows ? base + r : p.rows - 1;
+            const float* src = p.x + row * C + lane * V;
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                if (V == 4) {
+                    const float4 t = *reinterpret_cast<const float4*>(src + j * 128);
+                    x[r][j][0] = t.x; x[r][j][1] = t.y; x[r][j][2 % V] = t.z; x[r][j][3 % V] = t.w;
+                } else {
+                    const float2 t = *reinterpret_cast<const float2*>(src + j * 64);
+                    x[r][j][0] = t.x; x[r][j][1] = t.y;
+                }
+            }
+        }
+        if (p.n_partial > 0) {
+            for (int q = 0; q < p.n_partial; ++q)
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const long long row = base + r < p.rows ? base + r : p.rows - 1;
+                    const float* src = p.partial + ((long long)q * p.rows + row) * C + lane * V;
+#pragma unroll
+                    for (int j = 0; j < J; ++j)
+#pragma unroll
+                        for (int e = 0; e < V; ++e) x[r][j][e] += src[j * 32 * V + e];
+                }
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (base + r < p.rows) {
+                    float* dst = p.x_out + (base + r) * C + lane * V;
+#pragma unroll
+                    for (int j = 0; j < J; ++j)
+#pragma unroll
+                        for (int e = 0; e < V; ++e) dst[j * 32 * V + e] = x[r][j][e];
+                }
+        }
+        float s[R], ss[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            float a = 0.f;
+#pragma unroll
+            for (int j = 0; j < J; ++j)
+#pragma unroll
+                for (int e = 0; e < V; ++e) a += x[r][j][e];
+            s[r] = a;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int r = 0; r < R; ++r) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float mean = s[r] * (1.f / C);
+            float a = 0.f;
+#pragma unroll
+            for (int j = 0; j < J; ++j)
+#pragma unroll
+                for (int e = 0; e < V; ++e) { x[r][j][e] -= mean; a = fmaf(x[r][j][e], x[r][j][e], a); }
+            ss[r] = a;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int r = 0; r < R; ++r) ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], o);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float rstd = rsqrtf(ss[r] * (1.f / C) + LN_EPS);
+#pragma unroll
+            for (int j = 0; j < J; ++j)
+#pragma unroll
+                for (int e = 0; e < V; ++e) x[r][j][e] = fmaf(x[r][j][e] * rstd, gam[j][e], bet[j][e]);
+            if (p.planes && base + r < p.rows) {
+                __half* dst = p.planes + (base + r) * C + lane * V;
+#pragma unroll
+                for (int j = 0; j < J; ++j) {
+                    uint32_t h0, l0;
+                    split_f16x2(x[r][j][0], x[r][j][1], h0, l0);
+                    if (V == 4) {
+                        uint32_t h1, l1;
+                        split_f16x2(x[r][j][2 % V], x[r][j][3 % V], h1, l1);
+                        *reinterpret_cast<uint2*>(dst + j * 128) = make_uint2(h0, h1);
+                        *reinterpret_cast<uint2*>(dst + p.part_stride + j * 128) = make_uint2(l0, l1);
+                    } else {
+                        *reinterpret_cast<uint32_t*>(dst + j * 64) = h0;
+                        *reinterpret_cast<uint32_t*>(dst + p.part_stride + j * 64) = l0;
+                    }
+                }
+            }
+        }
+        if (NH > 0) {
+            constexpr int NV = NH > 0 ? R * NH : 1;
+            float acc[NV];
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) acc[h * R + r] = 0.f;
+#pragma unroll
+                for (int j = 0; j < J; ++j) {
+                    const float* w = head_s + h * C + (j * 32 + lane) * V;
+                    float wv[V];
+                    if (V == 4) {
+                        const float4 t = *reinterpret_cast<const float4*>(w);
+                        wv[0] = t.x; wv[1] = t.y; wv[2 % V] = t.z; wv[3 % V] = t.w;
+                    } else {
+                        const float2 t = *reinterpret_cast<const float2*>(w);
+                        wv[0] = t.x; wv[1] = t.y;
+                    }
+#pragma unroll
+                    for (int r = 0; r < R; ++r)
+#pragma unroll
+                        for (int e = 0; e < V; ++e) acc[h * R + r] = fmaf(x[r][j][e], wv[e], acc[h * R + r]);
+                }
+            }
+            lane_reduce<NV>(acc, lane);
+            const int b0 = reduced_base<NV>(lane);
+            constexpr int PER = NV >= 32 ? NV / 32 : 1, DUP = NV >= 32 ? 1 : 32 / NV;
+            if (lane % DUP == 0) {
+#pragma unroll
+                for (int i = 0; i < PER; ++i) {
+                    const int idx = b0 + i, h = idx / R;
+                    const long long row = base + idx % R;
+                    if (row < p.rows) {
+                        const long long at = p.transposed ? (row % p.n) * p.n + row / p.n : row;
+                        p.head_out[h * p.head_stride + at] = acc[i];
+                    }
+                }
+            }
+        }
+    }
+}
+
+bool ln_supported(int c) { return c == 64 || c == 128 || c == 256 || c == 384; }
+
+template <int C, int NH> static int ln_go(const LnArgs& a, cudaStream_t st) {
+    constexpr int R = NH == 16 ? 4 : NH > 0 ? 4 : (C >= 256 ? 2 : 4);
+    int dev = 0, sms = 148;
+    B200PF_CUDA(cudaGetDevice(&dev));
+    B200PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // few rows: one warp pass per block of fewer warps, so that every SM gets some
+    const int warps = a.rows >= (long long)sms * 8 * R ? 8 : 2;
+    const long long need = (a.rows + (long long)warps * R - 1) / ((long long)warps * R);
+    const long long most = (long long)sms * (NH > 0 ? 4 : 8);
+    return launch_pdl(ln_split_kernel<C, NH, R>, dim3((unsigned)(need < most ? need : most)), dim3(warps * 32), (size_t)NH * C * 4, st, a);
+}
+template <int C> static int ln_heads(const LnArgs& a, int heads, cudaStream_t st) {
+    switch (heads) {
+        case 0: return ln_go<C, 0>(a, st);
+        case 4: return ln_go<C, 4>(a, st);
+        case 8: return ln_go<C, 8>(a, st);
+        case 16: return ln_go<C, 16>(a, st);
+    }
+    B200PF_REQUIRE(false, B200PF_ERR_UNSUPPORTED, "layernorm: 0, 4, 8 or 16 head projections (got %d)", heads);
+}
+int launch_ln(const LnArgs& a, int c, int heads, cudaStream_t st) {
+    B200PF_REQUIRE(a.x && a.gamma && a.beta && aligned16(a.x) && (a.planes == nullptr || aligned16(a.planes)) && a.rows > 0, B200PF_ERR_INVALID,
+                   "layernorm: null or misaligned pointer");
+    switch (c) {
+        case 64: return ln_heads<64>(a, heads, st);
+        case 128: return ln_heads<128>(a, heads, st);
+        case 256: return ln_heads<256>(a, heads, st);
+        case 384: B200PF_REQUIRE(heads == 0, B200PF_ERR_UNSUPPORTED, "layernorm: no head projections at width 384"); return ln_go<384, 0>(a, st);
+    }
+    B200PF_REQUIRE(false, B200PF_ERR_UNSUPPORTED, "layernorm: width %d is not built", c);
+}
+
+// t[d][i][j] -> planes[(i, j)][d]: a block takes 32 positions of one row through shared memory ([D][33]: both the row-wise
+// fill and the column-wise reads are conflict free) and its warps normalise four positions each.
+template <int D>
+__global__ void __launch_bounds__(256) ln_channels_kernel(const float* t, long long plane_stride, int pitch, const float* gamma,
+                                                          const float* beta, __half* planes, long long part_stride, int n) {
+    extern __shared__ float ts[];
+    constexpr int E = D / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const int i = blockIdx.y, j0 = blockIdx.x * 32;
+    const float* src = t + (long long)i * pitch + j0 + lane;
+    const bool in = j0 + lane < n;
+#pragma unroll
+    for (int d0 = 0; d0 < D; d0 += 64) {
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = in ? *(src + (long long)(d0 + e * 8 + warp) * plane_stride) : 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ts[(d0 + e * 8 + warp) * 33 + lane] = v[e];
+    }
+    __syncthreads();
+    // lane: channels 2 lane + 64 e, 2 lane + 1 + 64 e
+    float g[E], b[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) { const int c = 2 * lane + 64 * (e >> 1) + (e & 1); g[e] = *(gamma + c); b[e] = *(beta + c); }
+    float x[4][E], s[4], ss[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        s[r] = 0.f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) { x[r][e] = ts[(2 * lane + 64 * (e >> 1) + (e & 1)) * 33 + warp * 4 + r]; s[r] += x[r][e]; }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const float mean = s[r] * (1.f / D);
+        ss[r] = 0.f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) { x[r][e] -= mean; ss[r] = fmaf(x[r][e], x[r][e], ss[r]); }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], o);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int j = j0 + warp * 4 + r;
+        if (j >= n) break;
+        const float rstd = rsqrtf(ss[r] * (1.f / D) + LN_EPS);
+        __half* dst = planes + ((long long)i * n + j) * D + 2 * lane;
+#pragma unroll
+        for (int e = 0; e < E; e += 2) {
+            uint32_t h, l;
+            split_f16x2(fmaf(x[r][e] * rstd, g[e], b[e]), fmaf(x[r][e + 1] * rstd, g[e + 1], b[e + 1]), h, l);
+            *reinterpret_cast<uint32_t*>(dst + 32 * e) = h;
+            *reinterpret_cast<uint32_t*>(dst + part_stride + 32 * e) = l;
+        }
+    }
+}
+
+template <int D> static int ln_channels_go(const float* t, long long plane_stride, int pitch, const float* gamma, const float* beta, __half* planes,
+                                           int n, cudaStream_t st) {
+    constexpr int smem = D * 33 * 4;
+    B200PF_SMEM_ATTR_ONCE(ln_channels_kernel<D>, smem);
+    return launch_pdl(ln_channels_kernel<D>, dim3((unsigned)((n + 31) / 32), (unsigned)n), dim3(256), smem, st, t, plane_stride, pitch, gamma, beta, planes,
+                      (long long)n * n * D, n);
+}
+int launch_ln_channels(const float* t, long long plane_stride, int pitch, const float* gamma, const float* beta, __half* planes, int n, int d,
+                       cudaStream_t st) {
+    switch (d) {
+        case 64: return ln_channels_go<64>(t, plane_stride, pitch, gamma, beta, planes, n, st);
+        case 128: return ln_channels_go<128>(t, plane_stride, pitch, gamma, beta, planes, n, st);
+        case 256: return ln_channels_go<256>(t, plane_stride, pitch, gamma, beta, planes, n, st);
+        case 384: return ln_channels_go<384>(t, plane_stride, pitch, gamma, beta, planes, n, st);
+    }
+    B200PF_REQUIRE(false, B200PF_ERR_UNSUPPORTED, "channel layernorm: width %d is not built", d);
+}
+
+__global__ void __launch_bounds__(256) parts_kernel(const float4* x, uint2* planes, long long count4) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < count4; i += (long long)gridDim.x * blockDim.x) {
+        const float4 v = *(x + i);
+        uint2 h, m, l;
+        split_bf16x3(v.x, v.y, h.x, m.x, l.x);
+        split_bf16x3(v.z, v.w, h.y, m.y, l.y);
+        planes[i] = h; planes[count4 + i] = m; planes[2 * count4 + i] = l;
+    }
+}
+int launch_parts(const float* x, __nv_bfloat16* planes, long long count, cudaStream_t st) {
+    B200PF_REQUIRE(x && planes && aligned16(x) && aligned16(planes) && count > 0 && count % 8 == 0, B200PF_ERR_INVALID, "parts: bad arguments");
+    const long long need = (count / 4 + 255) / 256, most = 148 * 16;
+    return launch_pdl(parts_kernel, dim3((unsigned)(need < most ? need : most)), dim3(256), 0, st, reinterpret_cast<const float4*>(x),
+                      reinterpret_cast<uint2*>(planes), count / 4);
+}
+
+__global__ void __launch_bounds__(256) add_partials_kernel(float4* x, const float4* partial, int n_partial, long long count4) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count4) return;
+    float4 v = x[i];
+    for (int q = 0; q < n_partial; ++q) {
+        const float4 t = *(partial + q * count4 + i);
+        v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+    }
+    x[i] = v;
+}
+int launch_add_partials(float* x, const float* partial, int n_partial, long long count, cudaStream_t st) {
+    B200PF_REQUIRE(x && partial && aligned16(x) && aligned16(partial) && count > 0 && count % 4 == 0, B200PF_ERR_INVALID, "add_partials: bad arguments");
+    return launch_pdl(add_partials_kernel, dim3((unsigned)((count / 4 + 255) / 256)), dim3(256), 0, st, reinterpret_cast<float4*>(x),
+                      reinterpret_cast<const float4*>(partial), n_partial, count / 4);
+}
+
+}  // namespace split
+}  // namespace b200pf

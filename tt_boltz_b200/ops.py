@@ -12,7 +12,7 @@ from typing import Dict, Optional
 
 import torch
 
-from . import _lib
+from . import _lib, weights
 from ._lib import PlaneOut, Planes, call, ptr, stream
 
 C_Z = 128
@@ -243,77 +243,152 @@ def transition_f32(x_res: torch.Tensor, w: Dict[str, torch.Tensor]) -> None:
     f32_linear(h, w["fc3.weight"], out=x_res, accumulate=True)
 
 
-def pair_bias_heads(z: torch.Tensor, w: Dict[str, torch.Tensor]) -> torch.Tensor:
-    """bias[h][i_local*N + j] of the single-track attention: one fp32 pass over the (local rows of) z."""
-    rows, c = z.shape[0] * z.shape[1], z.shape[-1]          # z may be a row shard [nr, N, c_z]
-    heads = w["proj_z.1.weight"].shape[0]
-    bias = torch.empty(heads, rows, dtype=torch.float32, device=z.device)
-    if c == C_Z and heads in (4, 16):
-        call("b200pf_ln_proj_heads", ptr(z), ptr(w["proj_z.0.weight"]), ptr(w["proj_z.0.bias"]),
-             ptr(w["proj_z.1.weight"]), ptr(bias), rows, rows, c, heads, stream())
-    else:
-        x = f32_layernorm(z, w["proj_z.0.weight"], w["proj_z.0.bias"])
-        call("b200pf_f32_linear_t", ptr(x), ptr(w["proj_z.1.weight"]), None, ptr(bias), rows, rows, c, heads, stream())
-    return bias
+# ------------------------------------------------------------------------------------------------
+# fp32-accurate tensor-core path (16-bit parts): pair track of the fp32 tier, single track of every tier
+# ------------------------------------------------------------------------------------------------
+class Scratch:
+    """A call's workspace: one buffer that grows to the largest request.  Made per call and per stream, never kept, so that
+    calls on several streams or threads do not meet in it."""
+
+    def __init__(self, device) -> None:
+        self.device, self.buf = device, None
+
+    def get(self, nbytes: int) -> int:
+        if self.buf is None or self.buf.numel() < nbytes:
+            self.buf = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+        return self.buf.data_ptr()
 
 
-def pack_single_track(w_att: Dict[str, torch.Tensor], w_trans: Dict[str, torch.Tensor]) -> Dict[str, torch.Tensor]:
-    """Concatenated fp32 weights so that q|g, k|v and fc1|fc2 are one GEMM launch each."""
-    cs = w_att["proj_q.weight"].shape[0]
-    return {
-        "w_qg": torch.cat([w_att["proj_q.weight"], w_att["proj_g.weight"]], 0).contiguous(),
-        "b_qg": torch.cat([w_att["proj_q.bias"], torch.zeros(cs, device=w_att["proj_q.bias"].device)], 0).contiguous(),
-        "w_kv": torch.cat([w_att["proj_k.weight"], w_att["proj_v.weight"]], 0).contiguous(),
-        "w_12": torch.cat([w_trans["fc1.weight"], w_trans["fc2.weight"]], 0).contiguous(),
-    }
+def _nbytes(name: str, *args) -> int:
+    return int(getattr(_lib.load(), name)(*args))
 
 
-def single_track_local(s: torch.Tensor, z_rows: torch.Tensor, tok_mask_u8: torch.Tensor, w_norm: Dict[str, torch.Tensor],
-                       w_att: Dict[str, torch.Tensor], fused: Dict[str, torch.Tensor], num_heads: int,
-                       r0: int = 0, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Gated attention output sigmoid(g) * softmax(...) v for the query rows [r0, r0 + z_rows.shape[0]) (fp32).
-    ``bias`` = pair_bias_heads(z_rows, w_att) when the caller has computed it already (then z_rows is only read
-    for its shape)."""
-    n, cs = s.shape
-    nq = z_rows.shape[0]
-    hd = cs // num_heads
-    st = stream()
-    sn = f32_layernorm(s, w_norm["weight"], w_norm["bias"])
-    qg = f32_linear(sn[r0:r0 + nq], fused["w_qg"], fused["b_qg"])                       # [nq, 2 cs]: q | g
-    pitch = _round_up(n, 4)
-    kvt = torch.empty(2 * cs, pitch, dtype=torch.float32, device=s.device)              # [k rows | v rows][key]
-    call("b200pf_f32_linear_t", ptr(sn), ptr(fused["w_kv"]), None, ptr(kvt), pitch, n, cs, 2 * cs, st)
-    if bias is None:
-        bias = pair_bias_heads(z_rows, w_att)                                            # [heads][nq * n]
-    o = torch.empty(nq, cs, dtype=torch.float32, device=s.device)
-    call("b200pf_f32_sattention", ptr(qg), 2 * cs, qg.data_ptr() + 4 * cs, 2 * cs, ptr(kvt), kvt.data_ptr() + 4 * cs * pitch, pitch,
-         ptr(o), cs, ptr(bias), nq * n, n, ptr(tok_mask_u8), nq, n, num_heads, hd, 1.0 / math.sqrt(hd), 1e6, st)
-    return o
+def tri_mul_split(z: torch.Tensor, mask_u8: torch.Tensor, pack, incoming: bool, scratch: Scratch) -> None:
+    n = z.shape[0]
+    ws = scratch.get(_nbytes("b200pf_split_pair_workspace", n, pack.struct.c, 0, 0, 0))
+    call("b200pf_split_tri_mul", ptr(z), ptr(mask_u8), C.byref(pack.struct), n, int(incoming), ws, stream())
 
 
-def single_track_finish(s: torch.Tensor, og_all: torch.Tensor, w_att: Dict[str, torch.Tensor],
-                        w_trans: Dict[str, torch.Tensor], fused: Dict[str, torch.Tensor]) -> None:
-    """s += proj_o(gated attention output); s += Transition(s) (tt_bio/reference.py:906-911)."""
-    n, cs = s.shape
-    f32_linear(og_all, w_att["proj_o.weight"], out=s, accumulate=True)
-    x = f32_layernorm(s, w_trans["norm.weight"], w_trans["norm.bias"])
-    h12 = f32_linear(x, fused["w_12"])                                                  # [n, 8 cs]: fc1 | fc2
-    hidden = h12.shape[1] // 2
-    h = torch.empty(n, hidden, dtype=torch.float32, device=s.device)
-    call("b200pf_f32_gate_strided", ptr(h12), 2 * hidden, h12.data_ptr() + 4 * hidden, 2 * hidden, ptr(h), hidden,
-         n, hidden, 1, stream())
-    f32_linear(h, w_trans["fc3.weight"], out=s, accumulate=True)
+def tri_att_split(z: torch.Tensor, mask_u8: torch.Tensor, pack, ending: bool, scratch: Scratch) -> None:
+    n, w = z.shape[0], pack.struct
+    ws = scratch.get(_nbytes("b200pf_split_pair_workspace", n, w.c, w.heads, w.hd, 0))
+    call("b200pf_split_tri_att", ptr(z), ptr(mask_u8), C.byref(w), n, int(ending), ws, stream())
 
 
-def single_track(s: torch.Tensor, z: torch.Tensor, tok_mask_u8: torch.Tensor, w_norm: Dict[str, torch.Tensor],
-                 w_att: Dict[str, torch.Tensor], w_trans: Dict[str, torch.Tensor], num_heads: int,
-                 fused: Optional[Dict[str, torch.Tensor]] = None, after_z_read=None) -> None:
-    """s += AttentionPairBias(LN(s), z); s += Transition(s) in fp32 (tt_bio/reference.py:906-912).
-    The pair-bias projection, the single track's only read of z, comes first; ``after_z_read`` is called behind it."""
-    if fused is None:
-        fused = pack_single_track(w_att, w_trans)
-    bias = pair_bias_heads(z, w_att)
+def transition_split(x: torch.Tensor, pack, scratch: Scratch) -> None:
+    w = pack.struct
+    n = math.isqrt(x.numel() // w.c - 1) + 1 if x.numel() > w.c else 1          # workspace of a square tensor at least as large
+    ws = scratch.get(_nbytes("b200pf_split_pair_workspace", n, w.c, 0, 0, w.hidden))
+    call("b200pf_split_transition", ptr(x), x.numel() // w.c, C.byref(w), ws, stream())
+
+
+def split_linear(x: torch.Tensor, w_parts: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, accumulate: bool, scratch: Scratch) -> None:
+    """out (+)= x w^T (+ bias) with ``w_parts`` = weights.bf16_parts(w): any finite fp32 x, all 24 bits of both factors."""
+    k, n = w_parts.shape[2], w_parts.shape[1]
+    rows = x.numel() // k
+    ws = scratch.get(_nbytes("b200pf_split_linear_workspace", rows, k))
+    call("b200pf_split_linear", ptr(x), ptr(w_parts), ptr(bias), ptr(out), rows, k, n, int(accumulate), ws, stream())
+
+
+class SingleTrack:
+    """s += AttentionPairBias(LN(s), z); s += Transition(s) in fp32 (tt_bio/reference.py:906-912) of one layer, on part
+    planes: ``bias`` (its only read of z), ``attention`` for a range of query rows, ``finish`` per row."""
+
+    def __init__(self, sd, pre: str, num_heads: int, device) -> None:
+        self.pack = weights.pack_single_track(sd, pre, num_heads, device)
+        self.z_bias = weights.pack_pair_bias(sd, pre + "attention.", device)
+
+    def bias(self, z_rows: torch.Tensor) -> torch.Tensor:
+        """bias[h][i_local * N + j], times log2(e): one fp32 pass over the (local rows of) z [nr, N, c_z]."""
+        rows, c = z_rows.shape[0] * z_rows.shape[1], z_rows.shape[-1]
+        w = self.z_bias
+        heads = w["w"].shape[0]
+        out = torch.empty(heads, rows, dtype=torch.float32, device=z_rows.device)
+        name = "b200pf_ln_proj_heads" if c == C_Z and heads in (4, 16) else "b200pf_ln_heads"
+        call(name, ptr(z_rows), ptr(w["gamma"]), ptr(w["beta"]), ptr(w["w"]), ptr(out), rows, rows, c, heads, stream())
+        return out
+
+    def attention(self, s: torch.Tensor, bias: torch.Tensor, tok_mask_u8: Optional[torch.Tensor], r0: int, nq: int, scratch: Scratch) -> torch.Tensor:
+        w = self.pack.struct
+        og = torch.empty(2, nq, w.cs, dtype=torch.float16, device=s.device)
+        ws = scratch.get(_nbytes("b200pf_single_track_workspace", s.shape[0], w.cs, w.hidden))
+        call("b200pf_single_track_attention", ptr(s), C.byref(w), ptr(bias), ptr(tok_mask_u8), ptr(og), s.shape[0], r0, nq, ws, stream())
+        return og
+
+    def finish(self, s_rows: torch.Tensor, og: torch.Tensor, scratch: Scratch) -> None:
+        w = self.pack.struct
+        ws = scratch.get(_nbytes("b200pf_single_track_workspace", s_rows.shape[0], w.cs, w.hidden))
+        call("b200pf_single_track_finish", ptr(s_rows), C.byref(w), ptr(og), s_rows.shape[0], ws, stream())
+
+
+class SingleTrackF32:
+    """The same on the un-fused fp32 kernels: widths the part-plane kernels are not built for."""
+
+    def __init__(self, sd, pre: str, num_heads: int, device) -> None:
+        f32 = lambda name: weights.to_device_f32(sd, pre + name, device)
+        self.num_heads = num_heads
+        self.w_norm, self.w_att, self.w_trans = f32("pre_norm_s."), f32("attention."), f32("transition_s.")
+        w_att, w_trans = self.w_att, self.w_trans
+        cs = w_att["proj_q.weight"].shape[0]
+        self.w_qg = torch.cat([w_att["proj_q.weight"], w_att["proj_g.weight"]], 0).contiguous()
+        self.b_qg = torch.cat([w_att["proj_q.bias"], torch.zeros(cs, device=device)], 0).contiguous()
+        self.w_kv = torch.cat([w_att["proj_k.weight"], w_att["proj_v.weight"]], 0).contiguous()
+        self.w_12 = torch.cat([w_trans["fc1.weight"], w_trans["fc2.weight"]], 0).contiguous()
+
+    def bias(self, z_rows: torch.Tensor) -> torch.Tensor:
+        """bias[h][i_local * N + j]: one fp32 pass over the (local rows of) z [nr, N, c_z]."""
+        w = self.w_att
+        rows, c = z_rows.shape[0] * z_rows.shape[1], z_rows.shape[-1]
+        heads = w["proj_z.1.weight"].shape[0]
+        out = torch.empty(heads, rows, dtype=torch.float32, device=z_rows.device)
+        if c == C_Z and heads in (4, 16):
+            call("b200pf_ln_proj_heads", ptr(z_rows), ptr(w["proj_z.0.weight"]), ptr(w["proj_z.0.bias"]),
+                 ptr(w["proj_z.1.weight"]), ptr(out), rows, rows, c, heads, stream())
+        else:
+            x = f32_layernorm(z_rows, w["proj_z.0.weight"], w["proj_z.0.bias"])
+            call("b200pf_f32_linear_t", ptr(x), ptr(w["proj_z.1.weight"]), None, ptr(out), rows, rows, c, heads, stream())
+        return out
+
+    def attention(self, s: torch.Tensor, bias: torch.Tensor, tok_mask_u8: Optional[torch.Tensor], r0: int, nq: int, scratch: Scratch) -> torch.Tensor:
+        n, cs = s.shape
+        hd, st = cs // self.num_heads, stream()
+        sn = f32_layernorm(s, self.w_norm["weight"], self.w_norm["bias"])
+        qg = f32_linear(sn[r0:r0 + nq], self.w_qg, self.b_qg)                           # [nq, 2 cs]: q | g
+        pitch = _round_up(n, 4)
+        kvt = torch.empty(2 * cs, pitch, dtype=torch.float32, device=s.device)          # [k rows | v rows][key]
+        call("b200pf_f32_linear_t", ptr(sn), ptr(self.w_kv), None, ptr(kvt), pitch, n, cs, 2 * cs, st)
+        o = torch.empty(nq, cs, dtype=torch.float32, device=s.device)
+        call("b200pf_f32_sattention", ptr(qg), 2 * cs, qg.data_ptr() + 4 * cs, 2 * cs, ptr(kvt), kvt.data_ptr() + 4 * cs * pitch, pitch,
+             ptr(o), cs, ptr(bias), nq * n, n, ptr(tok_mask_u8), nq, n, self.num_heads, hd, 1.0 / math.sqrt(hd), 1e6, st)
+        return o
+
+    def finish(self, s_rows: torch.Tensor, og: torch.Tensor, scratch: Scratch) -> None:
+        n = s_rows.shape[0]
+        f32_linear(og, self.w_att["proj_o.weight"], out=s_rows, accumulate=True)
+        x = f32_layernorm(s_rows, self.w_trans["norm.weight"], self.w_trans["norm.bias"])
+        h12 = f32_linear(x, self.w_12)                                                  # [n, 2 hidden]: fc1 | fc2
+        hidden = h12.shape[1] // 2
+        h = torch.empty(n, hidden, dtype=torch.float32, device=s_rows.device)
+        call("b200pf_f32_gate_strided", ptr(h12), 2 * hidden, h12.data_ptr() + 4 * hidden, 2 * hidden, ptr(h), hidden,
+             n, hidden, 1, stream())
+        f32_linear(h, self.w_trans["fc3.weight"], out=s_rows, accumulate=True)
+
+
+def pack_single_track(sd, pre: str, num_heads: int, device):
+    """Part-plane kernels where their widths fit: c_s = 384 (or 64, 128, 256), heads of 24 or 32, hidden a multiple of 64,
+    a pair width and head count the bias projection is built for; the un-fused fp32 kernels elsewhere."""
+    cs = sd[pre + "pre_norm_s.weight"].shape[0]
+    hidden = sd[pre + "transition_s.fc1.weight"].shape[0]
+    heads, cz = sd[pre + "attention.proj_z.1.weight"].shape
+    fits = (cs in weights.SPLIT_WIDTHS + (384,) and cs % num_heads == 0 and cs // num_heads in (24, 32) and hidden % 64 == 0
+            and cz in weights.SPLIT_WIDTHS and heads in (4, 8, 16))
+    return (SingleTrack if fits else SingleTrackF32)(sd, pre, num_heads, device)
+
+
+def single_track(s: torch.Tensor, z: torch.Tensor, tok_mask_u8: torch.Tensor, track, scratch: Scratch, after_z_read=None) -> None:
+    """The single track of one layer on all rows.  The pair-bias projection, its only read of z, comes first;
+    ``after_z_read`` is called behind it."""
+    bias = track.bias(z)
     if after_z_read is not None:
         after_z_read()
-    og = single_track_local(s, z, tok_mask_u8, w_norm, w_att, fused, num_heads, 0, bias)
-    single_track_finish(s, og, w_att, w_trans, fused)
+    track.finish(s, track.attention(s, bias, tok_mask_u8, 0, s.shape[0], scratch), scratch)

@@ -101,6 +101,9 @@ class B200PairformerLayer(nn.Module):
         self.token_s, self.token_z, self.num_heads = token_s, token_z, num_heads
         self.dropout, self.with_s, self.precision = dropout, with_s, precision
         self.fused = precision != "fp32"
+        # the fp32 tier's pair track runs on part planes where their kernels fit, on the un-fused fp32 kernels elsewhere
+        self.split = (not self.fused and token_z in weights.SPLIT_WIDTHS and pairwise_head_width == 32
+                      and pairwise_num_heads in (4, 8, 16))
         self.mx_contract_variant = 2   # 2 = block-scaled tcgen05, 0 = expand to bf16 + bf16 contraction (cross-check)
         for name, shape in layer_param_shapes(token_s, token_z, num_heads, pairwise_num_heads,
                                               pairwise_head_width, with_s):
@@ -118,27 +121,29 @@ class B200PairformerLayer(nn.Module):
             return self._packed
         sd = {k: v for k, v in self.state_dict().items()}
         pk: Dict[str, Dict[str, torch.Tensor]] = {"_device": device}
+        if self.fused:
+            pack_mul, pack_att, pack_trans = weights.pack_trimul, weights.pack_triatt, weights.pack_transition_z
+        elif self.split:
+            pack_mul, pack_att, pack_trans = weights.pack_split_trimul, weights.pack_split_triatt, weights.pack_split_transition
+        else:
+            pack_mul = pack_att = pack_trans = weights.to_device_f32
         for name in ("tri_mul_out", "tri_mul_in"):
-            pk[name] = (weights.pack_trimul(sd, name + ".", device) if self.fused
-                        else weights.to_device_f32(sd, name + ".", device))
+            pk[name] = pack_mul(sd, name + ".", device)
         for name in ("tri_att_start", "tri_att_end"):
-            pk[name] = (weights.pack_triatt(sd, name + ".", device) if self.fused
-                        else weights.to_device_f32(sd, name + ".", device))
-        pk["transition_z"] = (weights.pack_transition_z(sd, "transition_z.", device) if self.fused
-                              else weights.to_device_f32(sd, "transition_z.", device))
+            pk[name] = pack_att(sd, name + ".", device)
+        pk["transition_z"] = pack_trans(sd, "transition_z.", device)
         if self.with_s:
-            pk["pre_norm_s"] = weights.to_device_f32(sd, "pre_norm_s.", device)
-            pk["attention"] = weights.to_device_f32(sd, "attention.", device)
-            pk["transition_s"] = weights.to_device_f32(sd, "transition_s.", device)
-            pk["s_fused"] = ops.pack_single_track(pk["attention"], pk["transition_s"])
+            pk["single"] = ops.pack_single_track(sd, "", self.num_heads, device)
         self._packed = pk
         return pk
 
     def forward_inplace(self, s: Optional[torch.Tensor], z: torch.Tensor, tok_mask_u8: Optional[torch.Tensor],
-                        masks: ops.PairMasks, ws: Optional[ops.Workspace], side: Optional["SideTrack"] = None) -> None:
+                        masks: ops.PairMasks, ws: Optional[ops.Workspace], side: Optional["SideTrack"] = None,
+                        scratch: Optional[ops.Scratch] = None) -> None:
         """Update fp32 working copies z [N,N,128] and s [N,c_s] in place.  With a ``side`` track the update of s is
         only enqueued on its stream (the caller joins it before reading s)."""
         pk = self._pack(z.device)
+        scratch = scratch or ops.Scratch(z.device)
         wait_bias = side.before_z_write if side is not None else None
         if self.fused:
             if self.precision == "mxfp8":
@@ -150,6 +155,14 @@ class B200PairformerLayer(nn.Module):
             ops.tri_att_bf16(z, masks, pk["tri_att_start"], ws, False)
             ops.tri_att_bf16(z, masks, pk["tri_att_end"], ws, True)
             ops.transition_z_bf16(z, pk["transition_z"])
+        elif self.split:
+            if side is not None:
+                side.before_z_write()
+            ops.tri_mul_split(z, masks.pm, pk["tri_mul_out"], False, scratch)
+            ops.tri_mul_split(z, masks.pm, pk["tri_mul_in"], True, scratch)
+            ops.tri_att_split(z, masks.pm, pk["tri_att_start"], False, scratch)
+            ops.tri_att_split(z, masks.pm, pk["tri_att_end"], True, scratch)
+            ops.transition_split(z, pk["transition_z"], scratch)
         else:
             if side is not None:
                 side.before_z_write()
@@ -160,15 +173,13 @@ class B200PairformerLayer(nn.Module):
             ops.transition_f32(z, pk["transition_z"])
         if self.with_s and s is not None:
             if side is None:
-                ops.single_track(s, z, tok_mask_u8, pk["pre_norm_s"], pk["attention"], pk["transition_s"], self.num_heads,
-                                 pk["s_fused"])
+                ops.single_track(s, z, tok_mask_u8, pk["single"], scratch)
             else:
                 z_ready = torch.cuda.Event()
                 z_ready.record()
                 with torch.cuda.stream(side.stream):
                     side.stream.wait_event(z_ready)
-                    ops.single_track(s, z, tok_mask_u8, pk["pre_norm_s"], pk["attention"], pk["transition_s"], self.num_heads,
-                                     pk["s_fused"], side.mark_z_read)
+                    ops.single_track(s, z, tok_mask_u8, pk["single"], ops.Scratch(z.device), side.mark_z_read)
 
     def forward(self, s: Optional[torch.Tensor], z: torch.Tensor, mask: Optional[torch.Tensor] = None,
                 pair_mask: Optional[torch.Tensor] = None, chunk_size_tri_attn: Optional[int] = None,
@@ -196,12 +207,14 @@ class B200PairUpdateBlock(nn.Module):
     """The block of the ESMFold2 folding trunk (tt_bio/esmfold2.py:129-154): ``z += tri_mul_out(z); z += tri_mul_in(z);
     z += transition(z)``, no triangle attention, any pair width and transition width.  Keys as in the Pairformer layer
     (``tri_mul_out.*``, ``tri_mul_in.*``, ``transition_z.*``); ``remaps.esmfold2_pair_update_block`` produces them from
-    an ESMFold2 checkpoint.  Runs on the un-fused fp32 kernels."""
+    an ESMFold2 checkpoint.  fp32: on part planes where the widths fit (64, 128, 256 and a hidden width that is a
+    multiple of 64), on the un-fused fp32 kernels elsewhere."""
 
     def __init__(self, token_z: int = 256, hidden: Optional[int] = None) -> None:
         super().__init__()
         hidden = hidden or 4 * token_z
         self.token_z, self.hidden = token_z, hidden
+        self.split = token_z in weights.SPLIT_WIDTHS and hidden % 64 == 0
         for name in ("tri_mul_out", "tri_mul_in"):
             for leaf, shape in (("norm_in.weight", (token_z,)), ("norm_in.bias", (token_z,)),
                                 ("p_in.weight", (2 * token_z, token_z)), ("g_in.weight", (2 * token_z, token_z)),
@@ -218,13 +231,22 @@ class B200PairUpdateBlock(nn.Module):
         if self._packed is None or self._packed["_device"] != device:
             sd = dict(self.state_dict().items())
             self._packed = {"_device": device}
-            for name in ("tri_mul_out", "tri_mul_in", "transition_z"):
-                self._packed[name] = weights.to_device_f32(sd, name + ".", device)
+            pack_mul, pack_trans = ((weights.pack_split_trimul, weights.pack_split_transition) if self.split
+                                    else (weights.to_device_f32, weights.to_device_f32))
+            for name in ("tri_mul_out", "tri_mul_in"):
+                self._packed[name] = pack_mul(sd, name + ".", device)
+            self._packed["transition_z"] = pack_trans(sd, "transition_z.", device)
         return self._packed
 
     def forward_inplace(self, z: torch.Tensor, pair_mask_u8: torch.Tensor) -> None:
         """z [N, N, c_z] contiguous fp32, updated where it is; pair_mask_u8 [N, N]."""
         pk = self._pack(z.device)
+        if self.split:
+            scratch = ops.Scratch(z.device)
+            ops.tri_mul_split(z, pair_mask_u8, pk["tri_mul_out"], False, scratch)
+            ops.tri_mul_split(z, pair_mask_u8, pk["tri_mul_in"], True, scratch)
+            ops.transition_split(z, pk["transition_z"], scratch)
+            return
         ops.tri_mul_f32(z, pair_mask_u8, pk["tri_mul_out"], False)
         ops.tri_mul_f32(z, pair_mask_u8, pk["tri_mul_in"], True)
         ops.transition_f32(z, pk["transition_z"])
@@ -289,8 +311,9 @@ def _run_layers(layers, s, z, mask, pair_mask, ws_cache: Optional[dict] = None, 
         side = None
         if sw is not None and len(layers) > 1 and os.environ.get("B200PF_SIDE_TRACK", "0") == "1":
             side = SideTrack(z.device)
+        scratch = ops.Scratch(z.device)
         for layer in layers:
-            layer.forward_inplace(sw, zw, tm, pm, ws, side)
+            layer.forward_inplace(sw, zw, tm, pm, ws, side, scratch)
         if side is not None:
             side.join()
     if inplace:

@@ -370,14 +370,14 @@ def sharded_block(layer: B200PairformerLayer, s: Optional[torch.Tensor], z_loc: 
     # ---- single track: attention for the local query rows, the rest replicated --------------------
     if layer.with_s and s is not None:
         def single_track(channel: int) -> None:
-            bias = ops.pair_bias_heads(z_loc, pk["attention"])
+            track, scratch = pk["single"], ops.Scratch(z_loc.device)
+            bias = track.bias(z_loc)
             if side is not None:
                 side.mark_z_read()
-            og_loc = ops.single_track_local(s, z_loc, tok_mask_u8, pk["pre_norm_s"], pk["attention"], pk["s_fused"],
-                                            layer.num_heads, r0, bias)
+            og_loc = track.attention(s, bias, tok_mask_u8, r0, nr, scratch)
             # output projection and transition are per row: run them on the local rows, then gather s
             s_loc = s[r0:r0 + nr]
-            ops.single_track_finish(s_loc, og_loc, pk["attention"], pk["transition_s"], pk["s_fused"])
+            track.finish(s_loc, og_loc, scratch)
             s.copy_(all_gather_cat(s_loc, group, "s_rows", channel).view(n, s.shape[1]))
 
         if side is None:
