@@ -2,7 +2,7 @@
 // These exist so that the 1e-4-per-layer tier can be met on the GPU (tensor cores have no
 // fp32 mode) and they double as the single-track path, which the reference keeps in fp32
 // (tt_bio/reference.py:906-912).  Speed is secondary here; clarity and exactness come first.
-#include "common.cuh"
+#include "pdl.cuh"
 
 namespace b200pf {
 
@@ -431,11 +431,12 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], uint32_t a0, uint32_t a1
 }
 
 __global__ void __launch_bounds__(256)
-ln_proj_heads16_mma_kernel(const float* __restrict__ z, const float* __restrict__ gamma, const float* __restrict__ beta,
-                           const float* __restrict__ w, float* __restrict__ out, long long out_hs, long long rows) {
+ln_proj_heads16_mma_kernel(const float* z, const float* gamma, const float* beta, const float* w, float* out, long long out_hs, long long rows) {
     constexpr int C = 128, HEADS = 16;
     __shared__ uint2 w_hi[16][2][32], w_lo[16][2][32];       // [k step][n tile][lane] -> (b0, b1)
     __shared__ float cs[HEADS];
+    grid_dependency_wait();
+    grid_launch_dependents();
     for (int i = threadIdx.x; i < 16 * 2 * 32; i += blockDim.x) {
         const int ln = i & 31, nt = (i >> 5) & 1, ks = i >> 6;
         const int g = ln >> 2, t = ln & 3, h = nt * 8 + g, c0 = 16 * (ks >> 1) + 4 * t + 2 * (ks & 1);
@@ -466,7 +467,7 @@ ln_proj_heads16_mma_kernel(const float* __restrict__ z, const float* __restrict_
             const float4* src = reinterpret_cast<const float4*>(z + (row < rows ? row : 0) * C) + t;
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                const float4 v = row < rows ? __ldg(src + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 v = row < rows ? src[4 * q] : make_float4(0.f, 0.f, 0.f, 0.f);
                 x[r][4 * q] = v.x; x[r][4 * q + 1] = v.y; x[r][4 * q + 2] = v.z; x[r][4 * q + 3] = v.w;
             }
         }
@@ -922,12 +923,10 @@ int b200pf_ln_proj_heads(const float* z, const float* gamma, const float* beta, 
                    "ln_proj_heads: built for c = 128 and 4 or 16 heads (got c=%d heads=%d)", c, heads);
     B200PF_REQUIRE(aligned16(z), B200PF_ERR_INVALID, "ln_proj_heads: z must be 16-byte aligned");
     if (rows == 0) return B200PF_OK;
-    unsigned blocks = (unsigned)min((long long)148 * 4, (rows + 255) / 256);
-    if (heads == 4)
-        ln_proj_heads_kernel<4><<<blocks, 256, 0, (cudaStream_t)stream>>>(z, gamma, beta, w, out, out_hs, rows);
-    else
-        ln_proj_heads16_mma_kernel<<<(unsigned)min((long long)148 * 2, (rows + 127) / 128), 256, 0, (cudaStream_t)stream>>>(
-            z, gamma, beta, w, out, out_hs, rows);
+    if (heads == 16)
+        return launch_pdl(ln_proj_heads16_mma_kernel, dim3((unsigned)min((long long)148 * 2, (rows + 127) / 128)), dim3(256), 0, (cudaStream_t)stream,
+                          z, gamma, beta, w, out, out_hs, rows);
+    ln_proj_heads_kernel<4><<<(unsigned)min((long long)148 * 4, (rows + 255) / 256), 256, 0, (cudaStream_t)stream>>>(z, gamma, beta, w, out, out_hs, rows);
     B200PF_LAUNCH_CHECK();
     return B200PF_OK;
 }

@@ -5,7 +5,7 @@
 // Every GEMM operand is bf16 and K-major; the token axis is padded to a multiple of 8 (`np`) so that rows of
 // every operand start 16-byte aligned, with zero rows for the padding tokens (the pair-weighted averaging pads to
 // 32: its projected rows are written in groups of np columns).
-#include "common.cuh"
+#include "pdl.cuh"
 
 namespace b200pf {
 namespace msa {
@@ -48,8 +48,9 @@ ln_rows_bf16_kernel(const float* __restrict__ m, const float* __restrict__ gamma
 // w[h][i][j] = softmax_j(logit[h][i][j] - inf * (1 - mask[i][j])) as bf16 rows of `pitch` elements (zero beyond n).
 // One warp per (head, i).
 __global__ void __launch_bounds__(256)
-pwa_softmax_kernel(const float* __restrict__ logits, const uint8_t* __restrict__ mask, __nv_bfloat16* __restrict__ w,
-                   int n, int pitch, int heads, float inf_value) {
+pwa_softmax_kernel(const float* logits, const uint8_t* mask, __nv_bfloat16* w, int n, int pitch, int heads, float inf_value) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const int lane = threadIdx.x & 31;
     const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= (long long)heads * n) return;
@@ -182,10 +183,8 @@ extern "C" int b200pf_pwa_softmax(const float* logits, const uint8_t* mask, b200
                                   float inf_value, void* stream) {
     B200PF_REQUIRE(logits && mask && w && n > 0 && pitch >= n && heads > 0, B200PF_ERR_INVALID, "pwa_softmax: bad arguments");
     const long long rows = (long long)heads * n;
-    msa::pwa_softmax_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, (cudaStream_t)stream>>>(logits, mask, (__nv_bfloat16*)w, n, pitch,
-                                                                                          heads, inf_value);
-    B200PF_LAUNCH_CHECK();
-    return B200PF_OK;
+    return launch_pdl(msa::pwa_softmax_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, (cudaStream_t)stream, logits, mask, (__nv_bfloat16*)w, n, pitch,
+                      heads, inf_value);
 }
 
 extern "C" int b200pf_pwa_gate_transpose(const b200pf_bf16* o, const b200pf_bf16* g, b200pf_bf16* val, int s_len, int np,

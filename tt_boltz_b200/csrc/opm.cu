@@ -13,7 +13,7 @@
 //   opm_mask_bits_kernel: the MSA mask as one bit per sequence, 32 sequences per word and token.
 //   opm_finalize_kernel : pair counts by popcount of the two tokens' words, then y / count + bias added into (or
 //                         written over) the fp32 pair rows.
-#include "common.cuh"
+#include "pdl.cuh"
 
 namespace b200pf {
 namespace opm {
@@ -72,7 +72,9 @@ opm_producer_kernel(const float* __restrict__ m, const uint8_t* __restrict__ mas
     }
 }
 
-__global__ void opm_mask_bits_kernel(const uint8_t* __restrict__ mask, uint32_t* __restrict__ bits, int s_len, int n, int words) {
+__global__ void opm_mask_bits_kernel(const uint8_t* mask, uint32_t* bits, int s_len, int n, int words) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const int tok = blockIdx.x * blockDim.x + threadIdx.x, w = blockIdx.y;
     if (tok >= n) return;
     uint32_t v = 0;
@@ -84,8 +86,9 @@ __global__ void opm_mask_bits_kernel(const uint8_t* __restrict__ mask, uint32_t*
 }
 
 __global__ void __launch_bounds__(FIN_THREADS)
-opm_finalize_kernel(const __nv_bfloat16* __restrict__ y, const uint32_t* __restrict__ bits, const float* __restrict__ bias,
-                    float* __restrict__ z, int i0, int n, int words, int accumulate) {
+opm_finalize_kernel(const __nv_bfloat16* y, const uint32_t* bits, const float* bias, float* z, int i0, int n, int words, int accumulate) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     __shared__ uint32_t bi_s[MAX_WORDS];
     __shared__ float inv_s[FIN_J];
     const int il = blockIdx.y, i = i0 + il, j0 = blockIdx.x * FIN_J;
@@ -96,18 +99,18 @@ opm_finalize_kernel(const __nv_bfloat16* __restrict__ y, const uint32_t* __restr
         int cnt = 0;
         if (j < n) {
             const uint32_t* bj = bits + (long long)j * words;
-            for (int w = 0; w < words; ++w) cnt += __popc(bi_s[w] & __ldg(bj + w));
+            for (int w = 0; w < words; ++w) cnt += __popc(bi_s[w] & bj[w]);
         }
         inv_s[threadIdx.x] = 1.f / (float)(cnt > 0 ? cnt : 1);
     }
     __syncthreads();
     const int c4 = threadIdx.x & 31;                                  // four channels
-    const float4 b4 = __ldg(reinterpret_cast<const float4*>(bias) + c4);
+    const float4 b4 = reinterpret_cast<const float4*>(bias)[c4];
     for (int jl = threadIdx.x >> 5; jl < FIN_J; jl += FIN_THREADS / 32) {
         const int j = j0 + jl;
         if (j >= n) break;
         const long long row = (long long)il * n + j;
-        const uint2 yv = __ldg(reinterpret_cast<const uint2*>(y + row * 128) + c4);
+        const uint2 yv = reinterpret_cast<const uint2*>(y + row * 128)[c4];
         const float inv = inv_s[jl];
         float4 o;
         o.x = fmaf(bf16_lo(yv.x), inv, b4.x);
@@ -148,9 +151,7 @@ extern "C" int b200pf_opm_mask_bits(const uint8_t* mask, uint32_t* bits, int s_l
     const int words = (s_len + 31) / 32;
     B200PF_REQUIRE(words <= 65535, B200PF_ERR_UNSUPPORTED, "opm_mask_bits: too many sequences");
     dim3 grid((unsigned)((n + 127) / 128), (unsigned)words);
-    opm_mask_bits_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(mask, bits, s_len, n, words);
-    B200PF_LAUNCH_CHECK();
-    return B200PF_OK;
+    return launch_pdl(opm_mask_bits_kernel, grid, dim3(128), 0, (cudaStream_t)stream, mask, bits, s_len, n, words);
 }
 
 extern "C" int b200pf_opm_finalize(const b200pf_bf16* y, const uint32_t* bits, const float* bias, float* z, int s_len,
@@ -162,7 +163,5 @@ extern "C" int b200pf_opm_finalize(const b200pf_bf16* y, const uint32_t* bits, c
     B200PF_REQUIRE(s_len > 0 && words <= MAX_WORDS, B200PF_ERR_UNSUPPORTED, "opm_finalize: at most %d sequences", MAX_WORDS * 32);
     B200PF_REQUIRE(n > 0 && i0 >= 0 && n_i > 0 && i0 + n_i <= n && n_i <= 65535, B200PF_ERR_INVALID, "opm_finalize: bad sizes");
     dim3 grid((unsigned)((n + FIN_J - 1) / FIN_J), (unsigned)n_i);
-    opm_finalize_kernel<<<grid, FIN_THREADS, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)y, bits, bias, z, i0, n, words, accumulate);
-    B200PF_LAUNCH_CHECK();
-    return B200PF_OK;
+    return launch_pdl(opm_finalize_kernel, grid, dim3(FIN_THREADS), 0, (cudaStream_t)stream, (const __nv_bfloat16*)y, bits, bias, z, i0, n, words, accumulate);
 }

@@ -1,0 +1,51 @@
+// Programmatic dependent launch.
+//
+// A kernel launched with launch_pdl may start while its predecessor on the stream drains: what stands before
+// grid_dependency_wait() (barriers, tensor memory, descriptors) overlaps the predecessor's tail and the launch itself.
+// Nothing that the predecessor wrote, or reads, may be touched before the wait, and weights count as written: a program may
+// have updated them on the stream.  Every CTA executes the wait, on every path, so that a kernel's completion implies that of
+// all before it.  Kernels launched this way read global memory with plain loads: an ld.global.nc (__ldg, const __restrict__)
+// may be moved above the wait.
+#pragma once
+
+#include <utility>
+
+#include "common.cuh"
+
+namespace b200pf {
+
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... KArgs, class... Args>
+static inline int launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    B200PF_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+    count_launch();
+    return B200PF_OK;
+}
+
+// Multiprocessors of the current device, asked for once per device.
+static inline int multiprocessors(int* out) {
+    static int known[64] = {0};
+    int dev = 0;
+    B200PF_CUDA(cudaGetDevice(&dev));
+    int sms = dev >= 0 && dev < 64 ? known[dev] : 0;
+    if (sms == 0) {
+        B200PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        if (dev >= 0 && dev < 64) known[dev] = sms;
+    }
+    *out = sms;
+    return B200PF_OK;
+}
+
+}  // namespace b200pf

@@ -44,7 +44,7 @@ constexpr int SMEM_BYTES = OFF_BAR + 128;               // 231,552: the dynamic 
 constexpr int EPI_BAR_ID = 1;
 
 struct Bars {
-    uint64_t a_full[2], a_empty[2], acc_full[2], acc_empty[2];
+    uint64_t a_full[2], a_empty[2], acc_full[2], acc_empty[2], w_full;
     uint32_t tmem_slot;
     int abort_flag;
 };
@@ -70,10 +70,12 @@ __device__ __forceinline__ float tanh_approx(float x) {
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
 row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
-              const __grid_constant__ CUtensorMap map2, const __grid_constant__ CUtensorMap map3, Args p, unsigned int* status) {
+              const __grid_constant__ CUtensorMap map2, const __grid_constant__ CUtensorMap map3,
+              const __grid_constant__ CUtensorMap map_w, Args p, unsigned int* status) {
     using namespace sm100;
     extern __shared__ __align__(1024) uint8_t smem[];
     if ((smem_u32(smem) & 1023u) != 0) {       // swizzled tiles need 1024-byte alignment; there is no slack to fix it up
+        grid_dependency_wait();
         if (threadIdx.x == 0) atomicOr(status, DEV_STATUS_BAD_INDEX);
         return;
     }
@@ -85,21 +87,27 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
     const int span = p.transposed ? p.rows : p.n;                 // positions along a line
     const int n_lines = p.transposed ? p.n : p.rows;
     const int tpl = (span + TM - 1) / TM;
-    const long long tiles = (long long)n_lines * tpl;
+    const int tiles = n_lines * tpl;                              // below 2^31: a row is at least 256 bytes of memory
 
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(&B->a_full[i], LOAD_WARPS); mbar_init(&B->a_empty[i], MODE == MODE_TRIATT ? 1 + EPI_WARPS : 1);
             mbar_init(&B->acc_full[i], 1); mbar_init(&B->acc_empty[i], EPI_WARPS);
         }
+        mbar_init(&B->w_full, 1);
         B->abort_flag = 0;
         fence_barrier_init();
+        fence_proxy_async();
     }
-    load_weights_sw128(smem, p.w, 512, tid, THREADS);
+    if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (tid == 0) {
+        mbar_arrive_expect_tx(&B->w_full, W_BYTES);
+        load_weights_tma(smem, &map_w, 512, &B->w_full);
+    }
     if (MODE == MODE_TRIATT)
         for (int i = tid; i < 4 * 128; i += THREADS) wb_s[i] = p.w_bias_f32[i];
-    fence_proxy_async();
-    if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -116,13 +124,13 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         float4 gam[4], bet[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            gam[j] = __ldg(reinterpret_cast<const float4*>(p.ln_gamma) + j * 8 + sub);
-            bet[j] = __ldg(reinterpret_cast<const float4*>(p.ln_beta) + j * 8 + sub);
+            gam[j] = reinterpret_cast<const float4*>(p.ln_gamma)[j * 8 + sub];
+            bet[j] = reinterpret_cast<const float4*>(p.ln_beta)[j * 8 + sub];
         }
         uint32_t it = 0;
         bool ok = true;
-        for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
-            const int line = (int)(t / tpl), pos0 = (int)(t % tpl) * TM;
+        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
+            const int line = t / tpl, pos0 = (t - line * tpl) * TM;
             const uint32_t stage = it & 1, ph = (it >> 1) & 1;
             ok = mbar_wait(&B->a_empty[stage], ph ^ 1, abort_flag);
             if (!ok) break;
@@ -130,9 +138,9 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
             // this warp's 32 rows of the NEXT tile: one lane per row asks L2 for its four 128-byte lines, so the
             // loads of the next round find them there instead of paying the DRAM latency with only 4 warps in flight
             {
-                const long long tn = t + gridDim.x;
+                const int tn = t + (int)gridDim.x, ln = tn / tpl;
                 if (tn < tiles) {
-                    const long long f = flat_of((int)(tn / tpl), (int)(tn % tpl) * TM + warp * 32 + lane);
+                    const long long f = flat_of(ln, (tn - ln * tpl) * TM + warp * 32 + lane);
                     if (f >= 0) {
                         if (p.z_bf16) {
                             const char* rowp = reinterpret_cast<const char*>(p.z_bf16 + f * KC);
@@ -150,21 +158,24 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
             for (int pass = 0; pass < 2; ++pass) {
                 const int row0 = warp * 32 + pass * 16;
                 float4 v[4][4];
-                long long fl[4];
+                // rows 4 i of the pass: one flat index and a stride (positions of a column lie n rows apart)
+                const int pos_b = pos0 + row0 + rq;
+                const long long f0 = p.transposed ? (long long)pos_b * p.n + line : (long long)line * p.n + pos_b;
+                const long long fstep = p.transposed ? 4LL * p.n : 4LL;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    fl[i] = flat_of(line, pos0 + row0 + i * 4 + rq);
+                    const bool valid = pos_b + i * 4 < span;
                     if (p.z_bf16) {          // warp-uniform: four bf16 channels per lane and j, widened on the fly
-                        const uint2* src = reinterpret_cast<const uint2*>(p.z_bf16 + (fl[i] < 0 ? 0 : fl[i]) * KC);
+                        const uint2* src = reinterpret_cast<const uint2*>(p.z_bf16 + (f0 + i * fstep) * KC) + sub;
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            const uint2 w = fl[i] < 0 ? make_uint2(0u, 0u) : __ldg(src + j * 8 + sub);
+                            const uint2 w = valid ? src[j * 8] : make_uint2(0u, 0u);
                             v[i][j] = make_float4(bf16_lo(w.x), bf16_hi(w.x), bf16_lo(w.y), bf16_hi(w.y));
                         }
                     } else {
-                        const float4* src = reinterpret_cast<const float4*>(p.z + (fl[i] < 0 ? 0 : fl[i]) * KC);
+                        const float4* src = reinterpret_cast<const float4*>(p.z + (f0 + i * fstep) * KC) + sub;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) v[i][j] = fl[i] < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldg(src + j * 8 + sub);
+                        for (int j = 0; j < 4; ++j) v[i][j] = valid ? src[j * 8] : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
                 }
                 // The four rows of a pass are worked on stage by stage (all sums, then all shuffles, ...), not row by
@@ -172,8 +183,8 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
                 float kz[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    bool keep = fl[i] >= 0;
-                    if (MODE != MODE_TRIATT) keep = keep && __ldg(p.mask + (fl[i] < 0 ? 0 : fl[i])) != 0;
+                    bool keep = pos_b + i * 4 < span;
+                    if (MODE != MODE_TRIATT) keep = keep && p.mask[f0 + i * fstep] != 0;
                     kz[i] = keep ? 1.f : 0.f;
                 }
                 float s4[4];
@@ -235,8 +246,8 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         const uint64_t d_x0 = make_desc_k_sw128(smem_u32(smem + OFF_A));
         constexpr uint32_t W_KB16 = W_KB >> 4, A_KB16 = A_KB_BYTES >> 4;
         uint32_t it = 0, acc_cnt[2] = {0, 0};
-        bool ok = true;
-        for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
+        bool ok = mbar_wait_warp(&B->w_full, 0, abort_flag);
+        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
             const uint32_t stage = it & 1, ph = (it >> 1) & 1;
             ok = mbar_wait_warp(&B->a_full[stage], ph, abort_flag);
             if (!ok) break;
@@ -315,8 +326,8 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
                 bulk_commit();
             }
         };
-        for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++acc_cnt) {
-            const int line = (int)(t / tpl), pos0 = (int)(t % tpl) * TM;
+        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++acc_cnt) {
+            const int line = t / tpl, pos0 = (t - line * tpl) * TM;
             for (int half = 0; half < 2 && ok; ++half) {
                 ok = mbar_wait(&B->acc_full[half], acc_cnt & 1, abort_flag);
                 if (!ok) break;
@@ -481,17 +492,12 @@ static int launch(const Args& a, cudaStream_t st) {
     B200PF_REQUIRE(a.ln_gamma && a.ln_beta && aligned16(a.ln_gamma) && aligned16(a.ln_beta), B200PF_ERR_INVALID,
                    "row512: LayerNorm gain / offset must be given and 16-byte aligned");
     B200PF_SMEM_ATTR_ONCE(row512_kernel<MODE>, SMEM_BYTES);
-    int dev = 0, sms = 148;
-    B200PF_CUDA(cudaGetDevice(&dev));
-    B200PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     int span = a.transposed ? a.rows : a.n, lines = a.transposed ? a.n : a.rows;
     long long tiles = (long long)lines * ((span + TM - 1) / TM);
-    CUtensorMap m[4];
-    int rc = make_maps(MODE, a, m);
-    if (rc != B200PF_OK) return rc;
-    row512_kernel<MODE><<<(unsigned)(tiles < sms ? tiles : sms), THREADS, SMEM_BYTES, st>>>(m[0], m[1], m[2], m[3], a, status);
-    B200PF_LAUNCH_CHECK();
-    return B200PF_OK;
+    CUtensorMap m[4], m_w;
+    int sms, rc;
+    if ((rc = multiprocessors(&sms)) != B200PF_OK || (rc = make_maps(MODE, a, m)) != B200PF_OK || (rc = weight_map(&m_w, a.w, 512, "w")) != B200PF_OK) return rc;
+    return launch_pdl(row512_kernel<MODE>, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(THREADS), SMEM_BYTES, st, m[0], m[1], m[2], m[3], m_w, a, status);
 }
 
 int launch_trimul(const Args& a, cudaStream_t st) { return launch<MODE_TRIMUL>(a, st); }

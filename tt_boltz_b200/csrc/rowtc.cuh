@@ -4,7 +4,9 @@
 // shared memory in the same layout, epilogue warps read the fp32 result from TMEM.
 #pragma once
 
+#include "pdl.cuh"
 #include "sm100.cuh"
+#include "tmap.cuh"
 
 namespace b200pf {
 namespace rtc {
@@ -19,14 +21,21 @@ __device__ __forceinline__ uint32_t sw128(int row, int chunk) {
     return (uint32_t)(row * 128 + ((chunk ^ (row & 7)) << 4));
 }
 
-// Copy W[rows][128] (bf16, row-major in global memory) into shared memory as two k-blocks of
-// [rows][128 bytes] with the 128-byte swizzle.  All `nthreads` threads take part.
-__device__ __forceinline__ void load_weights_sw128(uint8_t* dst, const __nv_bfloat16* src, int rows, int tid, int nthreads) {
-    for (int i = tid; i < rows * 16; i += nthreads) {
-        int r = i >> 4, c16 = i & 15;
-        uint4 v = __ldg(reinterpret_cast<const uint4*>(src + (long long)r * KC) + c16);
-        *reinterpret_cast<uint4*>(dst + (c16 >> 3) * (rows * 128) + sw128(r, c16 & 7)) = v;
-    }
+// Fetch W[rows][128] (bf16, tensor map of weight_map) into shared memory as two k-blocks of [rows][128 bytes] with the
+// 128-byte swizzle, counted on `bar`; issued by one thread.  The copy runs under the first tile's LayerNorm: done by all
+// threads before anything else started (load, store, barrier), 128 KB of weights and the launch gap were 9 of the 22 us that
+// a producer took at 45 tokens, where every CTA has one tile (22.5 -> 13.1 us; 1024 tokens 248 -> 240 us).
+constexpr int W_BOX_ROWS = 128;
+__device__ __forceinline__ void load_weights_tma(uint8_t* dst, const CUtensorMap* map, int rows, uint64_t* bar) {
+    for (int kb = 0; kb < 2; ++kb)
+        for (int r = 0; r < rows; r += W_BOX_ROWS)
+            sm100::tma_load_4d(dst + kb * (rows * 128) + r * 128, map, bar, kb * 64, r, 0, 0);
+}
+static inline int weight_map(CUtensorMap* map, const void* w, int rows, const char* what) {
+    cuuint64_t dims[4] = {(cuuint64_t)KC, (cuuint64_t)rows, 1, 1};
+    cuuint64_t str[3] = {KC * 2, (cuuint64_t)rows * KC * 2, (cuuint64_t)rows * KC * 2};
+    cuuint32_t box[4] = {64, W_BOX_ROWS, 1, 1};
+    return tmap_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, w, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, what);
 }
 
 // LayerNorm (no affine) of 16 rows into the A tile; called by one warp.  Lane layout: 8 lanes per

@@ -119,7 +119,7 @@ __device__ __forceinline__ void zero_acc(float (&acc)[2][NT][4]) {
 __device__ __forceinline__ void load_weights_k128(__nv_bfloat16* dst, const __nv_bfloat16* src, int rows) {
     for (int i = threadIdx.x; i < rows * 16; i += blockDim.x) {
         int r = i >> 4, c = i & 15;
-        *reinterpret_cast<uint4*>(dst + r * APITCH + c * 8) = __ldg(reinterpret_cast<const uint4*>(src + r * KC + c * 8));
+        *reinterpret_cast<uint4*>(dst + r * APITCH + c * 8) = *reinterpret_cast<const uint4*>(src + r * KC + c * 8);
     }
 }
 

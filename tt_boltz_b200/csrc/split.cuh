@@ -11,18 +11,11 @@
 
 #include <cuda_fp16.h>
 
+#include "pdl.cuh"
 #include "sm100.cuh"
 
 namespace b200pf {
 namespace split {
-
-// ---- programmatic dependent launch ---------------------------------------------------------------
-// A kernel launched with launch_pdl may start while its predecessor on the stream drains: everything before
-// grid_dependency_wait() (barriers, tensor memory, descriptors) overlaps the predecessor's tail; nothing the
-// predecessor wrote, or reads, may be touched before it.  Kernels launched this way read global memory with plain loads only:
-// an ld.global.nc (__ldg, const __restrict__) may be moved above the wait.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
     __half2 t = __floats2half2_rn(lo, hi);
@@ -43,23 +36,6 @@ __device__ __forceinline__ void split_bf16x3(float a, float b, uint32_t& h, uint
 }
 
 // ---- host side -----------------------------------------------------------------------------------
-template <class... KArgs, class... Args>
-static inline int launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    B200PF_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
-    count_launch();
-    return B200PF_OK;
-}
-
 // Two-part (fp16) or three-part (bf16) operand of a GEMM: element (part, batch, row, col) at
 // ptr + part * part_stride + batch * batch_stride + row * row_stride + col (16-bit elements; strides multiples of 8).
 struct Operand {

@@ -83,6 +83,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_c
     using namespace sm100;
     extern __shared__ __align__(1024) uint8_t smem[];
     if ((smem_u32(smem) & 1023u) != 0) {
+        grid_dependency_wait();
         if (threadIdx.x == 0) atomicOr(status, DEV_STATUS_BAD_INDEX);
         return;
     }
@@ -103,6 +104,8 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_c
         fence_barrier_init();
     }
     if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
+    grid_dependency_wait();
+    grid_launch_dependents();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -114,8 +117,8 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_c
         float4 gam[4], bet[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            gam[j] = __ldg(reinterpret_cast<const float4*>(p.ln_gamma) + j * 8 + sub);
-            bet[j] = __ldg(reinterpret_cast<const float4*>(p.ln_beta) + j * 8 + sub);
+            gam[j] = reinterpret_cast<const float4*>(p.ln_gamma)[j * 8 + sub];
+            bet[j] = reinterpret_cast<const float4*>(p.ln_beta)[j * 8 + sub];
         }
         uint32_t it = 0;
         bool ok = true;
@@ -137,14 +140,13 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_c
             for (int pass = 0; pass < 2; ++pass) {
                 const int row0 = warp * 32 + pass * 16;
                 float4 v[4][4];
-                bool valid[4];
+                // rows beyond the last one repeat row 0: the reduce-add clips them
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const long long f = base + row0 + i * 4 + rq;
-                    valid[i] = f < p.rows_flat;
-                    const float4* src = reinterpret_cast<const float4*>(p.z + (valid[i] ? f : 0) * KC);
+                    const float4* src = reinterpret_cast<const float4*>(p.z + (f < p.rows_flat ? f : 0) * KC);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) v[i][j] = valid[i] ? __ldg(src + j * 8 + sub) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int j = 0; j < 4; ++j) v[i][j] = src[j * 8 + sub];
                 }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -166,12 +168,11 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_c
                     ss += __shfl_xor_sync(0xffffffffu, ss, 2);
                     ss += __shfl_xor_sync(0xffffffffu, ss, 4);
                     const float rstd = rsqrtf(ss * (1.f / KC) + LN_EPS);
-                    const float kz = valid[i] ? 1.f : 0.f;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         uint2 o;
-                        o.x = pack_bf16x2(fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x) * kz, fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y) * kz);
-                        o.y = pack_bf16x2(fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z) * kz, fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w) * kz);
+                        o.x = pack_bf16x2(fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x), fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y));
+                        o.y = pack_bf16x2(fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z), fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w));
                         const int chunk = (j & 1) * 4 + (sub >> 1);
                         *reinterpret_cast<uint2*>(a_tile + (j >> 1) * A_KB_BYTES + sw128(row, chunk) + (sub & 1) * 8) = o;
                     }
@@ -372,12 +373,9 @@ extern "C" int b200pf_transition_z_tc(float* z, const float* ln_gamma, const flo
     unsigned int* status = device_status_word();
     B200PF_REQUIRE(status, B200PF_ERR_CUDA, "transition_z_tc: no device status word");
     B200PF_SMEM_ATTR_ONCE(transition_tc_kernel, SMEM_BYTES);
-    int dev = 0, sms = 148;
-    B200PF_CUDA(cudaGetDevice(&dev));
-    B200PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms;
+    if ((rc = multiprocessors(&sms)) != B200PF_OK) return rc;
     long long tiles = (n_rows_flat + TM - 1) / TM;
     Args a{z, ln_gamma, ln_beta, n_rows_flat};
-    transition_tc_kernel<<<(unsigned)(tiles < sms ? tiles : sms), THREADS, SMEM_BYTES, (cudaStream_t)stream>>>(m12, m3, mz, a, status);
-    B200PF_LAUNCH_CHECK();
-    return B200PF_OK;
+    return launch_pdl(transition_tc_kernel, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, m12, m3, mz, a, status);
 }

@@ -23,6 +23,7 @@
 // (1.43 ms since the groups of a pair get their scores independently).
 // Scores are in the log2 domain (host folds log2(e)/sqrt(32) into W_q and log2(e) into the bias).
 // Every wait is bounded; a wait that runs out raises the status word and the CTA unwinds.
+#include "pdl.cuh"
 #include "sm100.cuh"
 #include "tmap.cuh"
 
@@ -180,6 +181,7 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     using namespace sm100;
     extern __shared__ __align__(1024) uint8_t smem[];
     if ((smem_u32(smem) & 1023u) != 0) {       // swizzled tiles need 1024-byte alignment; there is no slack to fix it up
+        grid_dependency_wait();
         if (threadIdx.x == 0) atomicOr(status, DEV_STATUS_BAD_INDEX);
         return;
     }
@@ -213,6 +215,8 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
     fence_proxy_async();
     if (warp == MMA_WARP0) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
+    grid_dependency_wait();
+    grid_launch_dependents();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -356,7 +360,7 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         // The key mask of a line is the same for every query row, i.e. uniform over the warp: lane l fetches the
         // mask bytes of keys 2l and 2l+1 of the NEXT tile, and two ballots turn them into one bit per key.
         auto mask_fetch = [&](const uint8_t* mrow, int j) -> uint32_t {
-            return (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(mrow + j * AK) + lane);
+            return (uint32_t)reinterpret_cast<const unsigned short*>(mrow + j * AK)[lane];
         };
         for (long long it = blockIdx.x; it < items && ok; it += gridDim.x) {
             int qt, h, line0;
@@ -558,13 +562,11 @@ extern "C" int b200pf_triatt_core_tc4(const b200pf_bf16* q, const b200pf_bf16* k
     unsigned int* status = device_status_word();
     B200PF_REQUIRE(status, B200PF_ERR_CUDA, "triatt_core_tc4: no device status word");
     B200PF_SMEM_ATTR_ONCE(triatt_core_tc4_kernel, SMEM_BYTES);
-    int dev = 0, sms = 148;
-    B200PF_CUDA(cudaGetDevice(&dev));
-    B200PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms;
+    if ((rc = multiprocessors(&sms)) != B200PF_OK) return rc;
     const long long items = (long long)((lines + NG - 1) / NG) * 4 * ((n + AQ - 1) / AQ);
     Args a{mask_lines, (__nv_bfloat16*)o, o_line_stride, o_pos_stride, mask_pitch, lines, n};
-    triatt_core_tc4_kernel<<<(unsigned)(items < sms ? items : sms), THREADS, SMEM_BYTES, (cudaStream_t)stream>>>(mq, mk, mvt, mb, a, status);
-    B200PF_LAUNCH_CHECK();
-    return B200PF_OK;
+    return launch_pdl(triatt_core_tc4_kernel, dim3((unsigned)(items < sms ? items : sms)), dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream,
+                      mq, mk, mvt, mb, a, status);
 }
 

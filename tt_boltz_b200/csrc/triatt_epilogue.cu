@@ -3,6 +3,7 @@
 //   producer : z -> LN -> [q | k | g | v] projection (128 -> 512) + 4-head triangle bias; the kernel is
 //              row512_kernel<1> in row512_tc.cu, this file holds its entry point
 //   epilogue : z += (o * g) W_o^T   (mma.sync; the residual is added by red.global.add, so z is not read)
+#include "pdl.cuh"
 #include "row512_tc.h"
 #include "rowtile.cuh"
 
@@ -21,6 +22,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1) triatt_epilogue_kernel(AttEpilo
     __nv_bfloat16* tiles = w_s + 128 * APITCH;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __nv_bfloat16* tile = tiles + warp * (UNIT * APITCH);
+    grid_dependency_wait();
+    grid_launch_dependents();
     load_weights_k128(w_s, p.w_o, 128);
     __syncthreads();
     const uint32_t w_addr = smem_u32(w_s), tile_addr = smem_u32(tile);
@@ -37,7 +40,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) triatt_epilogue_kernel(AttEpilo
             if (f < p.rows_flat) {
                 const uint4* op = reinterpret_cast<const uint4*>(p.o + f * KC) + sub * 2;
                 const uint4* gp = reinterpret_cast<const uint4*>(p.g + f * KC) + sub * 2;
-                ov[0] = __ldg(op); ov[1] = __ldg(op + 1); gv[0] = __ldg(gp); gv[1] = __ldg(gp + 1);
+                ov[0] = op[0]; ov[1] = op[1]; gv[0] = gp[0]; gv[1] = gp[1];
             } else {
                 ov[0] = ov[1] = gv[0] = gv[1] = make_uint4(0, 0, 0, 0);
             }
@@ -84,15 +87,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1) triatt_epilogue_kernel(AttEpilo
 }
 
 constexpr int ATT_EPILOGUE_SMEM = 128 * APITCH * 2 + WARPS * A_TILE_BYTES;             // 104,448
-
-static int grid_for_units(long long units, int ctas_per_sm) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    long long ctas = (units + WARPS - 1) / WARPS;
-    long long cap = (long long)sms * ctas_per_sm;
-    return (int)(ctas < cap ? ctas : cap);
-}
 
 }  // namespace b200pf
 
@@ -148,10 +142,10 @@ static int triatt_epilogue(float* z, b200pf_bf16* upd, const b200pf_bf16* o, con
                    "triatt_epilogue: pointers must be 16-byte aligned");
     AttEpilogueArgs p{z, (__nv_bfloat16*)upd, (const __nv_bfloat16*)o, (const __nv_bfloat16*)g, (const __nv_bfloat16*)w_o, n_rows_flat};
     B200PF_SMEM_ATTR_ONCE(triatt_epilogue_kernel, ATT_EPILOGUE_SMEM);
-    long long units = (n_rows_flat + UNIT - 1) / UNIT;
-    triatt_epilogue_kernel<<<grid_for_units(units, 2), WARPS * 32, ATT_EPILOGUE_SMEM, (cudaStream_t)stream>>>(p);
-    B200PF_LAUNCH_CHECK();
-    return B200PF_OK;
+    int sms, rc;
+    if ((rc = multiprocessors(&sms)) != B200PF_OK) return rc;
+    const long long units = (n_rows_flat + UNIT - 1) / UNIT, ctas = (units + WARPS - 1) / WARPS;
+    return launch_pdl(triatt_epilogue_kernel, dim3((unsigned)(ctas < 2 * sms ? ctas : 2 * sms)), dim3(WARPS * 32), ATT_EPILOGUE_SMEM, (cudaStream_t)stream, p);
 }
 
 extern "C" int b200pf_triatt_epilogue(float* z, const b200pf_bf16* o, const b200pf_bf16* g,

@@ -21,7 +21,7 @@ using namespace rtc;
 
 constexpr int LOAD_WARPS = 4, MMA_WARP = 4, EPI_WARP0 = 5, EPI_WARPS = 8, THREADS = 13 * 32;
 constexpr int W_TILE = 128 * 128 * 2;                    // 32 KB: two k-blocks of [128][128 B]
-constexpr int OFF_WP = 0, OFF_WG = W_TILE;
+constexpr int OFF_WP = 0, OFF_WG = W_TILE;               // 0.5 * W_pout * gamma_out, 0.5 * W_gout
 constexpr int OFF_AZ = 2 * W_TILE;                       // 2 stages
 constexpr int OFF_XT = OFF_AZ + 2 * A_TILE_BYTES;        // 1 stage: 2 boxes of [128 d][64 pos]
 constexpr int XT_BOX = 128 * 128;
@@ -38,15 +38,13 @@ struct Args {
     const float* z;                 // read for LN_in; the residual is added by TMA reduce
     const float* ln_in_gamma;
     const float* ln_in_beta;
-    const __nv_bfloat16* w_pout;    // [128][128] = 0.5 * W_pout * gamma_out
-    const __nv_bfloat16* w_gout;    // [128][128] = 0.5 * W_gout
     const float* wsum;              // [128] row sums of w_pout (as stored in bf16)
     const float* wb;                // [128] 0.5 * W_pout beta_out
     int rows, n;
 };
 
 struct Bars {
-    uint64_t x_full, x_empty, in_full[2], in_empty[2], acc_full[2], acc_empty[2];
+    uint64_t w_full, x_full, x_empty, in_full[2], in_empty[2], acc_full[2], acc_empty[2];
     uint32_t tmem_slot;
     int abort_flag;
 };
@@ -69,11 +67,13 @@ __device__ __forceinline__ float tanh_approx(float x) {
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
-trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_z, Args p,
+trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_z,
+                          const __grid_constant__ CUtensorMap map_wp, const __grid_constant__ CUtensorMap map_wg, Args p,
                           unsigned int* status) {
     using namespace sm100;
     extern __shared__ __align__(1024) uint8_t smem[];
     if ((smem_u32(smem) & 1023u) != 0) {
+        grid_dependency_wait();
         if (threadIdx.x == 0) atomicOr(status, DEV_STATUS_BAD_INDEX);
         return;
     }
@@ -86,6 +86,7 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
     const long long tiles = (long long)p.rows * tpl;
 
     if (tid == 0) {
+        mbar_init(&B->w_full, 1);
         mbar_init(&B->x_full, 1);
         mbar_init(&B->x_empty, 1 + EPI_WARPS);      // the MMAs and the epilogue warps' statistics pass both read the x tile
         for (int i = 0; i < 2; ++i) {
@@ -94,12 +95,17 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
         }
         B->abort_flag = 0;
         fence_barrier_init();
+        fence_proxy_async();
     }
-    load_weights_sw128(smem + OFF_WP, p.w_pout, 128, tid, THREADS);
-    load_weights_sw128(smem + OFF_WG, p.w_gout, 128, tid, THREADS);
-    if (tid < 128) { wsum_s[tid] = p.wsum[tid]; wb_s[tid] = p.wb[tid]; }
-    fence_proxy_async();
     if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (tid == 0) {
+        mbar_arrive_expect_tx(&B->w_full, 2 * W_TILE);
+        load_weights_tma(smem + OFF_WP, &map_wp, 128, &B->w_full);
+        load_weights_tma(smem + OFF_WG, &map_wg, 128, &B->w_full);
+    }
+    if (tid < 128) { wsum_s[tid] = p.wsum[tid]; wb_s[tid] = p.wb[tid]; }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -111,8 +117,8 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
         float4 gam[4], bet[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            gam[j] = __ldg(reinterpret_cast<const float4*>(p.ln_in_gamma) + j * 8 + sub);
-            bet[j] = __ldg(reinterpret_cast<const float4*>(p.ln_in_beta) + j * 8 + sub);
+            gam[j] = reinterpret_cast<const float4*>(p.ln_in_gamma)[j * 8 + sub];
+            bet[j] = reinterpret_cast<const float4*>(p.ln_in_beta)[j * 8 + sub];
         }
         uint32_t it = 0;
         bool ok = true;
@@ -124,9 +130,9 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
             uint8_t* a_tile = smem + OFF_AZ + stage * A_TILE_BYTES;
             {   // ask L2 for this warp's 32 rows of the NEXT tile (one lane per row, four 128-byte lines)
                 const long long tn = t + gridDim.x;
-                const int posn = (int)(tn % tpl) * TM + warp * 32 + lane;
+                const int rn = (int)(tn / tpl), posn = (int)(tn % tpl) * TM + warp * 32 + lane;
                 if (tn < tiles && posn < p.n) {
-                    const char* rowp = reinterpret_cast<const char*>(p.z + ((tn / tpl) * p.n + posn) * KC);
+                    const char* rowp = reinterpret_cast<const char*>(p.z + ((long long)rn * p.n + posn) * KC);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) asm volatile("prefetch.global.L2 [%0];" ::"l"(rowp + j * 128));
                 }
@@ -135,14 +141,14 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
             for (int pass = 0; pass < 2; ++pass) {
                 const int row0 = warp * 32 + pass * 16;
                 float4 v[4][4];
-                bool valid[4];
+                // positions beyond the row's end repeat its first one: the reduce-add clips them (zeroing them cost the
+                // loaders registers: with spills the kernel took 297 us at 1024 tokens, this way 270)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int pos = pos0 + row0 + i * 4 + rq;
-                    valid[i] = pos < p.n;
-                    const float4* src = reinterpret_cast<const float4*>(p.z + ((long long)r * p.n + (valid[i] ? pos : 0)) * KC);
+                    const float4* src = reinterpret_cast<const float4*>(p.z + ((long long)r * p.n + (pos < p.n ? pos : 0)) * KC);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) v[i][j] = valid[i] ? __ldg(src + j * 8 + sub) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int j = 0; j < 4; ++j) v[i][j] = src[j * 8 + sub];
                 }
                 if (pass == 0 && warp == 0 && lane == 0) {
                     // x tile of this tile: the buffer is free once the MMAs of the previous tile are done
@@ -186,12 +192,11 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
                 for (int i = 0; i < 4; ++i) {
                     const int row = row0 + i * 4 + rq;
                     const float rstd = rsqrtf(ss4[i] * (1.f / KC) + LN_EPS);
-                    const float kz = valid[i] ? 1.f : 0.f;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         uint2 o;
-                        o.x = pack_bf16x2(fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x) * kz, fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y) * kz);
-                        o.y = pack_bf16x2(fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z) * kz, fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w) * kz);
+                        o.x = pack_bf16x2(fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x), fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y));
+                        o.y = pack_bf16x2(fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z), fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w));
                         const int chunk = (j & 1) * 4 + (sub >> 1);
                         *reinterpret_cast<uint2*>(a_tile + (j >> 1) * A_KB_BYTES + sw128(row, chunk) + (sub & 1) * 8) = o;
                     }
@@ -211,7 +216,7 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
         constexpr uint32_t idesc_p = make_idesc_bf16(TM, 128) | (1u << 15);      // A operand MN-major
         const uint32_t wp_addr = smem_u32(smem + OFF_WP), wg_addr = smem_u32(smem + OFF_WG), xt_addr = smem_u32(smem + OFF_XT);
         uint32_t it = 0;
-        bool ok = true;
+        bool ok = mbar_wait_warp(&B->w_full, 0, abort_flag);
         for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
             const uint32_t stage = it & 1, ph = (it >> 1) & 1;
             ok = mbar_wait_warp(&B->in_full[stage], ph, abort_flag) && mbar_wait_warp(&B->x_full, it & 1, abort_flag) &&
@@ -328,8 +333,10 @@ extern "C" int b200pf_trimul_epilogue_tc(float* z, const b200pf_bf16* x, long lo
                    x_plane_stride >= (long long)x_pitch * rows, B200PF_ERR_INVALID, "trimul_epilogue_tc: bad sizes");
     B200PF_REQUIRE(aligned16(z) && aligned16(x) && aligned16(w_pout) && aligned16(w_gout) && aligned16(ln_in_gamma) &&
                    aligned16(ln_in_beta), B200PF_ERR_INVALID, "trimul_epilogue_tc: pointers must be 16-byte aligned");
-    CUtensorMap mx, mz;
-    int rc;
+    CUtensorMap mx, mz, mwp, mwg;
+    int sms, rc;
+    if ((rc = multiprocessors(&sms)) != B200PF_OK || (rc = weight_map(&mwp, w_pout, 128, "w_pout")) != B200PF_OK ||
+        (rc = weight_map(&mwg, w_gout, 128, "w_gout")) != B200PF_OK) return rc;
     {
         cuuint64_t dims[4] = {(cuuint64_t)n, (cuuint64_t)rows, 128, 1};
         cuuint64_t str[3] = {(cuuint64_t)x_pitch * 2, (cuuint64_t)x_plane_stride * 2, (cuuint64_t)x_plane_stride * 2 * 128};
@@ -345,12 +352,8 @@ extern "C" int b200pf_trimul_epilogue_tc(float* z, const b200pf_bf16* x, long lo
     unsigned int* status = device_status_word();
     B200PF_REQUIRE(status, B200PF_ERR_CUDA, "trimul_epilogue_tc: no device status word");
     B200PF_SMEM_ATTR_ONCE(trimul_epilogue_tc_kernel, SMEM_BYTES);
-    int dev = 0, sms = 148;
-    B200PF_CUDA(cudaGetDevice(&dev));
-    B200PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     long long tiles = (long long)rows * ((n + TM - 1) / TM);
-    Args a{z, ln_in_gamma, ln_in_beta, (const __nv_bfloat16*)w_pout, (const __nv_bfloat16*)w_gout, wsum, wb, rows, n};
-    trimul_epilogue_tc_kernel<<<(unsigned)(tiles < sms ? tiles : sms), THREADS, SMEM_BYTES, (cudaStream_t)stream>>>(mx, mz, a, status);
-    B200PF_LAUNCH_CHECK();
-    return B200PF_OK;
+    Args a{z, ln_in_gamma, ln_in_beta, wsum, wb, rows, n};
+    return launch_pdl(trimul_epilogue_tc_kernel, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream,
+                      mx, mz, mwp, mwg, a, status);
 }

@@ -8,7 +8,9 @@
 // Ragged sizes need no padding: TMA zero-fills out-of-range rows / columns, stores are guarded.
 #include <cstdlib>
 
+#include "pdl.cuh"
 #include "sm100.cuh"
+#include "tmap.cuh"
 
 namespace b200pf {
 
@@ -67,6 +69,8 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         fence_proxy_async();
     }
     if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+    grid_dependency_wait();
+    grid_launch_dependents();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -224,6 +228,8 @@ trimul_contract_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __g
         fence_proxy_async();
     }
     if (warp == 1) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
+    grid_dependency_wait();
+    grid_launch_dependents();
     tc_fence_before();
     __syncthreads();
     cluster_sync();                                              // the other CTA's barriers and tensor memory are ready
@@ -349,35 +355,12 @@ trimul_contract_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __g
 }
 
 // ---- host: tensor maps -----------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    }
-    return fn;
-}
-
 static int make_plane_map(CUtensorMap* map, const b200pf_planes* p, int channels, const char* what) {
-    EncodeTiledFn fn = encode_fn();
-    B200PF_REQUIRE(fn != nullptr, B200PF_ERR_CUDA, "cuTensorMapEncodeTiled not available from the driver");
     long long seg_stride = p->nseg > 1 ? p->seg_stride : p->plane_stride * channels;
     cuuint64_t dims[4] = {(cuuint64_t)p->cols, (cuuint64_t)p->rows, (cuuint64_t)channels, (cuuint64_t)p->nseg};
     cuuint64_t strides[3] = {(cuuint64_t)p->pitch * 2, (cuuint64_t)p->plane_stride * 2, (cuuint64_t)seg_stride * 2};
     cuuint32_t box[4] = {(cuuint32_t)BK, 128u, 1u, 1u};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(p->ptr), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    B200PF_REQUIRE(r == CUDA_SUCCESS, B200PF_ERR_CUDA, "cuTensorMapEncodeTiled(%s) failed with CUresult %d", what, (int)r);
-    return B200PF_OK;
+    return tmap_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, p->ptr, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, what);
 }
 
 static int check_planes(const b200pf_planes* p, const char* what) {
@@ -455,15 +438,11 @@ static int launch_contract_tc(const b200pf_planes* a, const b200pf_planes* b, b2
         }
         long long pairs = (dev >= 0 && dev < 64) ? resident_pairs[dev] : sms / 2;
         unsigned grid = 2u * (unsigned)(tiles < pairs ? tiles : pairs);
-        trimul_contract_pair_kernel<<<grid, GEMM_THREADS, PAIR_SMEM, st>>>(map_a, map_b, (__nv_bfloat16*)x, s, status);
-        B200PF_LAUNCH_CHECK();
-        return B200PF_OK;
+        return launch_pdl(trimul_contract_pair_kernel, dim3(grid), dim3(GEMM_THREADS), PAIR_SMEM, st, map_a, map_b, (__nv_bfloat16*)x, s, status);
     }
     long long tiles = (long long)s.channels * ((s.m_rows + BM - 1) / BM) * ((s.n_rows + BN - 1) / BN);
     unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
-    trimul_contract_tc_kernel<<<grid, GEMM_THREADS, GEMM_SMEM, st>>>(map_a, map_b, (__nv_bfloat16*)x, s, status);
-    B200PF_LAUNCH_CHECK();
-    return B200PF_OK;
+    return launch_pdl(trimul_contract_tc_kernel, dim3(grid), dim3(GEMM_THREADS), GEMM_SMEM, st, map_a, map_b, (__nv_bfloat16*)x, s, status);
 }
 
 namespace gemm_mx {   // block-scaled fp8 kernel, trimul_gemm_mx.cu

@@ -14,6 +14,7 @@
 //   * the 12 scale columns leave room for only one 256-column accumulator, so the epilogue of a
 //     tile does not overlap the MMAs of the next (TMA still runs ahead through the 4-stage ring).
 #include "mxfp8.cuh"
+#include "pdl.cuh"
 #include "sm100.cuh"
 #include "tmap.cuh"
 
@@ -51,8 +52,7 @@ __device__ __forceinline__ long long sf_block_offset(int d, int k0, int row0, in
 
 __global__ void __launch_bounds__(THREADS, 1)
 trimul_contract_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                          const uint8_t* __restrict__ sfa, const uint8_t* __restrict__ sfb,
-                          __nv_bfloat16* __restrict__ x, Shape s, unsigned int* status) {
+                          const uint8_t* sfa, const uint8_t* sfb, __nv_bfloat16* x, Shape s, unsigned int* status) {
     using namespace sm100;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -78,6 +78,8 @@ trimul_contract_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         fence_proxy_async();
     }
     if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+    grid_dependency_wait();
+    grid_launch_dependents();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -289,14 +291,11 @@ int launch_contract(const b200pf_planes* a, const b200pf_planes* b, const void* 
                               CU_TENSOR_MAP_SWIZZLE_128B, i ? "mx B" : "mx A")) != B200PF_OK) return rc;
     }
     B200PF_SMEM_ATTR_ONCE(trimul_contract_mx_kernel, SMEM);
-    int dev = 0, sms = 148;
-    B200PF_CUDA(cudaGetDevice(&dev));
-    B200PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms, rc_sm;
+    if ((rc_sm = multiprocessors(&sms)) != B200PF_OK) return rc_sm;
     const long long tiles = (long long)channels * ((s.m_rows + BM - 1) / BM) * ((s.n_rows + BN - 1) / BN);
-    trimul_contract_mx_kernel<<<(unsigned)(tiles < sms ? tiles : sms), THREADS, SMEM, st>>>(
-        maps[0], maps[1], static_cast<const uint8_t*>(a_scales), static_cast<const uint8_t*>(b_scales), (__nv_bfloat16*)x, s, status);
-    B200PF_LAUNCH_CHECK();
-    return B200PF_OK;
+    return launch_pdl(trimul_contract_mx_kernel, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(THREADS), SMEM, st, maps[0], maps[1],
+                      static_cast<const uint8_t*>(a_scales), static_cast<const uint8_t*>(b_scales), (__nv_bfloat16*)x, s, status);
 }
 
 }  // namespace gemm_mx
