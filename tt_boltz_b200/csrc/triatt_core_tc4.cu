@@ -12,7 +12,9 @@
 // both, made each group wait for the other to release its columns: 2 % slower.)  The softmax thread reads its row
 // in two halves, applies the key mask and computes p = exp2(s - m) in ONE pass with the reference m of the tiles
 // before (scaling by a stale reference is exact in floating point; a check keeps it far from overflow and hands the
-// rare tile that fails it, like the first tile of a line, to a two-pass path).  p goes back to TENSOR memory as
+// rare tile that fails it to a two-pass path).  A line's first tile takes its reference from its own first 32 keys and the
+// ragged last tile its excluded keys as -inf, so both run in one pass too: 41 -> 37 us at 203 tokens, 168 -> 154 at 400,
+// 402 -> 367 at 600, 1.64 -> 1.56 ms at 1024 with masked keys; without masks and raggedness, at 1024, 1.414 -> 1.427 ms.  p goes back to TENSOR memory as
 // packed bf16, the A operand of O_g += P_g V_g^T.  The running output stays in tensor memory and is rescaled only
 // when a row maximum has grown by more than 2^8; row sums are kept in fp32 registers.
 // TMEM columns: S 4 x 64 | P 4 x 32 | O 4 x 32 = 512.  S and P are single-buffered; S is released as soon as its
@@ -110,12 +112,21 @@ __device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-// Masked keys of a full tile get the score the reference's fp32 sum rounds to.  `even` / `odd` hold one bit per
-// key pair (bit l: key 2l / 2l+1 attends); they are uniform over the warp, so every test is a uniform branch and a
-// tile (or a group of 8 keys) without masked keys costs one compare.
+// Masked keys get the score the reference's fp32 sum rounds to.  `even` / `odd` hold one bit per key pair (bit l: key
+// 2l / 2l+1 attends); they are uniform over the warp, so every test is a uniform branch and a tile (or a group of 8 keys)
+// without masked keys costs one compare.  Keys at or beyond `left`, the number of keys the tile still has, are excluded
+// altogether.
 template <int HF>
-__device__ __forceinline__ void mask_half(uint32_t (&sr)[32], uint32_t even, uint32_t odd) {
+__device__ __forceinline__ void mask_half(uint32_t (&sr)[32], uint32_t even, uint32_t odd, int left) {
     const uint32_t e16 = (even >> (HF * 16)) & 0xffffu, o16 = (odd >> (HF * 16)) & 0xffffu, b16 = e16 & o16;
+    if (left < AK) {                // ragged last tile
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+            const uint32_t bit = (((e & 1) ? o16 : e16) >> (e >> 1)) & 1u;
+            sr[e] = HF * 32 + e >= left ? __float_as_uint(-INFINITY) : (bit ? sr[e] : __float_as_uint(MASKED_SCORE));
+        }
+        return;
+    }
     if (b16 == 0xffffu) return;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -126,16 +137,6 @@ __device__ __forceinline__ void mask_half(uint32_t (&sr)[32], uint32_t even, uin
             if (!((e16 >> pe) & 1u)) sr[2 * pe] = __float_as_uint(MASKED_SCORE);
             if (!((o16 >> pe) & 1u)) sr[2 * pe + 1] = __float_as_uint(MASKED_SCORE);
         }
-    }
-}
-// The same for any tile: keys at or beyond n (tile padding) are excluded altogether.
-__device__ __forceinline__ void mask_half_general(uint32_t (&sr)[32], uint32_t even, uint32_t odd, int hf, int key0, int n) {
-#pragma unroll
-    for (int e = 0; e < 32; ++e) {
-        const int pe = hf * 16 + (e >> 1);
-        const uint32_t bit = (((e & 1) ? odd : even) >> pe) & 1u;
-        const int key = key0 + hf * 32 + e;
-        sr[e] = (key >= n) ? __float_as_uint(-INFINITY) : (bit ? sr[e] : __float_as_uint(MASKED_SCORE));
     }
 }
 __device__ __forceinline__ void max_half(const uint32_t (&sr)[32], float (&m4)[4]) {
@@ -376,25 +377,33 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             for (int j = 0; j < T && ok; ++j, ++G) {
                 const uint32_t even = __ballot_sync(0xffffffffu, (vnext & 0x00ffu) != 0);    // bit l: key 2l attends
                 const uint32_t odd = __ballot_sync(0xffffffffu, (vnext & 0xff00u) != 0);     // bit l: key 2l+1 attends
-                const bool full_tile = (j * AK + AK <= n);
+                const int left = n - j * AK;                 // keys of this tile that exist (at least one)
                 if (j + 1 < T) vnext = mask_fetch(mrow, j + 1);
                 ok = mbar_wait(&B->s_full[g], G & 1, abort_flag);
                 if (!ok) break;
                 tc_fence_after();
                 bool done = false;
-                if (j > 0 && full_tile && !pending) {
-                    // ---- one pass: p = exp2(s - m_used) with the reference of the tiles before, no maximum first.
+                if (!pending) {
+                    // ---- one pass: p = exp2(s - m_used) with the reference of the tiles before (a line's first tile: the
+                    // maximum of its first 32 keys, which always hold key 0), no maximum of the whole tile first.
                     // Scaling by a stale reference is exact in floating point; it only has to stay far from
                     // overflow, which the check before the scores are released guarantees (otherwise the tile is
                     // redone by the two-pass path below, the scores being still in tensor memory).
-                    const uint64_t negm2 = f2_pack(-m_used, -m_used);
-                    uint64_t l2a = f2_pack(0.f, 0.f), l2b = l2a;
                     float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
                     uint32_t sr[32], pw[16];
                     tmem_ld_32x32(s_addr, sr);
                     tmem_ld_wait();
-                    mask_half<0>(sr, even, odd);
+                    mask_half<0>(sr, even, odd, left);
+                    if (j == 0) {       // a branch, not a select: every other tile's exponentials must not wait for a maximum
+                        float first = __uint_as_float(sr[0]);
+#pragma unroll
+                        for (int e = 1; e < 32; ++e) first = fmaxf(first, __uint_as_float(sr[e]));
+                        m_used = m_seen = first;
+                        __syncwarp();
+                    }
                     max_half(sr, m4);
+                    const uint64_t negm2 = f2_pack(-m_used, -m_used);
+                    uint64_t l2a = f2_pack(0.f, 0.f), l2b = l2a;
                     exp_half(sr, pw, negm2, l2a, l2b);
                     // the previous P V product of this group must have read its P operand before it is overwritten
                     ok = mbar_wait(&B->pv_done[g], (G & 1) ^ 1, abort_flag);
@@ -403,7 +412,7 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     tmem_st_32x16(p_addr, pw);
                     tmem_ld_32x32(s_addr + 32, sr);
                     tmem_ld_wait();
-                    mask_half<1>(sr, even, odd);
+                    mask_half<1>(sr, even, odd, left);
                     max_half(sr, m4);
                     const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
                     if (!__any_sync(0xffffffffu, mx > m_used + ONE_PASS_HEADROOM)) {
@@ -422,20 +431,20 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     }
                 }
                 if (!done) {
-                    // ---- two passes (first tile of a line, ragged last tile, a rescale that is due, or a tile the
-                    // one-pass path gave back): row maximum first, then the exponentials
-                    const bool plain = full_tile && (even & odd) == 0xffffffffu;
+                    // ---- two passes (a rescale that is due, or a tile the one-pass path gave back): row maximum first,
+                    // then the exponentials
                     float mx;
                     {
                         float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                        for (int hf = 0; hf < 2; ++hf) {
-                            uint32_t sr[32];
-                            tmem_ld_32x32(s_addr + hf * 32, sr);
-                            tmem_ld_wait();
-                            if (!plain) mask_half_general(sr, even, odd, hf, j * AK, n);
-                            max_half(sr, m4);
-                        }
+                        uint32_t sr[32];
+                        tmem_ld_32x32(s_addr, sr);
+                        tmem_ld_wait();
+                        mask_half<0>(sr, even, odd, left);
+                        max_half(sr, m4);
+                        tmem_ld_32x32(s_addr + 32, sr);
+                        tmem_ld_wait();
+                        mask_half<1>(sr, even, odd, left);
+                        max_half(sr, m4);
                         mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
                     }
                     // The previous P V product of this group has to be complete before its P operand is overwritten
@@ -473,7 +482,8 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                             __syncwarp();
                             if (lane == 0) mbar_arrive(&B->s_empty[g]);
                         }
-                        if (!plain) mask_half_general(sr, even, odd, hf, j * AK, n);
+                        if (hf == 0) mask_half<0>(sr, even, odd, left);
+                        else mask_half<1>(sr, even, odd, left);
                         exp_half(sr, pw, negm2, l2a, l2b);
                         tmem_st_32x16(p_addr + hf * 16, pw);
                     }
