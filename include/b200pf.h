@@ -368,6 +368,18 @@ int b200pf_pwa_gate_transpose(const b200pf_bf16* o, const b200pf_bf16* g, b200pf
 int b200pf_msa_swiglu(const b200pf_bf16* h, b200pf_bf16* out, long long rows, void* stream);
 /* m[s][i][:] += t[s*np + i][:]  (t bf16 rows of 64). */
 int b200pf_msa_add_rows(float* m, const b200pf_bf16* t, int s_len, int n, int np, void* stream);
+/* The same work with one kernel per stage, nothing but v and o in memory between them (weights bf16, accumulation and
+ * residual fp32).  np: tokens padded to a multiple of 8; elements of v at tokens >= n are zeros or left alone, those of o
+ * have no say.
+ * m[rows] += fc3 (silu(fc1 LN m) * fc2 LN m); w12 [4][64 rows of fc1, 64 rows of fc2][64], w3 = fc3 [64][256]. */
+int b200pf_msa_transition(float* m, const float* ln_gamma, const float* ln_beta, const b200pf_bf16* w12, const b200pf_bf16* w3,
+                          long long rows, void* stream);
+/* v[head][s][d][tok] = (proj_m LN m[s][tok])[32 head + d]: bf16 [8][S][32][np]; w_m = proj_m [256][64]. */
+int b200pf_pwa_value(const float* m, const float* ln_gamma, const float* ln_beta, const b200pf_bf16* w_m, b200pf_bf16* v, int s_len,
+                     int n, int np, void* stream);
+/* m[s][tok] += proj_o (sigmoid(proj_g LN m[s][tok]) * o[:][s][:][tok]); w_g = proj_g [256][64], w_o = proj_o [64][256]. */
+int b200pf_pwa_output(float* m, const float* ln_gamma, const float* ln_beta, const b200pf_bf16* w_g, const b200pf_bf16* w_o,
+                      const b200pf_bf16* o, int s_len, int n, int np, void* stream);
 /* m[s][i][:] += e[i][:] (fp32 rows of 64): the projected single representation added to every sequence's embedding
  * (MSAModule.forward, tt_bio/reference.py:1275-1276). */
 int b200pf_msa_add_token_rows(float* m, const float* e, int s_len, int n, void* stream);

@@ -90,6 +90,9 @@ SIGNATURES = {
     "b200pf_msa_swiglu": [_vp, _vp, _ll, _vp],
     "b200pf_msa_add_rows": [_vp, _vp, _i, _i, _i, _vp],
     "b200pf_msa_add_token_rows": [_vp, _vp, _i, _i, _vp],
+    "b200pf_msa_transition": [_vp, _vp, _vp, _vp, _vp, _ll, _vp],
+    "b200pf_pwa_value": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp],
+    "b200pf_pwa_output": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp],
     "b200pf_opm_producer": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp],
     "b200pf_opm_outer": [_vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "b200pf_opm_mask_bits": [_vp, _vp, _i, _i, _vp],

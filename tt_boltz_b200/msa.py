@@ -127,7 +127,7 @@ class B200OuterProductMean(nn.Module):
 # ------------------------------------------------------------------------------------------------
 # The MSA layer: pair-weighted averaging and transition on m, outer-product mean and a pair block on z
 # ------------------------------------------------------------------------------------------------
-ROWS_PER_CHUNK = 1 << 20           # (sequence, token) rows whose bf16 intermediates are held at a time
+ROWS_PER_CHUNK = 1 << 20           # (sequence, token) rows whose averaging operands are held at a time
 
 
 def _gemm(a, a_rows, k, b, b_rows, x, channels=1, a_plane=None, b_plane=None, a_pitch=None, b_pitch=None,
@@ -175,13 +175,14 @@ class B200PairWeightedAveraging(nn.Module):
         return super()._apply(fn, *args, **kwargs)
 
     def _pack(self, device):
-        if self._packed is None or self._packed["w_mg"].device != device:
+        if self._packed is None or self._packed["w_m"].device != device:
             with torch.no_grad():
                 f32 = dict(device=device, dtype=torch.float32)
                 self._packed = {
                     "gm": self.norm_m.weight.detach().to(**f32).contiguous(), "bm": self.norm_m.bias.detach().to(**f32).contiguous(),
                     "gz": self.norm_z.weight.detach().to(**f32).contiguous(), "bz": self.norm_z.bias.detach().to(**f32).contiguous(),
-                    "w_mg": torch.cat([self.proj_m.weight, self.proj_g.weight], 0).detach().to(device=device, dtype=torch.bfloat16).contiguous(),
+                    "w_m": self.proj_m.weight.detach().to(device=device, dtype=torch.bfloat16).contiguous(),
+                    "w_g": self.proj_g.weight.detach().to(device=device, dtype=torch.bfloat16).contiguous(),
                     # the LayerNorm + head projection kernel is built for 16 heads: 8 real rows, 8 zero rows
                     "w_z": torch.cat([self.proj_z.weight.detach().to(**f32), torch.zeros(8, self.c_z, **f32)], 0).contiguous(),
                     "w_o": self.proj_o.weight.detach().to(device=device, dtype=torch.bfloat16).contiguous(),
@@ -196,30 +197,21 @@ class B200PairWeightedAveraging(nn.Module):
             raise ValueError("z must be a contiguous fp32 tensor [N, N, 128]")
         w = self._pack(m.device)
         dev, st, heads = m.device, stream(), self.num_heads
-        np_, pw = _round_up(n, 32), _round_up(n, 8)          # the projected rows are written in column groups of np
+        np_ = pw = _round_up(n, 8)
         logits = torch.empty(16 * n * n, dtype=torch.float32, device=dev)
         call("b200pf_ln_proj_heads", ptr(z), ptr(w["gz"]), ptr(w["bz"]), ptr(w["w_z"]), ptr(logits), n * n, n * n, 128, 16, st)
         wt = torch.empty(heads * n * pw, dtype=torch.bfloat16, device=dev)
         call("b200pf_pwa_softmax", ptr(logits), ptr(mask_u8), ptr(wt), n, pw, heads, float(self.inf), st)
         sc = max(1, min(s_len, ROWS_PER_CHUNK // np_))
-        ln = torch.empty(sc * np_ * C_M, dtype=torch.bfloat16, device=dev)
-        vg = torch.empty(512 * sc * np_, dtype=torch.bfloat16, device=dev)
+        v = torch.empty(256 * sc * np_, dtype=torch.bfloat16, device=dev)         # [head][s][d][token]
         o = torch.empty(256 * sc * np_, dtype=torch.bfloat16, device=dev)
-        val = torch.empty(sc * np_ * 256, dtype=torch.bfloat16, device=dev)
-        t = torch.empty(sc * np_ * C_M, dtype=torch.bfloat16, device=dev)
         for s0 in range(0, s_len, sc):
             ns = min(sc, s_len - s0)
             p = ns * np_
-            call("b200pf_msa_ln_bf16", ptr(m[s0:]), ptr(w["gm"]), ptr(w["bm"]), ptr(ln), ns, n, np_, st)
-            # [v heads 0-7 ; g heads 0-7][s][d][token]: rows (head, d) in groups of 32, columns (s, token) in groups of np
-            pa = Planes(ptr(w["w_mg"]), 512 * C_M, 0, C_M, 512, C_M, 1, 0)
-            pb = Planes(ptr(ln), p * C_M, 0, C_M, p, C_M, 1, 0)
-            call("b200pf_gemm_grouped", C.byref(pa), C.byref(pb), ptr(vg), 0, np_, 32, ns * 32 * np_, np_, 32 * np_, 1, st)
-            _gemm(vg, self.c_h * ns, n, wt, n, o, channels=heads, a_plane=self.c_h * p, a_pitch=np_,
+            call("b200pf_pwa_value", ptr(m[s0:]), ptr(w["gm"]), ptr(w["bm"]), ptr(w["w_m"]), ptr(v), ns, n, np_, st)
+            _gemm(v, self.c_h * ns, n, wt, n, o, channels=heads, a_plane=self.c_h * p, a_pitch=np_,
                   b_plane=n * pw, b_pitch=pw, x_plane=self.c_h * p, x_pitch=np_, cols=n)
-            call("b200pf_pwa_gate_transpose", ptr(o), ptr(vg[256 * p:]), ptr(val), ns, np_, st)        # sigmoid(g) * o, K-major
-            _gemm(val, p, 256, w["w_o"], C_M, t)
-            call("b200pf_msa_add_rows", ptr(m[s0:]), ptr(t), ns, n, np_, st)
+            call("b200pf_pwa_output", ptr(m[s0:]), ptr(w["gm"]), ptr(w["bm"]), ptr(w["w_g"]), ptr(w["w_o"]), ptr(o), ns, n, np_, st)
 
     def add_into(self, m: torch.Tensor, z: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
         """m += pair_weighted_averaging(m, z, mask) in place; m [S, N, 64] fp32, z [N, N, 128] fp32, mask [N, N]."""
@@ -270,30 +262,16 @@ class B200MSATransition(nn.Module):
                 self._packed = {
                     "g": self.norm.weight.detach().to(device=device, dtype=torch.float32).contiguous(),
                     "b": self.norm.bias.detach().to(device=device, dtype=torch.float32).contiguous(),
-                    "w12": torch.cat([self.fc1.weight, self.fc2.weight], 0).detach().to(**bf).contiguous(),
+                    # 64 rows of fc1, the 64 of fc2 they are multiplied with, in turn
+                    "w12": torch.stack([self.fc1.weight.view(4, 64, C_M), self.fc2.weight.view(4, 64, C_M)], 1).detach().to(**bf).contiguous(),
                     "w3": self.fc3.weight.detach().to(**bf).contiguous(),
                 }
         return self._packed
 
     def _run(self, m: torch.Tensor) -> None:
         _check_m(m)
-        s_len, n = m.shape[0], m.shape[1]
         w = self._pack(m.device)
-        dev, st = m.device, stream()
-        np_ = _round_up(n, 8)
-        sc = max(1, min(s_len, ROWS_PER_CHUNK // np_))
-        ln = torch.empty(sc * np_ * C_M, dtype=torch.bfloat16, device=dev)
-        h12 = torch.empty(sc * np_ * 512, dtype=torch.bfloat16, device=dev)
-        hsw = torch.empty(sc * np_ * 256, dtype=torch.bfloat16, device=dev)
-        t = torch.empty(sc * np_ * C_M, dtype=torch.bfloat16, device=dev)
-        for s0 in range(0, s_len, sc):
-            ns = min(sc, s_len - s0)
-            p = ns * np_
-            call("b200pf_msa_ln_bf16", ptr(m[s0:]), ptr(w["g"]), ptr(w["b"]), ptr(ln), ns, n, np_, st)
-            _gemm(ln, p, C_M, w["w12"], 512, h12)
-            call("b200pf_msa_swiglu", ptr(h12), ptr(hsw), p, st)
-            _gemm(hsw, p, 256, w["w3"], C_M, t)
-            call("b200pf_msa_add_rows", ptr(m[s0:]), ptr(t), ns, n, np_, st)
+        call("b200pf_msa_transition", ptr(m), ptr(w["g"]), ptr(w["b"]), ptr(w["w12"]), ptr(w["w3"]), m.shape[0] * m.shape[1], stream())
 
     def add_into(self, m: torch.Tensor) -> torch.Tensor:
         with torch.no_grad():
