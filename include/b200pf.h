@@ -480,6 +480,41 @@ int b200pf_single_track_attention(const float* s, const b200pf_single_track_weig
 /* s[rows] += og W_o^T; s += Transition(s)  (tt_bio/reference.py:906-912). */
 int b200pf_single_track_finish(float* s, const b200pf_single_track_weights* w, const void* og, int rows, void* workspace, void* stream);
 
+/* The two calls above for all n query rows; the workspace also holds what passes between them. */
+long long b200pf_single_track_rows_workspace(int n, int cs, int hidden);
+int b200pf_single_track_rows(float* s, const b200pf_single_track_weights* w, const float* bias, const uint8_t* mask, int n, void* workspace, void* stream);
+
+/* ----------------------------------------------------------------------------------------
+ * The pair track of one block (tt_bio/reference.py:865-905) in the bf16 tier, enqueued by one call: both triangle
+ * multiplications, both triangle attentions and the transition, on z [n][n][128].
+ * ---------------------------------------------------------------------------------------- */
+typedef struct b200pf_trimul_weights {          /* as for b200pf_trimul_producer / b200pf_trimul_epilogue_tc */
+    const float *ln_in_gamma, *ln_in_beta;
+    const b200pf_bf16 *w_pg, *w_pout, *w_gout;
+    const float *wsum, *wb;
+} b200pf_trimul_weights;
+typedef struct b200pf_triatt_weights {          /* as for b200pf_triatt_producer / b200pf_triatt_epilogue */
+    const float *ln_gamma, *ln_beta, *w_bias;
+    const b200pf_bf16 *w_qkgv, *w_o;
+} b200pf_triatt_weights;
+typedef struct b200pf_transition_weights {      /* as for b200pf_transition_z_tc */
+    const float *ln_gamma, *ln_beta;
+    const b200pf_bf16 *w12, *w3;
+} b200pf_transition_weights;
+typedef struct b200pf_pair_weights {
+    b200pf_trimul_weights tri_mul_out, tri_mul_in;
+    b200pf_triatt_weights tri_att_start, tri_att_end;
+    b200pf_transition_weights transition;
+} b200pf_pair_weights;
+typedef struct b200pf_pair_scratch {
+    b200pf_bf16* buf[5];            /* n * pitch * 128 elements each */
+    b200pf_bf16* tri_bias;          /* 4 * n * pitch */
+    const uint8_t *mask;            /* [n][n] */
+    const uint8_t *mask_rows, *mask_cols;       /* the mask and its transpose, rows of mask_pitch (a multiple of 64) */
+    int n, pitch, mask_pitch;       /* pitch: n rounded up to a multiple of 8 */
+} b200pf_pair_scratch;
+int b200pf_pair_block(float* z, const b200pf_pair_weights* w, const b200pf_pair_scratch* scratch, void* stream);
+
 typedef struct b200pf_split_trimul_weights {
     const float *ln_in_gamma, *ln_in_beta;
     b200pf_split_weight in;         /* p_in rows, then g_in rows: [4 c][c] */

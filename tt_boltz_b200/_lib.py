@@ -63,6 +63,32 @@ class SplitTransitionWeights(C.Structure):
     _fields_ = [("ln_gamma", _vp), ("ln_beta", _vp), ("fc12", SplitWeight), ("fc3", SplitWeight), ("hidden_scale", _f), ("c", _i), ("hidden", _i)]
 
 
+class TriMulWeights(C.Structure):
+    """Mirror of ``b200pf_trimul_weights``."""
+    _fields_ = [(k, _vp) for k in ("ln_in_gamma", "ln_in_beta", "w_pg", "w_pout", "w_gout", "wsum", "wb")]
+
+
+class TriAttWeights(C.Structure):
+    """Mirror of ``b200pf_triatt_weights``."""
+    _fields_ = [(k, _vp) for k in ("ln_gamma", "ln_beta", "w_bias", "w_qkgv", "w_o")]
+
+
+class TransitionWeights(C.Structure):
+    """Mirror of ``b200pf_transition_weights``."""
+    _fields_ = [(k, _vp) for k in ("ln_gamma", "ln_beta", "w12", "w3")]
+
+
+class PairWeights(C.Structure):
+    """Mirror of ``b200pf_pair_weights``."""
+    _fields_ = [("tri_mul_out", TriMulWeights), ("tri_mul_in", TriMulWeights), ("tri_att_start", TriAttWeights), ("tri_att_end", TriAttWeights),
+                ("transition", TransitionWeights)]
+
+
+class PairScratch(C.Structure):
+    """Mirror of ``b200pf_pair_scratch``."""
+    _fields_ = [("buf", _vp * 5), ("tri_bias", _vp), ("mask", _vp), ("mask_rows", _vp), ("mask_cols", _vp), ("n", _i), ("pitch", _i), ("mask_pitch", _i)]
+
+
 # name -> argtypes (all return int unless listed in _RESTYPES)
 SIGNATURES = {
     "b200pf_version": [],
@@ -119,6 +145,9 @@ SIGNATURES = {
     "b200pf_single_track_workspace": [_i, _i, _i],
     "b200pf_single_track_attention": [_vp, C.POINTER(SingleTrackWeights), _vp, _vp, _vp, _i, _i, _i, _vp, _vp],
     "b200pf_single_track_finish": [_vp, C.POINTER(SingleTrackWeights), _vp, _i, _vp, _vp],
+    "b200pf_single_track_rows_workspace": [_i, _i, _i],
+    "b200pf_single_track_rows": [_vp, C.POINTER(SingleTrackWeights), _vp, _vp, _i, _vp, _vp],
+    "b200pf_pair_block": [_vp, C.POINTER(PairWeights), C.POINTER(PairScratch), _vp],
     "b200pf_split_pair_workspace": [_i, _i, _i, _i, _i],
     "b200pf_split_tri_mul": [_vp, _vp, C.POINTER(SplitTriMulWeights), _i, _i, _vp, _vp],
     "b200pf_split_tri_att": [_vp, _vp, C.POINTER(SplitTriAttWeights), _i, _i, _vp, _vp],
@@ -129,7 +158,7 @@ SIGNATURES = {
     "b200pf_split_ln_linear_workspace": [_ll, _i],
     "b200pf_split_ln_linear_add": [_vp, _vp, _vp, C.POINTER(SplitWeight), _vp, _ll, _i, _i, _vp, _vp],
 }
-_RESTYPES = {"b200pf_single_track_workspace": _ll, "b200pf_split_pair_workspace": _ll, "b200pf_split_linear_workspace": _ll,
+_RESTYPES = {"b200pf_single_track_workspace": _ll, "b200pf_single_track_rows_workspace": _ll, "b200pf_split_pair_workspace": _ll, "b200pf_split_linear_workspace": _ll,
              "b200pf_split_ln_linear_workspace": _ll,
              "b200pf_last_error": C.c_char_p, "b200pf_launch_count": _ll, "b200pf_mx_scale_bytes": _ll}
 

@@ -31,6 +31,11 @@ def _round_up(x: int, m: int) -> int:
     return (x + m - 1) // m * m
 
 
+def _u8(mask: torch.Tensor) -> torch.Tensor:
+    """A mask as uint8 (as it is when it is uint8 already)."""
+    return (mask if mask.dtype == torch.uint8 else (mask != 0).to(torch.uint8)).contiguous()
+
+
 class B200OuterProductMean(nn.Module):
     """Drop-in for ``OuterProductMean(c_in=64, c_hidden=32, c_out=128)``; other widths are refused."""
 
@@ -80,7 +85,7 @@ class B200OuterProductMean(nn.Module):
             raise ValueError("z must be contiguous fp32")
         w = self._pack(m.device)
         m = m.to(torch.float32).contiguous()
-        mask_u8 = (mask != 0).to(torch.uint8).contiguous()
+        mask_u8 = _u8(mask)
         dev, st = m.device, stream()
         pitch = _round_up(s_len, 8)
         a_t = torch.empty(n * C_HID * pitch, dtype=torch.bfloat16, device=dev)
@@ -216,7 +221,7 @@ class B200PairWeightedAveraging(nn.Module):
     def add_into(self, m: torch.Tensor, z: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
         """m += pair_weighted_averaging(m, z, mask) in place; m [S, N, 64] fp32, z [N, N, 128] fp32, mask [N, N]."""
         with torch.no_grad():
-            self._run(m, z, (mask != 0).to(torch.uint8).contiguous())
+            self._run(m, z, _u8(mask))
         return m
 
     def forward(self, m: torch.Tensor, z: torch.Tensor, mask: torch.Tensor, chunk_heads: bool = False) -> torch.Tensor:
@@ -228,7 +233,7 @@ class B200PairWeightedAveraging(nn.Module):
         with torch.no_grad():
             m0 = m[0].to(torch.float32).contiguous()
             work = m0.clone()
-            self._run(work, z[0].to(torch.float32).contiguous(), (mask[0] != 0).to(torch.uint8).contiguous())
+            self._run(work, z[0].to(torch.float32).contiguous(), _u8(mask[0]))
             return (work - m0)[None]
 
 
@@ -308,13 +313,15 @@ class B200MSALayer(nn.Module):
                                                          precision=precision)
         self.outer_product_mean = B200OuterProductMean(c_in=msa_s, c_hidden=32, c_out=token_z)
 
-    def forward_inplace(self, z: torch.Tensor, m: torch.Tensor, token_mask: torch.Tensor, msa_mask: torch.Tensor) -> None:
-        """z [N, N, 128] and m [S, N, 64], contiguous fp32, updated where they are; token_mask [N, N], msa_mask [S, N]."""
+    def forward_inplace(self, z: torch.Tensor, m: torch.Tensor, token_mask: torch.Tensor, msa_mask: torch.Tensor,
+                        ws_cache: Optional[dict] = None) -> None:
+        """z [N, N, 128] and m [S, N, 64], contiguous fp32, updated where they are; token_mask [N, N], msa_mask [S, N].
+        ``ws_cache``: a dict that the blocks of one call share, for the pair block's workspace."""
         from .pairformer import _run_layers
         self.pair_weighted_averaging.add_into(m, z, token_mask)
         self.msa_transition.add_into(m)
         self.outer_product_mean.add_into(z, m, msa_mask)
-        _run_layers([self.pairformer_layer], None, z, None, token_mask[None], inplace=True)
+        _run_layers([self.pairformer_layer], None, z, None, token_mask[None], ws_cache, inplace=True)
 
     def forward(self, z: torch.Tensor, m: torch.Tensor, token_mask: torch.Tensor, msa_mask: torch.Tensor,
                 chunk_heads_pwa: bool = False, chunk_size_transition_z: Optional[int] = None,
@@ -331,6 +338,14 @@ class B200MSALayer(nn.Module):
         return zw[None], mw[None]
 
 
+def _run_blocks(layers, z: torch.Tensor, m: torch.Tensor, token_mask: torch.Tensor, msa_mask: torch.Tensor) -> None:
+    """Every block on the resident z and m; what all blocks share (masks as uint8, the pair block's workspace) made once."""
+    with torch.no_grad():
+        pair_u8, msa_u8, ws_cache = _u8(token_mask), _u8(msa_mask), {}
+        for layer in layers:
+            layer.forward_inplace(z, m, pair_u8, msa_u8, ws_cache)
+
+
 class B200MSAStack(nn.Module):
     """The ``layers`` of the reference's MSA module (tt_bio/reference.py:1187-1201, loop at :1279-1307) on resident
     tensors: ``forward(z, m, token_mask, msa_mask) -> z`` runs every block on copies, ``run_inplace`` on the caller's
@@ -345,8 +360,7 @@ class B200MSAStack(nn.Module):
                                                  pairwise_num_heads, precision) for _ in range(msa_blocks))
 
     def run_inplace(self, z: torch.Tensor, m: torch.Tensor, token_mask: torch.Tensor, msa_mask: torch.Tensor) -> None:
-        for layer in self.layers:
-            layer.forward_inplace(z, m, token_mask, msa_mask)
+        _run_blocks(self.layers, z, m, token_mask, msa_mask)
 
     def forward(self, z: torch.Tensor, m: torch.Tensor, token_mask: torch.Tensor, msa_mask: torch.Tensor) -> torch.Tensor:
         """z [1, N, N, 128], m [1, S, N, 64], token_mask [1, N, N], msa_mask [1, S, N] -> z (what MSAModule.forward returns)."""
@@ -417,6 +431,5 @@ class B200MSAModule(nn.Module):
             token_mask = tok[:, None] * tok[None, :]
             m = self.embed(emb, feats)
             zw = z[0].to(torch.float32).clone(memory_format=torch.contiguous_format)
-            for layer in self.layers:
-                layer.forward_inplace(zw, m, token_mask, msa_mask)
+            _run_blocks(self.layers, zw, m, token_mask, msa_mask)
         return zw[None]

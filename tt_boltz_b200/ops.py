@@ -78,8 +78,7 @@ def trimul_epilogue(z, x, plane_stride, pitch, w, rows, n) -> None:
 
 
 def tri_mul_bf16(z: torch.Tensor, mask_u8: torch.Tensor, w: Dict[str, torch.Tensor], ws: Workspace,
-                 incoming: bool, before_z_write=None) -> None:
-    """``before_z_write`` is called (if given) right before the first kernel that writes z, the epilogue."""
+                 incoming: bool) -> None:
     n = z.shape[0]
     a, b, x = ws.buf[0], ws.buf[1], ws.buf[2]
     st = stream()
@@ -91,13 +90,11 @@ def tri_mul_bf16(z: torch.Tensor, mask_u8: torch.Tensor, w: Dict[str, torch.Tens
     pb = Planes(ptr(b), ws.plane_stride, 0, ws.pitch, n, n, 1, 0)
     call("b200pf_trimul_contract", C.byref(pa), C.byref(pb), None, None, ptr(x), ws.plane_stride, ws.pitch,
          0, 0, C_Z, 0, st)
-    if before_z_write is not None:
-        before_z_write()
     trimul_epilogue(z, x, ws.plane_stride, ws.pitch, w, n, n)
 
 
 def tri_mul_mxfp8(z: torch.Tensor, mask_u8: torch.Tensor, w: Dict[str, torch.Tensor], ws: Workspace,
-                  incoming: bool, contract_variant: int = 2, before_z_write=None) -> None:
+                  incoming: bool, contract_variant: int = 2) -> None:
     """Triangle multiplication with MXFP8 operands (e4m3 values, e8m0 scale per 32 along k).
 
     contract_variant 2 = block-scaled tcgen05 contraction; 0 = expand the operands to bf16
@@ -124,8 +121,6 @@ def tri_mul_mxfp8(z: torch.Tensor, mask_u8: torch.Tensor, w: Dict[str, torch.Ten
         pb = Planes(ptr(b), ws.plane_stride, 0, ws.pitch, n, n, 1, 0)
         call("b200pf_trimul_contract", C.byref(pa), C.byref(pb), None, None, ptr(x), ws.plane_stride, ws.pitch,
              0, 0, C_Z, 0, st)
-    if before_z_write is not None:
-        before_z_write()
     trimul_epilogue(z, x, ws.plane_stride, ws.pitch, w, n, n)
 
 
@@ -149,6 +144,23 @@ def tri_att_bf16(z: torch.Tensor, masks: PairMasks, w: Dict[str, torch.Tensor], 
 def transition_z_bf16(z: torch.Tensor, w: Dict[str, torch.Tensor]) -> None:
     rows = z.shape[0] * z.shape[1]
     call("b200pf_transition_z_tc", ptr(z), ptr(w["ln_gamma"]), ptr(w["ln_beta"]), ptr(w["w12_tc"]), ptr(w["w3"]), rows, stream())
+
+
+class PairBlock:
+    """The pair track of one block as a single call: the packed weights of the five sub-operations as the C structure."""
+
+    def __init__(self, pk) -> None:
+        mul = lambda w: _lib.TriMulWeights(ptr(w["ln_in_gamma"]), ptr(w["ln_in_beta"]), ptr(w["w_pg_tc"]), ptr(w["w_pout_tc"]), ptr(w["w_gout_tc"]),
+                                           ptr(w["wsum_tc"]), ptr(w["wb_tc"]))
+        att = lambda w: _lib.TriAttWeights(ptr(w["ln_gamma"]), ptr(w["ln_beta"]), ptr(w["w_bias_f32"]), ptr(w["w_qkgv_tc"]), ptr(w["w_o"]))
+        t = pk["transition_z"]
+        self.struct = _lib.PairWeights(mul(pk["tri_mul_out"]), mul(pk["tri_mul_in"]), att(pk["tri_att_start"]), att(pk["tri_att_end"]),
+                                       _lib.TransitionWeights(ptr(t["ln_gamma"]), ptr(t["ln_beta"]), ptr(t["w12_tc"]), ptr(t["w3"])))
+
+    def run(self, z: torch.Tensor, masks: PairMasks, ws: Workspace) -> None:
+        k = _lib.PairScratch((C.c_void_p * 5)(*[ptr(b) for b in ws.buf]), ptr(ws.tri_bias), ptr(masks.pm), ptr(masks.rows), ptr(masks.cols), ws.n, ws.pitch,
+                             masks.pitch)
+        call("b200pf_pair_block", ptr(z), C.byref(self.struct), C.byref(k), stream())
 
 
 # ------------------------------------------------------------------------------------------------
@@ -298,12 +310,13 @@ class SingleTrack:
         self.pack = weights.pack_single_track(sd, pre, num_heads, device)
         self.z_bias = weights.pack_pair_bias(sd, pre + "attention.", device)
 
-    def bias(self, z_rows: torch.Tensor) -> torch.Tensor:
+    def bias(self, z_rows: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """bias[h][i_local * N + j], times log2(e): one fp32 pass over the (local rows of) z [nr, N, c_z]."""
         rows, c = z_rows.shape[0] * z_rows.shape[1], z_rows.shape[-1]
         w = self.z_bias
         heads = w["w"].shape[0]
-        out = torch.empty(heads, rows, dtype=torch.float32, device=z_rows.device)
+        if out is None:
+            out = torch.empty(heads, rows, dtype=torch.float32, device=z_rows.device)
         name = "b200pf_ln_proj_heads" if c == C_Z and heads in (4, 16) else "b200pf_ln_heads"
         call(name, ptr(z_rows), ptr(w["gamma"]), ptr(w["beta"]), ptr(w["w"]), ptr(out), rows, rows, c, heads, stream())
         return out
@@ -314,6 +327,12 @@ class SingleTrack:
         ws = scratch.get(_nbytes("b200pf_single_track_workspace", s.shape[0], w.cs, w.hidden))
         call("b200pf_single_track_attention", ptr(s), C.byref(w), ptr(bias), ptr(tok_mask_u8), ptr(og), s.shape[0], r0, nq, ws, stream())
         return og
+
+    def rows(self, s: torch.Tensor, bias: torch.Tensor, tok_mask_u8: Optional[torch.Tensor], scratch: Scratch) -> None:
+        """``attention`` and ``finish`` for every row."""
+        w, n = self.pack.struct, s.shape[0]
+        ws = scratch.get(_nbytes("b200pf_single_track_rows_workspace", n, w.cs, w.hidden))
+        call("b200pf_single_track_rows", ptr(s), C.byref(w), ptr(bias), ptr(tok_mask_u8), n, ws, stream())
 
     def finish(self, s_rows: torch.Tensor, og: torch.Tensor, scratch: Scratch) -> None:
         w = self.pack.struct
@@ -335,12 +354,13 @@ class SingleTrackF32:
         self.w_kv = torch.cat([w_att["proj_k.weight"], w_att["proj_v.weight"]], 0).contiguous()
         self.w_12 = torch.cat([w_trans["fc1.weight"], w_trans["fc2.weight"]], 0).contiguous()
 
-    def bias(self, z_rows: torch.Tensor) -> torch.Tensor:
+    def bias(self, z_rows: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """bias[h][i_local * N + j]: one fp32 pass over the (local rows of) z [nr, N, c_z]."""
         w = self.w_att
         rows, c = z_rows.shape[0] * z_rows.shape[1], z_rows.shape[-1]
         heads = w["proj_z.1.weight"].shape[0]
-        out = torch.empty(heads, rows, dtype=torch.float32, device=z_rows.device)
+        if out is None:
+            out = torch.empty(heads, rows, dtype=torch.float32, device=z_rows.device)
         if c == C_Z and heads in (4, 16):
             call("b200pf_ln_proj_heads", ptr(z_rows), ptr(w["proj_z.0.weight"]), ptr(w["proj_z.0.bias"]),
                  ptr(w["proj_z.1.weight"]), ptr(out), rows, rows, c, heads, stream())
@@ -361,6 +381,9 @@ class SingleTrackF32:
         call("b200pf_f32_sattention", ptr(qg), 2 * cs, qg.data_ptr() + 4 * cs, 2 * cs, ptr(kvt), kvt.data_ptr() + 4 * cs * pitch, pitch,
              ptr(o), cs, ptr(bias), nq * n, n, ptr(tok_mask_u8), nq, n, self.num_heads, hd, 1.0 / math.sqrt(hd), 1e6, st)
         return o
+
+    def rows(self, s: torch.Tensor, bias: torch.Tensor, tok_mask_u8: Optional[torch.Tensor], scratch: Scratch) -> None:
+        self.finish(s, self.attention(s, bias, tok_mask_u8, 0, s.shape[0], scratch), scratch)
 
     def finish(self, s_rows: torch.Tensor, og: torch.Tensor, scratch: Scratch) -> None:
         n = s_rows.shape[0]
@@ -385,10 +408,6 @@ def pack_single_track(sd, pre: str, num_heads: int, device):
     return (SingleTrack if fits else SingleTrackF32)(sd, pre, num_heads, device)
 
 
-def single_track(s: torch.Tensor, z: torch.Tensor, tok_mask_u8: torch.Tensor, track, scratch: Scratch, after_z_read=None) -> None:
-    """The single track of one layer on all rows.  The pair-bias projection, its only read of z, comes first;
-    ``after_z_read`` is called behind it."""
-    bias = track.bias(z)
-    if after_z_read is not None:
-        after_z_read()
-    track.finish(s, track.attention(s, bias, tok_mask_u8, 0, s.shape[0], scratch), scratch)
+def single_track(s: torch.Tensor, z: torch.Tensor, tok_mask_u8: torch.Tensor, track, scratch: Scratch) -> None:
+    """The single track of one layer on all rows."""
+    track.rows(s, track.bias(z), tok_mask_u8, scratch)

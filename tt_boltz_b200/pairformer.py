@@ -38,7 +38,7 @@ from typing import Dict, Optional, Tuple
 import torch
 from torch import nn
 
-from . import ops, weights
+from . import _lib, ops, weights
 from .synthetic import layer_param_shapes
 
 
@@ -63,13 +63,28 @@ class SideTrack:
 
     The single track of block b needs z after block b's pair transition and s after block b-1, and nothing in the
     pair track ever reads s: so it can run on a stream of its own, under the next block's pair kernels (and, in the
-    sharded trunk, under its exchanges, which leave most SMs idle).  Its one read of z, the pair-bias projection,
-    has to be over before the next block first writes z: ``bias_read`` is the event the pair stream waits for
-    at that point."""
+    sharded trunk, under its exchanges, which leave most SMs idle).
+
+    On one GPU (``enqueue``) its one read of z, the pair-bias projection, stays on the pair stream, into one of two
+    buffers in turn, and the rest follows on this stream.  In the sharded trunk all of it runs on this stream, and
+    ``bias_read`` is the event the pair stream waits for before the next block first writes z."""
 
     def __init__(self, device: torch.device) -> None:
         self.stream = torch.cuda.Stream(device)
         self.bias_read: Optional[torch.cuda.Event] = None
+        self.turn, self.bias, self.done = 0, [None, None], [None, None]
+        self.scratch = ops.Scratch(device)
+
+    def enqueue(self, track, s: torch.Tensor, z: torch.Tensor, tok_mask_u8: Optional[torch.Tensor]) -> None:
+        i, self.turn = self.turn, 1 - self.turn
+        if self.done[i] is not None:                       # this buffer's reader was enqueued two blocks ago
+            torch.cuda.current_stream().wait_event(self.done[i])
+        self.bias[i] = track.bias(z, self.bias[i])
+        ready = torch.cuda.current_stream().record_event()
+        with torch.cuda.stream(self.stream):
+            self.stream.wait_event(ready)
+            track.rows(s, self.bias[i], tok_mask_u8, self.scratch)
+            self.done[i] = self.stream.record_event()
 
     def mark_z_read(self) -> None:
         self.bias_read = torch.cuda.Event()
@@ -132,6 +147,8 @@ class B200PairformerLayer(nn.Module):
         for name in ("tri_att_start", "tri_att_end"):
             pk[name] = pack_att(sd, name + ".", device)
         pk["transition_z"] = pack_trans(sd, "transition_z.", device)
+        if self.fused:
+            pk["pair"] = ops.PairBlock(pk)
         if self.with_s:
             pk["single"] = ops.pack_single_track(sd, "", self.num_heads, device)
         self._packed = pk
@@ -144,28 +161,25 @@ class B200PairformerLayer(nn.Module):
         only enqueued on its stream (the caller joins it before reading s)."""
         pk = self._pack(z.device)
         scratch = scratch or ops.Scratch(z.device)
-        wait_bias = side.before_z_write if side is not None else None
-        if self.fused:
+        if self.precision == "bf16" and _lib.timer is None:      # a timer wants the sub-operations one by one
+            pk["pair"].run(z, masks, ws)
+        elif self.fused:
             if self.precision == "mxfp8":
-                ops.tri_mul_mxfp8(z, masks.pm, pk["tri_mul_out"], ws, False, self.mx_contract_variant, wait_bias)
+                ops.tri_mul_mxfp8(z, masks.pm, pk["tri_mul_out"], ws, False, self.mx_contract_variant)
                 ops.tri_mul_mxfp8(z, masks.pm, pk["tri_mul_in"], ws, True, self.mx_contract_variant)
             else:
-                ops.tri_mul_bf16(z, masks.pm, pk["tri_mul_out"], ws, False, wait_bias)
+                ops.tri_mul_bf16(z, masks.pm, pk["tri_mul_out"], ws, False)
                 ops.tri_mul_bf16(z, masks.pm, pk["tri_mul_in"], ws, True)
             ops.tri_att_bf16(z, masks, pk["tri_att_start"], ws, False)
             ops.tri_att_bf16(z, masks, pk["tri_att_end"], ws, True)
             ops.transition_z_bf16(z, pk["transition_z"])
         elif self.split:
-            if side is not None:
-                side.before_z_write()
             ops.tri_mul_split(z, masks.pm, pk["tri_mul_out"], False, scratch)
             ops.tri_mul_split(z, masks.pm, pk["tri_mul_in"], True, scratch)
             ops.tri_att_split(z, masks.pm, pk["tri_att_start"], False, scratch)
             ops.tri_att_split(z, masks.pm, pk["tri_att_end"], True, scratch)
             ops.transition_split(z, pk["transition_z"], scratch)
         else:
-            if side is not None:
-                side.before_z_write()
             ops.tri_mul_f32(z, masks.pm, pk["tri_mul_out"], False)
             ops.tri_mul_f32(z, masks.pm, pk["tri_mul_in"], True)
             ops.tri_att_f32(z, masks.pm, pk["tri_att_start"], False)
@@ -175,11 +189,7 @@ class B200PairformerLayer(nn.Module):
             if side is None:
                 ops.single_track(s, z, tok_mask_u8, pk["single"], scratch)
             else:
-                z_ready = torch.cuda.Event()
-                z_ready.record()
-                with torch.cuda.stream(side.stream):
-                    side.stream.wait_event(z_ready)
-                    ops.single_track(s, z, tok_mask_u8, pk["single"], ops.Scratch(z.device), side.mark_z_read)
+                side.enqueue(pk["single"], s, z, tok_mask_u8)
 
     def forward(self, s: Optional[torch.Tensor], z: torch.Tensor, mask: Optional[torch.Tensor] = None,
                 pair_mask: Optional[torch.Tensor] = None, chunk_size_tri_attn: Optional[int] = None,
@@ -277,6 +287,17 @@ def _accept_backend_keys(state_dict, prefix, *_unused) -> None:
             state_dict[key[:m.end(1)] + "mha." + key[m.end(1):]] = state_dict.pop(key)
 
 
+# Up to this many tokens a pair kernel has one 128-position tile per line and at most one CTA per line: some of the chip is
+# idle, and the single track beside it costs the pair track nothing.  Beyond, its CTAs take SMs that the pair track's
+# persistent grids fill (17 % slower at 1024 tokens).
+SIDE_TRACK_TOKENS = 128
+
+
+def _side_track_wanted(n: int) -> bool:
+    forced = os.environ.get("B200PF_SIDE_TRACK")
+    return forced == "1" if forced is not None else n <= SIDE_TRACK_TOKENS
+
+
 def _run_layers(layers, s, z, mask, pair_mask, ws_cache: Optional[dict] = None, inplace: bool = False):
     """``inplace``: s [N, c_s] and z [N, N, C] are the caller's fp32 contiguous working tensors and are updated
     where they are (nothing is returned); otherwise [1, ...] inputs are copied and new tensors returned."""
@@ -309,13 +330,15 @@ def _run_layers(layers, s, z, mask, pair_mask, ws_cache: Optional[dict] = None, 
                     ws_cache.clear()
                     ws_cache[key] = ws
         side = None
-        if sw is not None and len(layers) > 1 and os.environ.get("B200PF_SIDE_TRACK", "0") == "1":
+        if sw is not None and len(layers) > 1 and _side_track_wanted(n):
             side = SideTrack(z.device)
         scratch = ops.Scratch(z.device)
-        for layer in layers:
-            layer.forward_inplace(sw, zw, tm, pm, ws, side, scratch)
-        if side is not None:
-            side.join()
+        try:
+            for layer in layers:
+                layer.forward_inplace(sw, zw, tm, pm, ws, side, scratch)
+        finally:                            # also when a layer raises: what is enqueued beside must not outlive its tensors
+            if side is not None:
+                side.join()
     if inplace:
         return None
     z_out = zw.unsqueeze(0).to(z.dtype)
