@@ -483,6 +483,15 @@ int b200pf_single_track_finish(float* s, const b200pf_single_track_weights* w, c
 /* The two calls above for all n query rows; the workspace also holds what passes between them. */
 long long b200pf_single_track_rows_workspace(int n, int cs, int hidden);
 int b200pf_single_track_rows(float* s, const b200pf_single_track_weights* w, const float* bias, const uint8_t* mask, int n, void* workspace, void* stream);
+/* The single track of one block beside the pair track: its read of z, the pair-bias projection into `bias` [heads][n][n], on
+ * pair_stream, the rest behind it on side_stream.  `ready` and `done` are CUDA events; `done` is recorded behind the last kernel
+ * (with wait_done, pair_stream first waits for its previous recording: the bias buffer's earlier reader). */
+typedef struct b200pf_pair_bias_weights {
+    const float *gamma, *beta, *w;      /* w [heads][cz] times log2 e */
+    int cz, heads;
+} b200pf_pair_bias_weights;
+int b200pf_single_track_beside(float* s, const float* z, const b200pf_pair_bias_weights* wb, const b200pf_single_track_weights* w, float* bias,
+                               const uint8_t* mask, int n, void* workspace, void* pair_stream, void* side_stream, void* ready, void* done, int wait_done);
 
 /* ----------------------------------------------------------------------------------------
  * The pair track of one block (tt_bio/reference.py:865-905) in the bf16 tier, enqueued by one call: both triangle

@@ -78,6 +78,11 @@ class TransitionWeights(C.Structure):
     _fields_ = [(k, _vp) for k in ("ln_gamma", "ln_beta", "w12", "w3")]
 
 
+class PairBiasWeights(C.Structure):
+    """Mirror of ``b200pf_pair_bias_weights``."""
+    _fields_ = [("gamma", _vp), ("beta", _vp), ("w", _vp), ("cz", _i), ("heads", _i)]
+
+
 class PairWeights(C.Structure):
     """Mirror of ``b200pf_pair_weights``."""
     _fields_ = [("tri_mul_out", TriMulWeights), ("tri_mul_in", TriMulWeights), ("tri_att_start", TriAttWeights), ("tri_att_end", TriAttWeights),
@@ -147,6 +152,7 @@ SIGNATURES = {
     "b200pf_single_track_finish": [_vp, C.POINTER(SingleTrackWeights), _vp, _i, _vp, _vp],
     "b200pf_single_track_rows_workspace": [_i, _i, _i],
     "b200pf_single_track_rows": [_vp, C.POINTER(SingleTrackWeights), _vp, _vp, _i, _vp, _vp],
+    "b200pf_single_track_beside": [_vp, _vp, C.POINTER(PairBiasWeights), C.POINTER(SingleTrackWeights), _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i],
     "b200pf_pair_block": [_vp, C.POINTER(PairWeights), C.POINTER(PairScratch), _vp],
     "b200pf_split_pair_workspace": [_i, _i, _i, _i, _i],
     "b200pf_split_tri_mul": [_vp, _vp, C.POINTER(SplitTriMulWeights), _i, _i, _vp, _vp],

@@ -53,3 +53,21 @@ extern "C" int b200pf_single_track_rows(float* s, const b200pf_single_track_weig
     B200PF_TRY(b200pf_single_track_attention(s, w, bias, mask, workspace, n, 0, n, rest, stream));
     return b200pf_single_track_finish(s, w, workspace, n, rest, stream);
 }
+
+extern "C" int b200pf_single_track_beside(float* s, const float* z, const b200pf_pair_bias_weights* wb, const b200pf_single_track_weights* w, float* bias,
+                                          const uint8_t* mask, int n, void* workspace, void* pair_stream, void* side_stream, void* ready, void* done,
+                                          int wait_done) {
+    B200PF_REQUIRE(s && z && wb && w && bias && workspace && ready && done && n > 0, B200PF_ERR_INVALID, "single_track_beside: bad argument");
+    cudaStream_t pair = (cudaStream_t)pair_stream, side = (cudaStream_t)side_stream;
+    const long long nn = (long long)n * n;
+    if (wait_done) B200PF_CUDA(cudaStreamWaitEvent(pair, (cudaEvent_t)done, 0));
+    if (wb->cz == 128 && (wb->heads == 4 || wb->heads == 16))
+        B200PF_TRY(b200pf_ln_proj_heads(z, wb->gamma, wb->beta, wb->w, bias, nn, nn, wb->cz, wb->heads, pair));
+    else
+        B200PF_TRY(b200pf_ln_heads(z, wb->gamma, wb->beta, wb->w, bias, nn, nn, wb->cz, wb->heads, pair));
+    B200PF_CUDA(cudaEventRecord((cudaEvent_t)ready, pair));
+    B200PF_CUDA(cudaStreamWaitEvent(side, (cudaEvent_t)ready, 0));
+    B200PF_TRY(b200pf_single_track_rows(s, w, bias, mask, n, workspace, side));
+    B200PF_CUDA(cudaEventRecord((cudaEvent_t)done, side));
+    return B200PF_OK;
+}

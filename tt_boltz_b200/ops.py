@@ -36,6 +36,11 @@ class PairMasks:
         self.cols = torch.zeros(n, self.pitch, dtype=torch.uint8, device=pair_mask_u8.device)
         self.cols[:, :n] = self.pm.t()
 
+    def scratch(self, ws: "Workspace") -> _lib.PairScratch:
+        """The workspace and the masks as ``b200pf_pair_block`` takes them."""
+        return _lib.PairScratch((C.c_void_p * 5)(*[ptr(b) for b in ws.buf]), ptr(ws.tri_bias), ptr(self.pm), ptr(self.rows), ptr(self.cols), ws.n, ws.pitch,
+                                self.pitch)
+
 
 class Workspace:
     """bf16 scratch for one token count: five [N*pitch*128] buffers shared by the sub-operations
@@ -157,10 +162,8 @@ class PairBlock:
         self.struct = _lib.PairWeights(mul(pk["tri_mul_out"]), mul(pk["tri_mul_in"]), att(pk["tri_att_start"]), att(pk["tri_att_end"]),
                                        _lib.TransitionWeights(ptr(t["ln_gamma"]), ptr(t["ln_beta"]), ptr(t["w12_tc"]), ptr(t["w3"])))
 
-    def run(self, z: torch.Tensor, masks: PairMasks, ws: Workspace) -> None:
-        k = _lib.PairScratch((C.c_void_p * 5)(*[ptr(b) for b in ws.buf]), ptr(ws.tri_bias), ptr(masks.pm), ptr(masks.rows), ptr(masks.cols), ws.n, ws.pitch,
-                             masks.pitch)
-        call("b200pf_pair_block", ptr(z), C.byref(self.struct), C.byref(k), stream())
+    def run(self, z: torch.Tensor, scratch: _lib.PairScratch) -> None:
+        call("b200pf_pair_block", ptr(z), C.byref(self.struct), C.byref(scratch), stream())
 
 
 # ------------------------------------------------------------------------------------------------
@@ -309,14 +312,15 @@ class SingleTrack:
     def __init__(self, sd, pre: str, num_heads: int, device) -> None:
         self.pack = weights.pack_single_track(sd, pre, num_heads, device)
         self.z_bias = weights.pack_pair_bias(sd, pre + "attention.", device)
+        b = self.z_bias
+        self.bias_struct = _lib.PairBiasWeights(ptr(b["gamma"]), ptr(b["beta"]), ptr(b["w"]), b["w"].shape[1], b["w"].shape[0])
 
-    def bias(self, z_rows: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    def bias(self, z_rows: torch.Tensor) -> torch.Tensor:
         """bias[h][i_local * N + j], times log2(e): one fp32 pass over the (local rows of) z [nr, N, c_z]."""
         rows, c = z_rows.shape[0] * z_rows.shape[1], z_rows.shape[-1]
         w = self.z_bias
         heads = w["w"].shape[0]
-        if out is None:
-            out = torch.empty(heads, rows, dtype=torch.float32, device=z_rows.device)
+        out = torch.empty(heads, rows, dtype=torch.float32, device=z_rows.device)
         name = "b200pf_ln_proj_heads" if c == C_Z and heads in (4, 16) else "b200pf_ln_heads"
         call(name, ptr(z_rows), ptr(w["gamma"]), ptr(w["beta"]), ptr(w["w"]), ptr(out), rows, rows, c, heads, stream())
         return out
@@ -333,6 +337,14 @@ class SingleTrack:
         w, n = self.pack.struct, s.shape[0]
         ws = scratch.get(_nbytes("b200pf_single_track_rows_workspace", n, w.cs, w.hidden))
         call("b200pf_single_track_rows", ptr(s), C.byref(w), ptr(bias), ptr(tok_mask_u8), n, ws, stream())
+
+    def beside(self, s: torch.Tensor, z: torch.Tensor, bias: torch.Tensor, tok_mask_u8: Optional[torch.Tensor], scratch: Scratch, side: int,
+               ready: int, done: int, wait_done: bool) -> None:
+        """``bias`` into the given buffer on the current stream, ``rows`` behind it on the stream ``side``."""
+        w, n = self.pack.struct, s.shape[0]
+        ws = scratch.get(_nbytes("b200pf_single_track_rows_workspace", n, w.cs, w.hidden))
+        call("b200pf_single_track_beside", ptr(s), ptr(z), C.byref(self.bias_struct), C.byref(w), ptr(bias), ptr(tok_mask_u8), n, ws, stream(), side,
+             ready, done, int(wait_done))
 
     def finish(self, s_rows: torch.Tensor, og: torch.Tensor, scratch: Scratch) -> None:
         w = self.pack.struct
@@ -354,13 +366,12 @@ class SingleTrackF32:
         self.w_kv = torch.cat([w_att["proj_k.weight"], w_att["proj_v.weight"]], 0).contiguous()
         self.w_12 = torch.cat([w_trans["fc1.weight"], w_trans["fc2.weight"]], 0).contiguous()
 
-    def bias(self, z_rows: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    def bias(self, z_rows: torch.Tensor) -> torch.Tensor:
         """bias[h][i_local * N + j]: one fp32 pass over the (local rows of) z [nr, N, c_z]."""
         w = self.w_att
         rows, c = z_rows.shape[0] * z_rows.shape[1], z_rows.shape[-1]
         heads = w["proj_z.1.weight"].shape[0]
-        if out is None:
-            out = torch.empty(heads, rows, dtype=torch.float32, device=z_rows.device)
+        out = torch.empty(heads, rows, dtype=torch.float32, device=z_rows.device)
         if c == C_Z and heads in (4, 16):
             call("b200pf_ln_proj_heads", ptr(z_rows), ptr(w["proj_z.0.weight"]), ptr(w["proj_z.0.bias"]),
                  ptr(w["proj_z.1.weight"]), ptr(out), rows, rows, c, heads, stream())

@@ -72,19 +72,22 @@ class SideTrack:
     def __init__(self, device: torch.device) -> None:
         self.stream = torch.cuda.Stream(device)
         self.bias_read: Optional[torch.cuda.Event] = None
-        self.turn, self.bias, self.done = 0, [None, None], [None, None]
-        self.scratch = ops.Scratch(device)
+        self.blocks, self.bias, self.held = 0, [None, None], []
+        self.ready, self.done = ([torch.cuda.Event(), torch.cuda.Event()] for _ in range(2))
+        self.scratch = ops.Scratch(device)          # from the pair stream's memory, given back to it after ``join``
 
     def enqueue(self, track, s: torch.Tensor, z: torch.Tensor, tok_mask_u8: Optional[torch.Tensor]) -> None:
-        i, self.turn = self.turn, 1 - self.turn
-        if self.done[i] is not None:                       # this buffer's reader was enqueued two blocks ago
-            torch.cuda.current_stream().wait_event(self.done[i])
-        self.bias[i] = track.bias(z, self.bias[i])
-        ready = torch.cuda.current_stream().record_event()
-        with torch.cuda.stream(self.stream):
-            self.stream.wait_event(ready)
-            track.rows(s, self.bias[i], tok_mask_u8, self.scratch)
-            self.done[i] = self.stream.record_event()
+        i, first = self.blocks & 1, self.blocks < 2
+        self.blocks += 1
+        if first:                                   # (an event exists from its first recording on)
+            self.bias[i] = torch.empty(track.bias_struct.heads, s.shape[0] ** 2, dtype=torch.float32, device=z.device)
+            self.ready[i].record()
+            self.done[i].record()
+        buf = self.scratch.buf
+        # the reader of this bias buffer was enqueued two blocks ago
+        track.beside(s, z, self.bias[i], tok_mask_u8, self.scratch, self.stream.cuda_stream, self.ready[i].cuda_event, self.done[i].cuda_event, not first)
+        if buf is not None and self.scratch.buf is not buf:
+            self.held.append(buf)                   # outgrown, but its kernels may still run
 
     def mark_z_read(self) -> None:
         self.bias_read = torch.cuda.Event()
@@ -156,13 +159,13 @@ class B200PairformerLayer(nn.Module):
 
     def forward_inplace(self, s: Optional[torch.Tensor], z: torch.Tensor, tok_mask_u8: Optional[torch.Tensor],
                         masks: ops.PairMasks, ws: Optional[ops.Workspace], side: Optional["SideTrack"] = None,
-                        scratch: Optional[ops.Scratch] = None) -> None:
+                        scratch: Optional[ops.Scratch] = None, pair_scratch=None) -> None:
         """Update fp32 working copies z [N,N,128] and s [N,c_s] in place.  With a ``side`` track the update of s is
         only enqueued on its stream (the caller joins it before reading s)."""
         pk = self._pack(z.device)
         scratch = scratch or ops.Scratch(z.device)
         if self.precision == "bf16" and _lib.timer is None:      # a timer wants the sub-operations one by one
-            pk["pair"].run(z, masks, ws)
+            pk["pair"].run(z, pair_scratch if pair_scratch is not None else masks.scratch(ws))
         elif self.fused:
             if self.precision == "mxfp8":
                 ops.tri_mul_mxfp8(z, masks.pm, pk["tri_mul_out"], ws, False, self.mx_contract_variant)
@@ -186,10 +189,13 @@ class B200PairformerLayer(nn.Module):
             ops.tri_att_f32(z, masks.pm, pk["tri_att_end"], True)
             ops.transition_f32(z, pk["transition_z"])
         if self.with_s and s is not None:
-            if side is None:
-                ops.single_track(s, z, tok_mask_u8, pk["single"], scratch)
+            track = pk["single"]
+            if side is not None and isinstance(track, ops.SingleTrack):
+                side.enqueue(track, s, z, tok_mask_u8)
             else:
-                side.enqueue(pk["single"], s, z, tok_mask_u8)
+                if side is not None:
+                    side.join()
+                ops.single_track(s, z, tok_mask_u8, track, scratch)
 
     def forward(self, s: Optional[torch.Tensor], z: torch.Tensor, mask: Optional[torch.Tensor] = None,
                 pair_mask: Optional[torch.Tensor] = None, chunk_size_tri_attn: Optional[int] = None,
@@ -287,10 +293,10 @@ def _accept_backend_keys(state_dict, prefix, *_unused) -> None:
             state_dict[key[:m.end(1)] + "mha." + key[m.end(1):]] = state_dict.pop(key)
 
 
-# Up to this many tokens a pair kernel has one 128-position tile per line and at most one CTA per line: some of the chip is
-# idle, and the single track beside it costs the pair track nothing.  Beyond, its CTAs take SMs that the pair track's
-# persistent grids fill (17 % slower at 1024 tokens).
-SIDE_TRACK_TOKENS = 128
+# Token count up to which the single track runs beside the pair track.  Its kernels are small and fill the tails and idle SMs
+# of the pair kernels: 16 blocks take 2.69 -> 2.26 ms at 45 tokens, 6.94 -> 6.47 at 256, 22.7 -> 22.3 at 512, 110 -> 109 at 1024;
+# at 1300 (225.5 and 225.6) nothing is left of it.
+SIDE_TRACK_TOKENS = 1024
 
 
 def _side_track_wanted(n: int) -> bool:
@@ -329,13 +335,14 @@ def _run_layers(layers, s, z, mask, pair_mask, ws_cache: Optional[dict] = None, 
                 if ws_cache is not None:
                     ws_cache.clear()
                     ws_cache[key] = ws
+        pair_scratch = pm.scratch(ws) if ws is not None else None
         side = None
         if sw is not None and len(layers) > 1 and _side_track_wanted(n):
             side = SideTrack(z.device)
         scratch = ops.Scratch(z.device)
         try:
             for layer in layers:
-                layer.forward_inplace(sw, zw, tm, pm, ws, side, scratch)
+                layer.forward_inplace(sw, zw, tm, pm, ws, side, scratch, pair_scratch)
         finally:                            # also when a layer raises: what is enqueued beside must not outlive its tensors
             if side is not None:
                 side.join()
