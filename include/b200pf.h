@@ -445,7 +445,7 @@ int b200pf_peer_barrier(const unsigned long long* pad_ptrs, unsigned int generat
 
 /* ------------------------------------------------------------------------------------------
  * fp32-accurate tensor-core path: every fp32 factor is multiplied as a sum of 16-bit parts (two fp16 parts of a scaled
- * value for linear layers, three bf16 parts for attention, the triangle contraction and unbounded inputs), fp32
+ * value for linear layers and attention, three bf16 parts for the triangle contraction and unbounded inputs), fp32
  * accumulation.  Widths that are multiples of 64 (64, 128, 256; 384 without head projections).  It carries the single
  * track of every tier and the pair track of the fp32 tier.
  * ---------------------------------------------------------------------------------------- */
@@ -462,7 +462,8 @@ typedef struct b200pf_single_track_weights {
     b200pf_split_weight qkvg;       /* rows q (times log2 e / sqrt(head width)) | k | v | g: [4 c_s][c_s] */
     const float* qkvg_bias;         /* [4 c_s], q part scaled like its rows */
     b200pf_split_weight o;          /* [c_s][c_s] */
-    float o_scale;                  /* scale of the gated attention output's parts */
+    float o_scale;                  /* scale of the parts of v and of the gated attention output */
+    float q_scale, k_scale;         /* scales of the parts of q and k */
     const float *ln2_gamma, *ln2_beta;
     b200pf_split_weight fc12;       /* 32 rows of fc1, then 32 of fc2, in turn: [2 hidden][c_s] */
     float hidden_scale;             /* scale of the hidden activations' parts */
@@ -536,7 +537,7 @@ typedef struct b200pf_split_triatt_weights {
     const float* head_w;            /* [heads][c] times log2 e over the planes' scale */
     b200pf_split_weight qkvg;       /* as in the single track: [4 heads hd][c] */
     b200pf_split_weight o;          /* [c][heads hd] */
-    float o_scale;
+    float o_scale, q_scale, k_scale;    /* as in the single track */
     int c, heads, hd;
 } b200pf_split_triatt_weights;
 typedef struct b200pf_split_transition_weights {

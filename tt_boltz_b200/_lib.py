@@ -42,7 +42,7 @@ class SplitWeight(C.Structure):
 class SingleTrackWeights(C.Structure):
     """Mirror of ``b200pf_single_track_weights``."""
     _fields_ = [("ln_gamma", _vp), ("ln_beta", _vp), ("qkvg", SplitWeight), ("qkvg_bias", _vp), ("o", SplitWeight), ("o_scale", _f),
-                ("ln2_gamma", _vp), ("ln2_beta", _vp), ("fc12", SplitWeight), ("hidden_scale", _f), ("fc3", SplitWeight),
+                ("q_scale", _f), ("k_scale", _f), ("ln2_gamma", _vp), ("ln2_beta", _vp), ("fc12", SplitWeight), ("hidden_scale", _f), ("fc3", SplitWeight),
                 ("cs", _i), ("heads", _i), ("hidden", _i)]
 
 
@@ -55,7 +55,7 @@ class SplitTriMulWeights(C.Structure):
 class SplitTriAttWeights(C.Structure):
     """Mirror of ``b200pf_split_triatt_weights``."""
     _fields_ = [("ln_gamma", _vp), ("ln_beta", _vp), ("head_w", _vp), ("qkvg", SplitWeight), ("o", SplitWeight), ("o_scale", _f),
-                ("c", _i), ("heads", _i), ("hd", _i)]
+                ("q_scale", _f), ("k_scale", _f), ("c", _i), ("heads", _i), ("hd", _i)]
 
 
 class SplitTransitionWeights(C.Structure):

@@ -69,7 +69,8 @@ struct Gemm {
     const float* bias = nullptr;    // [n_rows]
     const uint8_t* mask = nullptr;  // EPI_GATE_PLANES: position (batch, col) at mask + batch * mask_bs + col * mask_cs
     long long mask_bs = 0, mask_cs = 0;
-    int n_split = 0;                // EPI_QKVG: columns below it go out as three bf16 parts, the others as sigmoid, fp32
+    int n_split = 0;                // EPI_QKVG: columns below it (q | k | v, a third each) go out as two fp16 parts times
+    float qkv_scale[3] = {1.f, 1.f, 1.f};       // these, the others as sigmoid, fp32
     Output out[2];
 };
 int launch_gemm(const Gemm& g, cudaStream_t st);

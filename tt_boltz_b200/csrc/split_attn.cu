@@ -1,21 +1,25 @@
-// softmax(q k^T + bias + mask) v with a gate, at fp32 accuracy: one-pass softmax over 64-key tiles, both products as six
-// m16n8k16 bf16 MMAs on three-part operands (split.cuh: 24 bits of every factor, fp32 accumulation).
+// softmax(q k^T + bias + mask) v with a gate, at fp32 accuracy: one-pass softmax over 64-key tiles, both products as three
+// m16n8k16 fp16 MMAs on two-part operands (split.cuh; hi is rounded to 11 bits and lo to 11 bits of what is left, together
+// 2^-24 of the value, half an ulp of fp32), fp32 accumulation.
 //
-// mma.sync and not tcgen05: q, k, v rows are 24 or 32 wide and the probabilities need three parts of their own, so a tcgen05
-// form would have to push three times the probabilities through tensor memory; here they go from the accumulators of the
-// first product straight into the A fragments of the second.  A warp owns 16 queries; per 64-key tile it issues 192 MMAs
-// (8 clocks each and scheduler: the bound) against some 650 other instructions.  K and V tiles are shared by the CTA's
+// mma.sync and not tcgen05: q, k, v rows are 24 or 32 wide and the probabilities need parts of their own, so a tcgen05 form
+// would have to push both through tensor memory; here they go from the accumulators of the first product straight into the
+// A fragments of the second.  A warp owns 16 queries; per 64-key tile it issues 96 MMAs against some 700 other
+// instructions.  With three bf16 parts and six MMAs per product, and every lane fetching its own bias values, a launch took 462 us
+// at 292 tokens x 4 heads and 528 at 256 x 8; with two parts 390 and 430, with staged bias tiles 310 and 311.  Neither the
+// tensor pipe nor memory bounds it now.  K and V tiles are shared by the CTA's
 // warps, double buffered with cp.async; rows are 64 bytes with the 16-byte chunks swizzled by row so that ldmatrix is
-// conflict free.  Bias values are the accumulators' initial values.
+// conflict free.  Bias tiles come with them, as whole lines (read by
+// the lanes that want them, 8 bytes of eight rows at a time and behind the tile before, they were the longest wait of a tile), and are the accumulators' initial values.
 #include "split_attn.cuh"
 
 namespace b200pf {
 namespace split {
 
-constexpr int KT = 64, KV_PART = KT * 64, KV_STAGE = 6 * KV_PART;          // K parts | V parts
+constexpr int KT = 64, KV_PART = KT * 64, KV_STAGE = 4 * KV_PART;          // K parts | V parts
 
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
@@ -25,19 +29,24 @@ __device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
+constexpr int BP = KT + 8;               // bias tile pitch in floats: a half-warp's float2 reads of four rows meet no bank twice
+constexpr int bias_stage(int nw) { return nw * 16 * BP * 4; }
+constexpr float P_SCALE = 16384.f;      // probabilities are at most one: their parts use the upper half of fp16's range
+
 template <int HD, int NW>
 __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnArgs p) {
     constexpr int CH = HD / 8, NE = HD / 8, NT = NW * 32;
     static_assert(HD == 24 || HD == 32, "head width");
     extern __shared__ __align__(128) uint8_t at_smem[];
-    float* mterm = reinterpret_cast<float*>(at_smem + 2 * KV_STAGE);            // [2][KT]
+    uint8_t* bias_s = at_smem + 2 * KV_STAGE;                                    // [2][NW * 16 queries][BP]
+    float* mterm = reinterpret_cast<float*>(bias_s + 2 * bias_stage(NW));        // [2][KT]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int h = blockIdx.y, line = blockIdx.z;
     const int qw = blockIdx.x * (NW * 16) + warp * 16;                           // this warp's first query, relative to q0
     const bool active = qw < p.n_q;
     const int ht = p.heads * HD;
     if (HD == 24) {                                                              // the fourth chunk of every row stays zero
-        for (int i = tid; i < 2 * 6 * KT; i += NT) {
+        for (int i = tid; i < 2 * 4 * KT; i += NT) {
             const int key = i % KT, part = i / KT;
             *reinterpret_cast<uint4*>(at_smem + part * KV_PART + key * 64 + ((3 ^ ((key >> 1) & 3)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
         }
@@ -45,19 +54,39 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
     grid_dependency_wait();
     grid_launch_dependents();
 
-    const __nv_bfloat16* base = p.qkv + (long long)line * p.line_rows * p.ld + h * HD;
+    const __half* base = p.qkv + (long long)line * p.line_rows * p.ld + h * HD;
     const long long pos_ld = p.pos_rows * p.ld;
     auto load_tile = [&](int tile) {
         const int k0 = tile * KT;
         const uint32_t st = smem_u32(at_smem + (tile & 1) * KV_STAGE);
-        for (int i = tid; i < 6 * KT * CH; i += NT) {
-            const int c = i % CH, key = (i / CH) % KT, part = i / (CH * KT);     // parts 0-2: K, 3-5: V
+        for (int i = tid; i < 4 * KT * CH; i += NT) {
+            const int c = i % CH, key = (i / CH) % KT, part = i / (CH * KT);     // parts 0-1: K, 2-3: V
             const int kk = k0 + key;
             const bool in = kk < p.n_k;
-            const __nv_bfloat16* src = base + (part >= 3 ? 2 * ht : ht) + (long long)(part >= 3 ? part - 3 : part) * p.part_stride +
+            const __half* src = base + (part >= 2 ? 2 * ht : ht) + (long long)(part & 1) * p.part_stride +
                                        (in ? kk : 0) * pos_ld + c * 8;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(st + part * KV_PART + key * 64 + ((c ^ ((key >> 1) & 3)) << 4)),
                          "l"(src), "r"(in ? 16 : 0) : "memory");
+        }
+        const uint32_t bst = smem_u32(bias_s + (tile & 1) * bias_stage(NW));
+        const float* brow = p.bias + h * p.bias_hs;
+        const int qb = blockIdx.x * (NW * 16);
+        if (p.bias_vec) {
+#pragma unroll 2
+            for (int i = tid; i < NW * 16 * (KT / 4); i += NT) {
+                const int c = (i % (KT / 4)) * 4, r = i / (KT / 4);
+                const bool in = k0 + c < p.n_k;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(bst + (r * BP + c) * 4),
+                             "l"(brow + min(qb + r, p.n_q - 1) * p.bias_qs + (in ? k0 + c : 0)), "r"(in ? 16 : 0) : "memory");
+            }
+        } else {
+#pragma unroll 1
+            for (int i = tid; i < NW * 16 * KT; i += NT) {
+                const int c = i % KT, r = i / KT;
+                const bool in = k0 + c < p.n_k;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(bst + (r * BP + c) * 4),
+                             "l"(brow + min(qb + r, p.n_q - 1) * p.bias_qs + (in ? k0 + c : 0)), "r"(in ? 4 : 0) : "memory");
+            }
         }
         if (tid < KT) {
             const int kk = k0 + tid;
@@ -71,38 +100,28 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
     load_tile(0);
 
     const int r0 = min(qw + g, p.n_q - 1), r1 = min(qw + g + 8, p.n_q - 1);      // rows past the end repeat the last one
-    uint32_t q[3][2][4];
+    uint32_t q[2][2][4];
 #pragma unroll
-    for (int part = 0; part < 3; ++part)
+    for (int part = 0; part < 2; ++part)
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
-            const __nv_bfloat16* a = base + part * p.part_stride + (p.q0 + r0) * pos_ld + ks * 16 + 2 * t;
-            const __nv_bfloat16* b = base + part * p.part_stride + (p.q0 + r1) * pos_ld + ks * 16 + 2 * t;
+            const __half* a = base + part * p.part_stride + (p.q0 + r0) * pos_ld + ks * 16 + 2 * t;
+            const __half* b = base + part * p.part_stride + (p.q0 + r1) * pos_ld + ks * 16 + 2 * t;
             q[part][ks][0] = *reinterpret_cast<const uint32_t*>(a);
             q[part][ks][1] = *reinterpret_cast<const uint32_t*>(b);
             q[part][ks][2] = HD == 24 && ks == 1 ? 0u : *reinterpret_cast<const uint32_t*>(a + 8);
             q[part][ks][3] = HD == 24 && ks == 1 ? 0u : *reinterpret_cast<const uint32_t*>(b + 8);
         }
-    const float* bias0 = p.bias + h * p.bias_hs + r0 * p.bias_qs;
-    const float* bias1 = p.bias + h * p.bias_hs + r1 * p.bias_qs;
     float o[NE][4];
 #pragma unroll
     for (int e = 0; e < NE; ++e) { o[e][0] = o[e][1] = o[e][2] = o[e][3] = 0.f; }
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
     const int ntiles = (p.n_k + KT - 1) / KT;
+    const float qk = p.qk_scale, qk_inv = 1.f / p.qk_scale;                      // powers of two
     const uint32_t k_lane = (uint32_t)((lane & 7) * 64), k_sw = (uint32_t)(((lane >> 3) ^ ((lane >> 1) & 3)) << 4);     // row lane & 7, chunk lane / 8
 
 #pragma unroll 1
     for (int tile = 0; tile < ntiles; ++tile) {
-        float s[8][4];
-        {
-            const int k0 = tile * KT + 2 * t;
-#pragma unroll
-            for (int ni = 0; ni < 8; ++ni) {
-                const int c0 = min(k0 + 8 * ni, p.n_k - 1), c1 = min(k0 + 8 * ni + 1, p.n_k - 1);
-                s[ni][0] = bias0[c0]; s[ni][1] = bias0[c1]; s[ni][2] = bias1[c0]; s[ni][3] = bias1[c1];
-            }
-        }
         if (tile + 1 < ntiles) {
             load_tile(tile + 1);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -111,25 +130,30 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
         }
         __syncthreads();
         if (active) {
-            const uint32_t kst = smem_u32(at_smem + (tile & 1) * KV_STAGE), vst = kst + 3 * KV_PART;
+            float s[8][4];
+            const float* bt = reinterpret_cast<const float*>(bias_s + (tile & 1) * bias_stage(NW)) + (warp * 16 + g) * BP + 2 * t;
+#pragma unroll
+            for (int ni = 0; ni < 8; ++ni) {
+                const float2 b0 = *reinterpret_cast<const float2*>(bt + 8 * ni), b1 = *reinterpret_cast<const float2*>(bt + 8 * BP + 8 * ni);
+                s[ni][0] = b0.x * qk; s[ni][1] = b0.y * qk; s[ni][2] = b1.x * qk; s[ni][3] = b1.y * qk;
+            }
+            const uint32_t kst = smem_u32(at_smem + (tile & 1) * KV_STAGE), vst = kst + 2 * KV_PART;
             const float* mt = mterm + (tile & 1) * KT + 2 * t;
             float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
             for (int ni = 0; ni < 8; ++ni) {
-                uint32_t kb[3][4];
+                uint32_t kb[2][4];
 #pragma unroll
-                for (int part = 0; part < 3; ++part) ldsm4(kb[part], kst + part * KV_PART + ni * 512 + k_lane + k_sw);
+                for (int part = 0; part < 2; ++part) ldsm4(kb[part], kst + part * KV_PART + ni * 512 + k_lane + k_sw);
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks) {
-                    mma_bf16(s[ni], q[2][ks], kb[0][2 * ks], kb[0][2 * ks + 1]);
-                    mma_bf16(s[ni], q[1][ks], kb[1][2 * ks], kb[1][2 * ks + 1]);
-                    mma_bf16(s[ni], q[0][ks], kb[2][2 * ks], kb[2][2 * ks + 1]);
-                    mma_bf16(s[ni], q[1][ks], kb[0][2 * ks], kb[0][2 * ks + 1]);
-                    mma_bf16(s[ni], q[0][ks], kb[1][2 * ks], kb[1][2 * ks + 1]);
-                    mma_bf16(s[ni], q[0][ks], kb[0][2 * ks], kb[0][2 * ks + 1]);
+                    mma_f16(s[ni], q[1][ks], kb[0][2 * ks], kb[0][2 * ks + 1]);
+                    mma_f16(s[ni], q[0][ks], kb[1][2 * ks], kb[1][2 * ks + 1]);
+                    mma_f16(s[ni], q[0][ks], kb[0][2 * ks], kb[0][2 * ks + 1]);
                 }
                 const float2 mv = *reinterpret_cast<const float2*>(mt + 8 * ni);
-                s[ni][0] += mv.x; s[ni][1] += mv.y; s[ni][2] += mv.x; s[ni][3] += mv.y;
+                s[ni][0] = fmaf(s[ni][0], qk_inv, mv.x); s[ni][1] = fmaf(s[ni][1], qk_inv, mv.y);
+                s[ni][2] = fmaf(s[ni][2], qk_inv, mv.x); s[ni][3] = fmaf(s[ni][3], qk_inv, mv.y);
                 mx0 = fmaxf(mx0, fmaxf(s[ni][0], s[ni][1]));
                 mx1 = fmaxf(mx1, fmaxf(s[ni][2], s[ni][3]));
             }
@@ -145,33 +169,30 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
             for (int e = 0; e < NE; ++e) { ot[e][0] = ot[e][1] = ot[e][2] = ot[e][3] = 0.f; }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {                                        // 16 keys
-                uint32_t pf[3][4];
+                uint32_t pf[2][4];
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     float* sv = s[2 * j + u];
                     sv[0] = exp2f(sv[0] - n0); sv[1] = exp2f(sv[1] - n0); sv[2] = exp2f(sv[2] - n1); sv[3] = exp2f(sv[3] - n1);
                     l0 += sv[0] + sv[1]; l1 += sv[2] + sv[3];
-                    split_bf16x3(sv[0], sv[1], pf[0][2 * u], pf[1][2 * u], pf[2][2 * u]);
-                    split_bf16x3(sv[2], sv[3], pf[0][2 * u + 1], pf[1][2 * u + 1], pf[2][2 * u + 1]);
+                    split_f16x2(sv[0] * P_SCALE, sv[1] * P_SCALE, pf[0][2 * u], pf[1][2 * u]);
+                    split_f16x2(sv[2] * P_SCALE, sv[3] * P_SCALE, pf[0][2 * u + 1], pf[1][2 * u + 1]);
                 }
                 // matrices: (keys 0-7, chunk), (keys 8-15, chunk), (keys 0-7, chunk + 1), (keys 8-15, chunk + 1)
                 const int key = j * 16 + ((lane >> 3) & 1) * 8 + (lane & 7);
 #pragma unroll
                 for (int c2 = 0; c2 < 2; ++c2) {
-                    uint32_t vb[3][4];
+                    uint32_t vb[2][4];
                     const uint32_t off = (uint32_t)(key * 64 + (((c2 * 2 + (lane >> 4)) ^ ((key >> 1) & 3)) << 4));
 #pragma unroll
-                    for (int part = 0; part < 3; ++part) ldsm4_t(vb[part], vst + part * KV_PART + off);
+                    for (int part = 0; part < 2; ++part) ldsm4_t(vb[part], vst + part * KV_PART + off);
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
                         if (c2 * 2 + u >= NE) continue;
                         float (&oe)[4] = ot[(c2 * 2 + u) % NE];
-                        mma_bf16(oe, pf[2], vb[0][2 * u], vb[0][2 * u + 1]);
-                        mma_bf16(oe, pf[1], vb[1][2 * u], vb[1][2 * u + 1]);
-                        mma_bf16(oe, pf[0], vb[2][2 * u], vb[2][2 * u + 1]);
-                        mma_bf16(oe, pf[1], vb[0][2 * u], vb[0][2 * u + 1]);
-                        mma_bf16(oe, pf[0], vb[1][2 * u], vb[1][2 * u + 1]);
-                        mma_bf16(oe, pf[0], vb[0][2 * u], vb[0][2 * u + 1]);
+                        mma_f16(oe, pf[1], vb[0][2 * u], vb[0][2 * u + 1]);
+                        mma_f16(oe, pf[0], vb[1][2 * u], vb[1][2 * u + 1]);
+                        mma_f16(oe, pf[0], vb[0][2 * u], vb[0][2 * u + 1]);
                     }
                 }
             }
@@ -188,7 +209,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
     if (!active) return;
     l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-    const float inv[2] = {p.out_scale / l0, p.out_scale / l1};
+    const float inv[2] = {1.f / (l0 * P_SCALE), 1.f / (l1 * P_SCALE)};
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const int qi = qw + g + 8 * half;
@@ -208,13 +229,16 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
 }
 
 template <int HD, int NW> static int attn_go(const AttnArgs& a, cudaStream_t st) {
-    constexpr int smem = 2 * KV_STAGE + 2 * KT * 4;
+    constexpr int smem = 2 * KV_STAGE + 2 * bias_stage(NW) + 2 * KT * 4;         // NW = 8: 107,008, two CTAs per SM
     auto kern = split_attention_kernel<HD, NW>;
     B200PF_SMEM_ATTR_ONCE(kern, smem);
     return launch_pdl(kern, dim3((unsigned)((a.n_q + NW * 16 - 1) / (NW * 16)), (unsigned)a.heads, (unsigned)a.lines), dim3(NW * 32), smem, st, a);
 }
 
-int launch_attention(const AttnArgs& a, int hd, cudaStream_t st) {
+int launch_attention(const AttnArgs& args, int hd, cudaStream_t st) {
+    AttnArgs a = args;
+    // 16-byte pieces of the bias rows where every one starts on a 16-byte boundary and ends inside its row, single values elsewhere
+    a.bias_vec = aligned16(a.bias) && a.bias_hs % 4 == 0 && a.bias_qs % 4 == 0 && a.n_k % 4 == 0;
     B200PF_REQUIRE(a.qkv && a.gate && a.bias && a.out && aligned16(a.qkv) && a.part_stride % 8 == 0 && a.ld % 8 == 0, B200PF_ERR_INVALID,
                    "split attention: null or misaligned operand");
     B200PF_REQUIRE(a.lines > 0 && a.lines < 65536 && a.heads > 0 && a.n_q > 0 && a.n_k > 0, B200PF_ERR_INVALID, "split attention: bad sizes");

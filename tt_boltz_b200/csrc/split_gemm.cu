@@ -20,7 +20,7 @@ struct Dev {
     int m_rows, n_rows, batches, bn;
     int a_batched, b_batched, a_second_row;
     int k[2], k_splits, kb_per_split;
-    float alpha[2], out_scale;
+    float alpha[2], out_scale, qkv_scale[3];
     const float* bias;
     const uint8_t* mask;
     long long mask_bs, mask_cs;
@@ -248,8 +248,15 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
                         }
                         if (EPI == EPI_STORE) put_f32(v, &map_o0, false, col, m0, bt);
                         else if (EPI == EPI_ADD) put_f32(v, &map_o0, true, col, m0, bt);
-                        else if (col < p.n_split) put_bf16x3(v, &map_o0, col, m0, bt);
-                        else {
+                        else if (col < p.n_split) {
+                            const int third = p.n_split / 3;            // a multiple of 32: one of q, k, v per round
+                            const float sc = p.qkv_scale[col < third ? 0 : col < 2 * third ? 1 : 2];
+                            uint32_t w[2][16];
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) split_f16x2(v[2 * e] * sc, v[2 * e + 1] * sc, w[0][e], w[1][e]);
+                            put_part(w[0], &map_o0, col, m0, bt, 0);
+                            put_part(w[1], &map_o0, col, m0, bt, 1);
+                        } else {
 #pragma unroll
                             for (int e = 0; e < 32; ++e) v[e] = sigmoid_precise(v[e]);
                             put_f32(v, &map_o1, false, col - p.n_split, m0, bt);
@@ -342,6 +349,7 @@ static int launch_one(const Gemm& g, int bn, int sms, cudaStream_t st) {
     d.kb_per_split = ((g.k[0] + 63) / 64 + g.k_splits - 1) / g.k_splits;
     d.alpha[0] = g.alpha[0]; d.alpha[1] = g.alpha[1]; d.out_scale = g.out_scale;
     d.bias = g.bias; d.mask = g.mask; d.mask_bs = g.mask_bs; d.mask_cs = g.mask_cs;
+    for (int i = 0; i < 3; ++i) d.qkv_scale[i] = g.qkv_scale[i];
     d.n_split = g.n_split; d.rows_outer = g.out[0].rows_outer; d.n_out = g.out[0].cols;
     const long long tiles = (long long)d.batches * ((g.m_rows + 127) / 128) * ((g.n_rows + bn - 1) / bn);
     return launch_pdl(kern, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(THREADS), smem, st, a[0], a[1], b[0], b[1], o[0], o[1], d, status);

@@ -87,12 +87,12 @@ static int transition(float* x, long long rows, const float* gamma, const float*
 }
 constexpr long long TRANSITION_ROWS = 1 << 17;        // rows whose hidden activations are held at a time
 
-struct SingleWs { __half* x; __nv_bfloat16* qkv; float* gate; long long bytes; };
+struct SingleWs { __half *x, *qkv; float* gate; long long bytes; };
 static SingleWs single_ws(void* ws, int n, int cs) {
     Arena a(ws);
     SingleWs w;
     w.x = a.take<__half>(2LL * n * cs);
-    w.qkv = a.take<__nv_bfloat16>(3LL * n * 3 * cs);
+    w.qkv = a.take<__half>(2LL * n * 3 * cs);
     w.gate = a.take<float>((long long)n * cs);
     w.bytes = a.used;
     return w;
@@ -111,7 +111,7 @@ static TriMulWs trimul_ws(void* ws, int n, int c) {
     w.bytes = a.used;
     return w;
 }
-struct TriAttWs { __half *x, *og; __nv_bfloat16* qkv; float *gate, *bias; long long bytes; };
+struct TriAttWs { __half *x, *og, *qkv; float *gate, *bias; long long bytes; };
 static TriAttWs triatt_ws(void* ws, int n, int c, int heads, int hd) {
     Arena a(ws);
     const long long nn = (long long)n * n;
@@ -119,7 +119,7 @@ static TriAttWs triatt_ws(void* ws, int n, int c, int heads, int hd) {
     TriAttWs w;
     w.x = a.take<__half>(2 * nn * (c > ht ? c : ht));
     w.og = w.x;                                        // x is spent once q, k, v, g exist
-    w.qkv = a.take<__nv_bfloat16>(3 * nn * 3 * ht);
+    w.qkv = a.take<__half>(2 * nn * 3 * ht);
     w.gate = a.take<float>(nn * ht);
     w.bias = a.take<float>(nn * heads);
     w.bytes = a.used;
@@ -157,14 +157,15 @@ int b200pf_single_track_attention(const float* s, const b200pf_single_track_weig
     g.a[0] = matrix(k.x, n, cs);
     g.b[0] = matrix(w->qkvg.w, 4 * cs, cs);
     g.m_rows = n; g.n_rows = 4 * cs; g.k[0] = cs; g.alpha[0] = w->qkvg.alpha; g.bias = w->qkvg_bias; g.n_split = 3 * cs;
-    g.out[0] = dense(k.qkv, n, 3 * cs, 3);
+    g.qkv_scale[0] = w->q_scale; g.qkv_scale[1] = w->k_scale; g.qkv_scale[2] = w->o_scale;
+    g.out[0] = dense(k.qkv, n, 3 * cs, 2);
     g.out[1] = dense(k.gate, n, cs, 1);
     if ((rc = launch_gemm(g, st)) != B200PF_OK) return rc;
     AttnArgs a = {};
     a.qkv = k.qkv; a.part_stride = (long long)n * 3 * cs; a.ld = 3 * cs; a.line_rows = 0; a.pos_rows = 1;
     a.gate = k.gate; a.bias = bias; a.bias_hs = (long long)nq * n; a.bias_qs = n;
     a.mask = mask; a.mask_ls = 0; a.mask_ks = 1; a.mask_add = -1e6f * 1.4426950408889634f;
-    a.out = (__half*)og; a.out_part_stride = (long long)nq * cs; a.out_row0 = q0; a.out_scale = w->o_scale;
+    a.out = (__half*)og; a.out_part_stride = (long long)nq * cs; a.out_row0 = q0; a.qk_scale = w->q_scale * w->k_scale;
     a.lines = 1; a.heads = w->heads; a.q0 = q0; a.n_q = nq; a.n_k = n;
     return launch_attention(a, hd, st);
 }
@@ -252,7 +253,8 @@ int b200pf_split_tri_att(float* z, const uint8_t* mask, const b200pf_split_triat
         g.a[0] = matrix(k.x, nn, c);
         g.b[0] = matrix(w->qkvg.w, 4 * ht, c);
         g.m_rows = (int)nn; g.n_rows = 4 * ht; g.k[0] = c; g.alpha[0] = w->qkvg.alpha; g.n_split = 3 * ht;
-        g.out[0] = dense(k.qkv, nn, 3 * ht, 3);
+        g.qkv_scale[0] = w->q_scale; g.qkv_scale[1] = w->k_scale; g.qkv_scale[2] = w->o_scale;
+        g.out[0] = dense(k.qkv, nn, 3 * ht, 2);
         g.out[1] = dense(k.gate, nn, ht, 1);
         if ((rc = launch_gemm(g, st)) != B200PF_OK) return rc;
     }
@@ -261,7 +263,7 @@ int b200pf_split_tri_att(float* z, const uint8_t* mask, const b200pf_split_triat
     a.line_rows = ending ? 1 : n; a.pos_rows = ending ? n : 1;       // a line is a row of z, or a column
     a.gate = k.gate; a.bias = k.bias; a.bias_hs = nn; a.bias_qs = n;
     a.mask = mask; a.mask_ls = ending ? 1 : n; a.mask_ks = ending ? n : 1; a.mask_add = -1e9f * 1.4426950408889634f;
-    a.out = k.og; a.out_part_stride = nn * ht; a.out_row0 = 0; a.out_scale = w->o_scale;
+    a.out = k.og; a.out_part_stride = nn * ht; a.out_row0 = 0; a.qk_scale = w->q_scale * w->k_scale;
     a.lines = n; a.heads = heads; a.q0 = 0; a.n_q = n; a.n_k = n;
     if ((rc = launch_attention(a, hd, st)) != B200PF_OK) return rc;
     return residual_gemm(z, k.og, w->o, nn, ht, c, nullptr, st);

@@ -81,11 +81,14 @@ SPLIT_WIDTHS = (64, 128, 256)
 _F16_TARGET = 2.0 ** 14             # scaled values stay at or below this, a factor of four inside fp16's range
 
 
-def _pow2_scale(bound: float) -> float:
-    """Largest power of two that keeps ``bound`` at or below the fp16 target."""
+def _pow2_scale(bound: float, most: int = 100) -> float:
+    """Largest power of two (within 2^-most .. 2^most) that keeps ``bound`` at or below the fp16 target."""
     if not (bound > 0.0 and math.isfinite(bound)):
         return 1.0
-    return 2.0 ** max(-100, min(100, math.floor(math.log2(_F16_TARGET / bound))))
+    return 2.0 ** max(-most, min(most, math.floor(math.log2(_F16_TARGET / bound))))
+
+
+QK_MOST = 30        # scores times both scales stay far inside fp32's range; a smaller q or k has no say in a score of order one
 
 
 class SplitPack:
@@ -175,13 +178,15 @@ def pack_split_triatt(sd, pre: str, device):
     g, b = f["layer_norm.weight"], f["layer_norm.bias"]
     qkvg = torch.cat([f["mha.linear_q.weight"] * (LOG2E / math.sqrt(hd)), f["mha.linear_k.weight"], f["mha.linear_v.weight"],
                       f["mha.linear_g.weight"]], 0)
+    norm, ht = _row_norm(g, b), heads * hd
     v = _fetch(ln=_ln_bound(g, b), w=qkvg.abs().max(), o=f["mha.linear_o.weight"].abs().max(),
-               v=_projection_bound(f["mha.linear_v.weight"], _row_norm(g, b)))
+               q=_projection_bound(qkvg[:ht], norm), k=_projection_bound(qkvg[ht:2 * ht], norm), v=_projection_bound(qkvg[2 * ht:3 * ht], norm))
     s_in, o_scale = _pow2_scale(v["ln"]), _pow2_scale(v["v"])       # an attention output is an average of rows of v
     ln = _ln(keep, g, b, s_in)
     keep.append((f["linear.weight"] * (LOG2E / s_in)).contiguous())
     st = SplitTriAttWeights(*ln, keep[-1].data_ptr(), _split_weight(keep, qkvg, v["w"], s_in),
-                            _split_weight(keep, f["mha.linear_o.weight"], v["o"], o_scale), o_scale, c, heads, hd)
+                            _split_weight(keep, f["mha.linear_o.weight"], v["o"], o_scale), o_scale, _pow2_scale(v["q"], QK_MOST),
+                            _pow2_scale(v["k"], QK_MOST), c, heads, hd)
     return SplitPack(st, keep)
 
 
@@ -216,15 +221,17 @@ def pack_single_track(sd, pre: str, num_heads: int, device):
     g, b, cs = n["weight"], n["bias"], n["weight"].numel()
     qs = LOG2E / math.sqrt(cs // num_heads)
     qkvg = torch.cat([a["proj_q.weight"] * qs, a["proj_k.weight"], a["proj_v.weight"], a["proj_g.weight"]], 0)
+    norm = _row_norm(g, b)
     v = _fetch(ln=_ln_bound(g, b), w=qkvg.abs().max(), o=a["proj_o.weight"].abs().max(),
-               v=_projection_bound(a["proj_v.weight"], _row_norm(g, b)), **_swiglu_stats(t))
+               q=_projection_bound(qkvg[:cs], norm) + (a["proj_q.bias"] * qs).abs().max(), k=_projection_bound(qkvg[cs:2 * cs], norm),
+               v=_projection_bound(a["proj_v.weight"], norm), **_swiglu_stats(t))
     s_in, o_scale = _pow2_scale(v["ln"]), _pow2_scale(v["v"])
     ln = _ln(keep, g, b, s_in)
     keep.append(torch.nn.functional.pad(a["proj_q.bias"] * qs, (0, 3 * cs)))
     bias = keep[-1].data_ptr()
     w_qkvg, w_o = _split_weight(keep, qkvg, v["w"], s_in), _split_weight(keep, a["proj_o.weight"], v["o"], o_scale)
     gb2, fc12, fc3, hs = _pack_swiglu(t, keep, v)
-    return SplitPack(SingleTrackWeights(*ln, w_qkvg, bias, w_o, o_scale, *gb2, fc12, hs, fc3, cs, num_heads, t["fc1.weight"].shape[0]), keep)
+    return SplitPack(SingleTrackWeights(*ln, w_qkvg, bias, w_o, o_scale, _pow2_scale(v["q"], QK_MOST), _pow2_scale(v["k"], QK_MOST), *gb2, fc12, hs, fc3, cs, num_heads, t["fc1.weight"].shape[0]), keep)
 
 
 def pack_pair_bias(sd, pre: str, device) -> Dict[str, torch.Tensor]:
