@@ -445,7 +445,7 @@ int b200pf_peer_barrier(const unsigned long long* pad_ptrs, unsigned int generat
 
 /* ------------------------------------------------------------------------------------------
  * fp32-accurate tensor-core path: every fp32 factor is multiplied as a sum of 16-bit parts (two fp16 parts of a scaled
- * value for linear layers and attention, three bf16 parts for the triangle contraction and unbounded inputs), fp32
+ * value, three bf16 parts for inputs of unknown range), fp32
  * accumulation.  Widths that are multiples of 64 (64, 128, 256; 384 without head projections).  It carries the single
  * track of every tier and the pair track of the fp32 tier.
  * ---------------------------------------------------------------------------------------- */
@@ -530,6 +530,7 @@ typedef struct b200pf_split_trimul_weights {
     b200pf_split_weight in;         /* p_in rows, then g_in rows: [4 c][c] */
     const float *ln_out_gamma, *ln_out_beta;
     b200pf_split_weight p_out, g_out;
+    float u_scale;                  /* scale of the gated projections' parts */
     int c;
 } b200pf_split_trimul_weights;
 typedef struct b200pf_split_triatt_weights {

@@ -49,7 +49,7 @@ class SingleTrackWeights(C.Structure):
 class SplitTriMulWeights(C.Structure):
     """Mirror of ``b200pf_split_trimul_weights``."""
     _fields_ = [("ln_in_gamma", _vp), ("ln_in_beta", _vp), ("inp", SplitWeight), ("ln_out_gamma", _vp), ("ln_out_beta", _vp),
-                ("p_out", SplitWeight), ("g_out", SplitWeight), ("c", _i)]
+                ("p_out", SplitWeight), ("g_out", SplitWeight), ("u_scale", _f), ("c", _i)]
 
 
 class SplitTriAttWeights(C.Structure):

@@ -53,7 +53,7 @@ struct Output {
     bool rows_outer;
 };
 
-enum Epilogue { EPI_STORE, EPI_ADD, EPI_SWIGLU, EPI_QKVG, EPI_GATE_PLANES, EPI_GATE_ADD };
+enum Epilogue { EPI_STORE, EPI_ADD, EPI_SWIGLU, EPI_QKVG, EPI_GATE_PLANES, EPI_GATE_ADD, EPI_CONTRACT };
 
 struct Gemm {
     int parts = 2;                  // 2: F16X2, 3: BF16X3
@@ -65,7 +65,7 @@ struct Gemm {
     int k[2] = {0, 0};
     int k_splits = 1;               // > 1: batch index = K split, partial sums stored per batch (EPI_STORE only)
     float alpha[2] = {1.f, 1.f};
-    float out_scale = 1.f;          // EPI_SWIGLU: scale of the stored parts
+    float out_scale = 1.f;          // EPI_SWIGLU, EPI_GATE_PLANES: scale of the stored parts
     const float* bias = nullptr;    // [n_rows]
     const uint8_t* mask = nullptr;  // EPI_GATE_PLANES: position (batch, col) at mask + batch * mask_bs + col * mask_cs
     long long mask_bs = 0, mask_cs = 0;

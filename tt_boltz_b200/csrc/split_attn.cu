@@ -7,10 +7,10 @@
 // A fragments of the second.  A warp owns 16 queries; per 64-key tile it issues 96 MMAs against some 700 other
 // instructions.  With three bf16 parts and six MMAs per product, and every lane fetching its own bias values, a launch took 462 us
 // at 292 tokens x 4 heads and 528 at 256 x 8; with two parts 390 and 430, with staged bias tiles 310 and 311.  Neither the
-// tensor pipe nor memory bounds it now.  K and V tiles are shared by the CTA's
-// warps, double buffered with cp.async; rows are 64 bytes with the 16-byte chunks swizzled by row so that ldmatrix is
-// conflict free.  Bias tiles come with them, as whole lines (read by
-// the lanes that want them, 8 bytes of eight rows at a time and behind the tile before, they were the longest wait of a tile), and are the accumulators' initial values.
+// tensor pipe nor memory bounds it now.  K and V tiles are shared by the CTA's warps, double buffered with cp.async; rows are
+// 64 bytes with the 16-byte chunks swizzled by row so that ldmatrix is
+// conflict free.  Bias tiles come with them, as whole lines (read by the lanes that want them, 8 bytes of eight rows at a
+// time and behind the tile before, they were the longest wait of a tile), and are the accumulators' initial values.
 #include "split_attn.cuh"
 
 namespace b200pf {

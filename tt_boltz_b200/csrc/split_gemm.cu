@@ -48,10 +48,11 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
                   const __grid_constant__ CUtensorMap map_b0, const __grid_constant__ CUtensorMap map_b1,
                   const __grid_constant__ CUtensorMap map_o0, const __grid_constant__ CUtensorMap map_o1, Dev p, unsigned int* status) {
     using namespace sm100;
-    // PL == 3: the leading product and the five small ones have an accumulator each.  The tensor core truncates when it
-    // aligns an addend, so every MMA into a running sum costs up to an ulp of that sum, all in one direction: with 6 K / 16
-    // of them in one accumulator a 300-long contraction was biased by 7e-7; the small products' sums have no ulps to lose.
-    constexpr bool SMALL = PL == 3;
+    // The leading product and the small ones have an accumulator each, for three parts and for the long sums of a contraction.
+    // The tensor core truncates when it aligns an addend, so every MMA into a running sum costs up to an ulp of that sum, all in
+    // one direction: with 6 K / 16 of them in one accumulator a 300-long contraction was biased by 7e-7; the small products'
+    // sums have no ulps to lose.
+    constexpr bool SMALL = PL == 3 || EPI == EPI_CONTRACT;
     constexpr int NACC = SMALL ? 2 : NA * NK, ACC_COLS = NACC * BN, TMEM_COLS = 2 * ACC_COLS;
     constexpr int STAGES = stages_of(PL, BN, NA), A_PART = 128 * 128;
     static_assert(STAGES >= 2 && TMEM_COLS <= 512, "tile too large");
@@ -210,13 +211,6 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
             if (lane == 0) { tma_store_4d(map, s, c0, c1, c2, part); bulk_commit(); }
             slot ^= 1;
         };
-        auto put_bf16x3 = [&](const float (&v)[32], const CUtensorMap* map, int c0, int c1, int c2) {
-            uint32_t w[3][16];
-#pragma unroll
-            for (int e = 0; e < 16; ++e) split_bf16x3(v[2 * e], v[2 * e + 1], w[0][e], w[1][e], w[2][e]);
-#pragma unroll
-            for (int q = 0; q < 3; ++q) put_part(w[q], map, c0, c1, c2, q);
-        };
         for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
             const int bt = (int)(t / (mt * nt)), rem = (int)(t % (mt * nt));
             const int m0 = (rem / nt) * 128 + quarter * 32, n0 = (rem % nt) * bn;
@@ -239,14 +233,14 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
                     if (NACC == 2) tmem_ld_32x32(tb + BN + r * per, y);
                     tmem_ld_wait();
                     float v[32];
-                    if (EPI == EPI_STORE || EPI == EPI_ADD || EPI == EPI_QKVG) {
+                    if (EPI == EPI_STORE || EPI == EPI_CONTRACT || EPI == EPI_ADD || EPI == EPI_QKVG) {
 #pragma unroll
                         for (int e = 0; e < 32; ++e) v[e] = (SMALL ? __uint_as_float(x[e]) + __uint_as_float(y[e]) : __uint_as_float(x[e])) * p.alpha[0];
                         if (p.bias) {
 #pragma unroll
                             for (int e = 0; e < 32; ++e) v[e] += col + e < p.n_rows ? *(p.bias + col + e) : 0.f;
                         }
-                        if (EPI == EPI_STORE) put_f32(v, &map_o0, false, col, m0, bt);
+                        if (EPI == EPI_STORE || EPI == EPI_CONTRACT) put_f32(v, &map_o0, false, col, m0, bt);
                         else if (EPI == EPI_ADD) put_f32(v, &map_o0, true, col, m0, bt);
                         else if (col < p.n_split) {
                             const int third = p.n_split / 3;            // a multiple of 32: one of q, k, v per round
@@ -278,9 +272,13 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
 #pragma unroll
                         for (int e = 0; e < 32; ++e) {
                             const float u = __uint_as_float(x[e]) * p.alpha[0] * sigmoid_precise(__uint_as_float(y[e]) * p.alpha[0]);
-                            v[e] = (bits >> e) & 1u ? u : 0.f;
+                            v[e] = (bits >> e) & 1u ? u * p.out_scale : 0.f;
                         }
-                        put_bf16x3(v, &map_o0, col, bt, m0);
+                        uint32_t w[2][16];
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) split_f16x2(v[2 * e], v[2 * e + 1], w[0][e], w[1][e]);
+                        put_part(w[0], &map_o0, col, bt, m0, 0);
+                        put_part(w[1], &map_o0, col, bt, m0, 1);
                     } else {
 #pragma unroll
                         for (int e = 0; e < 32; ++e)
@@ -388,6 +386,7 @@ int launch_gemm(const Gemm& g, cudaStream_t st) {
             if (bn > 128) SG(2, 256, 1, 1, EPI_STORE);
             SG(2, 128, 1, 1, EPI_STORE);
         }
+        case EPI_CONTRACT: { const int bn = pick_bn(row_tiles, g.n_rows, 128, 32, sms); SG(2, 128, 1, 1, EPI_CONTRACT); }
         case EPI_ADD: {
             if (g.parts == 3) { const int bn = pick_bn(row_tiles, g.n_rows, 128, 32, sms); SG(3, 128, 1, 1, EPI_ADD); }
             const int bn = pick_bn(row_tiles, g.n_rows, 256, 32, sms);

@@ -98,15 +98,15 @@ static SingleWs single_ws(void* ws, int n, int cs) {
     return w;
 }
 
-struct TriMulWs { __half *x, *tn; __nv_bfloat16* ab; float* t; int pitch, tpitch; long long bytes; };
+struct TriMulWs { __half *x, *tn, *ab; float* t; int pitch, tpitch; long long bytes; };
 static TriMulWs trimul_ws(void* ws, int n, int c) {
     Arena a(ws);
     TriMulWs w;
     w.pitch = round_up(n, 8);
     w.tpitch = round_up(n, 4);
     w.x = a.take<__half>(2LL * n * n * c);
-    w.ab = a.take<__nv_bfloat16>(3LL * 2 * c * n * w.pitch);
-    w.tn = reinterpret_cast<__half*>(w.ab);            // the operands are spent when the normalised product is written
+    w.ab = a.take<__half>(2LL * 2 * c * n * w.pitch);
+    w.tn = w.ab;                                       // the operands are spent when the normalised product is written
     w.t = a.take<float>((long long)c * n * w.tpitch);
     w.bytes = a.used;
     return w;
@@ -209,12 +209,14 @@ int b200pf_split_tri_mul(float* z, const uint8_t* mask, const b200pf_split_trimu
         g.b_batched = true;
         g.m_rows = 2 * c; g.n_rows = n; g.batches = n; g.k[0] = c; g.alpha[0] = w->in.alpha;
         g.mask = mask; g.mask_bs = incoming ? 1 : n; g.mask_cs = incoming ? n : 1;
-        g.out[0] = Output{k.ab, 2 * c, n, n, 3, (long long)n * k.pitch, k.pitch, 2LL * c * n * k.pitch, true};
+        g.out_scale = w->u_scale;
+        g.out[0] = Output{k.ab, 2 * c, n, n, 2, (long long)n * k.pitch, k.pitch, 2LL * c * n * k.pitch, true};
         if ((rc = launch_gemm(g, st)) != B200PF_OK) return rc;
     }
     {   // t[channel][i][j] = sum_k a[channel][i][k] b[channel][j][k]
         Gemm g;
-        g.parts = 3;
+        g.epi = EPI_CONTRACT;
+        g.alpha[0] = 1.f / (w->u_scale * w->u_scale);
         g.a[0] = Operand{k.ab, n, n, c, k.pitch, (long long)n * k.pitch, 2LL * c * n * k.pitch};
         g.b[0] = Operand{k.ab + (long long)c * n * k.pitch, n, n, c, k.pitch, (long long)n * k.pitch, 2LL * c * n * k.pitch};
         g.a_batched = g.b_batched = true;

@@ -22,12 +22,13 @@ checkpoint slice works unchanged (tt_bio/tenstorrent.py:2179-2180 does the same 
 Inference only (eval-mode semantics: dropout masks are 1).  Inputs must be CUDA tensors; there
 is no CPU path.  The fused kernels are built for c_z = 128 with 4 x 32 triangle-attention heads (Boltz-2's trunk, MSA
 and confidence stacks); other widths (the template stack's c_z = 64, the c_z = 256 / 8-head trunks of sibling models)
-run on the un-fused fp32 kernels, which take any width: pass ``precision="fp32"`` or ``"auto"``.
+run in the fp32 tier, on part planes where their kernels fit and on the un-fused fp32 kernels at any other width: pass
+``precision="fp32"`` or ``"auto"``.
 ``precision``: "bf16" (fused tensor-core kernels, fp32 residual stream),
 "mxfp8" (as bf16, but the triangle-multiplication operands a / b are MXFP8: e4m3 values with one
 e8m0 scale per 32 elements along the contraction index, contracted by the block-scaled tensor-core
 instruction - the counterpart of the reference's block-fp8 fast mode, tt_bio/tenstorrent.py:178-181)
-or "fp32" (un-fused fp32 kernels, the validation tier).
+or "fp32" (fp32-accurate kernels, the validation tier).
 """
 from __future__ import annotations
 

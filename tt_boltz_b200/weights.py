@@ -88,7 +88,7 @@ def _pow2_scale(bound: float, most: int = 100) -> float:
     return 2.0 ** max(-most, min(most, math.floor(math.log2(_F16_TARGET / bound))))
 
 
-QK_MOST = 30        # scores times both scales stay far inside fp32's range; a smaller q or k has no say in a score of order one
+QK_MOST = 30        # of a factor whose products stay scaled in the accumulator: times both scales they stay far inside fp32's range
 
 
 class SplitPack:
@@ -162,11 +162,11 @@ def pack_split_trimul(sd, pre: str, device):
     w_in = torch.cat([f["p_in.weight"], f["g_in.weight"]], 0)
     gi, bi, go, bo = f["norm_in.weight"], f["norm_in.bias"], f["norm_out.weight"], f["norm_out.bias"]
     v = _fetch(ln_in=_ln_bound(gi, bi), ln_out=_ln_bound(go, bo), w_in=w_in.abs().max(), p=f["p_out.weight"].abs().max(),
-               g=f["g_out.weight"].abs().max())
+               g=f["g_out.weight"].abs().max(), u=_projection_bound(f["p_in.weight"], _row_norm(gi, bi)))
     s_in, s_out = _pow2_scale(v["ln_in"]), _pow2_scale(v["ln_out"])
     st = SplitTriMulWeights(*_ln(keep, gi, bi, s_in), _split_weight(keep, w_in, v["w_in"], s_in), *_ln(keep, go, bo, s_out),
                             _split_weight(keep, f["p_out.weight"], v["p"], s_out), _split_weight(keep, f["g_out.weight"], v["g"], s_in),
-                            gi.numel())
+                            _pow2_scale(v["u"], QK_MOST), gi.numel())
     return SplitPack(st, keep)
 
 
