@@ -33,6 +33,14 @@ constexpr int BP = KT + 8;               // bias tile pitch in floats: a half-wa
 constexpr int bias_stage(int nw) { return nw * 16 * BP * 4; }
 constexpr float P_SCALE = 16384.f;      // probabilities are at most one: their parts use the upper half of fp16's range
 
+// 2^x of a score below the row's maximum.  exp2f is this instruction with a range step around it that keeps results below 2^-126;
+// a row's largest probability is 1, so those have no bit to add to its sums.
+__device__ __forceinline__ float prob(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 template <int HD, int NW>
 __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnArgs p) {
     constexpr int CH = HD / 8, NE = HD / 8, NT = NW * 32;
@@ -173,7 +181,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     float* sv = s[2 * j + u];
-                    sv[0] = exp2f(sv[0] - n0); sv[1] = exp2f(sv[1] - n0); sv[2] = exp2f(sv[2] - n1); sv[3] = exp2f(sv[3] - n1);
+                    sv[0] = prob(sv[0] - n0); sv[1] = prob(sv[1] - n0); sv[2] = prob(sv[2] - n1); sv[3] = prob(sv[3] - n1);
                     l0 += sv[0] + sv[1]; l1 += sv[2] + sv[3];
                     split_f16x2(sv[0] * P_SCALE, sv[1] * P_SCALE, pf[0][2 * u], pf[1][2 * u]);
                     split_f16x2(sv[2] * P_SCALE, sv[3] * P_SCALE, pf[0][2 * u + 1], pf[1][2 * u + 1]);
