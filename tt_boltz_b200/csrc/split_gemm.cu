@@ -182,10 +182,11 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
         const int quarter = warp & 3, chalf = (warp - 2) >> 2;
         uint8_t* stg = stg_base + (warp - 2) * STG_BYTES;
         uint32_t it = 0, slot = 0;
-        bool ok = true;
+        bool ok = true, whole = false;      // whole: the last store was of all 4096 staging bytes
         // 32 rows x 32 fp32 values, 128-byte swizzle
         auto put_f32 = [&](const float (&v)[32], const CUtensorMap* map, bool add, int c0, int c1, int c2) {
             if (lane == 0) bulk_wait_read0();
+            whole = true;
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < 8; ++j)
@@ -198,9 +199,14 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
                 bulk_commit();
             }
         };
-        // 32 rows x 32 16-bit values of one part, 64-byte swizzle, two slots in turn
+        // 32 rows x 32 16-bit values of one part, 64-byte swizzle, two slots in turn: the store before may still read the other
+        // slot, unless it was put_f32's, which reads both (a gate tile whose CTA's next tile holds q, k or v)
         auto put_part = [&](const uint32_t (&w)[16], const CUtensorMap* map, int c0, int c1, int c2, int part) {
-            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            if (lane == 0) {
+                if (whole) bulk_wait_read0();
+                else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            }
+            whole = false;
             __syncwarp();
             uint8_t* s = stg + slot * 2048;
 #pragma unroll
