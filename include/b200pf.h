@@ -554,8 +554,10 @@ long long b200pf_split_pair_workspace(int n, int c, int heads, int hd, int hidde
 int b200pf_split_tri_mul(float* z, const uint8_t* mask, const b200pf_split_trimul_weights* w, int n, int incoming, void* workspace, void* stream);
 /* z += TriangleAttention(z) (tt_bio/reference.py:326-363); mask [n][n]. */
 int b200pf_split_tri_att(float* z, const uint8_t* mask, const b200pf_split_triatt_weights* w, int n, int ending, void* workspace, void* stream);
-/* x[rows] += Transition(x) (tt_bio/boltz2.py:1241-1246). */
-int b200pf_split_transition(float* x, long long rows, const b200pf_split_transition_weights* w, void* workspace, void* stream);
+/* x[rows] += Transition(x) (tt_bio/boltz2.py:1241-1246).  A workspace smaller than what its rows need is refused; one for more rows
+ * serves fewer. */
+long long b200pf_split_transition_workspace(long long rows, int c, int hidden);
+int b200pf_split_transition(float* x, long long rows, const b200pf_split_transition_weights* w, void* workspace, long long workspace_bytes, void* stream);
 
 /* out[h * head_stride + row] = <LN(x[row]), w[h]> in fp32, 4, 8 or 16 heads (tt_bio/boltz2.py:326-330). */
 int b200pf_ln_heads(const float* x, const float* gamma, const float* beta, const float* w, float* out, long long head_stride, long long rows,

@@ -59,13 +59,16 @@ static int residual_gemm(float* y, const void* planes, const b200pf_split_weight
 }
 
 // x += fc3(silu(fc1 LN x) * fc2 LN x)
+// Up to PARTIAL_ROWS rows may take partial sums.  Their room is in every workspace, so that one for more rows serves fewer.
+constexpr long long PARTIAL_ROWS = 2048;
 struct TransWs { __half *x, *h; float* partial; long long bytes; };
 static TransWs transition_ws(void* ws, long long rows, int c, int hidden) {
     Arena a(ws);
     TransWs w;
     w.x = a.take<__half>(2 * rows * c);
     w.h = a.take<__half>(2 * rows * hidden);
-    w.partial = rows <= 2048 ? a.take<float>(8 * rows * c) : nullptr;
+    float* partial = a.take<float>(8 * (rows < PARTIAL_ROWS ? rows : PARTIAL_ROWS) * c);
+    w.partial = rows <= PARTIAL_ROWS ? partial : nullptr;
     w.bytes = a.used;
     return w;
 }
@@ -271,10 +274,16 @@ int b200pf_split_tri_att(float* z, const uint8_t* mask, const b200pf_split_triat
     return residual_gemm(z, k.og, w->o, nn, ht, c, nullptr, st);
 }
 
-int b200pf_split_transition(float* x, long long rows, const b200pf_split_transition_weights* w, void* workspace, void* stream) {
+long long b200pf_split_transition_workspace(long long rows, int c, int hidden) {
+    return transition_ws(nullptr, rows < TRANSITION_ROWS ? rows : TRANSITION_ROWS, c, hidden).bytes;
+}
+
+int b200pf_split_transition(float* x, long long rows, const b200pf_split_transition_weights* w, void* workspace, long long workspace_bytes, void* stream) {
     B200PF_REQUIRE(x && w && workspace && aligned16(x) && aligned16(workspace) && rows > 0, B200PF_ERR_INVALID,
                    "split_transition: null or misaligned pointer");
     B200PF_REQUIRE(w->c % 64 == 0 && ln_supported(w->c) && w->hidden % 64 == 0, B200PF_ERR_UNSUPPORTED, "split_transition: %d -> %d is not built", w->c, w->hidden);
+    B200PF_REQUIRE(workspace_bytes >= b200pf_split_transition_workspace(rows, w->c, w->hidden), B200PF_ERR_INVALID,
+                   "split_transition: %lld bytes of workspace are too few for %lld rows", workspace_bytes, rows);
     for (long long r = 0; r < rows; r += TRANSITION_ROWS) {
         const long long m = rows - r < TRANSITION_ROWS ? rows - r : TRANSITION_ROWS;
         const int rc = transition(x + r * w->c, m, w->ln_gamma, w->ln_beta, w->fc12, w->hidden_scale, w->fc3, w->c, w->hidden, workspace, (cudaStream_t)stream);

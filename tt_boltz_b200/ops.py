@@ -291,10 +291,9 @@ def tri_att_split(z: torch.Tensor, mask_u8: torch.Tensor, pack, ending: bool, sc
 
 
 def transition_split(x: torch.Tensor, pack, scratch: Scratch) -> None:
-    w = pack.struct
-    n = math.isqrt(x.numel() // w.c - 1) + 1 if x.numel() > w.c else 1          # workspace of a square tensor at least as large
-    ws = scratch.get(_nbytes("b200pf_split_pair_workspace", n, w.c, 0, 0, w.hidden))
-    call("b200pf_split_transition", ptr(x), x.numel() // w.c, C.byref(w), ws, stream())
+    w, rows = pack.struct, x.numel() // pack.struct.c
+    nbytes = _nbytes("b200pf_split_transition_workspace", rows, w.c, w.hidden)
+    call("b200pf_split_transition", ptr(x), rows, C.byref(w), scratch.get(nbytes), nbytes, stream())
 
 
 def split_linear(x: torch.Tensor, w_parts: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, accumulate: bool, scratch: Scratch) -> None:
