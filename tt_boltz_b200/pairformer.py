@@ -135,6 +135,9 @@ class B200PairformerLayer(nn.Module):
     def reset_static_cache(self) -> None:
         self._packed = None
 
+    def __getstate__(self):             # a copy packs its own weights: a pack's C structures point into its tensors
+        return {**self.__dict__, "_packed": None}
+
     def _pack(self, device) -> Dict[str, Dict[str, torch.Tensor]]:
         if self._packed is not None and self._packed["_device"] == device:
             return self._packed
@@ -243,6 +246,9 @@ class B200PairUpdateBlock(nn.Module):
             _register_tree(self, f"transition_z.{leaf}", shape)
         self._packed = None
         self.register_load_state_dict_post_hook(lambda module, incompatible: setattr(module, "_packed", None))
+
+    def __getstate__(self):             # as in the layer
+        return {**self.__dict__, "_packed": None}
 
     def _pack(self, device):
         if self._packed is None or self._packed["_device"] != device:
