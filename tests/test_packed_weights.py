@@ -1,4 +1,5 @@
-"""What a module keeps of its weights between calls: copies of a module pack their own."""
+"""What a module keeps of its weights between calls: copies of a module pack their own, and the fp32 tier sees weights that are changed
+in place, as it does on the un-fused kernels, which read the parameters themselves."""
 import copy
 
 import pytest
@@ -30,6 +31,33 @@ def test_a_used_module_can_be_copied(i):
     assert module._packed is pack and twin._packed is None
     for (name, a), (_, b) in zip(module.named_parameters(), twin.named_parameters()):
         assert torch.equal(a, b) and a.data_ptr() != b.data_ptr(), name
+
+
+@pytest.mark.parametrize("i", [0, 1])
+def test_weights_changed_in_place_are_packed_anew(i):
+    module = _fill(_modules()[i])
+    pack = module._pack(CPU)
+    assert module._pack(CPU) is pack
+    with torch.no_grad():
+        next(p for name, p in module.named_parameters() if name == "transition_z.fc3.weight").mul_(3.0)
+    new = module._pack(CPU)
+    assert new is not pack and module._pack(CPU) is new
+    module.reset_static_cache()                          # for changes through .data
+    assert module._pack(CPU) is not new
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("c", [64, 96])                  # on part planes, on the un-fused kernels
+def test_the_fp32_tier_computes_with_weights_changed_in_place(c):
+    z = torch.randn(1, 21, 21, c, generator=torch.Generator().manual_seed(1)).cuda()
+    module = _fill(B200PairUpdateBlock(c, 128)).cuda()
+    module(z)
+    with torch.no_grad():
+        for p in module.parameters():
+            p.mul_(0.5)
+    other = B200PairUpdateBlock(c, 128)
+    other.load_state_dict(module.state_dict())
+    assert torch.equal(module(z), other.cuda()(z))
 
 
 @pytest.mark.gpu

@@ -133,16 +133,18 @@ class B200PairformerLayer(nn.Module):
 
     # same name as the reference backend's cache reset (tt_bio/tenstorrent.py:2185-2191)
     def reset_static_cache(self) -> None:
+        """Packs the weights anew at the next call.  ``load_state_dict`` does so by itself, and in the fp32 tier any change in place
+        that torch counts; a change through ``.data`` needs this call, and in the fused tiers every change does."""
         self._packed = None
 
     def __getstate__(self):             # a copy packs its own weights: a pack's C structures point into its tensors
         return {**self.__dict__, "_packed": None}
 
     def _pack(self, device) -> Dict[str, Dict[str, torch.Tensor]]:
-        if self._packed is not None and self._packed["_device"] == device:
+        if self._packed is not None and self._packed["_device"] == device and (self.fused or not self._packed["_versions"].changed()):
             return self._packed
         sd = {k: v for k, v in self.state_dict().items()}
-        pk: Dict[str, Dict[str, torch.Tensor]] = {"_device": device}
+        pk: Dict[str, Dict[str, torch.Tensor]] = {"_device": device, "_versions": weights.Versions(sd.values())}
         if self.fused:
             pack_mul, pack_att, pack_trans = weights.pack_trimul, weights.pack_triatt, weights.pack_transition_z
         elif self.split:
@@ -245,20 +247,25 @@ class B200PairUpdateBlock(nn.Module):
                             ("fc2.weight", (hidden, token_z)), ("fc3.weight", (token_z, hidden))):
             _register_tree(self, f"transition_z.{leaf}", shape)
         self._packed = None
-        self.register_load_state_dict_post_hook(lambda module, incompatible: setattr(module, "_packed", None))
+        self.register_load_state_dict_post_hook(lambda module, incompatible: module.reset_static_cache())
+
+    def reset_static_cache(self) -> None:
+        """As in the layer's fp32 tier: only a change through ``.data`` needs it."""
+        self._packed = None
 
     def __getstate__(self):             # as in the layer
         return {**self.__dict__, "_packed": None}
 
     def _pack(self, device):
-        if self._packed is None or self._packed["_device"] != device:
+        if self._packed is None or self._packed["_device"] != device or self._packed["_versions"].changed():
             sd = dict(self.state_dict().items())
-            self._packed = {"_device": device}
+            pk = {"_device": device, "_versions": weights.Versions(sd.values())}
             pack_mul, pack_trans = ((weights.pack_split_trimul, weights.pack_split_transition) if self.split
                                     else (weights.to_device_f32, weights.to_device_f32))
             for name in ("tri_mul_out", "tri_mul_in"):
-                self._packed[name] = pack_mul(sd, name + ".", device)
-            self._packed["transition_z"] = pack_trans(sd, "transition_z.", device)
+                pk[name] = pack_mul(sd, name + ".", device)
+            pk["transition_z"] = pack_trans(sd, "transition_z.", device)
+            self._packed = pk
         return self._packed
 
     def forward_inplace(self, z: torch.Tensor, pair_mask_u8: torch.Tensor) -> None:

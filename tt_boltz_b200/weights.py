@@ -91,6 +91,18 @@ def _pow2_scale(bound: float, most: int = 100) -> float:
 QK_MOST = 30        # of a factor whose products stay scaled in the accumulator: times both scales they stay far inside fp32's range
 
 
+class Versions:
+    """Tells whether any of the tensors was changed in place (by an operation that counts versions: one through ``.data`` does not,
+    nor do inference tensors)."""
+
+    def __init__(self, tensors) -> None:
+        self.tensors = [t for t in tensors if not t.is_inference()]
+        self.seen = [t._version for t in self.tensors]
+
+    def changed(self) -> bool:
+        return [t._version for t in self.tensors] != self.seen
+
+
 class SplitPack:
     """Device tensors of one packed layer and the C structure that points at them."""
 
