@@ -72,3 +72,25 @@ def test_a_copy_of_a_used_module_gives_its_results(precision):
     del module
     got = twin(s, z)
     assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["bf16", "fp32"])
+def test_a_pack_is_there_for_calls_on_other_streams(precision):
+    """The first call, which packs, stands behind 50 ms of other work on its stream; a second one on another stream gives its result."""
+    from tt_boltz_b200 import B200PairformerNoSeqModule, synthetic
+    module = B200PairformerNoSeqModule(128, 2, precision=precision)
+    module.load_state_dict(synthetic.make_weights(2, seed=3, std=0.05, affine_jitter=0.2, with_s=False), strict=True)
+    module = module.cuda()
+    z = synthetic.make_inputs(33, seed=1, with_s=False)[1].cuda()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(a):
+        torch.cuda._sleep(100_000_000)
+        first = module(z)
+    twin = copy.copy(module)                                 # shares the packed weights,
+    twin._ws_cache = {}                                      # but not the workspace
+    with torch.cuda.stream(b):
+        second = twin(z)
+    torch.cuda.synchronize()
+    assert torch.equal(first, second)

@@ -21,6 +21,7 @@ from typing import Optional
 import torch
 from torch import nn
 
+from . import weights
 from ._lib import Planes, call, ptr, stream
 
 C_M, C_HID, C_OUT = 64, 32, 128
@@ -62,15 +63,18 @@ class B200OuterProductMean(nn.Module):
 
     def _pack(self, device):
         if self._packed is None or self._packed["w_ab"].device != device:
+            old = self._packed and self._packed["w_ab"].device
             with torch.no_grad():
                 f32 = dict(device=device, dtype=torch.float32)
-                self._packed = {
+                packed = {
                     "gamma": self.norm.weight.detach().to(**f32).contiguous(),
                     "beta": self.norm.bias.detach().to(**f32).contiguous(),
                     "w_ab": torch.cat([self.proj_a.weight, self.proj_b.weight], 0).detach().to(**f32).contiguous(),
                     "w_o": self.proj_o.weight.detach().to(device=device, dtype=torch.bfloat16).contiguous(),
                     "bias": self.proj_o.bias.detach().to(**f32).contiguous(),
                 }
+            weights.settle(device, old)
+            self._packed = packed
         return self._packed
 
     # -- compute -------------------------------------------------------------------------------------
@@ -181,9 +185,10 @@ class B200PairWeightedAveraging(nn.Module):
 
     def _pack(self, device):
         if self._packed is None or self._packed["w_m"].device != device:
+            old = self._packed and self._packed["w_m"].device
             with torch.no_grad():
                 f32 = dict(device=device, dtype=torch.float32)
-                self._packed = {
+                packed = {
                     "gm": self.norm_m.weight.detach().to(**f32).contiguous(), "bm": self.norm_m.bias.detach().to(**f32).contiguous(),
                     "gz": self.norm_z.weight.detach().to(**f32).contiguous(), "bz": self.norm_z.bias.detach().to(**f32).contiguous(),
                     "w_m": self.proj_m.weight.detach().to(device=device, dtype=torch.bfloat16).contiguous(),
@@ -192,6 +197,8 @@ class B200PairWeightedAveraging(nn.Module):
                     "w_z": torch.cat([self.proj_z.weight.detach().to(**f32), torch.zeros(8, self.c_z, **f32)], 0).contiguous(),
                     "w_o": self.proj_o.weight.detach().to(device=device, dtype=torch.bfloat16).contiguous(),
                 }
+            weights.settle(device, old)
+            self._packed = packed
         return self._packed
 
     def _run(self, m: torch.Tensor, z: torch.Tensor, mask_u8: torch.Tensor) -> None:
@@ -262,15 +269,18 @@ class B200MSATransition(nn.Module):
 
     def _pack(self, device):
         if self._packed is None or self._packed["w12"].device != device:
+            old = self._packed and self._packed["w12"].device
             with torch.no_grad():
                 bf = dict(device=device, dtype=torch.bfloat16)
-                self._packed = {
+                packed = {
                     "g": self.norm.weight.detach().to(device=device, dtype=torch.float32).contiguous(),
                     "b": self.norm.bias.detach().to(device=device, dtype=torch.float32).contiguous(),
                     # 64 rows of fc1, the 64 of fc2 they are multiplied with, in turn
                     "w12": torch.stack([self.fc1.weight.view(4, 64, C_M), self.fc2.weight.view(4, 64, C_M)], 1).detach().to(**bf).contiguous(),
                     "w3": self.fc3.weight.detach().to(**bf).contiguous(),
                 }
+            weights.settle(device, old)
+            self._packed = packed
         return self._packed
 
     def _run(self, m: torch.Tensor) -> None:

@@ -160,6 +160,7 @@ class B200PairformerLayer(nn.Module):
             pk["pair"] = ops.PairBlock(pk)
         if self.with_s:
             pk["single"] = ops.pack_single_track(sd, "", self.num_heads, device)
+        weights.settle(device, self._packed and self._packed["_device"])
         self._packed = pk
         return pk
 
@@ -265,6 +266,7 @@ class B200PairUpdateBlock(nn.Module):
             for name in ("tri_mul_out", "tri_mul_in"):
                 pk[name] = pack_mul(sd, name + ".", device)
             pk["transition_z"] = pack_trans(sd, "transition_z.", device)
+            weights.settle(device, self._packed and self._packed["_device"])
             self._packed = pk
         return self._packed
 

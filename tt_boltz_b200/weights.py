@@ -103,6 +103,16 @@ class Versions:
         return [t._version for t in self.tensors] != self.seen
 
 
+def settle(device: torch.device, replaced) -> None:
+    """Waits for a pack that the current stream is making, so that a later call may read it on any stream.  ``replaced`` is the device
+    of a pack that is dropped for it (or None): kernels of any stream may still read that one, so they are waited for too.  A stream
+    that is being captured can't be waited for; its pack is the graph's own."""
+    if device.type == "cuda" and not torch.cuda.is_current_stream_capturing():
+        torch.cuda.current_stream(device).synchronize()
+        if replaced is not None and replaced.type == "cuda":
+            torch.cuda.synchronize(replaced)
+
+
 class SplitPack:
     """Device tensors of one packed layer and the C structure that points at them."""
 
