@@ -73,6 +73,7 @@ class SideTrack:
     def __init__(self, device: torch.device) -> None:
         self.stream = torch.cuda.Stream(device)
         self.bias_read: Optional[torch.cuda.Event] = None
+        self.used = False                           # (a capture can't wait for a stream that it has no part in)
         self.blocks, self.bias, self.held = 0, [None, None], []
         self.ready, self.done = ([torch.cuda.Event(), torch.cuda.Event()] for _ in range(2))
         self.scratch = ops.Scratch(device)          # from the pair stream's memory, given back to it after ``join``
@@ -80,6 +81,7 @@ class SideTrack:
     def enqueue(self, track, s: torch.Tensor, z: torch.Tensor, tok_mask_u8: Optional[torch.Tensor]) -> None:
         i, first = self.blocks & 1, self.blocks < 2
         self.blocks += 1
+        self.used = True
         if first:                                   # (an event exists from its first recording on)
             self.bias[i] = torch.empty(track.bias_struct.heads, s.shape[0] ** 2, dtype=torch.float32, device=z.device)
             self.ready[i].record()
@@ -89,6 +91,11 @@ class SideTrack:
         track.beside(s, z, self.bias[i], tok_mask_u8, self.scratch, self.stream.cuda_stream, self.ready[i].cuda_event, self.done[i].cuda_event, not first)
         if buf is not None and self.scratch.buf is not buf:
             self.held.append(buf)                   # outgrown, but its kernels may still run
+
+    def follow(self, event: torch.cuda.Event) -> None:
+        """What is put on this stream from here on comes behind ``event``."""
+        self.used = True
+        self.stream.wait_event(event)
 
     def mark_z_read(self) -> None:
         self.bias_read = torch.cuda.Event()
@@ -100,8 +107,9 @@ class SideTrack:
             self.bias_read = None
 
     def join(self) -> None:
-        torch.cuda.current_stream().wait_stream(self.stream)
-        self.bias_read = None
+        if self.used:
+            torch.cuda.current_stream().wait_stream(self.stream)
+        self.used, self.bias_read = False, None
 
 
 class B200PairformerLayer(nn.Module):

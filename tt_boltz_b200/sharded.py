@@ -386,7 +386,7 @@ def sharded_block(layer: B200PairformerLayer, s: Optional[torch.Tensor], z_loc: 
             z_ready = torch.cuda.Event()
             z_ready.record()
             with torch.cuda.stream(side.stream):
-                side.stream.wait_event(z_ready)
+                side.follow(z_ready)
                 single_track(1)
     return z_loc
 
