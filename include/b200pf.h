@@ -42,6 +42,10 @@ long long   b200pf_launch_count(void);
  * Synchronises `stream`.  0 = clean; bit 1 = an mbarrier wait inside a kernel ran out, bit 2 = an index
  * check failed, bit 4 = a cross-rank barrier gave up waiting for a peer. */
 int         b200pf_device_status(void* stream);
+/* Exchanges the calling thread's stream capture mode (0 global, 1 thread local, 2 relaxed) for *mode, as
+ * cudaThreadExchangeStreamCaptureMode does: work on a stream of its own, such as packing weights, is then allowed while another
+ * stream of the thread is being captured. */
+int         b200pf_exchange_capture_mode(int* mode);
 
 /* ------------------------------------------------------------------------------------------
  * fp32 validation tier: un-fused SIMT kernels, arithmetic in fp32 throughout.

@@ -6,6 +6,7 @@ library's own message.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import os
 from typing import Optional
@@ -100,6 +101,7 @@ SIGNATURES = {
     "b200pf_last_error": [],
     "b200pf_launch_count": [],
     "b200pf_device_status": [_vp],
+    "b200pf_exchange_capture_mode": [C.POINTER(_i)],
     "b200pf_f32_layernorm": [_vp, _vp, _vp, _vp, _ll, _i, _vp],
     "b200pf_f32_linear": [_vp, _vp, _vp, _vp, _ll, _i, _i, _i, _vp],
     "b200pf_f32_gate": [_vp, _vp, _vp, _vp, _ll, _i, _i, _vp],
@@ -242,6 +244,17 @@ def call(name: str, *args) -> None:
     if t is not None:
         b.record()
         t.events.append((name, a, b))
+
+
+@contextlib.contextmanager
+def relaxed_capture():
+    """Lets this thread work on other streams while one of its streams is being captured."""
+    mode = _i(2)
+    call("b200pf_exchange_capture_mode", C.byref(mode))
+    try:
+        yield
+    finally:
+        call("b200pf_exchange_capture_mode", C.byref(mode))
 
 
 def launch_count() -> int:

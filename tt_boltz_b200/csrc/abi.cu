@@ -47,6 +47,14 @@ const char* b200pf_last_error(void) { return b200pf::g_err; }
 
 long long b200pf_launch_count(void) { return b200pf::g_launches.load(); }
 
+int b200pf_exchange_capture_mode(int* mode) {
+    B200PF_REQUIRE(mode && *mode >= 0 && *mode <= 2, B200PF_ERR_INVALID, "exchange_capture_mode: bad argument");
+    cudaStreamCaptureMode m = static_cast<cudaStreamCaptureMode>(*mode);
+    B200PF_CUDA(cudaThreadExchangeStreamCaptureMode(&m));
+    *mode = static_cast<int>(m);
+    return B200PF_OK;
+}
+
 int b200pf_device_status(void* stream) {
     unsigned int* p = b200pf::device_status_word();
     B200PF_REQUIRE(p != nullptr, B200PF_ERR_CUDA, "no device status word (no CUDA device?)");

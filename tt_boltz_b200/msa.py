@@ -63,8 +63,7 @@ class B200OuterProductMean(nn.Module):
 
     def _pack(self, device):
         if self._packed is None or self._packed["w_ab"].device != device:
-            old = self._packed and self._packed["w_ab"].device
-            with torch.no_grad():
+            with torch.no_grad(), weights.packing(device, self._packed and self._packed["w_ab"].device):
                 f32 = dict(device=device, dtype=torch.float32)
                 packed = {
                     "gamma": self.norm.weight.detach().to(**f32).contiguous(),
@@ -73,7 +72,6 @@ class B200OuterProductMean(nn.Module):
                     "w_o": self.proj_o.weight.detach().to(device=device, dtype=torch.bfloat16).contiguous(),
                     "bias": self.proj_o.bias.detach().to(**f32).contiguous(),
                 }
-            weights.settle(device, old)
             self._packed = packed
         return self._packed
 
@@ -185,8 +183,7 @@ class B200PairWeightedAveraging(nn.Module):
 
     def _pack(self, device):
         if self._packed is None or self._packed["w_m"].device != device:
-            old = self._packed and self._packed["w_m"].device
-            with torch.no_grad():
+            with torch.no_grad(), weights.packing(device, self._packed and self._packed["w_m"].device):
                 f32 = dict(device=device, dtype=torch.float32)
                 packed = {
                     "gm": self.norm_m.weight.detach().to(**f32).contiguous(), "bm": self.norm_m.bias.detach().to(**f32).contiguous(),
@@ -197,7 +194,6 @@ class B200PairWeightedAveraging(nn.Module):
                     "w_z": torch.cat([self.proj_z.weight.detach().to(**f32), torch.zeros(8, self.c_z, **f32)], 0).contiguous(),
                     "w_o": self.proj_o.weight.detach().to(device=device, dtype=torch.bfloat16).contiguous(),
                 }
-            weights.settle(device, old)
             self._packed = packed
         return self._packed
 
@@ -269,8 +265,7 @@ class B200MSATransition(nn.Module):
 
     def _pack(self, device):
         if self._packed is None or self._packed["w12"].device != device:
-            old = self._packed and self._packed["w12"].device
-            with torch.no_grad():
+            with torch.no_grad(), weights.packing(device, self._packed and self._packed["w12"].device):
                 bf = dict(device=device, dtype=torch.bfloat16)
                 packed = {
                     "g": self.norm.weight.detach().to(device=device, dtype=torch.float32).contiguous(),
@@ -279,7 +274,6 @@ class B200MSATransition(nn.Module):
                     "w12": torch.stack([self.fc1.weight.view(4, 64, C_M), self.fc2.weight.view(4, 64, C_M)], 1).detach().to(**bf).contiguous(),
                     "w3": self.fc3.weight.detach().to(**bf).contiguous(),
                 }
-            weights.settle(device, old)
             self._packed = packed
         return self._packed
 

@@ -112,7 +112,45 @@ class SideTrack:
         self.used, self.bias_read = False, None
 
 
-class B200PairformerLayer(nn.Module):
+class _PackedModule(nn.Module):
+    """Weights packed at the first call on a device, and again after ``load_state_dict``, ``reset_static_cache`` or, in the fp32 tier,
+    a change in place."""
+
+    fused = False
+
+    def __init__(self) -> None:
+        super().__init__()
+        self._packed: Optional[Dict[str, Dict[str, torch.Tensor]]] = None
+        self._captured: list = []           # packs that a captured graph reads
+        self.register_load_state_dict_post_hook(lambda module, incompatible: module.reset_static_cache())
+
+    # same name as the reference backend's cache reset (tt_bio/tenstorrent.py:2185-2191)
+    def reset_static_cache(self) -> None:
+        """Packs the weights anew at the next call.  ``load_state_dict`` does so by itself, and in the fp32 tier any change in place
+        that torch counts; a change through ``.data`` needs this call, and in the fused tiers every change does."""
+        self._packed = None
+
+    def __getstate__(self):             # a copy packs its own weights: a pack's C structures point into its tensors
+        return {**self.__dict__, "_packed": None, "_captured": []}
+
+    def _pack(self, device) -> Dict[str, Dict[str, torch.Tensor]]:
+        old = self._packed
+        if old is not None and old["_device"] == device and (self.fused or not old["_versions"].changed()):
+            return old
+        sd = dict(self.state_dict().items())
+        pk = {"_device": device, "_versions": weights.Versions(sd.values())}
+        with weights.packing(device, old and old["_device"]):
+            self._build_pack(pk, sd, device)
+        self._packed = pk
+        return pk
+
+    def keep_for_capture(self) -> None:
+        """The graph being captured reads the present pack at every replay, whatever becomes of the weights."""
+        if not any(pk is self._packed for pk in self._captured):
+            self._captured.append(self._packed)
+
+
+class B200PairformerLayer(_PackedModule):
     """One Pairformer block (with or without the single track)."""
 
     def __init__(self, token_s: int = 384, token_z: int = 128, num_heads: int = 16, dropout: float = 0.25,
@@ -135,24 +173,9 @@ class B200PairformerLayer(nn.Module):
         for name, shape in layer_param_shapes(token_s, token_z, num_heads, pairwise_num_heads,
                                               pairwise_head_width, with_s):
             _register_tree(self, name, shape)
-        self._packed: Optional[Dict[str, Dict[str, torch.Tensor]]] = None
-        self.register_load_state_dict_post_hook(lambda module, incompatible: module.reset_static_cache())
         self._register_load_state_dict_pre_hook(_accept_backend_keys)
 
-    # same name as the reference backend's cache reset (tt_bio/tenstorrent.py:2185-2191)
-    def reset_static_cache(self) -> None:
-        """Packs the weights anew at the next call.  ``load_state_dict`` does so by itself, and in the fp32 tier any change in place
-        that torch counts; a change through ``.data`` needs this call, and in the fused tiers every change does."""
-        self._packed = None
-
-    def __getstate__(self):             # a copy packs its own weights: a pack's C structures point into its tensors
-        return {**self.__dict__, "_packed": None}
-
-    def _pack(self, device) -> Dict[str, Dict[str, torch.Tensor]]:
-        if self._packed is not None and self._packed["_device"] == device and (self.fused or not self._packed["_versions"].changed()):
-            return self._packed
-        sd = {k: v for k, v in self.state_dict().items()}
-        pk: Dict[str, Dict[str, torch.Tensor]] = {"_device": device, "_versions": weights.Versions(sd.values())}
+    def _build_pack(self, pk, sd, device) -> None:
         if self.fused:
             pack_mul, pack_att, pack_trans = weights.pack_trimul, weights.pack_triatt, weights.pack_transition_z
         elif self.split:
@@ -168,9 +191,6 @@ class B200PairformerLayer(nn.Module):
             pk["pair"] = ops.PairBlock(pk)
         if self.with_s:
             pk["single"] = ops.pack_single_track(sd, "", self.num_heads, device)
-        weights.settle(device, self._packed and self._packed["_device"])
-        self._packed = pk
-        return pk
 
     def forward_inplace(self, s: Optional[torch.Tensor], z: torch.Tensor, tok_mask_u8: Optional[torch.Tensor],
                         masks: ops.PairMasks, ws: Optional[ops.Workspace], side: Optional["SideTrack"] = None,
@@ -234,7 +254,7 @@ class B200PairformerNoSeqLayer(B200PairformerLayer):
         return _run_layers([self], None, z, None, pair_mask)[1]
 
 
-class B200PairUpdateBlock(nn.Module):
+class B200PairUpdateBlock(_PackedModule):
     """The block of the ESMFold2 folding trunk (tt_bio/esmfold2.py:129-154): ``z += tri_mul_out(z); z += tri_mul_in(z);
     z += transition(z)``, no triangle attention, any pair width and transition width.  Keys as in the Pairformer layer
     (``tri_mul_out.*``, ``tri_mul_in.*``, ``transition_z.*``); ``remaps.esmfold2_pair_update_block`` produces them from
@@ -255,28 +275,13 @@ class B200PairUpdateBlock(nn.Module):
         for leaf, shape in (("norm.weight", (token_z,)), ("norm.bias", (token_z,)), ("fc1.weight", (hidden, token_z)),
                             ("fc2.weight", (hidden, token_z)), ("fc3.weight", (token_z, hidden))):
             _register_tree(self, f"transition_z.{leaf}", shape)
-        self._packed = None
-        self.register_load_state_dict_post_hook(lambda module, incompatible: module.reset_static_cache())
 
-    def reset_static_cache(self) -> None:
-        """As in the layer's fp32 tier: only a change through ``.data`` needs it."""
-        self._packed = None
-
-    def __getstate__(self):             # as in the layer
-        return {**self.__dict__, "_packed": None}
-
-    def _pack(self, device):
-        if self._packed is None or self._packed["_device"] != device or self._packed["_versions"].changed():
-            sd = dict(self.state_dict().items())
-            pk = {"_device": device, "_versions": weights.Versions(sd.values())}
-            pack_mul, pack_trans = ((weights.pack_split_trimul, weights.pack_split_transition) if self.split
-                                    else (weights.to_device_f32, weights.to_device_f32))
-            for name in ("tri_mul_out", "tri_mul_in"):
-                pk[name] = pack_mul(sd, name + ".", device)
-            pk["transition_z"] = pack_trans(sd, "transition_z.", device)
-            weights.settle(device, self._packed and self._packed["_device"])
-            self._packed = pk
-        return self._packed
+    def _build_pack(self, pk, sd, device) -> None:
+        pack_mul, pack_trans = ((weights.pack_split_trimul, weights.pack_split_transition) if self.split
+                                else (weights.to_device_f32, weights.to_device_f32))
+        for name in ("tri_mul_out", "tri_mul_in"):
+            pk[name] = pack_mul(sd, name + ".", device)
+        pk["transition_z"] = pack_trans(sd, "transition_z.", device)
 
     def forward_inplace(self, z: torch.Tensor, pair_mask_u8: torch.Tensor) -> None:
         """z [N, N, c_z] contiguous fp32, updated where it is; pair_mask_u8 [N, N]."""
@@ -299,6 +304,8 @@ class B200PairUpdateBlock(nn.Module):
         with torch.cuda.device(z.device), torch.no_grad():
             zw = z[0].to(torch.float32).clone(memory_format=torch.contiguous_format)
             self.forward_inplace(zw, _mask_u8(mask, (n, n), z.device))
+            if torch.cuda.is_current_stream_capturing():
+                self.keep_for_capture()
         return zw[None]
 
 
@@ -349,7 +356,9 @@ def _run_layers(layers, s, z, mask, pair_mask, ws_cache: Optional[dict] = None, 
             sw = None if s is None else s[0].to(torch.float32).clone(memory_format=torch.contiguous_format)
         pm = ops.PairMasks(_mask_u8(pair_mask, (n, n), z.device))
         tm = _mask_u8(mask, (n,), z.device) if s is not None else None
-        ws = None
+        ws, capturing = None, torch.cuda.is_current_stream_capturing()
+        if capturing:
+            ws_cache = None                 # a graph's workspace is its own
         if any(l.fused for l in layers):
             key = (n, z.device)
             if ws_cache is not None and key in ws_cache:
@@ -367,6 +376,8 @@ def _run_layers(layers, s, z, mask, pair_mask, ws_cache: Optional[dict] = None, 
         try:
             for layer in layers:
                 layer.forward_inplace(sw, zw, tm, pm, ws, side, scratch, pair_scratch)
+                if capturing:
+                    layer.keep_for_capture()
         finally:                            # also when a layer raises: what is enqueued beside must not outlive its tensors
             if side is not None:
                 side.join()

@@ -7,10 +7,13 @@ LayerNorm gains / offsets as fp32 vectors the kernels apply themselves.
 """
 from __future__ import annotations
 
+import contextlib
 import math
 from typing import Dict
 
 import torch
+
+from . import _lib
 
 LOG2E = 1.4426950408889634
 C_Z = 128
@@ -103,14 +106,27 @@ class Versions:
         return [t._version for t in self.tensors] != self.seen
 
 
-def settle(device: torch.device, replaced) -> None:
-    """Waits for a pack that the current stream is making, so that a later call may read it on any stream.  ``replaced`` is the device
-    of a pack that is dropped for it (or None): kernels of any stream may still read that one, so they are waited for too.  A stream
-    that is being captured can't be waited for; its pack is the graph's own."""
-    if device.type == "cuda" and not torch.cuda.is_current_stream_capturing():
-        torch.cuda.current_stream(device).synchronize()
-        if replaced is not None and replaced.type == "cuda":
-            torch.cuda.synchronize(replaced)
+@contextlib.contextmanager
+def packing(device: torch.device, replaced):
+    """Around a module's packing, which is over when this is left, so that a later call may read the pack on any stream.  ``replaced``
+    is the device of a pack that is dropped for it (or None): kernels of any stream may still read that one, so they are waited for
+    too.  Under capture the packing runs at once, on a stream of its own, and not at every replay (nothing is dropped there)."""
+    if device.type != "cuda":
+        yield
+        return
+    with torch.cuda.device(device):
+        if torch.cuda.is_current_stream_capturing():
+            other = torch.cuda.Stream()
+            if other == torch.cuda.current_stream():        # streams come from a pool
+                other = torch.cuda.Stream()
+            with _lib.relaxed_capture(), torch.cuda.stream(other):
+                yield
+                other.synchronize()
+            return
+        yield
+        torch.cuda.current_stream().synchronize()
+    if replaced is not None and replaced.type == "cuda":
+        torch.cuda.synchronize(replaced)
 
 
 class SplitPack:
