@@ -71,3 +71,18 @@ def test_a_failing_layer_leaves_nothing_running_beside(monkeypatch):
     monkeypatch.undo()
     got = mod(*args)
     assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
+def test_a_timer_sees_the_single_track():
+    """Its kernels run behind the pair track then, as entry points of their own: an event pair on the pair stream would miss them on another."""
+    mod = _module(3)
+    args = _inputs(40)
+    want = mod(*args)
+    _lib.timer = _lib.KernelTimer()
+    try:
+        got = mod(*args)
+        seen = _lib.timer.summary()
+    finally:
+        _lib.timer = None
+    assert seen["b200pf_single_track_rows"][1] == 3 and "b200pf_single_track_beside" not in seen
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])

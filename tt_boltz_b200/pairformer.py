@@ -370,7 +370,8 @@ def _run_layers(layers, s, z, mask, pair_mask, ws_cache: Optional[dict] = None, 
                     ws_cache[key] = ws
         pair_scratch = pm.scratch(ws) if ws is not None else None
         side = None
-        if sw is not None and len(layers) > 1 and _side_track_wanted(n):
+        # under a timer the single track's kernels stand on the stream whose events time them
+        if sw is not None and len(layers) > 1 and _lib.timer is None and _side_track_wanted(n):
             side = SideTrack(z.device)
         scratch = ops.Scratch(z.device)
         try:
