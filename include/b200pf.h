@@ -460,6 +460,26 @@ typedef struct b200pf_split_weight {
     float       alpha;
 } b200pf_split_weight;
 
+/* What the scales of a layer's weights are chosen from: out[i] = {max |w|, max 2-norm of a row, max (sqrt(cols) |w| + |b|)} of
+ * w[rows][cols] and, for a LayerNorm (rows = 1), its offset b (else NULL: the third value is 0). */
+typedef struct b200pf_stat_item {
+    const float *w, *b;
+    int rows, cols;
+} b200pf_stat_item;
+int b200pf_weight_stats(const b200pf_stat_item* items, int n, float* out, void* stream);
+/* v = src * factor * scale (scale a power of two; src NULL: zeros) as fp32 values dst[rows][cols] (parts = 0) or as two fp16 parts, the
+ * second part_stride elements behind the first, from row row0 of dst on; interleave: rows in groups of 32, each followed by a gap
+ * of 32 (fc1 and fc2 in turn). */
+typedef struct b200pf_pack_item {
+    const float* src;
+    void* dst;
+    long long part_stride;
+    int rows, cols, row0;
+    float factor, scale;
+    short parts, interleave;
+} b200pf_pack_item;
+int b200pf_pack_parts(const b200pf_pack_item* items, int n, void* stream);
+
 /* LayerNorm gains and offsets below are given times the scale of the planes they produce. */
 typedef struct b200pf_single_track_weights {
     const float *ln_gamma, *ln_beta;

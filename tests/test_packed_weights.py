@@ -5,14 +5,14 @@ import copy
 import pytest
 import torch
 
-from tt_boltz_b200 import B200PairUpdateBlock
+from tt_boltz_b200 import B200PairUpdateBlock, _lib, weights
 from tt_boltz_b200.pairformer import B200PairformerNoSeqLayer
 
 CPU = torch.device("cpu")
 
 
-def _modules():
-    return [B200PairformerNoSeqLayer(64, precision="fp32"), B200PairUpdateBlock(64, 128)]
+def _modules():              # of a width whose pack a CPU can make: the part planes are packed on the GPU
+    return [B200PairformerNoSeqLayer(96, pairwise_num_heads=3, precision="fp32"), B200PairUpdateBlock(96, 128)]
 
 
 def _fill(module, seed=0):
@@ -27,6 +27,7 @@ def _fill(module, seed=0):
 def test_a_used_module_can_be_copied(i):
     module = _fill(_modules()[i])
     pack = module._pack(CPU)
+    pack["struct"] = weights.SplitPack(_lib.SplitTransitionWeights(c=96), [])        # as part planes have them
     twin = copy.deepcopy(module)
     assert module._packed is pack and twin._packed is None
     for (name, a), (_, b) in zip(module.named_parameters(), twin.named_parameters()):

@@ -40,6 +40,17 @@ class SplitWeight(C.Structure):
     _fields_ = [("w", _vp), ("alpha", _f)]
 
 
+class StatItem(C.Structure):
+    """Mirror of ``b200pf_stat_item``."""
+    _fields_ = [("w", _vp), ("b", _vp), ("rows", _i), ("cols", _i)]
+
+
+class PackItem(C.Structure):
+    """Mirror of ``b200pf_pack_item``."""
+    _fields_ = [("src", _vp), ("dst", _vp), ("part_stride", _ll), ("rows", _i), ("cols", _i), ("row0", _i), ("factor", _f), ("scale", _f),
+                ("parts", C.c_short), ("interleave", C.c_short)]
+
+
 class SingleTrackWeights(C.Structure):
     """Mirror of ``b200pf_single_track_weights``."""
     _fields_ = [("ln_gamma", _vp), ("ln_beta", _vp), ("qkvg", SplitWeight), ("qkvg_bias", _vp), ("o", SplitWeight), ("o_scale", _f),
@@ -156,6 +167,8 @@ SIGNATURES = {
     "b200pf_single_track_rows": [_vp, C.POINTER(SingleTrackWeights), _vp, _vp, _i, _vp, _vp],
     "b200pf_single_track_beside": [_vp, _vp, C.POINTER(PairBiasWeights), C.POINTER(SingleTrackWeights), _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i],
     "b200pf_pair_block": [_vp, C.POINTER(PairWeights), C.POINTER(PairScratch), _vp],
+    "b200pf_weight_stats": [C.POINTER(StatItem), _i, _vp, _vp],
+    "b200pf_pack_parts": [C.POINTER(PackItem), _i, _vp],
     "b200pf_split_pair_workspace": [_i, _i, _i, _i, _i],
     "b200pf_split_tri_mul": [_vp, _vp, C.POINTER(SplitTriMulWeights), _i, _i, _vp, _vp],
     "b200pf_split_tri_att": [_vp, _vp, C.POINTER(SplitTriAttWeights), _i, _i, _vp, _vp],

@@ -308,8 +308,8 @@ class SingleTrack:
     """s += AttentionPairBias(LN(s), z); s += Transition(s) in fp32 (tt_bio/reference.py:906-912) of one layer, on part
     planes: ``bias`` (its only read of z), ``attention`` for a range of query rows, ``finish`` per row."""
 
-    def __init__(self, sd, pre: str, num_heads: int, device) -> None:
-        self.pack = weights.pack_single_track(sd, pre, num_heads, device)
+    def __init__(self, sd, pre: str, num_heads: int, device, pack=None) -> None:
+        self.pack = pack or weights.pack_split([weights.single_builder(sd, pre, num_heads, device)], device)[0]
         self.z_bias = weights.pack_pair_bias(sd, pre + "attention.", device)
         b = self.z_bias
         self.bias_struct = _lib.PairBiasWeights(ptr(b["gamma"]), ptr(b["beta"]), ptr(b["w"]), b["w"].shape[1], b["w"].shape[0])
@@ -407,15 +407,22 @@ class SingleTrackF32:
         f32_linear(h, self.w_trans["fc3.weight"], out=s_rows, accumulate=True)
 
 
-def pack_single_track(sd, pre: str, num_heads: int, device):
-    """Part-plane kernels where their widths fit: c_s = 384 (or 64, 128, 256), heads of 24 or 32, hidden a multiple of 64,
-    a pair width and head count the bias projection is built for; the un-fused fp32 kernels elsewhere."""
+def single_track_fits(sd, pre: str, num_heads: int) -> bool:
+    """Whether the part-plane kernels are built for the single track's widths: c_s = 384 (or 64, 128, 256), heads of 24 or 32, hidden
+    a multiple of 64, a pair width and head count the bias projection is built for."""
     cs = sd[pre + "pre_norm_s.weight"].shape[0]
     hidden = sd[pre + "transition_s.fc1.weight"].shape[0]
     heads, cz = sd[pre + "attention.proj_z.1.weight"].shape
-    fits = (cs in weights.SPLIT_WIDTHS + (384,) and cs % num_heads == 0 and cs // num_heads in (24, 32) and hidden % 64 == 0
+    return (cs in weights.SPLIT_WIDTHS + (384,) and cs % num_heads == 0 and cs // num_heads in (24, 32) and hidden % 64 == 0
             and cz in weights.SPLIT_WIDTHS and heads in (4, 8, 16))
-    return (SingleTrack if fits else SingleTrackF32)(sd, pre, num_heads, device)
+
+
+def pack_single_track(sd, pre: str, num_heads: int, device, pack=None):
+    """Part-plane kernels where their widths fit (``pack``: their weights where the caller has packed them), the un-fused fp32 kernels
+    elsewhere."""
+    if single_track_fits(sd, pre, num_heads):
+        return SingleTrack(sd, pre, num_heads, device, pack)
+    return SingleTrackF32(sd, pre, num_heads, device)
 
 
 def single_track(s: torch.Tensor, z: torch.Tensor, tok_mask_u8: torch.Tensor, track, scratch: Scratch) -> None:

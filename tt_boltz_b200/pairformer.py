@@ -150,6 +150,14 @@ class _PackedModule(nn.Module):
             self._captured.append(self._packed)
 
 
+def _split_builders(sd, muls, atts, device):
+    """What ``weights.pack_split`` takes for a block on part planes, by name."""
+    out = {name: weights.split_trimul(sd, name + ".", device, name + ".") for name in muls}
+    out.update({name: weights.split_triatt(sd, name + ".", device, name + ".") for name in atts})
+    out["transition_z"] = weights.split_transition(sd, "transition_z.", device, "transition_z.")
+    return out
+
+
 class B200PairformerLayer(_PackedModule):
     """One Pairformer block (with or without the single track)."""
 
@@ -176,21 +184,25 @@ class B200PairformerLayer(_PackedModule):
         self._register_load_state_dict_pre_hook(_accept_backend_keys)
 
     def _build_pack(self, pk, sd, device) -> None:
-        if self.fused:
-            pack_mul, pack_att, pack_trans = weights.pack_trimul, weights.pack_triatt, weights.pack_transition_z
-        elif self.split:
-            pack_mul, pack_att, pack_trans = weights.pack_split_trimul, weights.pack_split_triatt, weights.pack_split_transition
-        else:
-            pack_mul = pack_att = pack_trans = weights.to_device_f32
-        for name in ("tri_mul_out", "tri_mul_in"):
-            pk[name] = pack_mul(sd, name + ".", device)
-        for name in ("tri_att_start", "tri_att_end"):
-            pk[name] = pack_att(sd, name + ".", device)
-        pk["transition_z"] = pack_trans(sd, "transition_z.", device)
+        builders = {}
+        if self.split:
+            builders = _split_builders(sd, ("tri_mul_out", "tri_mul_in"), ("tri_att_start", "tri_att_end"), device)
+        if self.with_s and ops.single_track_fits(sd, "", self.num_heads):
+            builders["single"] = weights.single_builder(sd, "", self.num_heads, device)
+        if builders:
+            pk.update(zip(builders, weights.pack_split(builders.values(), device)))
+        if not self.split:
+            pack_mul, pack_att, pack_trans = ((weights.pack_trimul, weights.pack_triatt, weights.pack_transition_z) if self.fused
+                                              else (weights.to_device_f32,) * 3)
+            for name in ("tri_mul_out", "tri_mul_in"):
+                pk[name] = pack_mul(sd, name + ".", device)
+            for name in ("tri_att_start", "tri_att_end"):
+                pk[name] = pack_att(sd, name + ".", device)
+            pk["transition_z"] = pack_trans(sd, "transition_z.", device)
         if self.fused:
             pk["pair"] = ops.PairBlock(pk)
         if self.with_s:
-            pk["single"] = ops.pack_single_track(sd, "", self.num_heads, device)
+            pk["single"] = ops.pack_single_track(sd, "", self.num_heads, device, pk.get("single"))
 
     def forward_inplace(self, s: Optional[torch.Tensor], z: torch.Tensor, tok_mask_u8: Optional[torch.Tensor],
                         masks: ops.PairMasks, ws: Optional[ops.Workspace], side: Optional["SideTrack"] = None,
@@ -277,11 +289,12 @@ class B200PairUpdateBlock(_PackedModule):
             _register_tree(self, f"transition_z.{leaf}", shape)
 
     def _build_pack(self, pk, sd, device) -> None:
-        pack_mul, pack_trans = ((weights.pack_split_trimul, weights.pack_split_transition) if self.split
-                                else (weights.to_device_f32, weights.to_device_f32))
-        for name in ("tri_mul_out", "tri_mul_in"):
-            pk[name] = pack_mul(sd, name + ".", device)
-        pk["transition_z"] = pack_trans(sd, "transition_z.", device)
+        if self.split:
+            builders = _split_builders(sd, ("tri_mul_out", "tri_mul_in"), (), device)
+            pk.update(zip(builders, weights.pack_split(builders.values(), device)))
+            return
+        for name in ("tri_mul_out", "tri_mul_in", "transition_z"):
+            pk[name] = weights.to_device_f32(sd, name + ".", device)
 
     def forward_inplace(self, z: torch.Tensor, pair_mask_u8: torch.Tensor) -> None:
         """z [N, N, c_z] contiguous fp32, updated where it is; pair_mask_u8 [N, N]."""

@@ -136,12 +136,6 @@ class SplitPack:
         self.struct, self.tensors = struct, tensors
 
 
-def _f16_parts(w: torch.Tensor, scale: float) -> torch.Tensor:
-    v = w * scale                       # exact: a power of two
-    hi = v.half()
-    return torch.stack([hi, (v - hi.float()).half()])
-
-
 def bf16_parts(w: torch.Tensor, device) -> torch.Tensor:
     """[3][...] bf16 parts whose sum is the fp32 value."""
     v = w.detach().float()
@@ -150,130 +144,186 @@ def bf16_parts(w: torch.Tensor, device) -> torch.Tensor:
     return torch.stack([h, m, (v - h.float() - m.float()).bfloat16()]).to(device).contiguous()
 
 
-def _fetch(**values: torch.Tensor) -> Dict[str, float]:
-    """Device scalars as host numbers, one synchronisation for all of them."""
-    return dict(zip(values, torch.stack([v.reshape(()).float() for v in values.values()]).tolist()))
+class _Plan:
+    """One sub-operation's tensors, the buffer its pack goes to and what is to be written there.
+
+    A plan's builder is a generator: it yields the tensors whose bounds it wants, (weight, None) or (LayerNorm gain, offset), gets for
+    each (largest entry, largest 2-norm of a row, bound of a normalised row's entries) and returns the C structure.  So the bounds of
+    all sub-operations of a layer are one launch and one synchronisation, and the parts another launch."""
+
+    def __init__(self, sd, pres, device) -> None:
+        self.f = {k: v.detach().to(device=device, dtype=torch.float32).contiguous() for k, v in sd.items() if k.startswith(pres)}
+        self.buf = torch.empty(sum(_padded(4 * t.numel()) for t in self.f.values()) + _padded(16 * max(t.shape[0] for t in self.f.values())),
+                               dtype=torch.uint8, device=device)
+        self.used, self.items = 0, []
+
+    def _take(self, nbytes: int) -> int:
+        at = self.buf.data_ptr() + self.used
+        self.used += _padded(nbytes)
+        assert self.used <= self.buf.numel()
+        return at
+
+    def vector(self, t: torch.Tensor, scale: float = 1.0, factor: float = 1.0, zeros: int = 0) -> int:
+        """fp32 values times factor and scale, and ``zeros`` zeros behind them."""
+        at = self._take(4 * (t.numel() + zeros))
+        self.items.append(_lib.PackItem(t.data_ptr(), at, 0, 1, t.numel(), 0, factor, scale, 0, 0))
+        if zeros:
+            self.items.append(_lib.PackItem(None, at + 4 * t.numel(), 0, 1, zeros, 0, 1.0, 1.0, 0, 0))
+        return at
+
+    def norm(self, gamma: torch.Tensor, beta: torch.Tensor, scale: float):
+        """Pointers of gain and offset times the planes' scale."""
+        return self.vector(gamma, scale), self.vector(beta, scale)
+
+    def weight(self, pieces, amax: float, operand_scale: float, interleave: bool = False):
+        """SplitWeight of the pieces' rows [(w[rows][k], factor)], one below the other or in turns of 32, for an operand that was
+        multiplied by ``operand_scale``."""
+        scale, k = _pow2_scale(amax), pieces[0][0].shape[1]
+        rows = sum(w.shape[0] for w, _ in pieces)
+        at, row0 = self._take(4 * rows * k), 0
+        for w, factor in pieces:
+            self.items.append(_lib.PackItem(w.data_ptr(), at, rows * k, w.shape[0], k, row0, factor, scale, 2, int(interleave)))
+            row0 += 32 if interleave else w.shape[0]
+        return _lib.SplitWeight(at, 1.0 / (scale * operand_scale))
 
 
-def _ln_bound(gamma: torch.Tensor, beta: torch.Tensor) -> torch.Tensor:
-    """Bound of a normalised row's entries."""
-    return (math.sqrt(gamma.numel()) * gamma.abs() + beta.abs()).max()
+def _padded(nbytes: int) -> int:
+    return (nbytes + 255) // 256 * 256
 
 
-def _row_norm(gamma: torch.Tensor, beta: torch.Tensor) -> torch.Tensor:
-    """Bound of a normalised row's 2-norm."""
-    return math.sqrt(gamma.numel()) * gamma.abs().max() + beta.norm()
+def _measure(wanted, device):
+    """A float triple per (tensor, offset or None); one synchronisation for all of them."""
+    items = [_lib.StatItem(t.data_ptr(), None if b is None else b.data_ptr(), t.numel() // t.shape[-1], t.shape[-1]) for t, b in wanted]
+    out = torch.empty(len(items), 3, dtype=torch.float32, device=device)
+    _lib.call("b200pf_weight_stats", (_lib.StatItem * len(items))(*items), len(items), out.data_ptr(), _lib.stream())
+    return out.tolist()
 
 
-def _projection_bound(w: torch.Tensor, row_norm: torch.Tensor) -> torch.Tensor:
-    """Bound of |x w^T| for rows x of at most that 2-norm."""
-    return w.norm(dim=1).max() * row_norm
+def pack_split(builders, device):
+    """SplitPacks of the builders' sub-operations (made by split_trimul, split_triatt, split_transition, split_single)."""
+    builders = list(builders)
+    if torch.device(device).type != "cuda":
+        raise RuntimeError("part planes are packed on the GPU (there is no CPU path)")
+    wanted = [next(b) for _, b in builders]
+    values, packs, items = iter(_measure([w for ws in wanted for w in ws], device)), [], []
+    for (plan, b), ws in zip(builders, wanted):
+        try:
+            b.send([next(values) for _ in ws])
+        except StopIteration as done:
+            packs.append(SplitPack(done.value, [plan.buf]))
+        items += plan.items
+    _lib.call("b200pf_pack_parts", (_lib.PackItem * len(items))(*items), len(items), _lib.stream())
+    return packs
 
 
-def _split_weight(keep, w: torch.Tensor, amax: float, operand_scale: float):
-    """SplitWeight of w[n][k] for an operand that was multiplied by ``operand_scale``; its tensor is appended to ``keep``."""
-    from ._lib import SplitWeight
-    scale = _pow2_scale(amax)
-    keep.append(_f16_parts(w, scale))
-    return SplitWeight(keep[-1].data_ptr(), 1.0 / (scale * operand_scale))
+def _builder(build):
+    """build(plan, ...) as (plan, generator) of a state dict's sub-operation."""
+    def make(sd, pres, device, *args):
+        plan = _Plan(sd, pres, device)
+        return plan, build(plan, *args)
+    return make
 
 
-def _ln(keep, gamma: torch.Tensor, beta: torch.Tensor, scale: float):
-    """Pointers of gain and offset times the planes' scale."""
-    keep += [gamma * scale, beta * scale]
-    return keep[-2].data_ptr(), keep[-1].data_ptr()
+def _row_norm(gamma, beta, c: int) -> float:
+    """Bound of a normalised row's 2-norm, from the triples of gain and offset."""
+    return math.sqrt(c) * gamma[0] + beta[1]
 
 
-def _on(sd, pre, device):
-    return {k[len(pre):]: v.detach().to(device=device, dtype=torch.float32) for k, v in sd.items() if k.startswith(pre)}
-
-
-def _swiglu_rows(fc1: torch.Tensor, fc2: torch.Tensor) -> torch.Tensor:
-    """32 rows of fc1, then 32 of fc2, in turn: a 64-column block of the product holds both factors of 32 hidden channels."""
-    h, k = fc1.shape
-    return torch.stack([fc1.view(h // 32, 32, k), fc2.view(h // 32, 32, k)], 1).reshape(2 * h, k)
-
-
-def pack_split_trimul(sd, pre: str, device):
-    from ._lib import SplitTriMulWeights
-    f, keep = _on(sd, pre, device), []
-    w_in = torch.cat([f["p_in.weight"], f["g_in.weight"]], 0)
+@_builder
+def split_trimul(plan, pre: str):
+    f = {k[len(pre):]: v for k, v in plan.f.items()}
     gi, bi, go, bo = f["norm_in.weight"], f["norm_in.bias"], f["norm_out.weight"], f["norm_out.bias"]
-    v = _fetch(ln_in=_ln_bound(gi, bi), ln_out=_ln_bound(go, bo), w_in=w_in.abs().max(), p=f["p_out.weight"].abs().max(),
-               g=f["g_out.weight"].abs().max(), u=_projection_bound(f["p_in.weight"], _row_norm(gi, bi)))
-    s_in, s_out = _pow2_scale(v["ln_in"]), _pow2_scale(v["ln_out"])
-    st = SplitTriMulWeights(*_ln(keep, gi, bi, s_in), _split_weight(keep, w_in, v["w_in"], s_in), *_ln(keep, go, bo, s_out),
-                            _split_weight(keep, f["p_out.weight"], v["p"], s_out), _split_weight(keep, f["g_out.weight"], v["g"], s_in),
-                            _pow2_scale(v["u"], QK_MOST), gi.numel())
-    return SplitPack(st, keep)
+    p_in, g_in, p_out, g_out = f["p_in.weight"], f["g_in.weight"], f["p_out.weight"], f["g_out.weight"]
+    ln_in, off, ln_out, pi, gg, po, gq = yield [(gi, bi), (bi, None), (go, bo), (p_in, None), (g_in, None), (p_out, None), (g_out, None)]
+    c = gi.numel()
+    s_in, s_out = _pow2_scale(ln_in[2]), _pow2_scale(ln_out[2])
+    return _lib.SplitTriMulWeights(*plan.norm(gi, bi, s_in), plan.weight([(p_in, 1.0), (g_in, 1.0)], max(pi[0], gg[0]), s_in), *plan.norm(go, bo, s_out),
+                                   plan.weight([(p_out, 1.0)], po[0], s_out), plan.weight([(g_out, 1.0)], gq[0], s_in),
+                                   _pow2_scale(pi[1] * _row_norm(ln_in, off, c), QK_MOST), c)
 
 
-def pack_split_triatt(sd, pre: str, device):
-    from ._lib import SplitTriAttWeights
-    f, keep = _on(sd, pre, device), []
-    heads, c = f["linear.weight"].shape
-    hd = f["mha.linear_q.weight"].shape[0] // heads
-    g, b = f["layer_norm.weight"], f["layer_norm.bias"]
-    qkvg = torch.cat([f["mha.linear_q.weight"] * (LOG2E / math.sqrt(hd)), f["mha.linear_k.weight"], f["mha.linear_v.weight"],
-                      f["mha.linear_g.weight"]], 0)
-    norm, ht = _row_norm(g, b), heads * hd
-    v = _fetch(ln=_ln_bound(g, b), w=qkvg.abs().max(), o=f["mha.linear_o.weight"].abs().max(),
-               q=_projection_bound(qkvg[:ht], norm), k=_projection_bound(qkvg[ht:2 * ht], norm), v=_projection_bound(qkvg[2 * ht:3 * ht], norm))
-    s_in, o_scale = _pow2_scale(v["ln"]), _pow2_scale(v["v"])       # an attention output is an average of rows of v
-    ln = _ln(keep, g, b, s_in)
-    keep.append((f["linear.weight"] * (LOG2E / s_in)).contiguous())
-    st = SplitTriAttWeights(*ln, keep[-1].data_ptr(), _split_weight(keep, qkvg, v["w"], s_in),
-                            _split_weight(keep, f["mha.linear_o.weight"], v["o"], o_scale), o_scale, _pow2_scale(v["q"], QK_MOST),
-                            _pow2_scale(v["k"], QK_MOST), c, heads, hd)
-    return SplitPack(st, keep)
+@_builder
+def split_triatt(plan, pre: str):
+    f = {k[len(pre):]: v for k, v in plan.f.items()}
+    g, b, head = f["layer_norm.weight"], f["layer_norm.bias"], f["linear.weight"]
+    qw, kw, vw, gw, ow = (f[f"mha.linear_{x}.weight"] for x in "qkvgo")
+    heads, c = head.shape
+    hd = qw.shape[0] // heads
+    qs = LOG2E / math.sqrt(hd)
+    ln, off, sq, sk, sv, sg, so = yield [(g, b), (b, None), (qw, None), (kw, None), (vw, None), (gw, None), (ow, None)]
+    norm = _row_norm(ln, off, c)
+    s_in, o_scale = _pow2_scale(ln[2]), _pow2_scale(sv[1] * norm)         # an attention output is an average of rows of v
+    return _lib.SplitTriAttWeights(*plan.norm(g, b, s_in), plan.vector(head, 1.0 / s_in, LOG2E),
+                                   plan.weight([(qw, qs), (kw, 1.0), (vw, 1.0), (gw, 1.0)], max(qs * sq[0], sk[0], sv[0], sg[0]), s_in),
+                                   plan.weight([(ow, 1.0)], so[0], o_scale), o_scale, _pow2_scale(qs * sq[1] * norm, QK_MOST),
+                                   _pow2_scale(sk[1] * norm, QK_MOST), c, heads, hd)
 
 
-def _swiglu_stats(f) -> Dict[str, torch.Tensor]:
-    """|silu(a) b| <= |a| |b|."""
+def _swiglu_wanted(f):
     g, b = f["norm.weight"], f["norm.bias"]
-    norm = _row_norm(g, b)
-    return {"t_ln": _ln_bound(g, b), "t_h": _projection_bound(f["fc1.weight"], norm) * _projection_bound(f["fc2.weight"], norm),
-            "t_12": torch.maximum(f["fc1.weight"].abs().max(), f["fc2.weight"].abs().max()), "t_3": f["fc3.weight"].abs().max()}
+    return [(g, b), (b, None), (f["fc1.weight"], None), (f["fc2.weight"], None), (f["fc3.weight"], None)]
 
 
-def _pack_swiglu(f, keep, v):
-    """(gain, offset), fc12, fc3, hidden scale."""
-    s_in, hs = _pow2_scale(v["t_ln"]), _pow2_scale(v["t_h"])
-    return (_ln(keep, f["norm.weight"], f["norm.bias"], s_in),
-            _split_weight(keep, _swiglu_rows(f["fc1.weight"], f["fc2.weight"]), v["t_12"], s_in),
-            _split_weight(keep, f["fc3.weight"], v["t_3"], hs), hs)
+def _swiglu(plan, f, values):
+    """(gain, offset), fc12, fc3, hidden scale; |silu(a) b| <= |a| |b|.  fc12: 32 rows of fc1, then 32 of fc2, in turn, so that a
+    64-column block of the product holds both factors of 32 hidden channels."""
+    ln, off, s1, s2, s3 = values
+    norm = _row_norm(ln, off, f["norm.weight"].numel())
+    s_in, hs = _pow2_scale(ln[2]), _pow2_scale(s1[1] * norm * s2[1] * norm)
+    return (plan.norm(f["norm.weight"], f["norm.bias"], s_in),
+            plan.weight([(f["fc1.weight"], 1.0), (f["fc2.weight"], 1.0)], max(s1[0], s2[0]), s_in, interleave=True),
+            plan.weight([(f["fc3.weight"], 1.0)], s3[0], hs), hs)
 
 
-def pack_split_transition(sd, pre: str, device):
-    from ._lib import SplitTransitionWeights
-    f, keep = _on(sd, pre, device), []
-    gb, fc12, fc3, hs = _pack_swiglu(f, keep, _fetch(**_swiglu_stats(f)))
-    return SplitPack(SplitTransitionWeights(*gb, fc12, fc3, hs, f["norm.weight"].numel(), f["fc1.weight"].shape[0]), keep)
+@_builder
+def split_transition(plan, pre: str):
+    f = {k[len(pre):]: v for k, v in plan.f.items()}
+    values = yield _swiglu_wanted(f)
+    gb, fc12, fc3, hs = _swiglu(plan, f, values)
+    return _lib.SplitTransitionWeights(*gb, fc12, fc3, hs, f["norm.weight"].numel(), f["fc1.weight"].shape[0])
 
 
-def pack_single_track(sd, pre: str, num_heads: int, device):
-    """Single track: pre_norm_s, attention (without the pair-bias projection) and transition_s of one layer."""
-    from ._lib import SingleTrackWeights
-    keep = []
-    n, a, t = (_on(sd, pre + part, device) for part in ("pre_norm_s.", "attention.", "transition_s."))
-    g, b, cs = n["weight"], n["bias"], n["weight"].numel()
+@_builder
+def split_single(plan, pre: str, num_heads: int):
+    """pre_norm_s, attention (without the pair-bias projection) and transition_s of one layer."""
+    f = {k[len(pre):]: v for k, v in plan.f.items()}
+    t = {k[len("transition_s."):]: v for k, v in f.items() if k.startswith("transition_s.")}
+    g, b, bias = f["pre_norm_s.weight"], f["pre_norm_s.bias"], f["attention.proj_q.bias"]
+    qw, kw, vw, gw, ow = (f[f"attention.proj_{x}.weight"] for x in "qkvgo")
+    cs = g.numel()
     qs = LOG2E / math.sqrt(cs // num_heads)
-    qkvg = torch.cat([a["proj_q.weight"] * qs, a["proj_k.weight"], a["proj_v.weight"], a["proj_g.weight"]], 0)
-    norm = _row_norm(g, b)
-    v = _fetch(ln=_ln_bound(g, b), w=qkvg.abs().max(), o=a["proj_o.weight"].abs().max(),
-               q=_projection_bound(qkvg[:cs], norm) + (a["proj_q.bias"] * qs).abs().max(), k=_projection_bound(qkvg[cs:2 * cs], norm),
-               v=_projection_bound(a["proj_v.weight"], norm), **_swiglu_stats(t))
-    s_in, o_scale = _pow2_scale(v["ln"]), _pow2_scale(v["v"])
-    ln = _ln(keep, g, b, s_in)
-    keep.append(torch.nn.functional.pad(a["proj_q.bias"] * qs, (0, 3 * cs)))
-    bias = keep[-1].data_ptr()
-    w_qkvg, w_o = _split_weight(keep, qkvg, v["w"], s_in), _split_weight(keep, a["proj_o.weight"], v["o"], o_scale)
-    gb2, fc12, fc3, hs = _pack_swiglu(t, keep, v)
-    return SplitPack(SingleTrackWeights(*ln, w_qkvg, bias, w_o, o_scale, _pow2_scale(v["q"], QK_MOST), _pow2_scale(v["k"], QK_MOST), *gb2, fc12, hs, fc3, cs, num_heads, t["fc1.weight"].shape[0]), keep)
+    ln, off, sq, sk, sv, sg, so, sb, *values = yield [(g, b), (b, None), (qw, None), (kw, None), (vw, None), (gw, None), (ow, None), (bias, None),
+                                                      *_swiglu_wanted(t)]
+    norm = _row_norm(ln, off, cs)
+    s_in, o_scale = _pow2_scale(ln[2]), _pow2_scale(sv[1] * norm)
+    ln_ptrs = plan.norm(g, b, s_in)
+    w_qkvg = plan.weight([(qw, qs), (kw, 1.0), (vw, 1.0), (gw, 1.0)], max(qs * sq[0], sk[0], sv[0], sg[0]), s_in)
+    bias_ptr, w_o = plan.vector(bias, 1.0, qs, zeros=3 * cs), plan.weight([(ow, 1.0)], so[0], o_scale)
+    gb, fc12, fc3, hs = _swiglu(plan, t, values)
+    return _lib.SingleTrackWeights(*ln_ptrs, w_qkvg, bias_ptr, w_o, o_scale, _pow2_scale(qs * (sq[1] * norm + sb[0]), QK_MOST),
+                                   _pow2_scale(sk[1] * norm, QK_MOST), *gb, fc12, hs, fc3, cs, num_heads, t["fc1.weight"].shape[0])
+
+
+def pack_split_trimul(sd, pre: str, device) -> SplitPack:
+    return pack_split([split_trimul(sd, pre, device, pre)], device)[0]
+
+
+def pack_split_triatt(sd, pre: str, device) -> SplitPack:
+    return pack_split([split_triatt(sd, pre, device, pre)], device)[0]
+
+
+def pack_split_transition(sd, pre: str, device) -> SplitPack:
+    return pack_split([split_transition(sd, pre, device, pre)], device)[0]
+
+
+def single_builder(sd, pre: str, num_heads: int, device):
+    # proj_z, the pair-bias projection, is packed by pack_pair_bias
+    own = {k: v for k, v in sd.items() if not k.startswith(pre + "attention.proj_z.")}
+    return split_single(own, (pre + "pre_norm_s.", pre + "attention.", pre + "transition_s."), device, pre, num_heads)
 
 
 def pack_pair_bias(sd, pre: str, device) -> Dict[str, torch.Tensor]:
     """The single track's only read of z: LayerNorm and the head projection, in the base-2 logarithms the attention works in."""
-    f = _on(sd, pre, device)
+    f = {k[len(pre):]: v.detach().to(device=device, dtype=torch.float32) for k, v in sd.items() if k.startswith(pre)}
     fp = lambda t: t.to(device=device, dtype=torch.float32).contiguous()
     return {"gamma": fp(f["proj_z.0.weight"]), "beta": fp(f["proj_z.0.bias"]), "w": fp(f["proj_z.1.weight"] * LOG2E)}
