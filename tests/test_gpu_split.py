@@ -1,8 +1,8 @@
 """The fp32-accurate path on 16-bit parts (csrc/split_*.cu) against the oracle in 64 bits, at the edges of its tiles: 128-row and
 32-column GEMM tiles, 64-key attention tiles, 32-position LayerNorm tiles, K splits.
 
-Tolerance on an update's relative 2-norm: two fp16 parts keep 22 bits of every factor (2^-22 relative per product, random),
-and every MMA truncates its addend to an ulp of the running sum (2^-24 of it, always towards zero); the longest sum here
+Tolerance on an update's relative 2-norm: two fp16 parts keep every factor to 2^-23 and a product leaves out at most 2^-22 (2^-21
+relative per product, random), and every MMA truncates its addend to an ulp of the running sum (2^-24 of it, always towards zero); the longest sum here
 takes 3 * 1536 / 16 = 288 of them, 1.7e-5 at worst.  2e-5 covers both."""
 import pytest
 import torch

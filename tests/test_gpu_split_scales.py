@@ -1,6 +1,6 @@
 """The fp32-accurate attention and triangle multiplication where their operands' scales and copies change: token counts whose bias
 rows are copied in 16-byte pieces (multiples of four) and not, and weights far from the size the fp16 parts are laid out for, so that
-the packed scales have to carry them.  Against the oracle in 64 bits; tolerance as in test_gpu_split (2^-22 relative per product, a
+the packed scales have to carry them.  Against the oracle in 64 bits; tolerance as in test_gpu_split (2^-21 relative per product, a
 sum of truncated additions: 2e-5), plus half an ulp of z where the update is read back as a difference."""
 import pytest
 import torch

@@ -1,9 +1,10 @@
 // Operands of the fp32-accurate tensor-core path: an fp32 value kept as a sum of 16-bit parts.
 //
-//   F16X2   v * scale = hi + lo, two fp16 parts (22 bits: what a 3xTF32 product keeps).  `scale` is a power of two chosen
-//           when the weights are packed from a bound of |v| (a LayerNorm output is at most sqrt(C) * gain + offset, a
-//           projection of it at most that times the row norm), so neither part can overflow and `lo` keeps its 11 bits
-//           down to 2^-17 of the bound.  Products: hi*hi + hi*lo + lo*hi, three MMAs.
+//   F16X2   v * scale = hi + lo, two fp16 parts.  hi is off by at most 2^-11 of the value, and lo by at most 2^-12 of what is left:
+//           2^-23 of the value together, one ulp of fp32.  `scale` is a power of two chosen when the weights are packed from a
+//           bound of |v| (a LayerNorm output is at most sqrt(C) * gain + offset, a projection of it at most that times the row
+//           norm), so neither part can overflow and this holds for values down to 2^-15 of the bound; below, the error is at most
+//           2^-38 of the bound.  Products: hi*hi + hi*lo + lo*hi, three MMAs; what is left out is at most 2^-22 of the product.
 //   BF16X3  v = h + m + l, three bf16 parts (24 bits, the whole fp32 mantissa, and fp32's own range: no scale).
 //           Products of total order <= 2: six MMAs.
 // Both accumulate in fp32.  A plane stack is [parts][rows][cols] of 16-bit values.

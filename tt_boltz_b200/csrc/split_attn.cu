@@ -1,6 +1,5 @@
 // softmax(q k^T + bias + mask) v with a gate, at fp32 accuracy: one-pass softmax over 64-key tiles, both products as three
-// m16n8k16 fp16 MMAs on two-part operands (split.cuh; hi is rounded to 11 bits and lo to 11 bits of what is left, together
-// 2^-24 of the value, half an ulp of fp32), fp32 accumulation.
+// m16n8k16 fp16 MMAs on two-part operands (split.cuh), fp32 accumulation.
 //
 // mma.sync and not tcgen05: q, k, v rows are 24 or 32 wide and the probabilities need parts of their own, so a tcgen05 form
 // would have to push both through tensor memory; here they go from the accumulators of the first product straight into the
@@ -33,8 +32,9 @@ constexpr int BP = KT + 8;               // bias tile pitch in floats: a half-wa
 constexpr int bias_stage(int nw) { return nw * 16 * BP * 4; }
 constexpr float P_SCALE = 16384.f;      // probabilities are at most one: their parts use the upper half of fp16's range
 
-// 2^x of a score below the row's maximum.  exp2f is this instruction with a range step around it that keeps results below 2^-126;
-// a row's largest probability is 1, so those have no bit to add to its sums.
+// 2^x of a score below the row's maximum.  PTX documents the instruction as an approximation good to some 2^-22 of its result, with
+// results below 2^-126 flushed to zero.  A row's largest probability is 1, so a flushed one is below 2^-126 of the row's sum, and each
+// of its products below 2^-126 of the largest value: nothing that 24 bits of either could show.
 __device__ __forceinline__ float prob(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
