@@ -48,8 +48,8 @@ int         b200pf_device_status(void* stream);
 int         b200pf_exchange_capture_mode(int* mode);
 
 /* ------------------------------------------------------------------------------------------
- * fp32 validation tier: un-fused SIMT kernels, arithmetic in fp32 throughout.
- * Stand in for torch.nn.functional calls of the reference's CPU path.
+ * Un-fused fp32 kernels, standing in for torch.nn.functional calls of the reference's CPU path: the fp32 tier and the single track
+ * at widths that the part-plane kernels below are not built for, the recycling and MSA embedding linears, the distogram.
  * ---------------------------------------------------------------------------------------- */
 
 /* y[r][:] = LayerNorm(x[r][:]) * gamma + beta, eps 1e-5, biased variance.
@@ -346,19 +346,15 @@ int b200pf_opm_finalize(const b200pf_bf16* y, const uint32_t* bits, const float*
                         int i0, int n_i, int n, int accumulate, void* stream);
 
 /* ----------------------------------------------------------------------------------------
- * Row kernels of the MSA stack (m fp32 [S][N][64]) around GEMMs run by b200pf_trimul_contract.  The token axis
- * of every bf16 operand is padded to np (a multiple of 8, >= n); padding rows are zero.
+ * Row kernels of the MSA stack (m fp32 [S][N][64]) around GEMMs run by b200pf_trimul_contract.  The token axis of every bf16
+ * operand is padded to np (a multiple of 8, >= n); padding rows are zero.  The MSA modules run one kernel per stage:
  *   pair-weighted averaging (tt_bio/tenstorrent.py:1542-1629, reference.py:672-800):
- *     ln = b200pf_msa_ln_bf16(m)                         [S*np][64]
- *     vg = b200pf_gemm_grouped(A = [proj_m ; proj_g] bf16 [512][64], B = ln) -> [16][S][32][np]: v groups 0-7 (heads),
- *          g groups 8-15; np a multiple of 32 here
- *     logits = b200pf_ln_proj_heads(z, norm_z, proj_z, 8 heads);  w = b200pf_pwa_softmax(logits, mask)
- *     o = contract over 8 heads (A = v as [8][S*32][np], B = w [8][n][pitch])   -> [8][S][32][np]
- *     val = b200pf_pwa_gate_transpose(o, g);  t = contract(A = val [S*np][256], B = proj_o bf16 [64][256]);
- *     b200pf_msa_add_rows(m, t)
- *   MSA transition (Transition(64, 256), tt_bio/boltz2.py:1188-1258):
- *     ln -> contract(A = ln, B = [fc1 ; fc2] bf16 [512][64]) -> b200pf_msa_swiglu -> contract(B = fc3 bf16 [64][256])
- *     -> b200pf_msa_add_rows
+ *     logits = b200pf_ln_proj_heads(z, norm_z, proj_z, 16 heads, 8 of them zero);  w = b200pf_pwa_softmax(logits, mask)
+ *     v = b200pf_pwa_value(m);  o = contract over 8 heads (A = v as [8][S*32][np], B = w [8][n][pitch]);  b200pf_pwa_output(m, o)
+ *   MSA transition (Transition(64, 256), tt_bio/boltz2.py:1188-1258): b200pf_msa_transition(m)
+ * The stages before and after a GEMM as kernels of their own, for hosts that keep the intermediates:
+ *   b200pf_msa_ln_bf16, b200pf_gemm_grouped (A = [proj_m ; proj_g], output [16][S][32][np], np a multiple of 32), b200pf_pwa_gate_transpose,
+ *   b200pf_msa_swiglu, b200pf_msa_add_rows.
  * ---------------------------------------------------------------------------------------- */
 int b200pf_msa_ln_bf16(const float* m, const float* gamma, const float* beta, b200pf_bf16* out, int s_len, int n, int np,
                        void* stream);
@@ -590,10 +586,6 @@ int b200pf_ln_heads(const float* x, const float* gamma, const float* beta, const
 long long b200pf_split_linear_workspace(long long rows, int k);
 int b200pf_split_linear(const float* x, const void* w, const float* bias, float* y, long long rows, int k, int n, int accumulate,
                         void* workspace, void* stream);
-/* y[rows][n] += LN(x)[rows][c] w[n][c]^T (the recycling projections, tt_bio/boltz2.py:5207-5208). */
-long long b200pf_split_ln_linear_workspace(long long rows, int c);
-int b200pf_split_ln_linear_add(const float* x, const float* gamma, const float* beta, const b200pf_split_weight* w, float* y, long long rows,
-                               int c, int n, void* workspace, void* stream);
 
 #ifdef __cplusplus
 }

@@ -177,11 +177,9 @@ SIGNATURES = {
     "b200pf_ln_heads": [_vp, _vp, _vp, _vp, _vp, _ll, _ll, _i, _i, _vp],
     "b200pf_split_linear_workspace": [_ll, _i],
     "b200pf_split_linear": [_vp, _vp, _vp, _vp, _ll, _i, _i, _i, _vp, _vp],
-    "b200pf_split_ln_linear_workspace": [_ll, _i],
-    "b200pf_split_ln_linear_add": [_vp, _vp, _vp, C.POINTER(SplitWeight), _vp, _ll, _i, _i, _vp, _vp],
 }
 _RESTYPES = {"b200pf_single_track_workspace": _ll, "b200pf_single_track_rows_workspace": _ll, "b200pf_split_pair_workspace": _ll, "b200pf_split_linear_workspace": _ll,
-             "b200pf_split_transition_workspace": _ll, "b200pf_split_ln_linear_workspace": _ll,
+             "b200pf_split_transition_workspace": _ll,
              "b200pf_last_error": C.c_char_p, "b200pf_launch_count": _ll, "b200pf_mx_scale_bytes": _ll}
 
 _lib: Optional[C.CDLL] = None

@@ -1,7 +1,6 @@
-// fp32 validation tier: plain SIMT kernels, fp32 arithmetic end to end.
-// These exist so that the 1e-4-per-layer tier can be met on the GPU (tensor cores have no
-// fp32 mode) and they double as the single-track path, which the reference keeps in fp32
-// (tt_bio/reference.py:906-912).  Speed is secondary here; clarity and exactness come first.
+// Un-fused fp32 kernels: the fp32 tier and the single track at widths that the part-plane kernels (split_*.cu) are not built
+// for, the recycling, distogram and MSA embedding linears, and an implementation of its own to compare the fused tiers
+// with.  SIMT, or 3xTF32 on mma.sync where a linear or an attention is large.
 #include "pdl.cuh"
 
 namespace b200pf {

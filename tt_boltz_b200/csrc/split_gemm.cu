@@ -24,7 +24,7 @@ struct Dev {
     const float* bias;
     const uint8_t* mask;
     long long mask_bs, mask_cs;
-    int n_split, rows_outer, n_out;      // n_out: output columns
+    int n_split;
 };
 
 // Products of the parts, smallest first: (lo, hi), (hi, lo), (hi, hi) and (l, h), (m, m), (h, l), (m, h), (h, m), (h, h).
@@ -354,7 +354,7 @@ static int launch_one(const Gemm& g, int bn, int sms, cudaStream_t st) {
     d.alpha[0] = g.alpha[0]; d.alpha[1] = g.alpha[1]; d.out_scale = g.out_scale;
     d.bias = g.bias; d.mask = g.mask; d.mask_bs = g.mask_bs; d.mask_cs = g.mask_cs;
     for (int i = 0; i < 3; ++i) d.qkv_scale[i] = g.qkv_scale[i];
-    d.n_split = g.n_split; d.rows_outer = g.out[0].rows_outer; d.n_out = g.out[0].cols;
+    d.n_split = g.n_split;
     const long long tiles = (long long)d.batches * ((g.m_rows + 127) / 128) * ((g.n_rows + bn - 1) / bn);
     return launch_pdl(kern, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(THREADS), smem, st, a[0], a[1], b[0], b[1], o[0], o[1], d, status);
 }
@@ -380,9 +380,8 @@ int launch_gemm(const Gemm& g, cudaStream_t st) {
     B200PF_REQUIRE(g.k_splits == 1 || (g.epi == EPI_STORE && g.batches == 1 && g.k_splits > 1 &&
                                        (g.k_splits - 1) * ((kb_total + g.k_splits - 1) / g.k_splits) < kb_total),
                    B200PF_ERR_INVALID, "split_gemm: every K split needs a k-block of its own");
-    int dev = 0, sms = 148;
-    B200PF_CUDA(cudaGetDevice(&dev));
-    B200PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms, rc;
+    if ((rc = multiprocessors(&sms)) != B200PF_OK) return rc;
     const long long row_tiles = (long long)(g.k_splits > 1 ? g.k_splits : g.batches) * ((g.m_rows + 127) / 128);
 #define SG(PL, BN, NA, NK, EPI) return launch_one<PL, BN, NA, NK, EPI>(g, bn, sms, st)
     switch (g.epi) {

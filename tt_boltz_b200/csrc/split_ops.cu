@@ -27,10 +27,10 @@ static int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
 // How many K splits a GEMM of few rows takes: enough CTAs to use the chip's bandwidth for its weights, at least three
 // k-blocks each, never more than eight partial sums for the reader to add.
-static int k_splits_for(int rows, int n, int k) {
+static int k_splits_for(int rows, int n, int k, int sms) {
     const int kb = (k + 63) / 64;
     const int tiles = ((rows + 127) / 128) * ((n + 31) / 32);
-    int want = 148 / (tiles > 0 ? tiles : 1);
+    int want = sms / (tiles > 0 ? tiles : 1);
     if (want > 8) want = 8;
     if (want > kb / 3) want = kb / 3;
     if (want < 2) return 1;
@@ -44,7 +44,9 @@ static int residual_gemm(float* y, const void* planes, const b200pf_split_weight
     g.a[0] = matrix(planes, rows, k);
     g.b[0] = matrix(w.w, n, k);
     g.m_rows = (int)rows; g.n_rows = n; g.k[0] = k; g.alpha[0] = w.alpha;
-    const int ks = partial ? k_splits_for((int)rows, n, k) : 1;
+    int sms, rc = multiprocessors(&sms);
+    if (rc != B200PF_OK) return rc;
+    const int ks = partial ? k_splits_for((int)rows, n, k, sms) : 1;
     if (ks == 1) {
         g.epi = EPI_ADD;
         g.out[0] = dense(y, rows, n, 1);
@@ -53,8 +55,7 @@ static int residual_gemm(float* y, const void* planes, const b200pf_split_weight
     g.epi = EPI_STORE;
     g.k_splits = ks;
     g.out[0] = Output{partial, (int)rows, n, ks, 1, n, rows * n, 0, false};
-    int rc = launch_gemm(g, st);
-    if (rc != B200PF_OK) return rc;
+    if ((rc = launch_gemm(g, st)) != B200PF_OK) return rc;
     return launch_add_partials(y, partial, ks, rows * n, st);
 }
 
@@ -321,21 +322,6 @@ int b200pf_split_linear(const float* x, const void* w, const float* bias, float*
     g.m_rows = (int)rows; g.n_rows = n; g.k[0] = k; g.bias = bias;
     g.out[0] = dense(y, rows, n, 1);
     return launch_gemm(g, st);
-}
-
-/* y[rows][n] += LN(x)[rows][c] w[n][c]^T */
-long long b200pf_split_ln_linear_workspace(long long rows, int c) { return 4 * rows * c; }
-
-int b200pf_split_ln_linear_add(const float* x, const float* gamma, const float* beta, const b200pf_split_weight* w, float* y, long long rows, int c, int n,
-                               void* workspace, void* stream) {
-    B200PF_REQUIRE(x && gamma && beta && w && y && workspace && aligned16(y) && aligned16(workspace), B200PF_ERR_INVALID,
-                   "split_ln_linear: null or misaligned pointer");
-    B200PF_REQUIRE(rows > 0 && rows <= 0x7fffffffLL && ln_supported(c) && n > 0 && n % 4 == 0, B200PF_ERR_UNSUPPORTED, "split_ln_linear: bad sizes");
-    LnArgs ln = {};
-    ln.x = x; ln.gamma = gamma; ln.beta = beta; ln.planes = (__half*)workspace; ln.part_stride = rows * c; ln.rows = rows;
-    int rc = launch_ln(ln, c, 0, (cudaStream_t)stream);
-    if (rc != B200PF_OK) return rc;
-    return residual_gemm(y, workspace, *w, rows, c, n, nullptr, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -70,27 +70,6 @@ __global__ void __launch_bounds__(256) ln_split_kernel(LnArgs p) {
                 }
             }
         }
-        if (p.n_partial > 0) {
-            for (int q = 0; q < p.n_partial; ++q)
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const long long row = base + r < p.rows ? base + r : p.rows - 1;
-                    const float* src = p.partial + ((long long)q * p.rows + row) * C + lane * V;
-#pragma unroll
-                    for (int j = 0; j < J; ++j)
-#pragma unroll
-                        for (int e = 0; e < V; ++e) x[r][j][e] += src[j * 32 * V + e];
-                }
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (base + r < p.rows) {
-                    float* dst = p.x_out + (base + r) * C + lane * V;
-#pragma unroll
-                    for (int j = 0; j < J; ++j)
-#pragma unroll
-                        for (int e = 0; e < V; ++e) dst[j * 32 * V + e] = x[r][j][e];
-                }
-        }
         float s[R], ss[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -190,9 +169,8 @@ bool ln_supported(int c) { return c == 64 || c == 128 || c == 256 || c == 384; }
 
 template <int C, int NH> static int ln_go(const LnArgs& a, cudaStream_t st) {
     constexpr int R = NH == 16 ? 4 : NH > 0 ? 4 : (C >= 256 ? 2 : 4);
-    int dev = 0, sms = 148;
-    B200PF_CUDA(cudaGetDevice(&dev));
-    B200PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms, rc;
+    if ((rc = multiprocessors(&sms)) != B200PF_OK) return rc;
     // few rows: one warp pass per block of fewer warps, so that every SM gets some
     const int warps = a.rows >= (long long)sms * 8 * R ? 8 : 2;
     const long long need = (a.rows + (long long)warps * R - 1) / ((long long)warps * R);
@@ -315,7 +293,9 @@ __global__ void __launch_bounds__(256) parts_kernel(const float4* x, uint2* plan
 }
 int launch_parts(const float* x, __nv_bfloat16* planes, long long count, cudaStream_t st) {
     B200PF_REQUIRE(x && planes && aligned16(x) && aligned16(planes) && count > 0 && count % 8 == 0, B200PF_ERR_INVALID, "parts: bad arguments");
-    const long long need = (count / 4 + 255) / 256, most = 148 * 16;
+    int sms, rc;
+    if ((rc = multiprocessors(&sms)) != B200PF_OK) return rc;
+    const long long need = (count / 4 + 255) / 256, most = 16LL * sms;
     return launch_pdl(parts_kernel, dim3((unsigned)(need < most ? need : most)), dim3(256), 0, st, reinterpret_cast<const float4*>(x),
                       reinterpret_cast<uint2*>(planes), count / 4);
 }

@@ -12,10 +12,6 @@ struct LnArgs {
     __half* planes;             // [2][rows][C], or null: heads only
     long long part_stride;
     long long rows;
-    // partial sums of a K-split GEMM that are still to be added: x += sum_p partial[p] (stored back to x_out)
-    const float* partial;
-    int n_partial;
-    float* x_out;
     // a few dot products per row with the normalised row: out[h][row], or, for a pair tensor of width n, out[h][j][i] of row (i, j)
     const float* head_w;        // [heads][C], divided by the planes' scale
     float* head_out;
