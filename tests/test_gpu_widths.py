@@ -1,6 +1,6 @@
 """Other pair widths than the trunk's 128: the template stack (c_z = 64), the c_z = 256 / 8-head blocks of the sibling
-models and the attention-free pair update block run on the un-fused fp32 kernels and must meet that tier's tolerance
-against the CPU oracle (1e-4 relative L2 per block; call sites: tt_bio/boltz2.py:3749-3753, tt_bio/protenix.py:947,
+models and the attention-free pair update block run in the fp32 tier, on part planes (the un-fused kernels at these and
+other widths are in test_gpu_unfused), and must meet that tier's tolerance against the CPU oracle (1e-4 relative L2 per block; call sites: tt_bio/boltz2.py:3749-3753, tt_bio/protenix.py:947,
 tt_bio/esmfold2.py:129-154)."""
 import pytest
 import torch
