@@ -167,7 +167,7 @@ class PairBlock:
 
 
 # ------------------------------------------------------------------------------------------------
-# fp32 tier (un-fused SIMT kernels) - also the single-track path of every tier
+# un-fused fp32 kernels: fp32 tier and single track at widths that the part-plane kernels below are not built for, recycling
 # ------------------------------------------------------------------------------------------------
 def _empty(rows: int, c: int, like: torch.Tensor) -> torch.Tensor:
     return torch.empty(rows, c, dtype=torch.float32, device=like.device)

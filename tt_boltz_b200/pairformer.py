@@ -167,7 +167,7 @@ class B200PairformerLayer(_PackedModule):
         super().__init__()
         if post_layer_norm:
             raise NotImplementedError("post_layer_norm=True is not used by Boltz-2 and is not built")
-        if precision == "auto":     # the fused kernels where their widths fit, the un-fused fp32 kernels elsewhere
+        if precision == "auto":     # the fused kernels where their widths fit, the fp32 tier elsewhere
             precision = "bf16" if (token_z, pairwise_num_heads, pairwise_head_width) == (128, 4, 32) else "fp32"
         if precision not in ("bf16", "mxfp8", "fp32"):
             raise ValueError("precision must be 'bf16', 'mxfp8', 'fp32' or 'auto'")

@@ -4,8 +4,8 @@ The reference runs Protenix-v2 (c_z = 256, 8 triangle-attention heads, 48 blocks
 (triangle multiplications + SwiGLU transition only, c_z = 256) on its Pairformer primitives after renaming their
 checkpoint keys (tt_bio/protenix_weights.py:17-137, tt_bio/esmfold2.py:102-126).  The same renames are expressed
 here as tables, so that such a checkpoint loads into ``B200PairformerModule`` / ``B200PairUpdateBlock`` /
-``B200OuterProductMean`` / ``B200PairWeightedAveraging`` with ``load_state_dict(strict=True)``.  These widths run on
-the un-fused fp32 kernels (``precision="fp32"`` or ``"auto"``).
+``B200OuterProductMean`` / ``B200PairWeightedAveraging`` with ``load_state_dict(strict=True)``.  These widths run in
+the fp32 tier (``precision="fp32"`` or ``"auto"``), on its tensor-core kernels.
 
 A table maps OUR key to the source key, or to a tuple of source keys whose rows are concatenated in that order.
 """

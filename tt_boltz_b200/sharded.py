@@ -196,7 +196,8 @@ def rows_to_cols(z_loc: torch.Tensor, group=None) -> torch.Tensor:
 
 
 # Around the sharded ending-node attention z crosses the wire in bf16 and only the update comes back (half the bytes
-# of the fp32 round trip); "0" keeps the fp32 exchange, which reproduces the one-GPU result bit for bit.
+# of the fp32 round trip); "0" keeps the fp32 exchange, which reproduces one GPU's z bit for bit.  (s differs in its last bits
+# either way: the single track's last GEMM is split along K by its row count, which a shard has less of.)
 _BF16_EXCHANGE = {"enabled": os.environ.get("B200PF_BF16_EXCHANGE", "1") != "0"}
 
 
