@@ -260,13 +260,7 @@ msa_transition_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_
                     const float a0 = __uint_as_float(f1[2 * e]), a1 = __uint_as_float(f1[2 * e + 1]);
                     hw[e] = pack_bf16x2(a0 * sigmoid_of(a0) * __uint_as_float(f2[2 * e]), a1 * sigmoid_of(a1) * __uint_as_float(f2[2 * e + 1]));
                 }
-                const uint32_t h = tmem + lane_off + COL_H + buf * 32 + half * 16;
-                asm volatile(
-                    "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-                    "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-                    ::"r"(h), "r"(hw[0]), "r"(hw[1]), "r"(hw[2]), "r"(hw[3]), "r"(hw[4]), "r"(hw[5]), "r"(hw[6]), "r"(hw[7]), "r"(hw[8]), "r"(hw[9]),
-                      "r"(hw[10]), "r"(hw[11]), "r"(hw[12]), "r"(hw[13]), "r"(hw[14]), "r"(hw[15])
-                    : "memory");
+                tmem_st_32x16(tmem + lane_off + COL_H + buf * 32 + half * 16, hw);
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();

@@ -68,14 +68,6 @@ __device__ __forceinline__ void tmem_ld_x16(uint32_t taddr, uint32_t (&r)[16]) {
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr) : "memory");
 }
-__device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
 
 __global__ void __launch_bounds__(THREADS, 1)
 transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_constant__ CUtensorMap map_w3,
@@ -291,7 +283,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_c
                     float h1 = fmaf(a1, tanh_approx(a1), a1) * __uint_as_float(f2[2 * e + 1]);
                     hw[e] = pack_bf16x2(h0, h1);
                 }
-                tmem_st_x16(tmem_base + lane_off + COL_H + buf * 32 + eh * 16, hw);
+                tmem_st_32x16(tmem_base + lane_off + COL_H + buf * 32 + eh * 16, hw);
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
