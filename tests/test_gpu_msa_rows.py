@@ -1,6 +1,7 @@
 """The MSA row kernels that stand between GEMMs as kernels of their own (the MSA modules run one kernel per stage instead) against torch
 in 64 bits, at ragged token counts.  Results are one fp32 computation rounded to bf16 once: 2^-9 relative per value (4e-3 with the
-largest entry's neighbours); the grouped GEMM's sums over 64 products of bf16 values are exact to fp32 before that."""
+largest entry's neighbours), 1e-5 where terms of order one cancel; the grouped GEMM's sums take four MMAs, each truncating a sum of up
+to 50 to its ulp: 4 * 50 * 2^-23 = 2.4e-5."""
 import ctypes as C
 
 import pytest
@@ -17,9 +18,9 @@ def _g(s, n):
     return torch.Generator().manual_seed(100 * s + n)
 
 
-def _close(got, want):
+def _close(got, want, slack=1e-5):
     assert torch.isfinite(got).all()
-    assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all())
+    assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + slack).all())
 
 
 @pytest.mark.parametrize("s, n", SIZES)
@@ -67,5 +68,5 @@ def test_grouped_gemm(s, n):
     pa, pb = Planes(ptr(w), 512 * 64, 0, 64, 512, 64, 1, 0), Planes(ptr(rows), s * np_ * 64, 0, 64, s * np_, 64, 1, 0)
     call("b200pf_gemm_grouped", C.byref(pa), C.byref(pb), ptr(out), 0, np_, 32, s * 32 * np_, np_, 32 * np_, 1, stream())
     want = (w.double() @ rows.double().T).view(16, 32, s, np_).permute(0, 2, 1, 3)
-    _close(out, want)
+    _close(out, want, 2.4e-5)
     assert device_status() == 0
