@@ -45,3 +45,9 @@ def test_first_and_ragged_tiles(n, kind):
         upd, want = (zd.cpu() - z[0]), (zf.cpu() - z[0])
         assert torch.isfinite(upd).all()
         assert rel_l2(upd, want) < 2e-2
+
+
+@pytest.mark.parametrize("n, kind", [(64, "ones"), (128, "late"), (128, "block"), (192, "none"), (192, "second_half"), (256, "ones")])
+def test_lines_of_whole_tiles(n, kind):
+    """The form of the core for token counts that are multiples of 64, which has no test for a short last tile."""
+    test_first_and_ragged_tiles(n, kind)

@@ -14,7 +14,7 @@
 // before (scaling by a stale reference is exact in floating point; a check keeps it far from overflow and hands the
 // rare tile that fails it to a two-pass path).  A line's first tile takes its reference from its own first 32 keys and the
 // ragged last tile its excluded keys as -inf, so both run in one pass too: 41 -> 37 us at 203 tokens, 168 -> 154 at 400,
-// 402 -> 367 at 600, 1.64 -> 1.56 ms at 1024 with masked keys; without masks and raggedness, at 1024, 1.414 -> 1.427 ms.  p goes back to TENSOR memory as
+// 402 -> 367 at 600, 1.62 -> 1.57 ms at 1024 with masked keys.  p goes back to TENSOR memory as
 // packed bf16, the A operand of O_g += P_g V_g^T.  The running output stays in tensor memory and is rescaled only
 // when a row maximum has grown by more than 2^8; row sums are kept in fp32 registers.
 // TMEM columns: S 4 x 64 | P 4 x 32 | O 4 x 32 = 512.  S and P are single-buffered; S is released as soon as its
@@ -167,6 +167,9 @@ struct IdleGuard {
     __device__ __forceinline__ void reset() { spins = 0; t0 = 0; }
 };
 
+// RAGGED: n is no multiple of a tile's keys.  Lines of whole tiles take a form without the tests for a short last one, which cost
+// them 2 to 5 % (1.505 -> 1.437 ms at 1024 tokens, 11.54 -> 10.97 at 2048, with masked keys 1.57 -> 1.53 at 1024).
+template <bool RAGGED>
 __global__ void __launch_bounds__(THREADS, 1)
 triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_vt, const __grid_constant__ CUtensorMap map_bias,
@@ -369,7 +372,7 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             for (int j = 0; j < T && ok; ++j, ++G) {
                 const uint32_t even = __ballot_sync(0xffffffffu, (vnext & 0x00ffu) != 0);    // bit l: key 2l attends
                 const uint32_t odd = __ballot_sync(0xffffffffu, (vnext & 0xff00u) != 0);     // bit l: key 2l+1 attends
-                const int left = n - j * AK;                 // keys of this tile that exist (at least one)
+                const int left = RAGGED ? n - j * AK : AK;   // keys of this tile that exist (at least one)
                 if (j + 1 < T) vnext = mask_fetch(mrow, j + 1);
                 ok = mbar_wait(&B->s_full[g], G & 1, abort_flag);
                 if (!ok) break;
@@ -563,12 +566,14 @@ extern "C" int b200pf_triatt_core_tc4(const b200pf_bf16* q, const b200pf_bf16* k
     }
     unsigned int* status = device_status_word();
     B200PF_REQUIRE(status, B200PF_ERR_CUDA, "triatt_core_tc4: no device status word");
-    B200PF_SMEM_ATTR_ONCE(triatt_core_tc4_kernel, SMEM_BYTES);
+    auto kern = n % AK != 0 ? triatt_core_tc4_kernel<true> : triatt_core_tc4_kernel<false>;
+    B200PF_SMEM_ATTR_ONCE(triatt_core_tc4_kernel<true>, SMEM_BYTES);
+    B200PF_SMEM_ATTR_ONCE(triatt_core_tc4_kernel<false>, SMEM_BYTES);
     int sms;
     if ((rc = multiprocessors(&sms)) != B200PF_OK) return rc;
     const long long items = (long long)((lines + NG - 1) / NG) * 4 * ((n + AQ - 1) / AQ);
     Args a{mask_lines, (__nv_bfloat16*)o, o_line_stride, o_pos_stride, mask_pitch, lines, n};
-    return launch_pdl(triatt_core_tc4_kernel, dim3((unsigned)(items < sms ? items : sms)), dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream,
+    return launch_pdl(kern, dim3((unsigned)(items < sms ? items : sms)), dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream,
                       mq, mk, mvt, mb, a, status);
 }
 
