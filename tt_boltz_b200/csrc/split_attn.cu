@@ -3,13 +3,14 @@
 //
 // mma.sync and not tcgen05: q, k, v rows are 24 or 32 wide and the probabilities need parts of their own, so a tcgen05 form
 // would have to push both through tensor memory; here they go from the accumulators of the first product straight into the
-// A fragments of the second.  A warp owns 16 queries; per 64-key tile it issues 96 MMAs against some 700 other
-// instructions.  With three bf16 parts and six MMAs per product, and every lane fetching its own bias values, a launch took 462 us
-// at 292 tokens x 4 heads and 528 at 256 x 8; with two parts 390 and 430, with staged bias tiles 310 and 311.  Neither the
-// tensor pipe nor memory bounds it now.  K and V tiles are shared by the CTA's warps, double buffered with cp.async; rows are
-// 64 bytes with the 16-byte chunks swizzled by row so that ldmatrix is
-// conflict free.  Bias tiles come with them, as whole lines (read by the lanes that want them, 8 bytes of eight rows at a
-// time and behind the tile before, they were the longest wait of a tile), and are the accumulators' initial values.
+// A fragments of the second.  A warp owns 16 queries; per 64-key tile it issues 96 MMAs.  With three bf16 parts and six MMAs per
+// product, and every lane fetching its own bias values, a launch took 462 us at 292 tokens x 4 heads and 528 at 256 x 8; with two
+// parts 390 and 430, with staged bias tiles 310 and 311, with one barrier a tile, interleaved accumulators, scores that stay in the
+// products' scale, packed fp32 arithmetic (1190 -> 745 instructions per warp and tile) and masks fetched a tile ahead 264 and 270.
+// K and V tiles are shared by the CTA's warps, double buffered with
+// cp.async; rows are 64 bytes with the 16-byte chunks swizzled by row so that ldmatrix is conflict free.  Bias tiles come with them,
+// as whole lines (read by the lanes that want them, 8 bytes of eight rows at a time and behind the tile before, they were the
+// longest wait of a tile), and are the accumulators' initial values.
 #include "split_attn.cuh"
 
 namespace b200pf {
@@ -18,7 +19,7 @@ namespace split {
 constexpr int KT = 64, KV_PART = KT * 64, KV_STAGE = 4 * KV_PART;          // K parts | V parts
 
 __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
@@ -30,7 +31,35 @@ __device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
 
 constexpr int BP = KT + 8;               // bias tile pitch in floats: a half-warp's float2 reads of four rows meet no bank twice
 constexpr int bias_stage(int nw) { return nw * 16 * BP * 4; }
-constexpr float P_SCALE = 16384.f;      // probabilities are at most one: their parts use the upper half of fp16's range
+constexpr float P_SHIFT = 14.f;          // probabilities are kept times 2^14: at most one, their parts use the upper half of fp16's range
+
+// Two fp32 values in one 64-bit register for the packed instructions (one issue slot, two results).
+__device__ __forceinline__ uint64_t f2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_get(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float m;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+    return m;
+}
 
 // 2^x of a score below the row's maximum.  PTX documents the instruction as an approximation good to some 2^-22 of its result, with
 // results below 2^-126 flushed to zero.  A row's largest probability is 1, so a flushed one is below 2^-126 of the row's sum, and each
@@ -64,46 +93,53 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
 
     const __half* base = p.qkv + (long long)line * p.line_rows * p.ld + h * HD;
     const long long pos_ld = p.pos_rows * p.ld;
+    const int qb = blockIdx.x * (NW * 16);
+    const float* brow = p.bias + h * p.bias_hs;
+    auto mask_term = [&](int kk) {
+        if (kk >= p.n_k) return -INFINITY;
+        return p.mask && p.mask[line * p.mask_ls + kk * p.mask_ks] == 0 ? p.mask_add : 0.f;
+    };
+    float m_next = tid < KT ? mask_term(tid) : 0.f;          // this thread's key of the next tile to be loaded, fetched a tile ahead
     auto load_tile = [&](int tile) {
         const int k0 = tile * KT;
-        const uint32_t st = smem_u32(at_smem + (tile & 1) * KV_STAGE);
-        for (int i = tid; i < 4 * KT * CH; i += NT) {
-            const int c = i % CH, key = (i / CH) % KT, part = i / (CH * KT);     // parts 0-1: K, 2-3: V
-            const int kk = k0 + key;
-            const bool in = kk < p.n_k;
-            const __half* src = base + (part >= 2 ? 2 * ht : ht) + (long long)(part & 1) * p.part_stride +
-                                       (in ? kk : 0) * pos_ld + c * 8;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(st + part * KV_PART + key * 64 + ((c ^ ((key >> 1) & 3)) << 4)),
-                         "l"(src), "r"(in ? 16 : 0) : "memory");
+        {   // K and V parts: four chunk slots per row (HD = 24 leaves the fourth out), NT / 4 rows at a time
+            const uint32_t st = smem_u32(at_smem + (tile & 1) * KV_STAGE);
+            const int c = tid & 3;
+            if (HD == 32 || c < CH) {
+#pragma unroll
+                for (int kr = 0; kr < KT; kr += NT / 4) {
+                    const int key = kr + (tid >> 2), kk = k0 + key;
+                    const bool in = kk < p.n_k;
+                    const __half* src = base + ht + (in ? kk : 0) * pos_ld + c * 8;
+                    const uint32_t dst = st + key * 64 + ((c ^ ((key >> 1) & 3)) << 4);
+#pragma unroll
+                    for (int part = 0; part < 4; ++part)                         // parts 0-1: K, 2-3: V
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + part * KV_PART),
+                                     "l"(src + (part >= 2 ? ht : 0) + (part & 1) * p.part_stride), "r"(in ? 16 : 0) : "memory");
+                }
+            }
         }
         const uint32_t bst = smem_u32(bias_s + (tile & 1) * bias_stage(NW));
-        const float* brow = p.bias + h * p.bias_hs;
-        const int qb = blockIdx.x * (NW * 16);
         if (p.bias_vec) {
-#pragma unroll 2
-            for (int i = tid; i < NW * 16 * (KT / 4); i += NT) {
-                const int c = (i % (KT / 4)) * 4, r = i / (KT / 4);
-                const bool in = k0 + c < p.n_k;
+            const int c = (tid % (KT / 4)) * 4, rt = tid / (KT / 4);
+            const bool in = k0 + c < p.n_k;
+            const float* src = brow + (in ? k0 + c : 0);
+#pragma unroll 4
+            for (int r = rt; r < NW * 16; r += NT / (KT / 4))
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(bst + (r * BP + c) * 4),
-                             "l"(brow + min(qb + r, p.n_q - 1) * p.bias_qs + (in ? k0 + c : 0)), "r"(in ? 16 : 0) : "memory");
-            }
+                             "l"(src + min(qb + r, p.n_q - 1) * p.bias_qs), "r"(in ? 16 : 0) : "memory");
         } else {
-#pragma unroll 1
-            for (int i = tid; i < NW * 16 * KT; i += NT) {
-                const int c = i % KT, r = i / KT;
-                const bool in = k0 + c < p.n_k;
+            const int c = tid % KT, rt = tid / KT;
+            const bool in = k0 + c < p.n_k;
+            const float* src = brow + (in ? k0 + c : 0);
+#pragma unroll 4
+            for (int r = rt; r < NW * 16; r += NT / KT)
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(bst + (r * BP + c) * 4),
-                             "l"(brow + min(qb + r, p.n_q - 1) * p.bias_qs + (in ? k0 + c : 0)), "r"(in ? 4 : 0) : "memory");
-            }
+                             "l"(src + min(qb + r, p.n_q - 1) * p.bias_qs), "r"(in ? 4 : 0) : "memory");
         }
-        if (tid < KT) {
-            const int kk = k0 + tid;
-            float m = 0.f;
-            if (kk >= p.n_k) m = -INFINITY;
-            else if (p.mask && p.mask[line * p.mask_ls + kk * p.mask_ks] == 0) m = p.mask_add;
-            mterm[(tile & 1) * KT + tid] = m;
-        }
+        if (tid < KT) mterm[(tile & 1) * KT + tid] = m_next;
         asm volatile("cp.async.commit_group;" ::: "memory");
+        if (tid < KT) m_next = mask_term(k0 + KT + tid);
     };
     load_tile(0);
 
@@ -123,101 +159,129 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
     float o[NE][4];
 #pragma unroll
     for (int e = 0; e < NE; ++e) { o[e][0] = o[e][1] = o[e][2] = o[e][3] = 0.f; }
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+    // Scores stay in the scaled domain of the products (qk is a power of two, so that moves no value); c0 / c1 are the rows'
+    // references as they enter the exponent, P_SHIFT minus the maximum so far, and l0 / l1 the sums of what they gave.
+    float c0 = INFINITY, c1 = INFINITY, mq0 = -INFINITY, mq1 = -INFINITY;
+    uint64_t l0 = f2(0.f, 0.f), l1 = l0;
     const int ntiles = (p.n_k + KT - 1) / KT;
     const float qk = p.qk_scale, qk_inv = 1.f / p.qk_scale;                      // powers of two
+    const uint64_t qk2 = f2(qk, qk), qk_inv2 = f2(qk_inv, qk_inv);
     const uint32_t k_lane = (uint32_t)((lane & 7) * 64), k_sw = (uint32_t)(((lane >> 3) ^ ((lane >> 1) & 3)) << 4);     // row lane & 7, chunk lane / 8
 
 #pragma unroll 1
     for (int tile = 0; tile < ntiles; ++tile) {
-        if (tile + 1 < ntiles) {
-            load_tile(tile + 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
+        // one barrier per tile: behind it this tile has arrived, and every warp is through the tile before, whose stage the
+        // next one overwrites
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
+        if (tile + 1 < ntiles) load_tile(tile + 1);
         if (active) {
             float s[8][4];
             const float* bt = reinterpret_cast<const float*>(bias_s + (tile & 1) * bias_stage(NW)) + (warp * 16 + g) * BP + 2 * t;
 #pragma unroll
             for (int ni = 0; ni < 8; ++ni) {
                 const float2 b0 = *reinterpret_cast<const float2*>(bt + 8 * ni), b1 = *reinterpret_cast<const float2*>(bt + 8 * BP + 8 * ni);
-                s[ni][0] = b0.x * qk; s[ni][1] = b0.y * qk; s[ni][2] = b1.x * qk; s[ni][3] = b1.y * qk;
+                f2_get(f2_mul(f2(b0.x, b0.y), qk2), s[ni][0], s[ni][1]);
+                f2_get(f2_mul(f2(b1.x, b1.y), qk2), s[ni][2], s[ni][3]);
             }
             const uint32_t kst = smem_u32(at_smem + (tile & 1) * KV_STAGE), vst = kst + 2 * KV_PART;
-            const float* mt = mterm + (tile & 1) * KT + 2 * t;
-            float mx0 = -INFINITY, mx1 = -INFINITY;
+            const float* mt = mterm + (tile & 1) * KT;
+            const float2 mine = *reinterpret_cast<const float2*>(mt + 2 * lane);
+            const bool masked = __any_sync(0xffffffffu, mine.x != 0.f || mine.y != 0.f);
 #pragma unroll
-            for (int ni = 0; ni < 8; ++ni) {
-                uint32_t kb[2][4];
+            for (int n2 = 0; n2 < 8; n2 += 2) {          // two column blocks at a time: their accumulators' chains interleave
+                uint32_t kb[2][2][4];
 #pragma unroll
-                for (int part = 0; part < 2; ++part) ldsm4(kb[part], kst + part * KV_PART + ni * 512 + k_lane + k_sw);
+                for (int u = 0; u < 2; ++u)
+#pragma unroll
+                    for (int part = 0; part < 2; ++part) ldsm4(kb[u][part], kst + part * KV_PART + (n2 + u) * 512 + k_lane + k_sw);
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks) {
-                    mma_f16(s[ni], q[1][ks], kb[0][2 * ks], kb[0][2 * ks + 1]);
-                    mma_f16(s[ni], q[0][ks], kb[1][2 * ks], kb[1][2 * ks + 1]);
-                    mma_f16(s[ni], q[0][ks], kb[0][2 * ks], kb[0][2 * ks + 1]);
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) mma_f16(s[n2 + u], q[1][ks], kb[u][0][2 * ks], kb[u][0][2 * ks + 1]);
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) mma_f16(s[n2 + u], q[0][ks], kb[u][1][2 * ks], kb[u][1][2 * ks + 1]);
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) mma_f16(s[n2 + u], q[0][ks], kb[u][0][2 * ks], kb[u][0][2 * ks + 1]);
                 }
-                const float2 mv = *reinterpret_cast<const float2*>(mt + 8 * ni);
-                s[ni][0] = fmaf(s[ni][0], qk_inv, mv.x); s[ni][1] = fmaf(s[ni][1], qk_inv, mv.y);
-                s[ni][2] = fmaf(s[ni][2], qk_inv, mv.x); s[ni][3] = fmaf(s[ni][3], qk_inv, mv.y);
-                mx0 = fmaxf(mx0, fmaxf(s[ni][0], s[ni][1]));
-                mx1 = fmaxf(mx1, fmaxf(s[ni][2], s[ni][3]));
             }
-            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+            if (masked) {
+#pragma unroll
+                for (int ni = 0; ni < 8; ++ni) {
+                    const float2 mv = *reinterpret_cast<const float2*>(mt + 8 * ni + 2 * t);
+                    s[ni][0] = fmaf(mv.x, qk, s[ni][0]); s[ni][1] = fmaf(mv.y, qk, s[ni][1]);
+                    s[ni][2] = fmaf(mv.x, qk, s[ni][2]); s[ni][3] = fmaf(mv.y, qk, s[ni][3]);
+                }
+            }
+            float mx0 = mq0, mx1 = mq1;
+#pragma unroll
+            for (int ni = 0; ni < 8; ++ni) {
+                mx0 = max3(mx0, s[ni][0], s[ni][1]);
+                mx1 = max3(mx1, s[ni][2], s[ni][3]);
+            }
+            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
             // every tile holds a key inside n_k, whose score is finite: the new maxima are finite
-            const float n0 = fmaxf(m0, mx0), n1 = fmaxf(m1, mx1);
-            const float a0 = exp2f(m0 - n0), a1 = exp2f(m1 - n1);                // 0 on the first tile
-            m0 = n0; m1 = n1;
-            l0 *= a0; l1 *= a1;
+            mq0 = mx0; mq1 = mx1;
+            // rounded down: no exponent may pass P_SHIFT, however large the scores, or a part would overflow
+            const float d0 = __fmaf_rd(-mx0, qk_inv, P_SHIFT), d1 = __fmaf_rd(-mx1, qk_inv, P_SHIFT);
+            const float a0 = exp2f(d0 - c0), a1 = exp2f(d1 - c1);                // 0 on the first tile
+            c0 = d0; c1 = d1;
+            const uint64_t c02 = f2(d0, d0), c12 = f2(d1, d1), a02 = f2(a0, a0), a12 = f2(a1, a1);
+            l0 = f2_mul(l0, a02); l1 = f2_mul(l1, a12);
             float ot[NE][4];
 #pragma unroll
             for (int e = 0; e < NE; ++e) { ot[e][0] = ot[e][1] = ot[e][2] = ot[e][3] = 0.f; }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {                                        // 16 keys
-                uint32_t pf[2][4];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    float* sv = s[2 * j + u];
-                    sv[0] = prob(sv[0] - n0); sv[1] = prob(sv[1] - n0); sv[2] = prob(sv[2] - n1); sv[3] = prob(sv[3] - n1);
-                    l0 += sv[0] + sv[1]; l1 += sv[2] + sv[3];
-                    split_f16x2(sv[0] * P_SCALE, sv[1] * P_SCALE, pf[0][2 * u], pf[1][2 * u]);
-                    split_f16x2(sv[2] * P_SCALE, sv[3] * P_SCALE, pf[0][2 * u + 1], pf[1][2 * u + 1]);
-                }
                 // matrices: (keys 0-7, chunk), (keys 8-15, chunk), (keys 0-7, chunk + 1), (keys 8-15, chunk + 1)
                 const int key = j * 16 + ((lane >> 3) & 1) * 8 + (lane & 7);
+                uint32_t vb[2][2][4];
 #pragma unroll
-                for (int c2 = 0; c2 < 2; ++c2) {
-                    uint32_t vb[2][4];
-                    const uint32_t off = (uint32_t)(key * 64 + (((c2 * 2 + (lane >> 4)) ^ ((key >> 1) & 3)) << 4));
+                for (int c2 = 0; c2 < 2; ++c2)
 #pragma unroll
-                    for (int part = 0; part < 2; ++part) ldsm4_t(vb[part], vst + part * KV_PART + off);
+                    for (int part = 0; part < 2; ++part)
+                        ldsm4_t(vb[c2][part], vst + part * KV_PART + (uint32_t)(key * 64 + (((c2 * 2 + (lane >> 4)) ^ ((key >> 1) & 3)) << 4)));
+                uint32_t pf[2][4];
 #pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        if (c2 * 2 + u >= NE) continue;
-                        float (&oe)[4] = ot[(c2 * 2 + u) % NE];
-                        mma_f16(oe, pf[1], vb[0][2 * u], vb[0][2 * u + 1]);
-                        mma_f16(oe, pf[0], vb[1][2 * u], vb[1][2 * u + 1]);
-                        mma_f16(oe, pf[0], vb[0][2 * u], vb[0][2 * u + 1]);
+                for (int u = 0; u < 2; ++u)
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const float* sv = s[2 * j + u] + 2 * r;
+                        float x0, x1;
+                        f2_get(f2_fma(f2(sv[0], sv[1]), qk_inv2, r ? c12 : c02), x0, x1);
+                        const float p0 = prob(x0), p1 = prob(x1);
+                        if (r) l1 = f2_add(l1, f2(p0, p1));
+                        else l0 = f2_add(l0, f2(p0, p1));
+                        split_f16x2(p0, p1, pf[0][2 * u + r], pf[1][2 * u + r]);
                     }
-                }
+#pragma unroll
+                for (int e = 0; e < NE; ++e) mma_f16(ot[e], pf[1], vb[e >> 1][0][2 * (e & 1)], vb[e >> 1][0][2 * (e & 1) + 1]);
+#pragma unroll
+                for (int e = 0; e < NE; ++e) mma_f16(ot[e], pf[0], vb[e >> 1][1][2 * (e & 1)], vb[e >> 1][1][2 * (e & 1) + 1]);
+#pragma unroll
+                for (int e = 0; e < NE; ++e) mma_f16(ot[e], pf[0], vb[e >> 1][0][2 * (e & 1)], vb[e >> 1][0][2 * (e & 1) + 1]);
             }
             // the tensor core truncates every addend to the running sum's ulp, always towards zero: a tile's products start
             // from zero and join the output with a rounded FMA
 #pragma unroll
             for (int e = 0; e < NE; ++e) {
-                o[e][0] = fmaf(o[e][0], a0, ot[e][0]); o[e][1] = fmaf(o[e][1], a0, ot[e][1]);
-                o[e][2] = fmaf(o[e][2], a1, ot[e][2]); o[e][3] = fmaf(o[e][3], a1, ot[e][3]);
+                f2_get(f2_fma(f2(o[e][0], o[e][1]), a02, f2(ot[e][0], ot[e][1])), o[e][0], o[e][1]);
+                f2_get(f2_fma(f2(o[e][2], o[e][3]), a12, f2(ot[e][2], ot[e][3])), o[e][2], o[e][3]);
             }
         }
-        __syncthreads();
     }
     if (!active) return;
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-    const float inv[2] = {1.f / (l0 * P_SCALE), 1.f / (l1 * P_SCALE)};
+    float inv[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        float x, y;
+        f2_get(r ? l1 : l0, x, y);
+        x += y;
+        x += __shfl_xor_sync(0xffffffffu, x, 1);
+        x += __shfl_xor_sync(0xffffffffu, x, 2);
+        inv[r] = 1.f / x;
+    }
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const int qi = qw + g + 8 * half;
