@@ -318,14 +318,15 @@ class B200MSALayer(nn.Module):
         self.outer_product_mean = B200OuterProductMean(c_in=msa_s, c_hidden=32, c_out=token_z)
 
     def forward_inplace(self, z: torch.Tensor, m: torch.Tensor, token_mask: torch.Tensor, msa_mask: torch.Tensor,
-                        ws_cache: Optional[dict] = None) -> None:
+                        ws_cache: Optional[dict] = None, masks=None) -> None:
         """z [N, N, 128] and m [S, N, 64], contiguous fp32, updated where they are; token_mask [N, N], msa_mask [S, N].
-        ``ws_cache``: a dict that the blocks of one call share, for the pair block's workspace."""
+        ``ws_cache``: a dict that the blocks of one call share, for the pair block's workspace; ``masks``: token_mask
+        as ``ops.PairMasks``, which they share too."""
         from .pairformer import _run_layers
         self.pair_weighted_averaging.add_into(m, z, token_mask)
         self.msa_transition.add_into(m)
         self.outer_product_mean.add_into(z, m, msa_mask)
-        _run_layers([self.pairformer_layer], None, z, None, token_mask[None], ws_cache, inplace=True)
+        _run_layers([self.pairformer_layer], None, z, None, token_mask[None], ws_cache, inplace=True, masks=masks)
 
     def forward(self, z: torch.Tensor, m: torch.Tensor, token_mask: torch.Tensor, msa_mask: torch.Tensor,
                 chunk_heads_pwa: bool = False, chunk_size_transition_z: Optional[int] = None,
@@ -343,11 +344,15 @@ class B200MSALayer(nn.Module):
 
 
 def _run_blocks(layers, z: torch.Tensor, m: torch.Tensor, token_mask: torch.Tensor, msa_mask: torch.Tensor) -> None:
-    """Every block on the resident z and m; what all blocks share (masks as uint8, the pair block's workspace) made once."""
+    """Every block on the resident z and m; what all blocks share (masks in the kernels' forms, the pair block's workspace) made
+    once: the pair mask's two padded forms are six small launches, 25 us a block at 171 tokens."""
+    from . import ops
+    from .pairformer import _mask_u8
     with torch.no_grad():
         pair_u8, msa_u8, ws_cache = _u8(token_mask), _u8(msa_mask), {}
+        masks = ops.PairMasks(_mask_u8(pair_u8, tuple(z.shape[:2]), z.device))
         for layer in layers:
-            layer.forward_inplace(z, m, pair_u8, msa_u8, ws_cache)
+            layer.forward_inplace(z, m, pair_u8, msa_u8, ws_cache, masks)
 
 
 class B200MSAStack(nn.Module):

@@ -348,9 +348,11 @@ def _side_track_wanted(n: int) -> bool:
     return forced == "1" if forced is not None else n <= SIDE_TRACK_TOKENS
 
 
-def _run_layers(layers, s, z, mask, pair_mask, ws_cache: Optional[dict] = None, inplace: bool = False):
+def _run_layers(layers, s, z, mask, pair_mask, ws_cache: Optional[dict] = None, inplace: bool = False,
+                masks: Optional[ops.PairMasks] = None):
     """``inplace``: s [N, c_s] and z [N, N, C] are the caller's fp32 contiguous working tensors and are updated
-    where they are (nothing is returned); otherwise [1, ...] inputs are copied and new tensors returned."""
+    where they are (nothing is returned); otherwise [1, ...] inputs are copied and new tensors returned.
+    ``masks``: the pair mask as the kernels take it, from a caller that makes it once for several calls."""
     if not z.is_cuda:
         raise RuntimeError("B200 Pairformer: inputs must be CUDA tensors (there is no CPU path)")
     if inplace:
@@ -367,7 +369,7 @@ def _run_layers(layers, s, z, mask, pair_mask, ws_cache: Optional[dict] = None, 
         else:
             zw = z[0].to(torch.float32).clone(memory_format=torch.contiguous_format)
             sw = None if s is None else s[0].to(torch.float32).clone(memory_format=torch.contiguous_format)
-        pm = ops.PairMasks(_mask_u8(pair_mask, (n, n), z.device))
+        pm = masks if masks is not None else ops.PairMasks(_mask_u8(pair_mask, (n, n), z.device))
         tm = _mask_u8(mask, (n,), z.device) if s is not None else None
         ws, capturing = None, torch.cuda.is_current_stream_capturing()
         if capturing:
