@@ -16,11 +16,14 @@
 //                 bf16 rows of the A tile: on the loader warps, one per scheduler, the same work
 //                 doubled the time of the whole kernel.
 // Output goes TMEM -> registers -> a swizzled staging tile -> TMA stores, so that global memory
-// only ever sees full, contiguous lines (thread-per-row 16-byte stores were 3x slower).
+// only ever sees full, contiguous lines (thread-per-row 16-byte stores were 3x slower).  Every epilogue
+// warp has a staging tile and stores of its own: no warp waits for another.
 // Roles (416 threads): warps 0-3 LayerNorm loaders (32 rows each), warp 4 MMA issuer, warps 5-12
 // epilogue (two warps per TMEM lane quarter, each taking half of the columns).  TMEM is used as
 // two halves of 256 columns so the epilogue of one half overlaps the MMAs of the next, and the x
-// tile is double buffered so the loaders run a tile ahead.
+// tile is double buffered so the loaders run a tile ahead.  A CTA's first tile is normalised by the
+// epilogue warps, 16 rows each, which have nothing else to do before its accumulators exist; the
+// loaders begin with the second.
 #include "mxfp8.cuh"
 #include "row512_tc.h"
 #include "rowtc.cuh"
@@ -36,9 +39,9 @@ constexpr int LOAD_WARPS = 4, MMA_WARP = 4, EPI_WARP0 = 5, EPI_WARPS = 8, THREAD
 constexpr int W_BYTES = 512 * 128 * 2;                 // two k-blocks of [512][128 B]
 constexpr int W_KB = 512 * 128;
 constexpr int OFF_A = W_BYTES;                          // 2 stages x 32 KB
-constexpr int OFF_STG = OFF_A + 2 * A_TILE_BYTES;       // output staging: 2 boxes of [128 rows][128 B], 128-byte swizzle
-constexpr int STG_BOX = 128 * 128;
-constexpr int OFF_WB = OFF_STG + 2 * STG_BOX;           // triangle-bias rows [4][128] fp32
+constexpr int OFF_STG = OFF_A + 2 * A_TILE_BYTES;       // output staging: per epilogue warp [32 rows][128 B], 128-byte swizzle
+constexpr int STG_BOX = 32 * 128;
+constexpr int OFF_WB = OFF_STG + EPI_WARPS * STG_BOX;           // triangle-bias rows [4][128] fp32
 constexpr int OFF_BAR = OFF_WB + 4 * 128 * 4;
 constexpr int SMEM_BYTES = OFF_BAR + 128;               // 231,552: the dynamic window must start 1024-byte aligned
 constexpr int EPI_BAR_ID = 1;
@@ -99,6 +102,10 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         fence_barrier_init();
         fence_proxy_async();
     }
+    if (tid == 32) {
+        tma_prefetch_desc(&map_w); tma_prefetch_desc(&map0); tma_prefetch_desc(&map1);
+        if (MODE == MODE_TRIATT) { tma_prefetch_desc(&map2); tma_prefetch_desc(&map3); }
+    }
     if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
     grid_dependency_wait();
     grid_launch_dependents();
@@ -118,18 +125,100 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         return p.transposed ? (long long)pos * p.n + line : (long long)line * p.n + pos;
     };
 
-    if (warp < LOAD_WARPS) {
-        // ---------------------------- LayerNorm loaders ----------------------------
-        const int sub = lane & 7, rq = lane >> 3;
-        float4 gam[4], bet[4];
+    // One warp's 16 rows of a tile: LayerNorm of positions pos0 + row0 .. of line `line` into the A tile; 8 lanes per row.
+    const int sub = lane & 7, rq = lane >> 3;
+    auto normalise16 = [&](int line, int pos0, int row0, uint8_t* a_tile, const float4 (&gam)[4], const float4 (&bet)[4]) {
+        float4 v[4][4];
+        // rows 4 i of the pass: one flat index and a stride (positions of a column lie n rows apart)
+        const int pos_b = pos0 + row0 + rq;
+        const long long f0 = p.transposed ? (long long)pos_b * p.n + line : (long long)line * p.n + pos_b;
+        const long long fstep = p.transposed ? 4LL * p.n : 4LL;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const bool valid = pos_b + i * 4 < span;
+            if (p.z_bf16) {          // warp-uniform: four bf16 channels per lane and j, widened on the fly
+                const uint2* src = reinterpret_cast<const uint2*>(p.z_bf16 + (f0 + i * fstep) * KC) + sub;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint2 w = valid ? src[j * 8] : make_uint2(0u, 0u);
+                    v[i][j] = make_float4(bf16_lo(w.x), bf16_hi(w.x), bf16_lo(w.y), bf16_hi(w.y));
+                }
+            } else {
+                const float4* src = reinterpret_cast<const float4*>(p.z + (f0 + i * fstep) * KC) + sub;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[i][j] = valid ? src[j * 8] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+        // The four rows of a pass are worked on stage by stage (all sums, then all shuffles, ...), not row by
+        // row: one loader warp per scheduler has nothing else to hide a dependent chain behind.
+        float kz[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            bool keep = pos_b + i * 4 < span;
+            if (MODE != MODE_TRIATT) keep = keep && p.mask[f0 + i * fstep] != 0;
+            kz[i] = keep ? 1.f : 0.f;
+        }
+        float s4[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s += (v[i][j].x + v[i][j].y) + (v[i][j].z + v[i][j].w);
+            s4[i] = s;
+        }
+#pragma unroll
+        for (int step = 1; step < 8; step <<= 1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s4[i] += __shfl_xor_sync(0xffffffffu, s4[i], step);
+        float ss4[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float mean = s4[i] * (1.f / KC);
+            float ss = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[i][j].x -= mean; v[i][j].y -= mean; v[i][j].z -= mean; v[i][j].w -= mean;
+                ss += (v[i][j].x * v[i][j].x + v[i][j].y * v[i][j].y) + (v[i][j].z * v[i][j].z + v[i][j].w * v[i][j].w);
+            }
+            ss4[i] = ss;
+        }
+#pragma unroll
+        for (int step = 1; step < 8; step <<= 1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ss4[i] += __shfl_xor_sync(0xffffffffu, ss4[i], step);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = row0 + i * 4 + rq;
+            const float rstd = rsqrtf(ss4[i] * (1.f / KC) + LN_EPS);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[i][j].x = fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x) * kz[i];
+                v[i][j].y = fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y) * kz[i];
+                v[i][j].z = fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z) * kz[i];
+                v[i][j].w = fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w) * kz[i];
+                uint2 o;
+                o.x = pack_bf16x2(v[i][j].x, v[i][j].y);
+                o.y = pack_bf16x2(v[i][j].z, v[i][j].w);
+                const int chunk = (j & 1) * 4 + (sub >> 1);
+                *reinterpret_cast<uint2*>(a_tile + (j >> 1) * A_KB_BYTES + sw128(row, chunk) + (sub & 1) * 8) = o;
+            }
+        }
+    };
+    auto load_affine = [&](float4 (&gam)[4], float4 (&bet)[4]) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             gam[j] = reinterpret_cast<const float4*>(p.ln_gamma)[j * 8 + sub];
             bet[j] = reinterpret_cast<const float4*>(p.ln_beta)[j * 8 + sub];
         }
-        uint32_t it = 0;
+    };
+
+    if (warp < LOAD_WARPS) {
+        // ---------------------------- LayerNorm loaders ----------------------------
+        float4 gam[4], bet[4];
+        load_affine(gam, bet);
+        uint32_t it = 1;                    // the epilogue warps normalise the CTA's first tile
         bool ok = true;
-        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
+        for (int t = (int)(blockIdx.x + gridDim.x); t < tiles && ok; t += gridDim.x, ++it) {
             const int line = t / tpl, pos0 = (t - line * tpl) * TM;
             const uint32_t stage = it & 1, ph = (it >> 1) & 1;
             ok = mbar_wait(&B->a_empty[stage], ph ^ 1, abort_flag);
@@ -156,82 +245,7 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
             }
 #pragma unroll 1
             for (int pass = 0; pass < 2; ++pass) {
-                const int row0 = warp * 32 + pass * 16;
-                float4 v[4][4];
-                // rows 4 i of the pass: one flat index and a stride (positions of a column lie n rows apart)
-                const int pos_b = pos0 + row0 + rq;
-                const long long f0 = p.transposed ? (long long)pos_b * p.n + line : (long long)line * p.n + pos_b;
-                const long long fstep = p.transposed ? 4LL * p.n : 4LL;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const bool valid = pos_b + i * 4 < span;
-                    if (p.z_bf16) {          // warp-uniform: four bf16 channels per lane and j, widened on the fly
-                        const uint2* src = reinterpret_cast<const uint2*>(p.z_bf16 + (f0 + i * fstep) * KC) + sub;
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const uint2 w = valid ? src[j * 8] : make_uint2(0u, 0u);
-                            v[i][j] = make_float4(bf16_lo(w.x), bf16_hi(w.x), bf16_lo(w.y), bf16_hi(w.y));
-                        }
-                    } else {
-                        const float4* src = reinterpret_cast<const float4*>(p.z + (f0 + i * fstep) * KC) + sub;
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) v[i][j] = valid ? src[j * 8] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
-                }
-                // The four rows of a pass are worked on stage by stage (all sums, then all shuffles, ...), not row by
-                // row: one loader warp per scheduler has nothing else to hide a dependent chain behind.
-                float kz[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    bool keep = pos_b + i * 4 < span;
-                    if (MODE != MODE_TRIATT) keep = keep && p.mask[f0 + i * fstep] != 0;
-                    kz[i] = keep ? 1.f : 0.f;
-                }
-                float s4[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    float s = 0.f;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) s += (v[i][j].x + v[i][j].y) + (v[i][j].z + v[i][j].w);
-                    s4[i] = s;
-                }
-#pragma unroll
-                for (int step = 1; step < 8; step <<= 1)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) s4[i] += __shfl_xor_sync(0xffffffffu, s4[i], step);
-                float ss4[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float mean = s4[i] * (1.f / KC);
-                    float ss = 0.f;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        v[i][j].x -= mean; v[i][j].y -= mean; v[i][j].z -= mean; v[i][j].w -= mean;
-                        ss += (v[i][j].x * v[i][j].x + v[i][j].y * v[i][j].y) + (v[i][j].z * v[i][j].z + v[i][j].w * v[i][j].w);
-                    }
-                    ss4[i] = ss;
-                }
-#pragma unroll
-                for (int step = 1; step < 8; step <<= 1)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) ss4[i] += __shfl_xor_sync(0xffffffffu, ss4[i], step);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int row = row0 + i * 4 + rq;
-                    const float rstd = rsqrtf(ss4[i] * (1.f / KC) + LN_EPS);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        v[i][j].x = fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x) * kz[i];
-                        v[i][j].y = fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y) * kz[i];
-                        v[i][j].z = fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z) * kz[i];
-                        v[i][j].w = fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w) * kz[i];
-                        uint2 o;
-                        o.x = pack_bf16x2(v[i][j].x, v[i][j].y);
-                        o.y = pack_bf16x2(v[i][j].z, v[i][j].w);
-                        const int chunk = (j & 1) * 4 + (sub >> 1);
-                        *reinterpret_cast<uint2*>(a_tile + (j >> 1) * A_KB_BYTES + sw128(row, chunk) + (sub & 1) * 8) = o;
-                    }
-                }
+                normalise16(line, pos0, warp * 32 + pass * 16, a_tile, gam, bet);
             }
             fence_proxy_async();
             __syncwarp();
@@ -280,12 +294,22 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
     } else {
         // ---------------------------- epilogue ----------------------------
         // Each round moves one [128 x 128] bf16 block out: TMEM -> registers -> swizzled staging tile
-        // -> two TMA stores of [128 rows x 64 elements], so global memory only sees full lines.
+        // -> a TMA store of [32 rows x 64 elements] per warp, so global memory only sees full lines.
         const int quarter = warp & 3, chalf = (warp - EPI_WARP0) >> 2;
-        const int epi_tid = threadIdx.x - EPI_WARP0 * 32;
+        if ((int)blockIdx.x < tiles) {
+            // the first tile's LayerNorm, 16 rows a warp.  At 45 tokens, one tile per CTA, four loader warps in two passes each
+            // took 3.6 of the kernel's 9 us.
+            float4 gam[4], bet[4];
+            load_affine(gam, bet);
+            const int line = (int)blockIdx.x / tpl;
+            normalise16(line, ((int)blockIdx.x - line * tpl) * TM, (warp - EPI_WARP0) * 16, smem + OFF_A, gam, bet);
+            fence_proxy_async();
+            named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
+            if (warp - EPI_WARP0 < LOAD_WARPS && lane == 0) mbar_arrive(&B->a_full[0]);       // the loaders' arrivals of this phase
+        }
         const int lrow = quarter * 32 + lane;                     // TMEM lane of this thread = staging row
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
-        uint8_t* stg = smem + OFF_STG;
+        uint8_t* stg = smem + OFF_STG + (warp - EPI_WARP0) * STG_BOX;
         uint32_t acc_cnt = 0;
         bool ok = true;
         // tanh_mode: 0 = copy, 1 = p' + p' * tanh(g')  (gate columns at +128), 2 = 0.5 + 0.5 * tanh(x)
@@ -313,21 +337,21 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
                 w[e] = pack_bf16x2(v0, v1);
             }
         };
-        auto store_round = [&](const uint4 (&o)[8], const CUtensorMap* map, int c0, int c1, int c2, int c3) {
-            if (epi_tid == 0) bulk_wait_read0();               // the previous round's stores have read the staging tile
-            named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
+        // This warp's 32 staging rows x 128 bytes; `inside`: the box is not wholly beyond the tensor's edge.
+        auto store_round = [&](const uint4 (&o)[8], const CUtensorMap* map, bool inside, int c0, int c1, int c2, int c3) {
+            if (lane == 0) bulk_wait_read0();                  // this warp's previous store has read the staging tile
+            __syncwarp();
 #pragma unroll
-            for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(stg + chalf * STG_BOX + sw128(lrow, j)) = o[j];
+            for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(stg + sw128(lane, j)) = o[j];
             fence_proxy_async();
-            named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
-            if (epi_tid == 0) {
+            __syncwarp();
+            if (lane == 0 && inside) {
                 tma_store_4d(map, stg, c0, c1, c2, c3);
-                tma_store_4d(map, stg + STG_BOX, c0 + 64, c1, c2, c3);
                 bulk_commit();
             }
         };
         for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++acc_cnt) {
-            const int line = t / tpl, pos0 = (t - line * tpl) * TM;
+            const int line = t / tpl, pos0 = (t - line * tpl) * TM, pos_w = pos0 + quarter * 32;
             for (int half = 0; half < 2 && ok; ++half) {
                 ok = mbar_wait(&B->acc_full[half], acc_cnt & 1, abort_flag);
                 if (!ok) break;
@@ -362,21 +386,23 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
                     }
                     *reinterpret_cast<uint16_t*>(p.scales[half] + mx::scale_offset(lrow, line, (pos0 >> 5) + chalf * 2,
                                                                                    p.sf_kgroups, p.sf_row_blocks)) = (uint16_t)sc;
-                    if (epi_tid == 0) bulk_wait_read0();
-                    named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
+                    if (lane == 0) bulk_wait_read0();
+                    __syncwarp();
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(stg + sw128(lrow, chalf * 4 + j)) = o[j];
+                    for (int j = 0; j < 4; ++j)               // 64-byte rows, 64-byte swizzle
+                        *reinterpret_cast<uint4*>(stg + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = o[j];
                     fence_proxy_async();
-                    named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
-                    if (epi_tid == 0) {
-                        tma_store_4d(half == 0 ? &map0 : &map1, stg, pos0, line, 0, 0);
+                    __syncwarp();
+                    if (lane == 0 && pos0 + chalf * 64 < p.pitch) {
+                        tma_store_4d(half == 0 ? &map0 : &map1, stg, pos0 + chalf * 64, line, quarter * 32, 0);
                         bulk_commit();
                     }
                 } else if (MODE == MODE_TRIMUL) {
                     // lane = channel of operand `half`, columns = positions; this warp's 64 positions = box `chalf`
                     load64(tbase + chalf * 64, 1, o);
                     const int rg = p.row_group[half];
-                    store_round(o, half == 0 ? &map0 : &map1, pos0, line % rg, 0, line / rg);
+                    const int c0 = pos0 + chalf * 64;
+                    store_round(o, half == 0 ? &map0 : &map1, c0 < p.pitch, c0, line % rg, quarter * 32, line / rg);
                 } else if (half == 0) {
                     {   // The 4 triangle-bias heads of this tile, from the normalised bf16 rows still in the A tile (the
                         // accumulator being ready means the loaders' writes are visible): thread = position `lrow`,
@@ -411,22 +437,22 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
                     }
                     // lane = position, columns = channels of q then k; box `chalf` = channels 64*chalf ..
                     load64(tbase + chalf * 64, 0, o);
-                    store_round(o, &map0, 0, pos0, line, 0);
+                    store_round(o, &map0, pos_w < span, chalf * 64, pos_w, line, 0);
                     load64(tbase + 128 + chalf * 64, 0, o);
-                    store_round(o, &map1, 0, pos0, line, 0);
+                    store_round(o, &map1, pos_w < span, chalf * 64, pos_w, line, 0);
                 } else {
                     load64(tbase + chalf * 64, 2, o);                       // gate: sigmoid
-                    if (p.transposed) store_round(o, &map2, 0, line, pos0, 0);
-                    else store_round(o, &map2, 0, pos0, line, 0);
+                    if (p.transposed) store_round(o, &map2, pos_w < span, chalf * 64, line, pos_w, 0);
+                    else store_round(o, &map2, pos_w < span, chalf * 64, pos_w, line, 0);
                     load64(tbase + 128 + chalf * 64, 0, o);                 // v^T: lane = v channel, columns = positions
-                    store_round(o, &map3, pos0, 0, line, 0);
+                    store_round(o, &map3, pos0 + chalf * 64 < p.vt_pitch, pos0 + chalf * 64, quarter * 32, line, 0);
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&B->acc_empty[half]);
             }
         }
-        if (epi_tid == 0) bulk_wait0();
+        if (lane == 0) bulk_wait0();
         if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
     }
     tc_fence_before();
@@ -442,8 +468,8 @@ static int make_maps(int mode, const Args& a, CUtensorMap (&m)[4]) {
         for (int i = 0; i < 2; ++i) {     // byte planes [d][line][pitch]
             cuuint64_t dims[4] = {(cuuint64_t)a.pitch, (cuuint64_t)lines, 128, 1};
             cuuint64_t str[3] = {(cuuint64_t)a.pitch, (cuuint64_t)a.plane_stride[i], (cuuint64_t)a.plane_stride[i] * 128};
-            cuuint32_t box[4] = {128, 1, 128, 1};
-            if ((rc = tmap_encode(&m[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, a.planes[i], 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B,
+            cuuint32_t box[4] = {64, 1, 32, 1};
+            if ((rc = tmap_encode(&m[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, a.planes[i], 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_64B,
                                   "mx planes")) != B200PF_OK) return rc;
         }
         m[2] = m[0];
@@ -456,7 +482,7 @@ static int make_maps(int mode, const Args& a, CUtensorMap (&m)[4]) {
             cuuint64_t dims[4] = {(cuuint64_t)a.pitch, (cuuint64_t)(rg < lines ? rg : lines), 128, (cuuint64_t)groups};
             cuuint64_t str[3] = {(cuuint64_t)a.pitch * 2, (cuuint64_t)a.plane_stride[i] * 2,
                                  (cuuint64_t)(groups > 1 ? a.group_stride[i] : a.plane_stride[i] * 128) * 2};
-            cuuint32_t box[4] = {64, 1, 128, 1};
+            cuuint32_t box[4] = {64, 1, 32, 1};
             if ((rc = tmap_encode(&m[i], bf, a.planes[i], 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, "planes")) != B200PF_OK) return rc;
         }
         m[2] = m[0];
@@ -466,20 +492,20 @@ static int make_maps(int mode, const Args& a, CUtensorMap (&m)[4]) {
     {   // q, k: [line][pos][128]
         cuuint64_t dims[4] = {128, (cuuint64_t)span, (cuuint64_t)lines, 1};
         cuuint64_t str[3] = {256, (cuuint64_t)span * 256, (cuuint64_t)span * 256 * lines};
-        cuuint32_t box[4] = {64, 128, 1, 1};
+        cuuint32_t box[4] = {64, 32, 1, 1};
         if ((rc = tmap_encode(&m[0], bf, a.q, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, "q")) != B200PF_OK) return rc;
         if ((rc = tmap_encode(&m[1], bf, a.k, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, "k")) != B200PF_OK) return rc;
     }
     {   // g in the layout of the z view [rows][n][128]
         cuuint64_t dims[4] = {128, (cuuint64_t)a.n, (cuuint64_t)a.rows, 1};
         cuuint64_t str[3] = {256, (cuuint64_t)a.n * 256, (cuuint64_t)a.n * 256 * a.rows};
-        cuuint32_t box_rows[4] = {64, 128, 1, 1}, box_cols[4] = {64, 1, 128, 1};
+        cuuint32_t box_rows[4] = {64, 32, 1, 1}, box_cols[4] = {64, 1, 32, 1};
         if ((rc = tmap_encode(&m[2], bf, a.g, 4, dims, str, a.transposed ? box_cols : box_rows, CU_TENSOR_MAP_SWIZZLE_128B, "g")) != B200PF_OK) return rc;
     }
     {   // v transposed: [line][head*32 + d][vt_pitch]
         cuuint64_t dims[4] = {(cuuint64_t)a.vt_pitch, 128, (cuuint64_t)lines, 1};
         cuuint64_t str[3] = {(cuuint64_t)a.vt_pitch * 2, (cuuint64_t)a.vt_pitch * 256, (cuuint64_t)a.vt_pitch * 256 * lines};
-        cuuint32_t box[4] = {64, 128, 1, 1};
+        cuuint32_t box[4] = {64, 32, 1, 1};
         if ((rc = tmap_encode(&m[3], bf, a.v, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, "vt")) != B200PF_OK) return rc;
     }
     return B200PF_OK;
