@@ -9,8 +9,10 @@
 // The gate GEMM uses LN_in(z) (affine applied by the loader warps) against 0.5 * W_gout, so that
 // p * sigmoid(g) = p' + p' * tanh(g').  The fp32 update leaves through TMA reduce-add straight
 // into z: the kernel never reads z for the residual.
-// Roles (416 threads): warps 0-3 loaders (LN of z rows, x statistics, TMA issue), warp 4 MMA issuer,
-// warps 5-12 epilogue.
+// Roles (416 threads): warps 0-3 loaders (LN of z rows, TMA issue), warp 4 MMA issuer, warps 5-12 epilogue (x statistics, gate,
+// update; each with a staging tile and reductions of its own, so that no warp waits for another).  A CTA's first tile is
+// normalised by the epilogue warps, 16 rows each, which have nothing else to do before its accumulators exist; the loaders begin
+// with the second.
 #include "rowtc.cuh"
 #include "tmap.cuh"
 
@@ -25,12 +27,11 @@ constexpr int OFF_WP = 0, OFF_WG = W_TILE;               // 0.5 * W_pout * gamma
 constexpr int OFF_AZ = 2 * W_TILE;                       // 2 stages
 constexpr int OFF_XT = OFF_AZ + 2 * A_TILE_BYTES;        // 1 stage: 2 boxes of [128 d][64 pos]
 constexpr int XT_BOX = 128 * 128;
-constexpr int OFF_STG = OFF_XT + 2 * XT_BOX;             // staging: 2 boxes of [128 pos][32 fp32], 128-byte swizzle
-constexpr int STG_BOX = 128 * 128, STG_BUF = 2 * STG_BOX;
-constexpr int OFF_CONST = OFF_STG + STG_BUF;             // wsum[128], wb[128] fp32
-constexpr int OFF_STATS = OFF_CONST + 1024;              // [2][128] float2 (mean, rstd)
-constexpr int OFF_BAR = OFF_STATS + 2048;
-constexpr int SMEM_BYTES = OFF_BAR + 128;                // 199,808; the dynamic window must start 1024-byte aligned
+constexpr int OFF_STG = OFF_XT + 2 * XT_BOX;             // staging: per epilogue warp [32 pos][32 fp32], 128-byte swizzle
+constexpr int STG_BOX = 32 * 128;
+constexpr int OFF_CONST = OFF_STG + EPI_WARPS * STG_BOX; // wsum[128], wb[128] fp32
+constexpr int OFF_BAR = OFF_CONST + 1024;
+constexpr int SMEM_BYTES = OFF_BAR + 128;                // 197,760; the dynamic window must start 1024-byte aligned
 static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 constexpr int EPI_BAR_ID = 1;
 
@@ -97,6 +98,7 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
         fence_barrier_init();
         fence_proxy_async();
     }
+    if (tid == 32) { tma_prefetch_desc(&map_x); tma_prefetch_desc(&map_wp); tma_prefetch_desc(&map_wg); tma_prefetch_desc(&map_z); }
     if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
     grid_dependency_wait();
     grid_launch_dependents();
@@ -111,18 +113,86 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
     tc_fence_after();
     const uint32_t tmem_base = B->tmem_slot;
 
-    if (warp < LOAD_WARPS) {
-        // ---------------------------- loaders ----------------------------
-        const int sub = lane & 7, rq = lane >> 3;
-        float4 gam[4], bet[4];
+    // One warp's 16 rows of a tile, 8 lanes per row: fetched, and normalised into the A tile.  Positions beyond the row's end repeat
+    // its first one: the reduce-add clips them (zeroing them cost the loaders registers: with spills the kernel took 297 us at
+    // 1024 tokens, this way 270).
+    const int sub = lane & 7, rq = lane >> 3;
+    auto fetch16 = [&](int r, int pos0, int row0, float4 (&v)[4][4]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int pos = pos0 + row0 + i * 4 + rq;
+            const float4* src = reinterpret_cast<const float4*>(p.z + ((long long)r * p.n + (pos < p.n ? pos : 0)) * KC);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[i][j] = src[j * 8 + sub];
+        }
+    };
+    auto normalise16 = [&](int row0, float4 (&v)[4][4], uint8_t* a_tile, const float4 (&gam)[4], const float4 (&bet)[4]) {
+        // the four rows of a pass stage by stage (sums, shuffles, variance, ...): instruction-level parallelism
+        // for a warp that has its scheduler almost to itself
+        float s4[4], ss4[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s += (v[i][j].x + v[i][j].y) + (v[i][j].z + v[i][j].w);
+            s4[i] = s;
+        }
+#pragma unroll
+        for (int step = 1; step < 8; step <<= 1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s4[i] += __shfl_xor_sync(0xffffffffu, s4[i], step);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float mean = s4[i] * (1.f / KC);
+            float ss = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[i][j].x -= mean; v[i][j].y -= mean; v[i][j].z -= mean; v[i][j].w -= mean;
+                ss += (v[i][j].x * v[i][j].x + v[i][j].y * v[i][j].y) + (v[i][j].z * v[i][j].z + v[i][j].w * v[i][j].w);
+            }
+            ss4[i] = ss;
+        }
+#pragma unroll
+        for (int step = 1; step < 8; step <<= 1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ss4[i] += __shfl_xor_sync(0xffffffffu, ss4[i], step);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = row0 + i * 4 + rq;
+            const float rstd = rsqrtf(ss4[i] * (1.f / KC) + LN_EPS);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                uint2 o;
+                o.x = pack_bf16x2(fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x), fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y));
+                o.y = pack_bf16x2(fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z), fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w));
+                const int chunk = (j & 1) * 4 + (sub >> 1);
+                *reinterpret_cast<uint2*>(a_tile + (j >> 1) * A_KB_BYTES + sw128(row, chunk) + (sub & 1) * 8) = o;
+            }
+        }
+    };
+    auto load_affine = [&](float4 (&gam)[4], float4 (&bet)[4]) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             gam[j] = reinterpret_cast<const float4*>(p.ln_in_gamma)[j * 8 + sub];
             bet[j] = reinterpret_cast<const float4*>(p.ln_in_beta)[j * 8 + sub];
         }
-        uint32_t it = 0;
+    };
+    // x tile of the CTA's tile number `it`; the buffer is free once the MMAs of the tile before are done
+    auto load_x = [&](int r, int pos0, uint32_t it) {
+        if (!mbar_wait(&B->x_empty, (it & 1) ^ 1, abort_flag)) return false;
+        mbar_arrive_expect_tx(&B->x_full, 2 * XT_BOX);
+        tma_load_4d(smem + OFF_XT, &map_x, &B->x_full, pos0, r, 0, 0);
+        tma_load_4d(smem + OFF_XT + XT_BOX, &map_x, &B->x_full, pos0 + 64, r, 0, 0);
+        return true;
+    };
+
+    if (warp < LOAD_WARPS) {
+        // ---------------------------- loaders ----------------------------
+        float4 gam[4], bet[4];
+        load_affine(gam, bet);
+        uint32_t it = 1;                    // the epilogue warps normalise the CTA's first tile
         bool ok = true;
-        for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
+        for (long long t = blockIdx.x + gridDim.x; t < tiles && ok; t += gridDim.x, ++it) {
             const int r = (int)(t / tpl), pos0 = (int)(t % tpl) * TM;
             const uint32_t stage = it & 1, ph = (it >> 1) & 1;
             ok = mbar_wait(&B->in_empty[stage], ph ^ 1, abort_flag) && mbar_wait(&B->acc_empty[stage], ph ^ 1, abort_flag);
@@ -141,66 +211,9 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
             for (int pass = 0; pass < 2; ++pass) {
                 const int row0 = warp * 32 + pass * 16;
                 float4 v[4][4];
-                // positions beyond the row's end repeat its first one: the reduce-add clips them (zeroing them cost the
-                // loaders registers: with spills the kernel took 297 us at 1024 tokens, this way 270)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int pos = pos0 + row0 + i * 4 + rq;
-                    const float4* src = reinterpret_cast<const float4*>(p.z + ((long long)r * p.n + (pos < p.n ? pos : 0)) * KC);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) v[i][j] = src[j * 8 + sub];
-                }
-                if (pass == 0 && warp == 0 && lane == 0) {
-                    // x tile of this tile: the buffer is free once the MMAs of the previous tile are done
-                    ok = mbar_wait(&B->x_empty, (it & 1) ^ 1, abort_flag);
-                    if (ok) {
-                        mbar_arrive_expect_tx(&B->x_full, 2 * XT_BOX);
-                        tma_load_4d(smem + OFF_XT, &map_x, &B->x_full, pos0, r, 0, 0);
-                        tma_load_4d(smem + OFF_XT + XT_BOX, &map_x, &B->x_full, pos0 + 64, r, 0, 0);
-                    }
-                }
-                // the four rows of a pass stage by stage (sums, shuffles, variance, ...): instruction-level parallelism
-                // for a warp that has its scheduler almost to itself
-                float s4[4], ss4[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    float s = 0.f;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) s += (v[i][j].x + v[i][j].y) + (v[i][j].z + v[i][j].w);
-                    s4[i] = s;
-                }
-#pragma unroll
-                for (int step = 1; step < 8; step <<= 1)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) s4[i] += __shfl_xor_sync(0xffffffffu, s4[i], step);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float mean = s4[i] * (1.f / KC);
-                    float ss = 0.f;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        v[i][j].x -= mean; v[i][j].y -= mean; v[i][j].z -= mean; v[i][j].w -= mean;
-                        ss += (v[i][j].x * v[i][j].x + v[i][j].y * v[i][j].y) + (v[i][j].z * v[i][j].z + v[i][j].w * v[i][j].w);
-                    }
-                    ss4[i] = ss;
-                }
-#pragma unroll
-                for (int step = 1; step < 8; step <<= 1)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) ss4[i] += __shfl_xor_sync(0xffffffffu, ss4[i], step);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int row = row0 + i * 4 + rq;
-                    const float rstd = rsqrtf(ss4[i] * (1.f / KC) + LN_EPS);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        uint2 o;
-                        o.x = pack_bf16x2(fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x), fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y));
-                        o.y = pack_bf16x2(fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z), fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w));
-                        const int chunk = (j & 1) * 4 + (sub >> 1);
-                        *reinterpret_cast<uint2*>(a_tile + (j >> 1) * A_KB_BYTES + sw128(row, chunk) + (sub & 1) * 8) = o;
-                    }
-                }
+                fetch16(r, pos0, row0, v);
+                if (pass == 0 && warp == 0 && lane == 0) ok = load_x(r, pos0, it);
+                normalise16(row0, v, a_tile, gam, bet);
             }
             if (warp == 0) ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;     // lane 0 waited for the x buffer
             if (!ok) break;
@@ -244,11 +257,25 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
     } else {
         // ---------------------------- epilogue ----------------------------
         const int quarter = warp & 3, chalf = (warp - EPI_WARP0) >> 2;
-        const int epi_tid = threadIdx.x - EPI_WARP0 * 32;
         const int lrow = quarter * 32 + lane;                     // position inside the tile
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
-        uint32_t it = 0, round = 0;
+        uint8_t* stg = smem + OFF_STG + (warp - EPI_WARP0) * STG_BOX;
+        uint32_t it = 0;
         bool ok = true;
+        if (blockIdx.x < tiles) {
+            // the first tile's x and LayerNorm, 16 rows a warp.  At 45 tokens, one tile per CTA, four loader warps in two passes each
+            // took 3.7 of the kernel's 7 us.
+            const int r = (int)blockIdx.x / tpl, pos0 = ((int)blockIdx.x % tpl) * TM, row0 = (warp - EPI_WARP0) * 16;
+            if (warp == EPI_WARP0 && lane == 0) ok = load_x(r, pos0, 0);
+            float4 v[4][4], gam[4], bet[4];
+            fetch16(r, pos0, row0, v);
+            load_affine(gam, bet);
+            normalise16(row0, v, smem + OFF_AZ, gam, bet);
+            fence_proxy_async();
+            named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
+            if (warp - EPI_WARP0 < LOAD_WARPS && lane == 0) mbar_arrive(&B->in_full[0]);      // the loaders' arrivals of this phase
+            ok = __all_sync(0xffffffffu, ok) != 0;
+        }
         for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
             const int r = (int)(t / tpl), pos0 = (int)(t % tpl) * TM;
             const uint32_t stage = it & 1, ph = (it >> 1) & 1;
@@ -279,7 +306,7 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
             tc_fence_after();
             const uint32_t tbase = tmem_base + lane_off + stage * 256;
 #pragma unroll 1
-            for (int rd = 0; rd < 2; ++rd, ++round) {
+            for (int rd = 0; rd < 2; ++rd) {
                 const int c0 = rd * 64 + chalf * 32;
                 uint32_t pr[32], gr[32];
                 tmem_ld_32x32(tbase + c0, pr);
@@ -292,16 +319,14 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
                     float ph2 = fmaf(st.y, fmaf(-st.x, wsum_s[c0 + e], __uint_as_float(pr[e])), wb_s[c0 + e]);
                     of[e] = fmaf(ph2, tanh_approx(__uint_as_float(gr[e])), ph2);
                 }
-                uint8_t* stg = smem + OFF_STG;
-                if (epi_tid == 0) bulk_wait_read0();               // the previous round's reduce has read the staging tile
-                named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
+                if (lane == 0) bulk_wait_read0();                  // this warp's previous reduction has read the staging tile
+                __syncwarp();
 #pragma unroll
-                for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(stg + chalf * STG_BOX + sw128(lrow, j)) = o[j];
+                for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(stg + sw128(lane, j)) = o[j];
                 fence_proxy_async();
-                named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
-                if (epi_tid == 0) {
-                    tma_reduce_add_4d(&map_z, stg, rd * 64, pos0, r, 0);
-                    tma_reduce_add_4d(&map_z, stg + STG_BOX, rd * 64 + 32, pos0, r, 0);
+                __syncwarp();
+                if (lane == 0 && pos0 + quarter * 32 < p.n) {
+                    tma_reduce_add_4d(&map_z, stg, c0, pos0 + quarter * 32, r, 0);
                     bulk_commit();
                 }
             }
@@ -309,7 +334,7 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
             __syncwarp();
             if (lane == 0) mbar_arrive(&B->acc_empty[stage]);
         }
-        if (epi_tid == 0) bulk_wait0();
+        if (lane == 0) bulk_wait0();
         if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
     }
     tc_fence_before();
@@ -346,7 +371,7 @@ extern "C" int b200pf_trimul_epilogue_tc(float* z, const b200pf_bf16* x, long lo
     {
         cuuint64_t dims[4] = {128, (cuuint64_t)n, (cuuint64_t)rows, 1};
         cuuint64_t str[3] = {512, (cuuint64_t)n * 512, (cuuint64_t)n * 512 * rows};
-        cuuint32_t box[4] = {32, 128, 1, 1};
+        cuuint32_t box[4] = {32, 32, 1, 1};
         if ((rc = tmap_encode(&mz, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, z, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, "z")) != B200PF_OK) return rc;
     }
     unsigned int* status = device_status_word();
