@@ -10,7 +10,9 @@
 // a = f1/2:  silu(f1) = a + a*tanh(a).
 // Weights (384 KB bf16) do not fit in shared memory: a dedicated warp streams the chunk pair
 // (32 KB + 16 KB) from L2 with TMA through a three-stage ring.
-// Roles (448 threads): warps 0-3 LayerNorm loaders, warp 4 MMA issuer, warp 5 weight TMA, warps 6-13 epilogue.
+// Roles (448 threads): warps 0-3 LayerNorm loaders, warp 4 MMA issuer, warp 5 weight TMA, warps 6-13 epilogue (each with a
+// staging tile and reductions of its own).  A CTA's first tile is normalised by the epilogue warps, 16 rows each, which have nothing
+// else to do before its first products exist; the loaders begin with the second.
 #include "rowtc.cuh"
 #include "tmap.cuh"
 
@@ -28,9 +30,9 @@ constexpr int OFF_W = 0;                                  // 2 stages
 constexpr int WSTAGES = 3;                                // the weight stream comes from L2 for every tile: the MMA
                                                           // issuer waited ~6.4 k clocks per tile on it with 2 stages
 constexpr int OFF_A = WSTAGES * WSTAGE;                   // 2 stages x 32 KB
-constexpr int OFF_STG = OFF_A + 2 * A_TILE_BYTES;         // staging: one box of [128 pos][32 fp32]
-constexpr int STG_BOX = 128 * 128;
-constexpr int OFF_BAR = OFF_STG + STG_BOX;
+constexpr int OFF_STG = OFF_A + 2 * A_TILE_BYTES;         // staging: per epilogue warp [16 pos][32 fp32], 128-byte swizzle
+constexpr int STG_BOX = 16 * 128;
+constexpr int OFF_BAR = OFF_STG + EPI_WARPS * STG_BOX;
 constexpr int SMEM_BYTES = OFF_BAR + 256;                 // 229,632
 constexpr int EPI_BAR_ID = 1;
 // TMEM columns
@@ -95,6 +97,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_c
         B->abort_flag = 0;
         fence_barrier_init();
     }
+    if (tid == 32) { tma_prefetch_desc(&map_w12); tma_prefetch_desc(&map_w3); tma_prefetch_desc(&map_z); }
     if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
     grid_dependency_wait();
     grid_launch_dependents();
@@ -103,18 +106,63 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_c
     tc_fence_after();
     const uint32_t tmem_base = B->tmem_slot;
 
-    if (warp < LOAD_WARPS) {
-        // ---------------------------- LayerNorm loaders ----------------------------
-        const int sub = lane & 7, rq = lane >> 3;
-        float4 gam[4], bet[4];
+    // One warp's 16 rows of a tile, 8 lanes per row, normalised into the A tile.
+    const int sub = lane & 7, rq = lane >> 3;
+    auto normalise16 = [&](long long base, int row0, uint8_t* a_tile, const float4 (&gam)[4], const float4 (&bet)[4]) {
+        float4 v[4][4];
+        // rows beyond the last one repeat row 0: the reduce-add clips them
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const long long f = base + row0 + i * 4 + rq;
+            const float4* src = reinterpret_cast<const float4*>(p.z + (f < p.rows_flat ? f : 0) * KC);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[i][j] = src[j * 8 + sub];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = row0 + i * 4 + rq;
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s += (v[i][j].x + v[i][j].y) + (v[i][j].z + v[i][j].w);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            s += __shfl_xor_sync(0xffffffffu, s, 4);
+            const float mean = s * (1.f / KC);
+            float ss = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[i][j].x -= mean; v[i][j].y -= mean; v[i][j].z -= mean; v[i][j].w -= mean;
+                ss += (v[i][j].x * v[i][j].x + v[i][j].y * v[i][j].y) + (v[i][j].z * v[i][j].z + v[i][j].w * v[i][j].w);
+            }
+            ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+            ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+            ss += __shfl_xor_sync(0xffffffffu, ss, 4);
+            const float rstd = rsqrtf(ss * (1.f / KC) + LN_EPS);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                uint2 o;
+                o.x = pack_bf16x2(fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x), fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y));
+                o.y = pack_bf16x2(fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z), fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w));
+                const int chunk = (j & 1) * 4 + (sub >> 1);
+                *reinterpret_cast<uint2*>(a_tile + (j >> 1) * A_KB_BYTES + sw128(row, chunk) + (sub & 1) * 8) = o;
+            }
+        }
+    };
+    auto load_affine = [&](float4 (&gam)[4], float4 (&bet)[4]) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             gam[j] = reinterpret_cast<const float4*>(p.ln_gamma)[j * 8 + sub];
             bet[j] = reinterpret_cast<const float4*>(p.ln_beta)[j * 8 + sub];
         }
-        uint32_t it = 0;
+    };
+
+    if (warp < LOAD_WARPS) {
+        // ---------------------------- LayerNorm loaders ----------------------------
+        float4 gam[4], bet[4];
+        load_affine(gam, bet);
+        uint32_t it = 1;                    // the epilogue warps normalise the CTA's first tile
         bool ok = true;
-        for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
+        for (long long t = blockIdx.x + gridDim.x; t < tiles && ok; t += gridDim.x, ++it) {
             const long long base = t * TM;
             const uint32_t stage = it & 1, ph = (it >> 1) & 1;
             ok = mbar_wait(&B->a_empty[stage], ph ^ 1, abort_flag);
@@ -130,45 +178,7 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_c
             }
 #pragma unroll 1
             for (int pass = 0; pass < 2; ++pass) {
-                const int row0 = warp * 32 + pass * 16;
-                float4 v[4][4];
-                // rows beyond the last one repeat row 0: the reduce-add clips them
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const long long f = base + row0 + i * 4 + rq;
-                    const float4* src = reinterpret_cast<const float4*>(p.z + (f < p.rows_flat ? f : 0) * KC);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) v[i][j] = src[j * 8 + sub];
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int row = row0 + i * 4 + rq;
-                    float s = 0.f;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) s += (v[i][j].x + v[i][j].y) + (v[i][j].z + v[i][j].w);
-                    s += __shfl_xor_sync(0xffffffffu, s, 1);
-                    s += __shfl_xor_sync(0xffffffffu, s, 2);
-                    s += __shfl_xor_sync(0xffffffffu, s, 4);
-                    const float mean = s * (1.f / KC);
-                    float ss = 0.f;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        v[i][j].x -= mean; v[i][j].y -= mean; v[i][j].z -= mean; v[i][j].w -= mean;
-                        ss += (v[i][j].x * v[i][j].x + v[i][j].y * v[i][j].y) + (v[i][j].z * v[i][j].z + v[i][j].w * v[i][j].w);
-                    }
-                    ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-                    ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-                    ss += __shfl_xor_sync(0xffffffffu, ss, 4);
-                    const float rstd = rsqrtf(ss * (1.f / KC) + LN_EPS);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        uint2 o;
-                        o.x = pack_bf16x2(fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x), fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y));
-                        o.y = pack_bf16x2(fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z), fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w));
-                        const int chunk = (j & 1) * 4 + (sub >> 1);
-                        *reinterpret_cast<uint2*>(a_tile + (j >> 1) * A_KB_BYTES + sw128(row, chunk) + (sub & 1) * 8) = o;
-                    }
-                }
+                normalise16(base, warp * 32 + pass * 16, a_tile, gam, bet);
             }
             fence_proxy_async();
             __syncwarp();
@@ -258,11 +268,18 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_c
     } else {
         // ---------------------------- epilogue ----------------------------
         const int quarter = warp & 3, eh = (warp - EPI_WARP0) >> 2;
-        const int epi_tid = threadIdx.x - EPI_WARP0 * 32;
-        const int lrow = quarter * 32 + lane;
+        uint8_t* stg = smem + OFF_STG + (warp - EPI_WARP0) * STG_BOX;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         uint32_t it = 0, d1_cnt[2] = {0, 0};
         bool ok = true;
+        if (blockIdx.x < tiles) {
+            float4 gam[4], bet[4];
+            load_affine(gam, bet);
+            normalise16((long long)blockIdx.x * TM, (warp - EPI_WARP0) * 16, smem + OFF_A, gam, bet);
+            fence_proxy_async();
+            named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
+            if (warp - EPI_WARP0 < LOAD_WARPS && lane == 0) mbar_arrive(&B->a_full[0]);       // the loaders' arrivals of this phase
+        }
         for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
             for (int c = 0; c < CHUNKS && ok; ++c) {
                 const uint32_t buf = c & 1;
@@ -301,28 +318,29 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_c
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&B->d2_empty);
-            const long long base = t * TM;
+            // four rounds of 16 positions x 32 channels: the lanes of the upper and the lower half of the warp in turn
+            const long long row_w = t * TM + quarter * 32;
 #pragma unroll
             for (int rd = 0; rd < 4; ++rd) {
-                // round rd stores channels [32 rd, +32): they are held by the warps with eh == rd / 2 (register half rd % 2)
-                if (epi_tid == 0) bulk_wait_read0();
-                named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
-                if (eh == (rd >> 1)) {
+                if (lane == 0) bulk_wait_read0();
+                __syncwarp();
+                if ((lane >> 4) == (rd & 1)) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        uint4 v = make_uint4(d[rd & 1][4 * j], d[rd & 1][4 * j + 1], d[rd & 1][4 * j + 2], d[rd & 1][4 * j + 3]);
-                        *reinterpret_cast<uint4*>(smem + OFF_STG + sw128(lrow, j)) = v;
+                        uint4 v = make_uint4(d[rd >> 1][4 * j], d[rd >> 1][4 * j + 1], d[rd >> 1][4 * j + 2], d[rd >> 1][4 * j + 3]);
+                        *reinterpret_cast<uint4*>(stg + sw128(lane & 15, j)) = v;
                     }
                 }
                 fence_proxy_async();
-                named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
-                if (epi_tid == 0) {
-                    tma_reduce_add_4d(&map_z, smem + OFF_STG, rd * 32, (int)(base & 0x7fffffff), 0, 0);
+                __syncwarp();
+                const long long row = row_w + (rd & 1) * 16;
+                if (lane == 0 && row < p.rows_flat) {
+                    tma_reduce_add_4d(&map_z, stg, eh * 64 + (rd >> 1) * 32, (int)row, 0, 0);
                     bulk_commit();
                 }
             }
         }
-        if (epi_tid == 0) bulk_wait0();
+        if (lane == 0) bulk_wait0();
         if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
     }
     tc_fence_before();
@@ -359,7 +377,7 @@ extern "C" int b200pf_transition_z_tc(float* z, const float* ln_gamma, const flo
     {
         cuuint64_t dims[4] = {128, (cuuint64_t)n_rows_flat, 1, 1};
         cuuint64_t str[3] = {512, (cuuint64_t)n_rows_flat * 512, (cuuint64_t)n_rows_flat * 512};
-        cuuint32_t box[4] = {32, 128, 1, 1};
+        cuuint32_t box[4] = {32, 16, 1, 1};
         if ((rc = tmap_encode(&mz, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, z, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, "z")) != B200PF_OK) return rc;
     }
     unsigned int* status = device_status_word();
