@@ -16,7 +16,10 @@ struct AttEpilogueArgs {
     long long rows_flat;
 };
 
-__global__ void __launch_bounds__(WARPS * 32, 1) triatt_epilogue_kernel(AttEpilogueArgs p) {
+// Units of 32 positions go round robin over the CTAs first and their warps second: the residual's red.global traffic is bound per SM
+// (some 2.4 clocks per 32-byte sector), and 64 units on 8 CTAs, all warps filled first, took 5 us of a 10 us launch at 45 tokens.  The
+// weights arrive by cp.async under the first unit's gather.
+__global__ void __launch_bounds__(WARPS * 32, 2) triatt_epilogue_kernel(AttEpilogueArgs p) {
     extern __shared__ __align__(16) uint8_t smem[];
     __nv_bfloat16* w_s = reinterpret_cast<__nv_bfloat16*>(smem);
     __nv_bfloat16* tiles = w_s + 128 * APITCH;
@@ -24,15 +27,14 @@ __global__ void __launch_bounds__(WARPS * 32, 1) triatt_epilogue_kernel(AttEpilo
     __nv_bfloat16* tile = tiles + warp * (UNIT * APITCH);
     grid_dependency_wait();
     grid_launch_dependents();
-    load_weights_k128(w_s, p.w_o, 128);
-    __syncthreads();
+    for (int i = threadIdx.x; i < 128 * 16; i += WARPS * 32) cp_async16(w_s + (i >> 4) * APITCH + (i & 15) * 8, p.w_o + (i >> 4) * KC + (i & 15) * 8);
+    cp_async_commit();
     const uint32_t w_addr = smem_u32(w_s), tile_addr = smem_u32(tile);
     const long long units = (p.rows_flat + UNIT - 1) / UNIT;
     const int g = lane >> 2, t = lane & 3;
-    for (long long u = (long long)blockIdx.x * WARPS + warp; u < units; u += (long long)gridDim.x * WARPS) {
-        const long long base = u * UNIT;
-        // gather o * g into the operand tile: 8 lanes per row, 16 channels per lane
-#pragma unroll 2
+    // o * g of a unit's rows into the operand tile: 8 lanes per row, 16 channels per lane
+    auto gather = [&](long long base) {
+#pragma unroll 4
         for (int it = 0; it < 8; ++it) {
             int l = it * 4 + (lane >> 3), sub = lane & 7;
             long long f = base + l;
@@ -58,6 +60,13 @@ __global__ void __launch_bounds__(WARPS * 32, 1) triatt_epilogue_kernel(AttEpilo
             dst[1] = r[1];
         }
         __syncwarp();
+    };
+    long long u = (long long)warp * gridDim.x + blockIdx.x;
+    if (u < units) gather(u * UNIT);
+    cp_async_wait<0>();
+    __syncthreads();
+    while (u < units) {
+        const long long base = u * UNIT;
 #pragma unroll 1
         for (int c = 0; c < 2; ++c) {
             float acc[2][8][4];
@@ -83,6 +92,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1) triatt_epilogue_kernel(AttEpilo
                 }
         }
         __syncwarp();
+        u += (long long)gridDim.x * WARPS;
+        if (u < units) gather(u * UNIT);
     }
 }
 
@@ -144,8 +155,8 @@ static int triatt_epilogue(float* z, b200pf_bf16* upd, const b200pf_bf16* o, con
     B200PF_SMEM_ATTR_ONCE(triatt_epilogue_kernel, ATT_EPILOGUE_SMEM);
     int sms, rc;
     if ((rc = multiprocessors(&sms)) != B200PF_OK) return rc;
-    const long long units = (n_rows_flat + UNIT - 1) / UNIT, ctas = (units + WARPS - 1) / WARPS;
-    return launch_pdl(triatt_epilogue_kernel, dim3((unsigned)(ctas < 2 * sms ? ctas : 2 * sms)), dim3(WARPS * 32), ATT_EPILOGUE_SMEM, (cudaStream_t)stream, p);
+    const long long units = (n_rows_flat + UNIT - 1) / UNIT;
+    return launch_pdl(triatt_epilogue_kernel, dim3((unsigned)(units < 2 * sms ? units : 2 * sms)), dim3(WARPS * 32), ATT_EPILOGUE_SMEM, (cudaStream_t)stream, p);
 }
 
 extern "C" int b200pf_triatt_epilogue(float* z, const b200pf_bf16* o, const b200pf_bf16* g,
