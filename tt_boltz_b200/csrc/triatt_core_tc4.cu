@@ -24,6 +24,7 @@
 // bias product alone 0.22 ms); with the softmax arithmetic and only the Q K^T products 1.36 ms; together 1.45 ms
 // (1.43 ms since the groups of a pair get their scores independently).
 // Scores are in the log2 domain (host folds log2(e)/sqrt(32) into W_q and log2(e) into the bias).
+// A last tile of at most 32 keys (every other line length) takes half of the softmax work and half of the P V products.
 // Every wait is bounded; a wait that runs out raises the status word and the CTA unwinds.
 #include "pdl.cuh"
 #include "sm100.cuh"
@@ -210,6 +211,7 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         *reinterpret_cast<uint4*>(smem + OFF_IDENT + row * 128 + ((chunk ^ (row & 7)) << 4)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
     }
     fence_proxy_async();
+    if (tid == TMA_WARP * 32) { tma_prefetch_desc(&map_q); tma_prefetch_desc(&map_k); tma_prefetch_desc(&map_vt); tma_prefetch_desc(&map_bias); }
     if (warp == MMA_WARP0) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
     grid_dependency_wait();
     grid_launch_dependents();
@@ -282,6 +284,7 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const uint32_t t_s = tmem_base + COL_S + (uint32_t)(g0 * AK);
         const uint32_t t_p = tmem_base + COL_P + (uint32_t)(g0 * (AK / 2));
         const uint32_t t_o = tmem_base + COL_O + (uint32_t)(g0 * HD);
+        const uint32_t short_j = RAGGED && n - (T - 1) * AK <= AK / 2 ? (uint32_t)T - 1 : (uint32_t)T;     // the tile of half the keys, if any
         uint32_t Gs[2] = {0u, 0u}, Gp[2] = {0u, 0u};
         uint32_t js[2] = {0u, 0u}, ks[2] = {0u, 0u}, stage_s[2] = {0u, 0u}, phase_s[2] = {0u, 0u};   // per group: the next S
         uint32_t jp[2] = {0u, 0u}, stage_p[2] = {0u, 0u};
@@ -328,7 +331,8 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                         if (jp[i] == 0) umma_bf16_ts(d, a, dv, idesc_pv, 0u);
                         else umma_bf16_ts(d, a, dv, idesc_pv, 1u);
 #pragma unroll
-                        for (int kk = 1; kk < AK / 16; ++kk) umma_bf16_ts(d, a + (uint32_t)(kk * 8), dv + 2 * kk, idesc_pv, 1u);
+                        for (int kk = 1; kk < AK / 16; ++kk)
+                            if (!RAGGED || kk < AK / 32 || jp[i] != short_j) umma_bf16_ts(d, a + (uint32_t)(kk * 8), dv + 2 * kk, idesc_pv, 1u);
                         umma_commit(&B->pv_done[g0 + i]);
                         if (Gp[1 - i] > G) umma_commit(&B->kv_empty[stage_p[i]]);     // both groups of the pair are through this stage
                     }
@@ -405,17 +409,22 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     if (!ok) break;
                     tc_fence_after();
                     tmem_st_32x16(p_addr, pw);
-                    tmem_ld_32x32(s_addr + 32, sr);
-                    tmem_ld_wait();
-                    mask_half<1>(sr, even, odd, left);
-                    max_half(sr, m4);
+                    const bool whole = !RAGGED || left > AK / 2;     // a last tile of at most 32 keys has no second half to work on
+                    if (whole) {
+                        tmem_ld_32x32(s_addr + 32, sr);
+                        tmem_ld_wait();
+                        mask_half<1>(sr, even, odd, left);
+                        max_half(sr, m4);
+                    }
                     const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
                     if (!__any_sync(0xffffffffu, mx > m_used + ONE_PASS_HEADROOM)) {
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&B->s_empty[g]);          // S may be overwritten by the next tile
-                        exp_half(sr, pw, negm2, l2a, l2b);
-                        tmem_st_32x16(p_addr + 16, pw);
+                        if (whole) {
+                            exp_half(sr, pw, negm2, l2a, l2b);
+                            tmem_st_32x16(p_addr + 16, pw);
+                        }
                         float a0, a1, b0, b1;
                         f2_unpack(l2a, a0, a1);
                         f2_unpack(l2b, b0, b1);
