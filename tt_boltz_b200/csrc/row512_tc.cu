@@ -107,17 +107,11 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         if (MODE == MODE_TRIATT) { tma_prefetch_desc(&map2); tma_prefetch_desc(&map3); }
     }
     if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
-    grid_dependency_wait();
-    grid_launch_dependents();
-    if (tid == 0) {
-        mbar_arrive_expect_tx(&B->w_full, W_BYTES);
-        load_weights_tma(smem, &map_w, 512, &B->w_full);
-    }
-    if (MODE == MODE_TRIATT)
-        for (int i = tid; i < 4 * 128; i += THREADS) wb_s[i] = p.w_bias_f32[i];
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dependency_wait();                 // behind the CTA's barrier: every warp goes to work by itself from here on
+    grid_launch_dependents();
     const uint32_t tmem_base = B->tmem_slot;
 
     auto flat_of = [&](int line, int pos) -> long long {   // flat (r * n + c) index, or -1 outside
@@ -259,6 +253,11 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         const uint64_t d_w = make_desc_k_sw128(smem_u32(smem));            // weight row r starts 8 r units further
         const uint64_t d_x0 = make_desc_k_sw128(smem_u32(smem + OFF_A));
         constexpr uint32_t W_KB16 = W_KB >> 4, A_KB16 = A_KB_BYTES >> 4;
+        if (elect_one()) {
+            mbar_arrive_expect_tx(&B->w_full, W_BYTES);
+            load_weights_tma(smem, &map_w, 512, &B->w_full);
+        }
+        __syncwarp();
         uint32_t it = 0, acc_cnt[2] = {0, 0};
         bool ok = mbar_wait_warp(&B->w_full, 0, abort_flag);
         for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
@@ -299,6 +298,8 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         if ((int)blockIdx.x < tiles) {
             // the first tile's LayerNorm, 16 rows a warp.  At 45 tokens, one tile per CTA, four loader warps in two passes each
             // took 3.6 of the kernel's 9 us.
+            if (MODE == MODE_TRIATT)
+                for (int i = (int)threadIdx.x - EPI_WARP0 * 32; i < 4 * 128; i += EPI_WARPS * 32) wb_s[i] = p.w_bias_f32[i];
             float4 gam[4], bet[4];
             load_affine(gam, bet);
             const int line = (int)blockIdx.x / tpl;

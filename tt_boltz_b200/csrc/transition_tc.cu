@@ -99,11 +99,11 @@ transition_tc_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_c
     }
     if (tid == 32) { tma_prefetch_desc(&map_w12); tma_prefetch_desc(&map_w3); tma_prefetch_desc(&map_z); }
     if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
-    grid_dependency_wait();
-    grid_launch_dependents();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dependency_wait();                 // behind the CTA's barrier: every warp goes to work by itself from here on
+    grid_launch_dependents();
     const uint32_t tmem_base = B->tmem_slot;
 
     // One warp's 16 rows of a tile, 8 lanes per row, normalised into the A tile.

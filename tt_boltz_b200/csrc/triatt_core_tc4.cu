@@ -213,11 +213,11 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     fence_proxy_async();
     if (tid == TMA_WARP * 32) { tma_prefetch_desc(&map_q); tma_prefetch_desc(&map_k); tma_prefetch_desc(&map_vt); tma_prefetch_desc(&map_bias); }
     if (warp == MMA_WARP0) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
-    grid_dependency_wait();
-    grid_launch_dependents();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dependency_wait();                 // behind the CTA's barrier: every warp goes to work by itself from here on
+    grid_launch_dependents();
     const uint32_t tmem_base = B->tmem_slot;
 
     auto decode = [&](long long it, int& qt, int& h, int& line0) {
@@ -239,8 +239,8 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 ok = mbar_wait(&B->q_empty[qb], ((k >> 1) & 1) ^ 1, abort_flag);
                 if (!ok) break;
                 mbar_arrive_expect_tx(&B->q_full[qb], NG * Q_BYTES);
-                for (int g = 0; g < NG; ++g)
-                    tma_load_4d(smem + OFF_Q + (qb * NG + g) * Q_BYTES, &map_q, &B->q_full[qb], 0, h, qt * AQ, clamp_line(line0 + g));
+                // one box for all four lines; those past the last one arrive as zeros
+                tma_load_4d(smem + OFF_Q + qb * NG * Q_BYTES, &map_q, &B->q_full[qb], 0, h, qt * AQ, line0);
                 for (int j = 0; j < T; ++j, ++G) {
                     const uint32_t stage = G % ST;
                     ok = mbar_wait(&B->kv_empty[stage], ((G / ST) & 1) ^ 1, abort_flag);
@@ -248,11 +248,8 @@ triatt_core_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     uint8_t* st = smem + stage * STAGE_BYTES;
                     mbar_arrive_expect_tx(&B->kv_full[stage], STAGE_BYTES);
                     tma_load_3d(st, &map_bias, &B->kv_full[stage], j * AK, h, qt * AQ);
-                    for (int g = 0; g < NG; ++g) {
-                        const int line = clamp_line(line0 + g);
-                        tma_load_4d(st + BIAS_BYTES + g * K_BYTES, &map_k, &B->kv_full[stage], 0, h, j * AK, line);
-                        tma_load_4d(st + BIAS_BYTES + NG * K_BYTES + g * VT_BYTES, &map_vt, &B->kv_full[stage], j * AK, 0, h, line);
-                    }
+                    tma_load_4d(st + BIAS_BYTES, &map_k, &B->kv_full[stage], 0, h, j * AK, line0);
+                    tma_load_4d(st + BIAS_BYTES + NG * K_BYTES, &map_vt, &B->kv_full[stage], j * AK, 0, h, line0);
                 }
             }
             if (!ok) {
@@ -557,14 +554,14 @@ extern "C" int b200pf_triatt_core_tc4(const b200pf_bf16* q, const b200pf_bf16* k
     {   // q, k: [line][pos][head][32]; coordinates (d, head, pos, line)
         cuuint64_t dims[4] = {(cuuint64_t)HD, 4, (cuuint64_t)n, (cuuint64_t)lines};
         cuuint64_t str[3] = {(cuuint64_t)HD * 2, (cuuint64_t)4 * HD * 2, (cuuint64_t)n * 4 * HD * 2};
-        cuuint32_t boxq[4] = {HD, 1, AQ, 1}, boxk[4] = {HD, 1, AK, 1};
+        cuuint32_t boxq[4] = {HD, 1, AQ, NG}, boxk[4] = {HD, 1, AK, NG};
         if ((rc = tmap_encode(&mq, bf, q, 4, dims, str, boxq, CU_TENSOR_MAP_SWIZZLE_64B, "q")) != B200PF_OK) return rc;
         if ((rc = tmap_encode(&mk, bf, k, 4, dims, str, boxk, CU_TENSOR_MAP_SWIZZLE_64B, "k")) != B200PF_OK) return rc;
     }
     {   // v transposed: [line][head][32][vt_pitch]; coordinates (key, d, head, line)
         cuuint64_t dims[4] = {(cuuint64_t)n, (cuuint64_t)HD, 4, (cuuint64_t)lines};
         cuuint64_t str[3] = {(cuuint64_t)vt_pitch * 2, (cuuint64_t)HD * vt_pitch * 2, (cuuint64_t)4 * HD * vt_pitch * 2};
-        cuuint32_t box[4] = {AK, HD, 1, 1};
+        cuuint32_t box[4] = {AK, HD, 1, NG};
         if ((rc = tmap_encode(&mvt, bf, vt, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, "vt")) != B200PF_OK) return rc;
     }
     {   // bias: [query][head][key]

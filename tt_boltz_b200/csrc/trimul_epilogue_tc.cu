@@ -102,11 +102,6 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
     if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
     grid_dependency_wait();
     grid_launch_dependents();
-    if (tid == 0) {
-        mbar_arrive_expect_tx(&B->w_full, 2 * W_TILE);
-        load_weights_tma(smem + OFF_WP, &map_wp, 128, &B->w_full);
-        load_weights_tma(smem + OFF_WG, &map_wg, 128, &B->w_full);
-    }
     if (tid < 128) { wsum_s[tid] = p.wsum[tid]; wb_s[tid] = p.wb[tid]; }
     tc_fence_before();
     __syncthreads();
@@ -228,6 +223,12 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
         constexpr uint32_t idesc_g = make_idesc_bf16(TM, 128);
         constexpr uint32_t idesc_p = make_idesc_bf16(TM, 128) | (1u << 15);      // A operand MN-major
         const uint32_t wp_addr = smem_u32(smem + OFF_WP), wg_addr = smem_u32(smem + OFF_WG), xt_addr = smem_u32(smem + OFF_XT);
+        if (elect_one()) {
+            mbar_arrive_expect_tx(&B->w_full, 2 * W_TILE);
+            load_weights_tma(smem + OFF_WP, &map_wp, 128, &B->w_full);
+            load_weights_tma(smem + OFF_WG, &map_wg, 128, &B->w_full);
+        }
+        __syncwarp();
         uint32_t it = 0;
         bool ok = mbar_wait_warp(&B->w_full, 0, abort_flag);
         for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
