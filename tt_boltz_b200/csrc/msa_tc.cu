@@ -20,7 +20,6 @@ constexpr int CM = 64;                                    // MSA channels: one 1
 constexpr int X_BYTES = TM * 128;                         // normalised tile: [128 rows][64] bf16
 constexpr int BOX = 128 * 128;                            // [128 rows][128 bytes], 128-byte swizzle
 constexpr int LOAD_WARPS = 4, MMA_WARP = 4, TMA_WARP = 5, EPI_WARP0 = 6, EPI_WARPS = 8, THREADS = 14 * 32;
-constexpr int EPI_BAR_ID = 1;
 
 // 32 rows of 64 channels -> bf16 rows row0 .. row0 + 31 of the tile; called by one warp.  Eight lanes per row, two float4
 // each; eight rows per lane at once, so that a warp has all of its loads in flight.  Rows >= valid are written as zeros.
@@ -119,20 +118,20 @@ __device__ __forceinline__ bool load_loop(const LnRows& p, uint8_t* x0, uint64_t
 
 __device__ __forceinline__ float sigmoid_of(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 
-// Two 32-column blocks [128 rows][32 fp32] of an update into m by TMA reduce-add; called by the epilogue warps together, each
-// with the 32 columns of its half for row `lrow`.
-__device__ __forceinline__ void reduce_update(const CUtensorMap* map_m, uint8_t* stg, const uint32_t (&d)[32], int half, int lrow, int epi_tid, int pos0, int line) {
+// A warp's [32 rows][32 fp32] block of an update into m by TMA reduce-add, through a staging tile of its own (STG_WARP bytes): no warp
+// waits for another.
+constexpr int STG_WARP = 32 * 128;
+__device__ __forceinline__ void reduce_update(const CUtensorMap* map_m, uint8_t* stg, const uint32_t (&d)[32], int lane, int col, int pos, int span, int line) {
     using namespace sm100;
-    if (epi_tid == 0) bulk_wait_read0();                       // the tile before has left the staging boxes
-    named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
+    if (lane == 0) bulk_wait_read0();                          // the tile before has left the staging tile
+    __syncwarp();
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-        *reinterpret_cast<uint4*>(stg + half * BOX + sw128(lrow, j)) = make_uint4(d[4 * j], d[4 * j + 1], d[4 * j + 2], d[4 * j + 3]);
+        *reinterpret_cast<uint4*>(stg + sw128(lane, j)) = make_uint4(d[4 * j], d[4 * j + 1], d[4 * j + 2], d[4 * j + 3]);
     fence_proxy_async();
-    named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
-    if (epi_tid == 0) {
-        tma_reduce_add_4d(map_m, stg, 0, pos0, line, 0);
-        tma_reduce_add_4d(map_m, stg + BOX, 32, pos0, line, 0);
+    __syncwarp();
+    if (lane == 0 && pos < span) {
+        tma_reduce_add_4d(map_m, stg, col, pos, line, 0);
         bulk_commit();
     }
 }
@@ -179,19 +178,13 @@ msa_transition_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_
         fence_proxy_async();
     }
     if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
-    grid_dependency_wait();
-    grid_launch_dependents();
-    if (tid == 0) {
-        mbar_arrive_expect_tx(&B->w_full, CHUNKS * (BOX + W3_KB));
-        for (int c = 0; c < CHUNKS; ++c) {
-            tma_load_4d(smem + OFF_W12 + c * BOX, &map_w12, &B->w_full, 0, c * 128, 0, 0);
-            tma_load_4d(smem + OFF_W3 + c * W3_KB, &map_w3, &B->w_full, c * 64, 0, 0, 0);
-        }
-    }
+    if (tid == 32) { tma_prefetch_desc(&map_w12); tma_prefetch_desc(&map_w3); tma_prefetch_desc(&map_m); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = B->tmem_slot;
+    grid_dependency_wait();                 // behind the CTA's barrier: every warp goes to work by itself from here on
+    grid_launch_dependents();
 
     bool ok = true;
     if (warp < LOAD_WARPS) {
@@ -202,6 +195,14 @@ msa_transition_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_
         const uint64_t d_x = make_desc_k_sw128(smem_u32(smem + OFF_X)), d_w12 = make_desc_k_sw128(smem_u32(smem + OFF_W12)),
                        d_w3 = make_desc_k_sw128(smem_u32(smem + OFF_W3));
         uint32_t it = 0, h_cnt[2] = {0, 0};
+        if (elect_one()) {
+            mbar_arrive_expect_tx(&B->w_full, CHUNKS * (BOX + W3_KB));
+            for (int c = 0; c < CHUNKS; ++c) {
+                tma_load_4d(smem + OFF_W12 + c * BOX, &map_w12, &B->w_full, 0, c * 128, 0, 0);
+                tma_load_4d(smem + OFF_W3 + c * W3_KB, &map_w3, &B->w_full, c * 64, 0, 0, 0);
+            }
+        }
+        __syncwarp();
         ok = mbar_wait_warp(&B->w_full, 0, abort_flag);
         auto gemm1 = [&](uint32_t stage, int c) {
             if (elect_one()) {
@@ -238,7 +239,7 @@ msa_transition_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_
             }
         }
     } else if (warp >= EPI_WARP0) {
-        const int quarter = warp & 3, half = (warp - EPI_WARP0) >> 2, epi_tid = threadIdx.x - EPI_WARP0 * 32, lrow = quarter * 32 + lane;
+        const int quarter = warp & 3, half = (warp - EPI_WARP0) >> 2;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         uint32_t it = 0, d1_cnt[2] = {0, 0};
         for (int t = blockIdx.x; t < p.t.tiles && ok; t += gridDim.x, ++it) {
@@ -277,9 +278,9 @@ msa_transition_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_
             __syncwarp();
             if (lane == 0) mbar_arrive(&B->d2_empty[stage]);
             const int line = t / p.t.tpl, pos0 = (t - line * p.t.tpl) * TM;
-            reduce_update(&map_m, smem + OFF_STG, d, half, lrow, epi_tid, pos0, line);
+            reduce_update(&map_m, smem + OFF_STG + (warp - EPI_WARP0) * STG_WARP, d, lane, half * 32, pos0 + quarter * 32, p.t.span, line);
         }
-        if (epi_tid == 0) bulk_wait0();
+        if (lane == 0) bulk_wait0();
     }
     if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
     tc_fence_before();
@@ -323,16 +324,13 @@ pwa_value_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         fence_proxy_async();
     }
     if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
-    grid_dependency_wait();
-    grid_launch_dependents();
-    if (tid == 0) {
-        mbar_arrive_expect_tx(&B->w_full, 2 * BOX);
-        for (int h = 0; h < 2; ++h) tma_load_4d(smem + OFF_W + h * BOX, &map_w, &B->w_full, 0, h * 128, 0, 0);
-    }
+    if (tid == 32) { tma_prefetch_desc(&map_w); tma_prefetch_desc(&map_v); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = B->tmem_slot;
+    grid_dependency_wait();                 // behind the CTA's barrier: every warp goes to work by itself from here on
+    grid_launch_dependents();
 
     bool ok = true;
     if (warp < LOAD_WARPS) {
@@ -342,6 +340,11 @@ pwa_value_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         constexpr uint32_t idesc = make_idesc_bf16(128, TM);
         const uint64_t d_w = make_desc_k_sw128(smem_u32(smem + OFF_W)), d_x = make_desc_k_sw128(smem_u32(smem + OFF_X));
         uint32_t it = 0;
+        if (elect_one()) {
+            mbar_arrive_expect_tx(&B->w_full, 2 * BOX);
+            for (int h = 0; h < 2; ++h) tma_load_4d(smem + OFF_W + h * BOX, &map_w, &B->w_full, 0, h * 128, 0, 0);
+        }
+        __syncwarp();
         ok = mbar_wait_warp(&B->w_full, 0, abort_flag);
         for (int t = blockIdx.x; t < p.t.tiles && ok; t += gridDim.x, ++it) {
             const uint32_t stage = it & 1, ph = (it >> 1) & 1;
@@ -361,18 +364,18 @@ pwa_value_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             __syncwarp();
         }
     } else if (warp >= EPI_WARP0) {
-        // thread = channel 128 h + lrow, 64 tokens of its half; box (h, half) = [4 heads x 32 d][64 tokens]
-        const int quarter = warp & 3, half = (warp - EPI_WARP0) >> 2, epi_tid = threadIdx.x - EPI_WARP0 * 32, lrow = quarter * 32 + lane;
+        // thread = channel 128 h + 32 quarter + lane, i.e. head 4 h + quarter, 64 tokens of its half; a box is [32 d][64 tokens]
+        const int quarter = warp & 3, half = (warp - EPI_WARP0) >> 2;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
-        uint8_t* stg = smem + OFF_STG;
+        uint8_t* stg = smem + OFF_STG + (warp - EPI_WARP0) * 2 * STG_WARP;
         uint32_t it = 0;
         for (int t = blockIdx.x; t < p.t.tiles && ok; t += gridDim.x, ++it) {
             const uint32_t stage = it & 1, ph = (it >> 1) & 1;
             ok = mbar_wait(&B->d_full[stage], ph, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            if (epi_tid == 0) bulk_wait_read0();
-            named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
+            if (lane == 0) bulk_wait_read0();
+            __syncwarp();
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 uint32_t r[2][32];
@@ -387,22 +390,21 @@ pwa_value_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                         const int e = j * 8 + q * 2;
                         w[q] = pack_bf16x2(__uint_as_float(r[e >> 5][e & 31]), __uint_as_float(r[e >> 5][(e & 31) + 1]));
                     }
-                    *reinterpret_cast<uint4*>(stg + (h * 2 + half) * BOX + sw128(lrow, j)) = make_uint4(w[0], w[1], w[2], w[3]);
+                    *reinterpret_cast<uint4*>(stg + h * STG_WARP + sw128(lane, j)) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&B->d_empty[stage]);
             fence_proxy_async();
-            named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
-            if (epi_tid == 0) {
-                const int line = t / p.t.tpl, pos0 = (t - line * p.t.tpl) * TM;
-                for (int b = 0; b < 4; ++b)      // the second token half may lie beyond the line's end: nothing to store
-                    if (pos0 + (b & 1) * 64 < p.t.span) tma_store_4d(&map_v, stg + b * BOX, pos0 + (b & 1) * 64, 0, line, (b >> 1) * 4);
+            __syncwarp();
+            const int line = t / p.t.tpl, pos = (t - line * p.t.tpl) * TM + half * 64;
+            if (lane == 0 && pos < p.t.span) {      // the second token half may lie beyond the line's end: nothing to store
+                for (int h = 0; h < 2; ++h) tma_store_4d(&map_v, stg + h * STG_WARP, pos, 0, line, h * 4 + quarter);
                 bulk_commit();
             }
         }
-        if (epi_tid == 0) bulk_wait0();
+        if (lane == 0) bulk_wait0();
     }
     if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
     tc_fence_before();
@@ -465,17 +467,13 @@ pwa_output_kernel(const __grid_constant__ CUtensorMap map_wg, const __grid_const
         fence_proxy_async();
     }
     if (warp == MMA_WARP) { tmem_alloc(&B->tmem_slot, 512); tmem_relinquish(); }
-    grid_dependency_wait();
-    grid_launch_dependents();
-    if (tid == 0) {
-        mbar_arrive_expect_tx(&B->w_full, 2 * BOX + 4 * WO_KB);
-        for (int h = 0; h < 2; ++h) tma_load_4d(smem + OFF_WG + h * BOX, &map_wg, &B->w_full, 0, h * 128, 0, 0);
-        for (int k = 0; k < 4; ++k) tma_load_4d(smem + OFF_WO + k * WO_KB, &map_wo, &B->w_full, k * 64, 0, 0, 0);
-    }
+    if (tid == 32) { tma_prefetch_desc(&map_wg); tma_prefetch_desc(&map_wo); tma_prefetch_desc(&map_o); tma_prefetch_desc(&map_m); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = B->tmem_slot;
+    grid_dependency_wait();                 // behind the CTA's barrier: every warp goes to work by itself from here on
+    grid_launch_dependents();
 
     bool ok = true;
     if (warp < LOAD_WARPS) {
@@ -506,6 +504,12 @@ pwa_output_kernel(const __grid_constant__ CUtensorMap map_wg, const __grid_const
         constexpr uint32_t idesc_g = make_idesc_bf16(128, TM), idesc_o = make_idesc_bf16(TM, 64) | (1u << 15);      // A MN-major
         const uint64_t d_wg = make_desc_k_sw128(smem_u32(smem + OFF_WG)), d_x = make_desc_k_sw128(smem_u32(smem + OFF_X)),
                        d_wo = make_desc_k_sw128(smem_u32(smem + OFF_WO)), d_o = desc_mn_sw128(smem_u32(smem + OFF_O));
+        if (elect_one()) {
+            mbar_arrive_expect_tx(&B->w_full, 2 * BOX + 4 * WO_KB);
+            for (int h = 0; h < 2; ++h) tma_load_4d(smem + OFF_WG + h * BOX, &map_wg, &B->w_full, 0, h * 128, 0, 0);
+            for (int k = 0; k < 4; ++k) tma_load_4d(smem + OFF_WO + k * WO_KB, &map_wo, &B->w_full, k * 64, 0, 0, 0);
+        }
+        __syncwarp();
         ok = mbar_wait_warp(&B->w_full, 0, abort_flag);
         auto gate = [&](uint32_t tile, int h) {           // tile: this CTA's running number
             const uint32_t stage = tile & 1;
@@ -547,7 +551,7 @@ pwa_output_kernel(const __grid_constant__ CUtensorMap map_wg, const __grid_const
             }
         }
     } else {
-        const int quarter = warp & 3, half = (warp - EPI_WARP0) >> 2, epi_tid = threadIdx.x - EPI_WARP0 * 32, lrow = quarter * 32 + lane;
+        const int quarter = warp & 3, half = (warp - EPI_WARP0) >> 2, lrow = quarter * 32 + lane;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         auto update = [&](uint32_t tile, int t) {         // D2 of this CTA's tile number `tile` (global tile t) into m
             const uint32_t acc = tile & 1;
@@ -561,7 +565,7 @@ pwa_output_kernel(const __grid_constant__ CUtensorMap map_wg, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive(&B->d2_empty[acc]);
             const int line = t / p.t.tpl, pos0 = (t - line * p.t.tpl) * TM;
-            reduce_update(&map_m, smem + OFF_STG, d, half, lrow, epi_tid, pos0, line);
+            reduce_update(&map_m, smem + OFF_STG + (warp - EPI_WARP0) * STG_WARP, d, lane, half * 32, pos0 + quarter * 32, p.t.span, line);
         };
         uint32_t it = 0, slot = 0, ph = 0;
         int t = blockIdx.x;
@@ -600,7 +604,7 @@ pwa_output_kernel(const __grid_constant__ CUtensorMap map_wg, const __grid_const
             if (ok && it > 0) update(it - 1, t - (int)gridDim.x);      // the tile before, whose product ran under this one's gate
         }
         if (ok) update(it - 1, t - (int)gridDim.x);
-        if (epi_tid == 0) bulk_wait0();
+        if (lane == 0) bulk_wait0();
     }
     if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
     tc_fence_before();
@@ -618,13 +622,13 @@ static int map_rows64(CUtensorMap* map, const void* w, int rows, int cols, int b
 static int map_update(CUtensorMap* map, const float* m, const Tiling& t) {
     cuuint64_t dims[4] = {CM, (cuuint64_t)t.span, (cuuint64_t)t.lines, 1};
     cuuint64_t str[3] = {CM * 4, (cuuint64_t)t.span * CM * 4, (cuuint64_t)t.span * t.lines * CM * 4};
-    cuuint32_t box[4] = {32, 128, 1, 1};
+    cuuint32_t box[4] = {32, 32, 1, 1};
     return tmap_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, m, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, "m");
 }
-static int map_heads(CUtensorMap* map, const void* v, int s_len, int n, int np, const char* what) {               // [8][S][32][np] bf16
+static int map_heads(CUtensorMap* map, const void* v, int s_len, int n, int np, int box_heads, const char* what) {      // [8][S][32][np] bf16
     cuuint64_t dims[4] = {(cuuint64_t)n, 32, (cuuint64_t)s_len, 8};
     cuuint64_t str[3] = {(cuuint64_t)np * 2, (cuuint64_t)np * 64, (cuuint64_t)np * 64 * s_len};
-    cuuint32_t box[4] = {64, 32, 1, 4};
+    cuuint32_t box[4] = {64, 32, 1, (cuuint32_t)box_heads};
     return tmap_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, v, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, what);
 }
 static Tiling tiling(int lines, int span) {
@@ -667,7 +671,7 @@ extern "C" int b200pf_pwa_value(const float* m, const float* ln_gamma, const flo
     CUtensorMap mw, mv;
     int sms, rc;
     if ((rc = multiprocessors(&sms)) != B200PF_OK || (rc = map_rows64(&mw, w_m, 256, CM, 128, "w_m")) != B200PF_OK ||
-        (rc = map_heads(&mv, v, s_len, n, np, "v")) != B200PF_OK) return rc;
+        (rc = map_heads(&mv, v, s_len, n, np, 1, "v")) != B200PF_OK) return rc;
     B200PF_SMEM_ATTR_ONCE(pwa_value_kernel, va::SMEM);
     return launch_pdl(pwa_value_kernel, dim3((unsigned)(t.tiles < sms ? t.tiles : sms)), dim3(THREADS), va::SMEM, (cudaStream_t)stream, mw, mv,
                       LnRows{m, ln_gamma, ln_beta, t}, status);
@@ -685,7 +689,7 @@ extern "C" int b200pf_pwa_output(float* m, const float* ln_gamma, const float* l
     CUtensorMap mg, mo, mov, mm;
     int sms, rc;
     if ((rc = multiprocessors(&sms)) != B200PF_OK || (rc = map_rows64(&mg, w_g, 256, CM, 128, "w_g")) != B200PF_OK ||
-        (rc = map_rows64(&mo, w_o, 64, 256, 64, "w_o")) != B200PF_OK || (rc = map_heads(&mov, o, s_len, n, np, "o")) != B200PF_OK ||
+        (rc = map_rows64(&mo, w_o, 64, 256, 64, "w_o")) != B200PF_OK || (rc = map_heads(&mov, o, s_len, n, np, 4, "o")) != B200PF_OK ||
         (rc = map_update(&mm, m, t)) != B200PF_OK) return rc;
     B200PF_SMEM_ATTR_ONCE(pwa_output_kernel, ou::SMEM);
     return launch_pdl(pwa_output_kernel, dim3((unsigned)(t.tiles < sms ? t.tiles : sms)), dim3(THREADS), ou::SMEM, (cudaStream_t)stream, mg, mo, mov, mm,
