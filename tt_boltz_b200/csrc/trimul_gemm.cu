@@ -3,7 +3,7 @@
 // One batched K-major GEMM over the 128 channels.  Persistent, warp-specialised kernel:
 //   warp 0   : TMA producer (one lane) - 128x64 bf16 boxes, 128-byte swizzle, 4-stage ring
 //   warp 1   : TMEM owner + MMA issuer (one lane) - tcgen05.mma 128x256x16, fp32 accumulators
-//   warps 2-5: epilogue - tcgen05.ld the finished 128x256 accumulator, round to bf16, store
+//   warps 2-5: epilogue - tcgen05.ld the finished 128x256 accumulator, round to bf16, stage, TMA store
 // Two accumulators (2 x 256 TMEM columns) let the epilogue of tile t overlap the MMAs of t+1.
 // Ragged sizes need no padding: TMA zero-fills out-of-range rows / columns, stores are guarded.
 #include <cstdlib>
@@ -17,7 +17,8 @@ namespace b200pf {
 constexpr int BM = 128, BN = 256, BK = 64, STAGES = 4;
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int GEMM_THREADS = 192;
-constexpr int GEMM_SMEM = STAGES * STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+constexpr int STG_BYTES = 32 * 128, STG_TOTAL = 4 * 2 * STG_BYTES;           // two [32 rows][64 columns] tiles per epilogue warp
+constexpr int GEMM_SMEM = STAGES * STAGE_BYTES + STG_TOTAL + 1024 /*align slack*/ + 256 /*barriers*/;
 
 struct GemmShape {
     int m_rows;          // rows of A (output rows)
@@ -35,6 +36,7 @@ struct GemmShape {
     int x_cols;          // columns written (whole 8-column vectors below this bound)
     int x_col_group;     // > 0: output columns in groups of this many (a multiple of 32), x_colgroup_stride elements apart
     long long x_colgroup_stride;
+    int x_tma;           // the output leaves through map_x (see store_tile)
 };
 // Output element (d, row, col) lives at (row / x_row_group) * x_group_stride + d * x_plane_stride + (row % x_row_group) * x_pitch + col.
 __device__ __forceinline__ long long x_row_offset(const GemmShape& s, int d, int row) {
@@ -42,13 +44,81 @@ __device__ __forceinline__ long long x_row_offset(const GemmShape& s, int d, int
     return (long long)grp * s.x_group_stride + (long long)d * s.x_plane_stride + (long long)(row - grp * s.x_row_group) * s.x_pitch;
 }
 
+// One epilogue warp's 32 rows (from `row0`) x 256 columns of a finished accumulator.  Plain planes leave through a swizzled staging tile and
+// TMA stores of [32 rows][64 columns].  As 16-byte stores of a thread per row, 4096 partial sectors a tile, they took 11 k clocks a tile
+// against 3.6 k to 8.2 k of MMAs: 11.7 -> 9.7 us at 203 tokens, 43 -> 35 at 400, 112 -> 94 at 600, 238 -> 224 at 1024 (what is left is
+// the operands, some 9 TB/s out of L2).  Columns in groups (the
+// outer product's blocks of contiguous 2 KB) and row groups that 32 does not divide stay with the direct stores.
+__device__ __forceinline__ void store_tile(const CUtensorMap* map_x, __nv_bfloat16* x, const GemmShape& s, uint32_t taddr, uint8_t* stg, uint32_t& slot, int d, int row0,
+                                           int n0, int lane) {
+    using namespace sm100;
+    const int row = row0 + lane;
+    if (s.x_tma) {
+        const int grp = row0 / s.x_row_group, row_in = row0 - grp * s.x_row_group;
+#pragma unroll 1
+        for (int c = 0; c < BN / 64; ++c) {
+            const int col = n0 + c * 64;
+            if (col >= s.x_cols || row0 >= s.m_rows) break;          // warp-uniform
+            uint32_t r[2][32];
+            tmem_ld_32x32(taddr + c * 64, r[0]);
+            tmem_ld_32x32(taddr + c * 64 + 32, r[1]);
+            tmem_ld_wait();
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");      // the store before last has read this tile
+            __syncwarp();
+            uint8_t* tile = stg + slot * STG_BYTES;
+            slot ^= 1;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                uint32_t w[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int e = j * 8 + q * 2;
+                    w[q] = pack_bf16x2(__uint_as_float(r[e >> 5][e & 31]), __uint_as_float(r[e >> 5][(e & 31) + 1]));
+                }
+                *reinterpret_cast<uint4*>(tile + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+                tma_store_4d(map_x, tile, col, row_in, d, grp);
+                bulk_commit();
+            }
+        }
+        return;
+    }
+    __nv_bfloat16* xrow = x + x_row_offset(s, d, row < s.m_rows ? row : 0);
+#pragma unroll 1
+    for (int c = 0; c < BN / 32; ++c) {
+        const int col = n0 + c * 32;
+        if (col >= s.x_cols) break;                                  // warp-uniform
+        __nv_bfloat16* xdst = s.x_col_group > 0 ? xrow + (long long)(col / s.x_col_group) * s.x_colgroup_stride + (col % s.x_col_group) : xrow + col;
+        uint32_t r[32];
+        tmem_ld_32x32(taddr + c * 32, r);
+        tmem_ld_wait();
+        if (row < s.m_rows) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                if (col + v * 8 + 8 <= s.x_cols) {
+                    uint4 o;
+                    o.x = pack_bf16x2(__uint_as_float(r[v * 8 + 0]), __uint_as_float(r[v * 8 + 1]));
+                    o.y = pack_bf16x2(__uint_as_float(r[v * 8 + 2]), __uint_as_float(r[v * 8 + 3]));
+                    o.z = pack_bf16x2(__uint_as_float(r[v * 8 + 4]), __uint_as_float(r[v * 8 + 5]));
+                    o.w = pack_bf16x2(__uint_as_float(r[v * 8 + 6]), __uint_as_float(r[v * 8 + 7]));
+                    *reinterpret_cast<uint4*>(xdst + v * 8) = o;
+                }
+            }
+        }
+    }
+}
+
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_x,
                           __nv_bfloat16* __restrict__ x, GemmShape s, unsigned int* status) {
     using namespace sm100;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+    uint8_t* stg = smem + STAGES * STAGE_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(stg + STG_TOTAL);
     uint64_t* full = bars;                    // [STAGES]
     uint64_t* empty = bars + STAGES;          // [STAGES]
     uint64_t* acc_full = bars + 2 * STAGES;   // [2]
@@ -142,6 +212,7 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     } else if (warp >= 2) {
         // ---------------- epilogue ----------------
         const int quarter = warp & 3;                 // TMEM lanes this warp may touch: 32*quarter ..
+        uint32_t slot = 0;                            // staging tile of the next store
         bool ok = true;
         long long it = 0;
         for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
@@ -152,36 +223,12 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             ok = mbar_wait(&acc_full[ab], aphase, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            int row = m0 + quarter * 32 + lane;
-            __nv_bfloat16* xrow = x + x_row_offset(s, d, row < s.m_rows ? row : 0);
-#pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
-                int col = n0 + c * 32;
-                if (col >= s.x_cols) break;           // warp-uniform
-                __nv_bfloat16* xdst = s.x_col_group > 0
-                                          ? xrow + (long long)(col / s.x_col_group) * s.x_colgroup_stride + (col % s.x_col_group)
-                                          : xrow + col;
-                uint32_t r[32];
-                tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + ab * BN + c * 32, r);
-                tmem_ld_wait();
-                if (row < s.m_rows) {
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        if (col + v * 8 + 8 <= s.x_cols) {
-                            uint4 o;
-                            o.x = pack_bf16x2(__uint_as_float(r[v * 8 + 0]), __uint_as_float(r[v * 8 + 1]));
-                            o.y = pack_bf16x2(__uint_as_float(r[v * 8 + 2]), __uint_as_float(r[v * 8 + 3]));
-                            o.z = pack_bf16x2(__uint_as_float(r[v * 8 + 4]), __uint_as_float(r[v * 8 + 5]));
-                            o.w = pack_bf16x2(__uint_as_float(r[v * 8 + 6]), __uint_as_float(r[v * 8 + 7]));
-                            *reinterpret_cast<uint4*>(xdst + v * 8) = o;
-                        }
-                    }
-                }
-            }
+            store_tile(&map_x, x, s, tmem_base + ((uint32_t)(quarter * 32) << 16) + ab * BN, stg + quarter * 2 * STG_BYTES, slot, d, m0 + quarter * 32, n0, lane);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[ab]);
         }
+        if (lane == 0) bulk_wait0();
         if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
     }
     tc_fence_before();
@@ -197,15 +244,16 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 // multicast); their bytes are counted on the even CTA's barrier.  Every role of both CTAs always reaches the two
 // cluster barriers, also after a wait ran out.
 constexpr int P_STAGES = 6, P_STAGE_BYTES = 2 * (128 * BK * 2);
-constexpr int PAIR_SMEM = P_STAGES * P_STAGE_BYTES + 1024 + 256;
+constexpr int PAIR_SMEM = P_STAGES * P_STAGE_BYTES + STG_TOTAL + 1024 + 256;
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
-trimul_contract_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+trimul_contract_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_x,
                             __nv_bfloat16* __restrict__ x, GemmShape s, unsigned int* status) {
     using namespace sm100;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + P_STAGES * P_STAGE_BYTES);
+    uint8_t* stg = smem + P_STAGES * P_STAGE_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(stg + STG_TOTAL);
     uint64_t* full = bars;                      // [P_STAGES]  used in the even CTA: both CTAs' loads
     uint64_t* empty = bars + P_STAGES;          // [P_STAGES]  one per CTA
     uint64_t* acc_full = bars + 2 * P_STAGES;   // [2]         one per CTA
@@ -306,6 +354,7 @@ trimul_contract_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     } else if (warp >= 2) {
         // ---------------- epilogue: this CTA's 128 rows of the tile ----------------
         const int quarter = warp & 3;
+        uint32_t slot = 0;                            // staging tile of the next store
         bool ok = true;
         long long it = 0;
         for (long long t = pair; t < tiles && ok; t += pairs, ++it) {
@@ -316,36 +365,12 @@ trimul_contract_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __g
             ok = mbar_wait(&acc_full[ab], aphase, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            int row = m0 + quarter * 32 + lane;
-            __nv_bfloat16* xrow = x + x_row_offset(s, d, row < s.m_rows ? row : 0);
-#pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
-                int col = n0 + c * 32;
-                if (col >= s.x_cols) break;           // warp-uniform
-                __nv_bfloat16* xdst = s.x_col_group > 0
-                                          ? xrow + (long long)(col / s.x_col_group) * s.x_colgroup_stride + (col % s.x_col_group)
-                                          : xrow + col;
-                uint32_t r[32];
-                tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + ab * BN + c * 32, r);
-                tmem_ld_wait();
-                if (row < s.m_rows) {
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        if (col + v * 8 + 8 <= s.x_cols) {
-                            uint4 o;
-                            o.x = pack_bf16x2(__uint_as_float(r[v * 8 + 0]), __uint_as_float(r[v * 8 + 1]));
-                            o.y = pack_bf16x2(__uint_as_float(r[v * 8 + 2]), __uint_as_float(r[v * 8 + 3]));
-                            o.z = pack_bf16x2(__uint_as_float(r[v * 8 + 4]), __uint_as_float(r[v * 8 + 5]));
-                            o.w = pack_bf16x2(__uint_as_float(r[v * 8 + 6]), __uint_as_float(r[v * 8 + 7]));
-                            *reinterpret_cast<uint4*>(xdst + v * 8) = o;
-                        }
-                    }
-                }
-            }
+            store_tile(&map_x, x, s, tmem_base + ((uint32_t)(quarter * 32) << 16) + ab * BN, stg + quarter * 2 * STG_BYTES, slot, d, m0 + quarter * 32, n0, lane);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(&acc_empty[ab], 0));
         }
+        if (lane == 0) bulk_wait0();
         if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
     }
     tc_fence_before();
@@ -394,13 +419,25 @@ static bool use_pair_kernel() {
 }
 static bool pair_attr_set[64] = {false};
 
-static int launch_contract_tc(const b200pf_planes* a, const b200pf_planes* b, b200pf_bf16* x, const GemmShape& s, cudaStream_t st) {
+static int launch_contract_tc(const b200pf_planes* a, const b200pf_planes* b, b200pf_bf16* x, const GemmShape& shape, cudaStream_t st) {
     unsigned int* status = device_status_word();
     B200PF_REQUIRE(status, B200PF_ERR_CUDA, "trimul_contract: no device status word");
-    CUtensorMap map_a, map_b;
+    CUtensorMap map_a, map_b, map_x;
     int rc;
-    if ((rc = make_plane_map(&map_a, a, s.channels, "A")) != B200PF_OK) return rc;
-    if ((rc = make_plane_map(&map_b, b, s.channels, "B")) != B200PF_OK) return rc;
+    if ((rc = make_plane_map(&map_a, a, shape.channels, "A")) != B200PF_OK) return rc;
+    if ((rc = make_plane_map(&map_b, b, shape.channels, "B")) != B200PF_OK) return rc;
+    GemmShape s = shape;
+    const int groups = s.m_rows > s.x_row_group ? s.m_rows / s.x_row_group : 1;
+    s.x_tma = s.x_col_group == 0 && (groups == 1 ? s.m_rows <= s.x_row_group : s.m_rows % s.x_row_group == 0 && s.x_row_group % 32 == 0);
+    map_x = map_a;
+    if (s.x_tma) {
+        const int rows = s.m_rows < s.x_row_group ? s.m_rows : s.x_row_group;
+        const long long plane = s.channels > 1 ? s.x_plane_stride : (long long)rows * s.x_pitch;      // stride of an extent of 1: anything valid
+        cuuint64_t dims[4] = {(cuuint64_t)s.x_cols, (cuuint64_t)rows, (cuuint64_t)s.channels, (cuuint64_t)groups};
+        cuuint64_t str[3] = {(cuuint64_t)s.x_pitch * 2, (cuuint64_t)plane * 2, (cuuint64_t)(groups > 1 ? s.x_group_stride : plane * s.channels) * 2};
+        cuuint32_t box[4] = {64, 32, 1, 1};
+        if ((rc = tmap_encode(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, "x")) != B200PF_OK) return rc;
+    }
     static bool attr_set[64] = {false};
     int dev = 0;
     B200PF_CUDA(cudaGetDevice(&dev));
@@ -438,11 +475,11 @@ static int launch_contract_tc(const b200pf_planes* a, const b200pf_planes* b, b2
         }
         long long pairs = (dev >= 0 && dev < 64) ? resident_pairs[dev] : sms / 2;
         unsigned grid = 2u * (unsigned)(tiles < pairs ? tiles : pairs);
-        return launch_pdl(trimul_contract_pair_kernel, dim3(grid), dim3(GEMM_THREADS), PAIR_SMEM, st, map_a, map_b, (__nv_bfloat16*)x, s, status);
+        return launch_pdl(trimul_contract_pair_kernel, dim3(grid), dim3(GEMM_THREADS), PAIR_SMEM, st, map_a, map_b, map_x, (__nv_bfloat16*)x, s, status);
     }
     long long tiles = (long long)s.channels * ((s.m_rows + BM - 1) / BM) * ((s.n_rows + BN - 1) / BN);
     unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
-    return launch_pdl(trimul_contract_tc_kernel, dim3(grid), dim3(GEMM_THREADS), GEMM_SMEM, st, map_a, map_b, (__nv_bfloat16*)x, s, status);
+    return launch_pdl(trimul_contract_tc_kernel, dim3(grid), dim3(GEMM_THREADS), GEMM_SMEM, st, map_a, map_b, map_x, (__nv_bfloat16*)x, s, status);
 }
 
 namespace gemm_mx {   // block-scaled fp8 kernel, trimul_gemm_mx.cu
@@ -468,7 +505,7 @@ extern "C" int b200pf_trimul_contract(const b200pf_planes* a, const b200pf_plane
     if ((rc = check_planes(a, "A")) != B200PF_OK) return rc;
     if ((rc = check_planes(b, "B")) != B200PF_OK) return rc;
     B200PF_REQUIRE(x && aligned16(x) && channels > 0, B200PF_ERR_INVALID, "trimul_contract: bad output");
-    GemmShape s;
+    GemmShape s = {};
     s.m_rows = (a->nseg > 1 && !a->seg_is_k) ? a->rows * a->nseg : a->rows;
     s.n_rows = (b->nseg > 1 && !b->seg_is_k) ? b->rows * b->nseg : b->rows;
     int ka = (a->nseg > 1 && a->seg_is_k) ? a->cols * a->nseg : a->cols;
@@ -513,7 +550,7 @@ extern "C" int b200pf_gemm_grouped(const b200pf_planes* a, const b200pf_planes* 
     B200PF_REQUIRE(x_col_group > 0 && x_col_group % 32 == 0 && x_colgroup_stride % 8 == 0 && x_pitch % 8 == 0 &&
                        x_pitch >= x_col_group && x_plane_stride % 8 == 0 && x_group_stride % 8 == 0,
                    B200PF_ERR_INVALID, "gemm_grouped: column groups must be multiples of 32 and every stride a multiple of 8");
-    GemmShape s;
+    GemmShape s = {};
     s.m_rows = a->rows;
     s.n_rows = b->rows;
     s.k_total = a->cols;
@@ -544,7 +581,7 @@ extern "C" int b200pf_opm_outer(const b200pf_bf16* a_t, const b200pf_bf16* b_t, 
                    "opm_outer: too many tokens");
     b200pf_planes a{a_t, (long long)pitch * n_i * 32, 0, pitch, n_i * 32, s_len, 1, 0};
     b200pf_planes b{b_t, (long long)pitch * n_j * 32, 0, pitch, n_j * 32, s_len, 1, 0};
-    GemmShape s;
+    GemmShape s = {};
     s.m_rows = n_i * 32;
     s.n_rows = n_j * 32;
     s.k_total = s_len;
