@@ -1,7 +1,7 @@
 // A block's kernels enqueued by one call: the pair track of the bf16 tier and the single track.  Only the order of the launches
 // is kept here; the work is behind the entry points of the sub-operations.  A block is some 23 launches: enqueued one by one from
 // an interpreter they cost the host 7.8 us each, 180 us a block, more than a block of 45 tokens keeps the GPU busy.
-#include "common.cuh"
+#include "pdl.cuh"
 
 using namespace b200pf;
 
@@ -67,7 +67,14 @@ extern "C" int b200pf_single_track_beside(float* s, const float* z, const b200pf
         B200PF_TRY(b200pf_ln_heads(z, wb->gamma, wb->beta, wb->w, bias, nn, nn, wb->cz, wb->heads, pair));
     B200PF_CUDA(cudaEventRecord((cudaEvent_t)ready, pair));
     B200PF_CUDA(cudaStreamWaitEvent(side, (cudaEvent_t)ready, 0));
-    B200PF_TRY(b200pf_single_track_rows(s, w, bias, mask, n, workspace, side));
+    {
+        // Up to 128 tokens a row kernel of the pair track has a CTA per line and leaves the other SMs idle.  The single track's kernels
+        // keep to those: spread over the whole chip they held SMs that the pair track's next kernel then waited for.
+        int sms;
+        B200PF_TRY(device_multiprocessors(&sms));
+        const CtaLimit limit(n <= 128 && sms - n >= 16 ? sms - n : 0);
+        B200PF_TRY(b200pf_single_track_rows(s, w, bias, mask, n, workspace, side));
+    }
     B200PF_CUDA(cudaEventRecord((cudaEvent_t)done, side));
     return B200PF_OK;
 }

@@ -35,7 +35,7 @@ static inline int launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size
 }
 
 // Multiprocessors of the current device, asked for once per device.
-static inline int multiprocessors(int* out) {
+static inline int device_multiprocessors(int* out) {
     static int known[64] = {0};
     int dev = 0;
     B200PF_CUDA(cudaGetDevice(&dev));
@@ -46,6 +46,21 @@ static inline int multiprocessors(int* out) {
     }
     *out = sms;
     return B200PF_OK;
+}
+
+// The multiprocessors that a launch sizes its grid for: the device's, or fewer while this thread holds a CtaLimit.
+inline thread_local int cta_limit = 0;
+struct CtaLimit {
+    const int before;
+    explicit CtaLimit(int n) : before(cta_limit) { cta_limit = n; }
+    ~CtaLimit() { cta_limit = before; }
+    CtaLimit(const CtaLimit&) = delete;
+    CtaLimit& operator=(const CtaLimit&) = delete;
+};
+static inline int multiprocessors(int* out) {
+    const int rc = device_multiprocessors(out);
+    if (rc == B200PF_OK && cta_limit > 0 && cta_limit < *out) *out = cta_limit;
+    return rc;
 }
 
 }  // namespace b200pf

@@ -44,7 +44,7 @@ static int residual_gemm(float* y, const void* planes, const b200pf_split_weight
     g.a[0] = matrix(planes, rows, k);
     g.b[0] = matrix(w.w, n, k);
     g.m_rows = (int)rows; g.n_rows = n; g.k[0] = k; g.alpha[0] = w.alpha;
-    int sms, rc = multiprocessors(&sms);
+    int sms, rc = device_multiprocessors(&sms);       // not the launch's share: the sums' order must not depend on it
     if (rc != B200PF_OK) return rc;
     const int ks = partial ? k_splits_for((int)rows, n, k, sms) : 1;
     if (ks == 1) {
