@@ -47,8 +47,8 @@ __device__ __forceinline__ long long x_row_offset(const GemmShape& s, int d, int
 // One epilogue warp's 32 rows (from `row0`) x 256 columns of a finished accumulator.  Plain planes leave through a swizzled staging tile and
 // TMA stores of [32 rows][64 columns].  As 16-byte stores of a thread per row, 4096 partial sectors a tile, they took 11 k clocks a tile
 // against 3.6 k to 8.2 k of MMAs: 11.7 -> 9.7 us at 203 tokens, 43 -> 35 at 400, 112 -> 94 at 600, 238 -> 224 at 1024 (what is left is
-// the operands, some 9 TB/s out of L2).  Columns in groups (the
-// outer product's blocks of contiguous 2 KB) and row groups that 32 does not divide stay with the direct stores.
+// the operands, some 9 TB/s out of L2).  Columns in groups (the outer product's blocks of contiguous 2 KB) and row groups that 32 does
+// not divide stay with the direct stores.
 __device__ __forceinline__ void store_tile(const CUtensorMap* map_x, __nv_bfloat16* x, const GemmShape& s, uint32_t taddr, uint8_t* stg, uint32_t& slot, int d, int row0,
                                            int n0, int lane) {
     using namespace sm100;
