@@ -8,10 +8,11 @@
 // contiguously), the projection a second one over the 1024 (c, d) products (b200pf_trimul_contract with one
 // channel).  This file holds what feeds and drains them:
 //   opm_producer_kernel : LayerNorm + both projections + mask, written TRANSPOSED (sequence index contiguous) as
-//                         the GEMM's K-major operands; fp32 factors as two tf32 parts on mma.sync, bf16 on store.
+//                         the GEMM's K-major operands; fp32 throughout, bf16 on store.
 //   opm_mask_bits_kernel: the MSA mask as one bit per sequence, 32 sequences per word and token.
 //   opm_finalize_kernel : pair counts by popcount of the two tokens' words, then y / count + bias added into (or
 //                         written over) the fp32 pair rows.
+#include "mma.cuh"
 #include "pdl.cuh"
 
 namespace b200pf {
@@ -19,130 +20,134 @@ namespace opm {
 
 constexpr int CM = 64;            // MSA channels
 constexpr int CH = 32;            // projected channels per side
-constexpr int PROD_WARPS = 4, PROD_THREADS = PROD_WARPS * 32, PROD_ROWS = PROD_WARPS * 32;      // sequences per CTA and token
-constexpr int WF_ENTRIES = 4 * 8 * 32;                           // weight fragments: 4 row blocks of 16, 8 K steps, 32 lanes
-constexpr int STG_PITCH = 80;                                    // bytes per staged output row: 32 bf16 and 16 to spread the banks
-constexpr int PROD_SMEM = 2 * WF_ENTRIES * 16 + PROD_WARPS * 2 * CH * STG_PITCH;                // 53,248
+constexpr int PROD_THREADS = 128, PROD_ROWS = 64;                // sequences per CTA and token
+constexpr int XP = CM + 4;        // pitch of a staged row in floats: 16-byte reads of eight rows meet no bank twice
+constexpr int PROD_SMEM = (CM * 2 * CH + PROD_ROWS * (XP + CM + 1) + 2 * CM) * 4;               // 50,944: four CTAs per SM
 constexpr int FIN_THREADS = 256, FIN_J = 64;
 constexpr int MAX_WORDS = 512;    // sequences / 32 the finalize kernel keeps in shared memory (S <= 16384)
 
-// v = hi + lo, both rounded to tf32's 11 significant bits: 2^-23 of v is left.  cvt and not integer arithmetic: a NaN stays one.
-__device__ __forceinline__ void split_tf32(float v, uint32_t& hi, uint32_t& lo) {
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(v));
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(v - __uint_as_float(hi)));
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+__device__ __forceinline__ uint64_t twice(float w) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(w));
+    return r;
 }
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint4& a, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
-}
+__device__ __forceinline__ void both(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
 
-// A warp takes 32 sequences of one token: D[output][sequence] = W x^T, three tf32 MMAs per product (hi*hi, hi*lo, lo*hi: 2^-22 of
-// a product is left out), so every output lies as the operands want it.  The sum over the 64 channels may run in any order, so
-// lane (g, t) owns channels 16 q + 4 t .. + 3 of row g: the rows arrive as whole 64-byte pieces straight into B fragments, and the
-// weights are laid out once per CTA as A fragments in the same order.  A CTA walks several tokens.  One thread per row with the
-// weights broadcast from shared memory (4096 FMAs and 1024 shared loads a row, every lane on lines of its own) took 230 us at
-// 1024 sequences x 600 tokens.
+// A CTA takes 64 sequences of one token at a time: rows into shared memory, a thread per row for the LayerNorm, then a thread per
+// 8 sequences x 8 outputs, all in fp32 and every sum in one order: the mean and the variance over the channels in turn, an output as
+// two chains of FMAs (channels 0-3, 8-11, .. on warps 0 and 1, channels 4-7, 12-15, .. on warps 2 and 3) that are added at the end.  The
+// operands are rounded to bf16 right behind, and a last bit that flips there moves the whole MSA module's result by 2e-3 of its norm:
+// products of two tf32 parts (2^-22 of a product left out) on the tensor cores did that, in 119 us at 1024 sequences x 600 tokens.  The
+// same sums by a thread per row, the weights broadcast from shared memory (a 16-byte load per four FMAs), took 226 us there and 19 at
+// 122 x 171; here a load serves sixteen FMAs, packed two sequences each: 138 and 12.  What bounds it are those loads, 512 bytes a warp
+// into registers at 128 a clock, beside the FMAs.
 __global__ void __launch_bounds__(PROD_THREADS, 4)
 opm_producer_kernel(const float* m, const uint8_t* mask, const float* gamma, const float* beta, const float* w_ab, __nv_bfloat16* a_t,
                     __nv_bfloat16* b_t, int s_len, int n, int pitch, int vec) {
     extern __shared__ __align__(16) uint8_t smem[];
-    uint4* wf = reinterpret_cast<uint4*>(smem);                  // [part][row block][K step][lane]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    uint8_t* stg = smem + 2 * WF_ENTRIES * 16 + warp * (2 * CH * STG_PITCH);
+    float* w_s = reinterpret_cast<float*>(smem);                          // [channel][output]
+    float* in_s = w_s + CM * 2 * CH;                                      // [row][XP] as loaded
+    float* x_s = in_s + PROD_ROWS * XP;                                   // [channel][row] normalised
+    float* keep_s = x_s + CM * PROD_ROWS;
+    float* gb_s = keep_s + PROD_ROWS;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, s0 = blockIdx.x * PROD_ROWS;
+    const int chain = tid >> 6, u = tid & 63, rg = (u & 7) * 4, o0 = (u >> 3) * 8;       // rows rg .. + 3 and 32 + rg .. + 3, outputs o0 .. + 7
     grid_dependency_wait();
     grid_launch_dependents();
-    for (int i = threadIdx.x; i < WF_ENTRIES; i += PROD_THREADS) {
-        const int ln = i & 31, ks = (i >> 5) & 7, mb = i >> 8;
-        const float* w0 = w_ab + (mb * 16 + (ln >> 2)) * CM + (ks >> 1) * 16 + (ln & 3) * 4 + (ks & 1) * 2;
-        const float2 lo8 = *reinterpret_cast<const float2*>(w0), hi8 = *reinterpret_cast<const float2*>(w0 + 8 * CM);
-        uint4 h, l;
-        split_tf32(lo8.x, h.x, l.x); split_tf32(hi8.x, h.y, l.y); split_tf32(lo8.y, h.z, l.z); split_tf32(hi8.y, h.w, l.w);
-        wf[i] = h;
-        wf[WF_ENTRIES + i] = l;
-    }
-    float4 gam[4], bet[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        gam[q] = make_float4(gamma[q * 16 + 4 * t], gamma[q * 16 + 4 * t + 1], gamma[q * 16 + 4 * t + 2], gamma[q * 16 + 4 * t + 3]);
-        bet[q] = make_float4(beta[q * 16 + 4 * t], beta[q * 16 + 4 * t + 1], beta[q * 16 + 4 * t + 2], beta[q * 16 + 4 * t + 3]);
-    }
-    __syncthreads();
-    const int s_base = blockIdx.x * PROD_ROWS + warp * 32;
-    if (s_base >= s_len) return;
-    for (int tok = blockIdx.y; tok < n; tok += gridDim.y) {
-#pragma unroll 1
-        for (int half = 0; half < 2; ++half) {                   // 16 sequences: two column blocks of 8
-            uint32_t xh[2][16], xl[2][16];
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                const int s = s_base + half * 16 + nt * 8 + g;
-                const long long row = (long long)(s < s_len ? s : s_len - 1) * n + tok;     // rows past the end repeat the last one
-                const float4* src = reinterpret_cast<const float4*>(m + row * CM) + t;
-                float4 v[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) v[q] = src[q * 4];
-                const float keep = mask[row] ? 1.f : 0.f;
-                float sum = 0.f;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) sum += (v[q].x + v[q].y) + (v[q].z + v[q].w);
-                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-                const float mean = sum * (1.f / CM);
-                float ss = 0.f;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    v[q].x -= mean; v[q].y -= mean; v[q].z -= mean; v[q].w -= mean;
-                    ss += (v[q].x * v[q].x + v[q].y * v[q].y) + (v[q].z * v[q].z + v[q].w * v[q].w);
-                }
-                ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-                ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-                const float rstd = rsqrtf(ss * (1.f / CM) + LN_EPS);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    split_tf32(fmaf(v[q].x * rstd, gam[q].x, bet[q].x) * keep, xh[nt][4 * q], xl[nt][4 * q]);
-                    split_tf32(fmaf(v[q].y * rstd, gam[q].y, bet[q].y) * keep, xh[nt][4 * q + 1], xl[nt][4 * q + 1]);
-                    split_tf32(fmaf(v[q].z * rstd, gam[q].z, bet[q].z) * keep, xh[nt][4 * q + 2], xl[nt][4 * q + 2]);
-                    split_tf32(fmaf(v[q].w * rstd, gam[q].w, bet[q].w) * keep, xh[nt][4 * q + 3], xl[nt][4 * q + 3]);
-                }
-            }
-#pragma unroll 1
-            for (int mb = 0; mb < 4; ++mb) {
-                float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, small[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-                for (int ks = 0; ks < 8; ++ks) {
-                    const uint4 wh = wf[(mb * 8 + ks) * 32 + lane], wl = wf[WF_ENTRIES + (mb * 8 + ks) * 32 + lane];
-                    const int e = (ks >> 1) * 4 + (ks & 1) * 2;
-#pragma unroll
-                    for (int nt = 0; nt < 2; ++nt) {
-                        mma_tf32(acc[nt], wh, xh[nt][e], xh[nt][e + 1]);
-                        mma_tf32(small[nt], wh, xl[nt][e], xl[nt][e + 1]);
-                        mma_tf32(small[nt], wl, xh[nt][e], xh[nt][e + 1]);
-                    }
-                }
-#pragma unroll
-                for (int nt = 0; nt < 2; ++nt) {
-                    uint8_t* at = stg + (mb * 16 + g) * STG_PITCH + (half * 16 + nt * 8 + 2 * t) * 2;
-                    *reinterpret_cast<uint32_t*>(at) = pack_bf16x2(acc[nt][0] + small[nt][0], acc[nt][1] + small[nt][1]);
-                    *reinterpret_cast<uint32_t*>(at + 8 * STG_PITCH) = pack_bf16x2(acc[nt][2] + small[nt][2], acc[nt][3] + small[nt][3]);
-                }
-            }
+    auto load_rows = [&](int tok) {                                       // 16 lanes per row; rows past the end repeat the last one
+        for (int i = tid; i < PROD_ROWS * (CM / 4); i += PROD_THREADS) {
+            const int r = i >> 4, c = (i & 15) * 4, s = s0 + r;
+            cp_async16(in_s + r * XP + c, m + ((long long)(s < s_len ? s : s_len - 1) * n + tok) * CM + c);
         }
-        __syncwarp();
+        cp_async_commit();
+    };
+    load_rows(blockIdx.y);
+    gb_s[tid] = tid < CM ? gamma[tid] : beta[tid - CM];
+    for (int i = tid; i < 2 * CH * (CM / 4); i += PROD_THREADS) {
+        const int o = i & (2 * CH - 1), k = (i >> 6) * 4;
+        const float4 w = *reinterpret_cast<const float4*>(w_ab + o * CM + k);
+        w_s[k * 2 * CH + o] = w.x;
+        w_s[(k + 1) * 2 * CH + o] = w.y;
+        w_s[(k + 2) * 2 * CH + o] = w.z;
+        w_s[(k + 3) * 2 * CH + o] = w.w;
+    }
+    int turn = 0;
+#pragma unroll 1
+    for (int tok = blockIdx.y; tok < n; tok += gridDim.y, turn ^= 2) {
+        cp_async_wait<0>();
+        __syncthreads();
+        const int row = ((warp + turn) & 3) * 32 + lane;                  // two warps normalise, the other two the next time: a warp
+        const bool ln = row < PROD_ROWS;                                  // stays on its scheduler
+        if (ln) {
+            const int s = s0 + row;
+            const bool keep = mask[(long long)(s < s_len ? s : s_len - 1) * n + tok] != 0;
+            float x[CM], sum = 0.f, ss = 0.f;
 #pragma unroll
-        for (int it = 0; it < 8; ++it) {                         // 64 output rows of 64 bytes, four lanes each
-            const int o = it * 8 + g, s = s_base + t * 8;
-            const uint4 v = *reinterpret_cast<const uint4*>(stg + o * STG_PITCH + t * 16);
-            __nv_bfloat16* dst = (o < CH ? a_t : b_t) + ((long long)tok * CH + (o & (CH - 1))) * pitch + s;
-            if (vec && s + 8 <= s_len) {
-                *reinterpret_cast<uint4*>(dst) = v;
+            for (int j = 0; j < CM / 4; ++j) {
+                const float4 v = *reinterpret_cast<const float4*>(in_s + row * XP + 4 * j);
+                x[4 * j] = v.x; x[4 * j + 1] = v.y; x[4 * j + 2] = v.z; x[4 * j + 3] = v.w;
+            }
+#pragma unroll
+            for (int k = 0; k < CM; ++k) sum += x[k];
+            const float mean = sum * (1.f / CM);
+#pragma unroll
+            for (int k = 0; k < CM; ++k) { x[k] -= mean; ss = fmaf(x[k], x[k], ss); }
+            const float rstd = rsqrtf(ss * (1.f / CM) + LN_EPS);
+#pragma unroll
+            for (int k = 0; k < CM; ++k) x_s[k * PROD_ROWS + row] = fmaf(x[k] * rstd, gb_s[k], gb_s[CM + k]);
+            keep_s[row] = keep ? 1.f : 0.f;
+        }
+        __syncthreads();
+        if (tok + (int)gridDim.y < n) load_rows(tok + gridDim.y);         // the next rows arrive under the products
+        uint64_t acc[8][4] = {};                                          // output, pair of rows
+#pragma unroll 1
+        for (int k4 = chain * 4; k4 < CM; k4 += 8)
+#pragma unroll
+            for (int e = 3; e >= 0; --e) {
+                const float* xk = x_s + (k4 + e) * PROD_ROWS + rg;
+                const float* wk = w_s + (k4 + e) * 2 * CH + o0;
+                const ulonglong2 xa = *reinterpret_cast<const ulonglong2*>(xk), xb = *reinterpret_cast<const ulonglong2*>(xk + PROD_ROWS / 2);
+                const float4 wa = *reinterpret_cast<const float4*>(wk), wb = *reinterpret_cast<const float4*>(wk + 4);
+                const uint64_t w[8] = {twice(wa.x), twice(wa.y), twice(wa.z), twice(wa.w), twice(wb.x), twice(wb.y), twice(wb.z), twice(wb.w)};
+#pragma unroll
+                for (int o = 0; o < 8; ++o) {
+                    fma2(acc[o][0], w[o], xa.x);
+                    fma2(acc[o][1], w[o], xa.y);
+                    fma2(acc[o][2], w[o], xb.x);
+                    fma2(acc[o][3], w[o], xb.y);
+                }
+            }
+        // the chains meet: each thread gives four of its outputs to the one with the other chain and finishes the other four
+        __syncthreads();
+        ulonglong2* ex = reinterpret_cast<ulonglong2*>(x_s);              // [chain][output, half of the rows][thread]
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int o = j >> 1, h = 2 * (j & 1);
+            ex[(chain * 8 + j) * 64 + u] = chain ? make_ulonglong2(acc[o][h], acc[o][h + 1]) : make_ulonglong2(acc[4 + o][h], acc[4 + o][h + 1]);
+        }
+        __syncthreads();
+        const int oo = o0 + 4 * chain;
+        __nv_bfloat16* dst = (oo < CH ? a_t : b_t) + ((long long)tok * CH + (oo & (CH - 1))) * pitch + s0 + rg;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int o = j >> 1, h = 2 * (j & 1);
+            const float4 other = *reinterpret_cast<const float4*>(ex + ((chain ^ 1) * 8 + j) * 64 + u);
+            const float4 keep = *reinterpret_cast<const float4*>(keep_s + (j & 1) * (PROD_ROWS / 2) + rg);
+            float v[4];
+            both(chain ? acc[4 + o][h] : acc[o][h], v[0], v[1]);
+            both(chain ? acc[4 + o][h + 1] : acc[o][h + 1], v[2], v[3]);
+            v[0] = (v[0] + other.x) * keep.x; v[1] = (v[1] + other.y) * keep.y; v[2] = (v[2] + other.z) * keep.z; v[3] = (v[3] + other.w) * keep.w;
+            const int s = s0 + (j & 1) * (PROD_ROWS / 2) + rg;
+            __nv_bfloat16* at = dst + o * (long long)pitch + (j & 1) * (PROD_ROWS / 2);
+            if (vec && s + 4 <= s_len) {
+                *reinterpret_cast<uint2*>(at) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
             } else {
-                const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    if (s + e < s_len) reinterpret_cast<uint16_t*>(dst)[e] = (uint16_t)(w4[e >> 1] >> (16 * (e & 1)));
+                for (int e = 0; e < 4; ++e)
+                    if (s + e < s_len) at[e] = __float2bfloat16(v[e]);
             }
         }
-        __syncwarp();
     }
 }
 
@@ -215,9 +220,9 @@ extern "C" int b200pf_opm_producer(const float* m, const uint8_t* mask, const fl
     int sms, rc;
     if ((rc = multiprocessors(&sms)) != B200PF_OK) return rc;
     B200PF_SMEM_ATTR_ONCE(opm_producer_kernel, PROD_SMEM);
-    // four CTAs fit an SM; each takes every gridDim.y-th token of its sequences, so that its weight fragments serve several
+    // four CTAs fit an SM; each takes every gridDim.y-th token of its sequences, so that its copy of the weights serves several
     const int tiles = (s_len + PROD_ROWS - 1) / PROD_ROWS, want = (4 * sms + tiles - 1) / tiles, per = (n + want - 1) / want;
-    const int vec = aligned16(a_t) && aligned16(b_t) && pitch % 8 == 0;
+    const int vec = aligned16(a_t) && aligned16(b_t) && pitch % 4 == 0;
     return launch_pdl(opm_producer_kernel, dim3((unsigned)tiles, (unsigned)((n + per - 1) / per)), dim3(PROD_THREADS), PROD_SMEM, (cudaStream_t)stream,
                       m, mask, ln_gamma, ln_beta, w_ab, (__nv_bfloat16*)a_t, (__nv_bfloat16*)b_t, s_len, n, pitch, vec);
 }
