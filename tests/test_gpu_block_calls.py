@@ -53,6 +53,21 @@ def test_single_track_beside_the_pair_track(n, precision, monkeypatch):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("n", [100, 128])
+def test_single_track_beside_a_wide_pair_track(n, monkeypatch):
+    """256 pair channels: the single track's kernels take the whole chip there, next to 128 channels they keep to a part of it."""
+    mod = B200PairformerModule(384, 256, 3, pairwise_num_heads=8, v2=True, precision="auto")
+    mod.load_state_dict(synthetic.make_weights(3, seed=3, std=0.05, affine_jitter=0.2, c_z=256, tri_heads=8), strict=True)
+    s, z = synthetic.make_inputs(n, c_z=256, seed=n)
+    args = [t.cuda() for t in (s, z, *synthetic.tail_padding_mask(n, n // 8))]
+    monkeypatch.setenv("B200PF_SIDE_TRACK", "0")
+    behind = mod(*args)
+    monkeypatch.setenv("B200PF_SIDE_TRACK", "1")
+    beside = mod(*args)
+    assert torch.equal(behind[0], beside[0]) and torch.equal(behind[1], beside[1])
+    assert _lib.device_status() == 0
+
+
 def test_a_failing_layer_leaves_nothing_running_beside(monkeypatch):
     mod = _module(3)
     args = _inputs(40)

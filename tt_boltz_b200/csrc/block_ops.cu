@@ -1,7 +1,7 @@
 // A block's kernels enqueued by one call: the pair track of the bf16 tier and the single track.  Only the order of the launches
 // is kept here; the work is behind the entry points of the sub-operations.  A block is some 23 launches: enqueued one by one from
 // an interpreter they cost the host 7.8 us each, 180 us a block, more than a block of 45 tokens keeps the GPU busy.
-#include "pdl.cuh"
+#include "rowtc.cuh"
 
 using namespace b200pf;
 
@@ -68,11 +68,16 @@ extern "C" int b200pf_single_track_beside(float* s, const float* z, const b200pf
     B200PF_CUDA(cudaEventRecord((cudaEvent_t)ready, pair));
     B200PF_CUDA(cudaStreamWaitEvent(side, (cudaEvent_t)ready, 0));
     {
-        // Up to 128 tokens a row kernel of the pair track has a CTA per line and leaves the other SMs idle.  The single track's kernels
-        // keep to those: spread over the whole chip they held SMs that the pair track's next kernel then waited for.
+        // Up to one tile of positions per line, the producers and the tri-mul epilogue of a 128-wide pair track have a CTA per line and
+        // leave the other SMs idle most of the time.  The single track's GEMMs, whose CTAs take an SM each, are sized for those: spread
+        // over the whole chip they hold SMs that the pair track's next kernel then waits for.  (Its LayerNorms, attention and partial sums
+        // are small CTAs that fit beside others.)  Eight blocks at 128 tokens 1199 -> 1136 us, at 117 1158 -> 1151, at 90 1035 -> 1025.
+        // With 12, 16 or 20 SMs it is the same at 128, with 8 the single track becomes the longer one (1161; 1168 at 117).  The GEMMs of a
+        // 256-wide pair track fill the chip at any size: four of its blocks at 110 tokens lose by the limit (1604 -> 1610 us).
+        constexpr int LEAST_SMS = 12;
         int sms;
         B200PF_TRY(device_multiprocessors(&sms));
-        const CtaLimit limit(n <= 128 && sms - n >= 16 ? sms - n : 0);
+        const CtaLimit limit(wb->cz == rtc::KC && n <= rtc::TM && sms - n >= LEAST_SMS ? sms - n : 0);
         B200PF_TRY(b200pf_single_track_rows(s, w, bias, mask, n, workspace, side));
     }
     B200PF_CUDA(cudaEventRecord((cudaEvent_t)done, side));

@@ -321,7 +321,7 @@ int launch_attention(const AttnArgs& args, int hd, cudaStream_t st) {
     B200PF_REQUIRE(hd == 24 || hd == 32, B200PF_ERR_UNSUPPORTED, "split attention: head width 24 or 32 (got %d)", hd);
     // eight warps share a K / V tile; with fewer than two such CTAs per SM, four warps per CTA spread the queries further
     int sms, rc;
-    if ((rc = multiprocessors(&sms)) != B200PF_OK) return rc;
+    if ((rc = device_multiprocessors(&sms)) != B200PF_OK) return rc;      // its CTAs share an SM: a CtaLimit does not mean them
     const bool wide = (long long)a.lines * a.heads * ((a.n_q + 127) / 128) >= 2LL * sms;
     if (hd == 24) return wide ? attn_go<24, 8>(a, st) : attn_go<24, 4>(a, st);
     return wide ? attn_go<32, 8>(a, st) : attn_go<32, 4>(a, st);
