@@ -114,13 +114,4 @@ __device__ __forceinline__ void zero_acc(float (&acc)[2][NT][4]) {
             for (int e = 0; e < 4; ++e) acc[mi][nt][e] = 0.f;
 }
 
-// Copy a [rows][128] bf16 weight matrix from global memory into shared memory with row pitch
-// APITCH; all threads of the CTA take part.  Caller synchronises.
-__device__ __forceinline__ void load_weights_k128(__nv_bfloat16* dst, const __nv_bfloat16* src, int rows) {
-    for (int i = threadIdx.x; i < rows * 16; i += blockDim.x) {
-        int r = i >> 4, c = i & 15;
-        *reinterpret_cast<uint4*>(dst + r * APITCH + c * 8) = *reinterpret_cast<const uint4*>(src + r * KC + c * 8);
-    }
-}
-
 }  // namespace b200pf
