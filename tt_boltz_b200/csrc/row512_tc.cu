@@ -102,7 +102,9 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         fence_barrier_init();
         fence_proxy_async();
     }
-    if (tid == 32) {
+    // Fetched by warp 1, the multiplication's producers spill in their loaders (at 1024 tokens outgoing 257 us for 242, incoming 326 for 289);
+    // by the MMA warp, the attention's does (18.4 us for 17.8 at 203).
+    if (MODE == MODE_TRIATT ? tid == 32 : warp == MMA_WARP && elect_one()) {
         tma_prefetch_desc(&map_w); tma_prefetch_desc(&map0); tma_prefetch_desc(&map1);
         if (MODE == MODE_TRIATT) { tma_prefetch_desc(&map2); tma_prefetch_desc(&map3); }
     }
@@ -118,9 +120,17 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         return p.transposed ? (long long)pos * p.n + line : (long long)line * p.n + pos;
     };
 
+    // Mask byte of row `row` of tile `t`, 0 where there is none.  The bf16 multiplication's loaders ask for it a tile ahead, a lane per row:
+    // eight lanes asking with the row itself, in a column each on a line of its own, took 293 us for 278 incoming at 1024 tokens.  The MXFP8
+    // producer is slower that way (279 us for 260) and asks with the row.
+    auto mask_of = [&](int t, int row) -> uint32_t {
+        const int line = t / tpl;
+        const long long f = t < tiles ? flat_of(line, (t - line * tpl) * TM + row) : -1;
+        return f >= 0 ? p.mask[f] : 0u;
+    };
     // One warp's 16 rows of a tile: LayerNorm of positions pos0 + row0 .. of line `line` into the A tile; 8 lanes per row.
     const int sub = lane & 7, rq = lane >> 3;
-    auto normalise16 = [&](int line, int pos0, int row0, uint8_t* a_tile, const float4 (&gam)[4], const float4 (&bet)[4]) {
+    auto normalise16 = [&](int line, int pos0, int row0, uint32_t kept, uint8_t* a_tile, const float4 (&gam)[4], const float4 (&bet)[4]) {
         float4 v[4][4];
         // rows 4 i of the pass: one flat index and a stride (positions of a column lie n rows apart)
         const int pos_b = pos0 + row0 + rq;
@@ -129,7 +139,7 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const bool valid = pos_b + i * 4 < span;
-            if (p.z_bf16) {          // warp-uniform: four bf16 channels per lane and j, widened on the fly
+            if (MODE != MODE_TRIMUL && p.z_bf16) {          // warp-uniform: four bf16 channels per lane and j, widened on the fly
                 const uint2* src = reinterpret_cast<const uint2*>(p.z_bf16 + (f0 + i * fstep) * KC) + sub;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -148,7 +158,8 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             bool keep = pos_b + i * 4 < span;
-            if (MODE != MODE_TRIATT) keep = keep && p.mask[f0 + i * fstep] != 0;
+            if (MODE == MODE_TRIMUL) keep = (kept >> (i * 4 + rq)) & 1u;
+            if (MODE == MODE_TRIMUL_MX) keep = keep && p.mask[f0 + i * fstep] != 0;
             kz[i] = keep ? 1.f : 0.f;
         }
         float s4[4];
@@ -210,6 +221,8 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         float4 gam[4], bet[4];
         load_affine(gam, bet);
         uint32_t it = 1;                    // the epilogue warps normalise the CTA's first tile
+        uint32_t mine = 0;                  // mask of this lane's row of the next tile
+        if (MODE == MODE_TRIMUL) mine = mask_of((int)(blockIdx.x + gridDim.x), warp * 32 + lane);
         bool ok = true;
         for (int t = (int)(blockIdx.x + gridDim.x); t < tiles && ok; t += gridDim.x, ++it) {
             const int line = t / tpl, pos0 = (t - line * tpl) * TM;
@@ -217,6 +230,8 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
             ok = mbar_wait(&B->a_empty[stage], ph ^ 1, abort_flag);
             if (!ok) break;
             uint8_t* a_tile = smem + OFF_A + stage * A_TILE_BYTES;
+            const uint32_t kept = MODE != MODE_TRIMUL ? 0u : __ballot_sync(0xffffffffu, mine != 0);
+            if (MODE == MODE_TRIMUL) mine = 0;
             // this warp's 32 rows of the NEXT tile: one lane per row asks L2 for its four 128-byte lines, so the
             // loads of the next round find them there instead of paying the DRAM latency with only 4 warps in flight
             {
@@ -224,7 +239,8 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
                 if (tn < tiles) {
                     const long long f = flat_of(ln, (tn - ln * tpl) * TM + warp * 32 + lane);
                     if (f >= 0) {
-                        if (p.z_bf16) {
+                        if (MODE == MODE_TRIMUL) mine = p.mask[f];
+                        if (MODE != MODE_TRIMUL && p.z_bf16) {
                             const char* rowp = reinterpret_cast<const char*>(p.z_bf16 + f * KC);
 #pragma unroll
                             for (int j = 0; j < 2; ++j) asm volatile("prefetch.global.L2 [%0];" ::"l"(rowp + j * 128));
@@ -238,7 +254,7 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
             }
 #pragma unroll 1
             for (int pass = 0; pass < 2; ++pass) {
-                normalise16(line, pos0, warp * 32 + pass * 16, a_tile, gam, bet);
+                normalise16(line, pos0, warp * 32 + pass * 16, kept >> (pass * 16), a_tile, gam, bet);
             }
             fence_proxy_async();
             __syncwarp();
@@ -302,7 +318,9 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
             float4 gam[4], bet[4];
             load_affine(gam, bet);
             const int line = (int)blockIdx.x / tpl;
-            normalise16(line, ((int)blockIdx.x - line * tpl) * TM, (warp - EPI_WARP0) * 16, smem + OFF_A, gam, bet);
+            const int row0 = (warp - EPI_WARP0) * 16;
+            const uint32_t kept = MODE != MODE_TRIMUL ? 0u : __ballot_sync(0xffffffffu, mask_of((int)blockIdx.x, row0 + (lane & 15)) != 0);
+            normalise16(line, ((int)blockIdx.x - line * tpl) * TM, row0, kept, smem + OFF_A, gam, bet);
             fence_proxy_async();
             named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
             if (warp - EPI_WARP0 < LOAD_WARPS && lane == 0) mbar_arrive(&B->a_full[0]);       // the loaders' arrivals of this phase
