@@ -130,7 +130,7 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
     };
     // One warp's 16 rows of a tile: LayerNorm of positions pos0 + row0 .. of line `line` into the A tile; 8 lanes per row.
     const int sub = lane & 7, rq = lane >> 3;
-    auto normalise16 = [&](int line, int pos0, int row0, uint32_t kept, uint8_t* a_tile, const float4 (&gam)[4], const float4 (&bet)[4]) {
+    auto normalise16 = [&](int line, int pos0, int row0, auto kept_bits, uint8_t* a_tile, const float4 (&gam)[4], const float4 (&bet)[4]) {
         float4 v[4][4];
         // rows 4 i of the pass: one flat index and a stride (positions of a column lie n rows apart)
         const int pos_b = pos0 + row0 + rq;
@@ -154,6 +154,7 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         }
         // The four rows of a pass are worked on stage by stage (all sums, then all shuffles, ...), not row by
         // row: one loader warp per scheduler has nothing else to hide a dependent chain behind.
+        const uint32_t kept = kept_bits();       // asked for behind the rows' loads: nothing waits for a mask ahead of them
         float kz[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -254,7 +255,7 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
             }
 #pragma unroll 1
             for (int pass = 0; pass < 2; ++pass) {
-                normalise16(line, pos0, warp * 32 + pass * 16, kept >> (pass * 16), a_tile, gam, bet);
+                normalise16(line, pos0, warp * 32 + pass * 16, [&] { return kept >> (pass * 16); }, a_tile, gam, bet);
             }
             fence_proxy_async();
             __syncwarp();
@@ -319,8 +320,9 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
             load_affine(gam, bet);
             const int line = (int)blockIdx.x / tpl;
             const int row0 = (warp - EPI_WARP0) * 16;
-            const uint32_t kept = MODE != MODE_TRIMUL ? 0u : __ballot_sync(0xffffffffu, mask_of((int)blockIdx.x, row0 + (lane & 15)) != 0);
-            normalise16(line, ((int)blockIdx.x - line * tpl) * TM, row0, kept, smem + OFF_A, gam, bet);
+            const uint32_t mine = MODE != MODE_TRIMUL ? 0u : mask_of((int)blockIdx.x, row0 + (lane & 15));
+            normalise16(line, ((int)blockIdx.x - line * tpl) * TM, row0, [&] { return MODE != MODE_TRIMUL ? 0u : __ballot_sync(0xffffffffu, mine != 0); },
+                        smem + OFF_A, gam, bet);
             fence_proxy_async();
             named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
             if (warp - EPI_WARP0 < LOAD_WARPS && lane == 0) mbar_arrive(&B->a_full[0]);       // the loaders' arrivals of this phase
