@@ -6,7 +6,7 @@
 // A fragments of the second.  A warp owns 16 queries; per 64-key tile it issues 96 MMAs.  With three bf16 parts and six MMAs per
 // product, and every lane fetching its own bias values, a launch took 462 us at 292 tokens x 4 heads and 528 at 256 x 8; with two
 // parts 390 and 430, with staged bias tiles 310 and 311, with one barrier a tile, interleaved accumulators, scores that stay in the
-// products' scale, packed fp32 arithmetic (1190 -> 761 instructions per warp and tile) and masks fetched a tile ahead 258 and 245.
+// products' scale, packed fp32 arithmetic (1190 -> 779 instructions per warp and tile) and masks fetched a tile ahead 258 and 245.
 // K and V tiles are shared by the CTA's warps, double buffered with
 // cp.async; rows are 64 bytes with the 16-byte chunks swizzled by row so that ldmatrix is conflict free.  Bias tiles come with them,
 // as whole lines (read by the lanes that want them, 8 bytes of eight rows at a time and behind the tile before, they were the
