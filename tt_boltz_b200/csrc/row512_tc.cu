@@ -18,12 +18,17 @@
 // Output goes TMEM -> registers -> a swizzled staging tile -> TMA stores, so that global memory
 // only ever sees full, contiguous lines (thread-per-row 16-byte stores were 3x slower).  Every epilogue
 // warp has a staging tile and stores of its own: no warp waits for another.
-// Roles (416 threads): warps 0-3 LayerNorm loaders (32 rows each), warp 4 MMA issuer, warps 5-12
+// Roles (480 threads): warps 0-5 LayerNorm loaders (16 rows at a time, round robin), warp 6 MMA issuer, warps 7-14
 // epilogue (two warps per TMEM lane quarter, each taking half of the columns).  TMEM is used as
 // two halves of 256 columns so the epilogue of one half overlaps the MMAs of the next, and the x
 // tile is double buffered so the loaders run a tile ahead.  A CTA's first tile is normalised by the
 // epilogue warps, 16 rows each, which have nothing else to do before its accumulators exist; the
 // loaders begin with the second.
+// The loaders bound it: a pass is one long chain (loads, two reductions, stores) with nothing to interleave, and four warps took
+// some 9 k clocks for a tile.  Up to 16 warps cost no registers (four per scheduler, 128 a thread, as with 13).  Six loaders against
+// four with 32 rows each: 269 / 290 -> 232 / 247 us (multiplication, outgoing / incoming) and 352 / 356 -> 326 / 330 (attention, rows /
+// columns) at 1024 tokens, 47.8 -> 43.4 and 61.3 -> 60.2 at 400, the same at 203, where a CTA has three tiles; five are slower
+// everywhere (252 / 273 and 334 / 333), seven no faster (238 / 251 and 324 / 334) and spill in the MXFP8 form.
 #include "mxfp8.cuh"
 #include "row512_tc.h"
 #include "rowtc.cuh"
@@ -35,7 +40,8 @@ namespace r512 {
 using namespace rtc;
 
 constexpr int MODE_TRIMUL = 0, MODE_TRIATT = 1, MODE_TRIMUL_MX = 2;   // MX: e4m3 planes + e8m0 scales (mxfp8.cuh)
-constexpr int LOAD_WARPS = 4, MMA_WARP = 4, EPI_WARP0 = 5, EPI_WARPS = 8, THREADS = 13 * 32;
+constexpr int LOAD_WARPS = 6, MMA_WARP = 6, EPI_WARP0 = 7, EPI_WARPS = 8, THREADS = 15 * 32;
+constexpr int PASS_ROWS = 16, PASSES = TM / PASS_ROWS;  // a loader warp's unit of work
 constexpr int W_BYTES = 512 * 128 * 2;                 // two k-blocks of [512][128 B]
 constexpr int W_KB = 512 * 128;
 constexpr int OFF_A = W_BYTES;                          // 2 stages x 32 KB
@@ -94,7 +100,7 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
 
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&B->a_full[i], LOAD_WARPS); mbar_init(&B->a_empty[i], MODE == MODE_TRIATT ? 1 + EPI_WARPS : 1);
+            mbar_init(&B->a_full[i], PASSES); mbar_init(&B->a_empty[i], MODE == MODE_TRIATT ? 1 + EPI_WARPS : 1);
             mbar_init(&B->acc_full[i], 1); mbar_init(&B->acc_empty[i], EPI_WARPS);
         }
         mbar_init(&B->w_full, 1);
@@ -221,42 +227,42 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         // ---------------------------- LayerNorm loaders ----------------------------
         float4 gam[4], bet[4];
         load_affine(gam, bet);
-        uint32_t it = 1;                    // the epilogue warps normalise the CTA's first tile
-        uint32_t mine = 0;                  // mask of this lane's row of the next tile
-        if (MODE == MODE_TRIMUL) mine = mask_of((int)(blockIdx.x + gridDim.x), warp * 32 + lane);
+        // Passes of 16 rows go round robin over the loader warps: pass u is rows 16 (u % 8) of tile 1 + u / 8 of this CTA
+        // (the epilogue warps normalise its first).
+        auto tile_of = [&](uint32_t u) { return (int)(blockIdx.x + (1 + u / PASSES) * gridDim.x); };
+        uint32_t mine = 0;                  // mask of this lane's row of the next pass
+        if (MODE == MODE_TRIMUL) mine = mask_of(tile_of(warp), (warp % PASSES) * PASS_ROWS + (lane & 15));
         bool ok = true;
-        for (int t = (int)(blockIdx.x + gridDim.x); t < tiles && ok; t += gridDim.x, ++it) {
+        for (uint32_t u = warp; ok; u += LOAD_WARPS) {
+            const int t = tile_of(u);
+            if (t >= tiles) break;
             const int line = t / tpl, pos0 = (t - line * tpl) * TM;
-            const uint32_t stage = it & 1, ph = (it >> 1) & 1;
+            const uint32_t it = 1 + u / PASSES, stage = it & 1, ph = (it >> 1) & 1;
+            const int row0 = (int)(u % PASSES) * PASS_ROWS;
             ok = mbar_wait(&B->a_empty[stage], ph ^ 1, abort_flag);
             if (!ok) break;
             uint8_t* a_tile = smem + OFF_A + stage * A_TILE_BYTES;
             const uint32_t kept = MODE != MODE_TRIMUL ? 0u : __ballot_sync(0xffffffffu, mine != 0);
             if (MODE == MODE_TRIMUL) mine = 0;
-            // this warp's 32 rows of the NEXT tile: one lane per row asks L2 for its four 128-byte lines, so the
-            // loads of the next round find them there instead of paying the DRAM latency with only 4 warps in flight
+            // this warp's NEXT 16 rows: two lanes per row ask L2 for its 128-byte lines, so the loads of the next pass find
+            // them there instead of paying the DRAM latency
             {
-                const int tn = t + (int)gridDim.x, ln = tn / tpl;
+                const int tn = tile_of(u + LOAD_WARPS), ln = tn / tpl;
                 if (tn < tiles) {
-                    const long long f = flat_of(ln, (tn - ln * tpl) * TM + warp * 32 + lane);
+                    const long long f = flat_of(ln, (tn - ln * tpl) * TM + (int)((u + LOAD_WARPS) % PASSES) * PASS_ROWS + (lane & 15));
                     if (f >= 0) {
                         if (MODE == MODE_TRIMUL) mine = p.mask[f];
                         if (MODE != MODE_TRIMUL && p.z_bf16) {
-                            const char* rowp = reinterpret_cast<const char*>(p.z_bf16 + f * KC);
+                            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(p.z_bf16 + f * KC) + (lane >> 4) * 128));
+                        } else {
+                            const char* rowp = reinterpret_cast<const char*>(p.z + f * KC) + (lane >> 4) * 256;
 #pragma unroll
                             for (int j = 0; j < 2; ++j) asm volatile("prefetch.global.L2 [%0];" ::"l"(rowp + j * 128));
-                        } else {
-                            const char* rowp = reinterpret_cast<const char*>(p.z + f * KC);
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) asm volatile("prefetch.global.L2 [%0];" ::"l"(rowp + j * 128));
                         }
                     }
                 }
             }
-#pragma unroll 1
-            for (int pass = 0; pass < 2; ++pass) {
-                normalise16(line, pos0, warp * 32 + pass * 16, [&] { return kept >> (pass * 16); }, a_tile, gam, bet);
-            }
+            normalise16(line, pos0, row0, [&] { return kept; }, a_tile, gam, bet);
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(&B->a_full[stage]);
@@ -324,8 +330,9 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
             normalise16(line, ((int)blockIdx.x - line * tpl) * TM, row0, [&] { return MODE != MODE_TRIMUL ? 0u : __ballot_sync(0xffffffffu, mine != 0); },
                         smem + OFF_A, gam, bet);
             fence_proxy_async();
-            named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
-            if (warp - EPI_WARP0 < LOAD_WARPS && lane == 0) mbar_arrive(&B->a_full[0]);       // the loaders' arrivals of this phase
+            if (MODE == MODE_TRIATT) named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);              // wb_s is there
+            else __syncwarp();
+            if (lane == 0) mbar_arrive(&B->a_full[0]);
         }
         const int lrow = quarter * 32 + lane;                     // TMEM lane of this thread = staging row
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
