@@ -9,10 +9,14 @@
 // The gate GEMM uses LN_in(z) (affine applied by the loader warps) against 0.5 * W_gout, so that
 // p * sigmoid(g) = p' + p' * tanh(g').  The fp32 update leaves through TMA reduce-add straight
 // into z: the kernel never reads z for the residual.
-// Roles (416 threads): warps 0-3 loaders (LN of z rows, TMA issue), warp 4 MMA issuer, warps 5-12 epilogue (x statistics, gate,
-// update; each with a staging tile and reductions of its own, so that no warp waits for another).  A CTA's first tile is
-// normalised by the epilogue warps, 16 rows each, which have nothing else to do before its accumulators exist; the loaders begin
-// with the second.
+// Roles (512 threads): warps 0-5 loaders (LN of z rows, 16 at a time, round robin), warp 6 TMA of the x tiles, warp 7 MMA issuer,
+// warps 8-15 epilogue (x statistics, gate, update; each with a staging tile and reductions of its own, so that no warp waits for
+// another).  A CTA's first tile is normalised by the epilogue warps, 16 rows each, which have nothing else to do before its
+// accumulators exist; the loaders begin with the second.
+// What bounded it was the chain x tile -> statistics -> accumulators -> update of ONE x buffer, whose copy could only start when the tile
+// before had been read twice, and the statistics' 128 two-byte reads and 400 scalar instructions per thread.  With two x buffers,
+// packed statistics of two positions per lane and six loader warps for four: 22.0 -> 14.0 us at 203 tokens, 65.8 -> 47.4 at 400,
+// 288 -> 225 at 1024 (6.0 TB/s of its 10 E bytes, 0.91 of the copy rate).
 #include "rowtc.cuh"
 #include "tmap.cuh"
 
@@ -21,19 +25,19 @@ namespace tme {
 
 using namespace rtc;
 
-constexpr int LOAD_WARPS = 4, MMA_WARP = 4, EPI_WARP0 = 5, EPI_WARPS = 8, THREADS = 13 * 32;
+constexpr int LOAD_WARPS = 6, X_WARP = 6, MMA_WARP = 7, EPI_WARP0 = 8, EPI_WARPS = 8, THREADS = 16 * 32;
+constexpr int PASS_ROWS = 16, PASSES = TM / PASS_ROWS;   // a loader warp's unit of work
 constexpr int W_TILE = 128 * 128 * 2;                    // 32 KB: two k-blocks of [128][128 B]
 constexpr int OFF_WP = 0, OFF_WG = W_TILE;               // 0.5 * W_pout * gamma_out, 0.5 * W_gout
 constexpr int OFF_AZ = 2 * W_TILE;                       // 2 stages
-constexpr int OFF_XT = OFF_AZ + 2 * A_TILE_BYTES;        // 1 stage: 2 boxes of [128 d][64 pos]
+constexpr int OFF_XT = OFF_AZ + 2 * A_TILE_BYTES;        // 2 stages of 2 boxes of [128 d][64 pos]
 constexpr int XT_BOX = 128 * 128;
-constexpr int OFF_STG = OFF_XT + 2 * XT_BOX;             // staging: per epilogue warp [32 pos][32 fp32], 128-byte swizzle
+constexpr int OFF_STG = OFF_XT + 4 * XT_BOX;             // staging: per epilogue warp [32 pos][32 fp32], 128-byte swizzle
 constexpr int STG_BOX = 32 * 128;
 constexpr int OFF_CONST = OFF_STG + EPI_WARPS * STG_BOX; // wsum[128], wb[128] fp32
 constexpr int OFF_BAR = OFF_CONST + 1024;
-constexpr int SMEM_BYTES = OFF_BAR + 128;                // 197,760; the dynamic window must start 1024-byte aligned
+constexpr int SMEM_BYTES = OFF_BAR + 128;                // 230,528; the dynamic window must start 1024-byte aligned
 static_assert(SMEM_BYTES <= 232448, "shared memory budget");
-constexpr int EPI_BAR_ID = 1;
 
 struct Args {
     const float* z;                 // read for LN_in; the residual is added by TMA reduce
@@ -45,7 +49,7 @@ struct Args {
 };
 
 struct Bars {
-    uint64_t w_full, x_full, x_empty, in_full[2], in_empty[2], acc_full[2], acc_empty[2];
+    uint64_t w_full, x_full[2], x_empty[2], in_full[2], in_empty[2], acc_full[2], acc_empty[2];
     uint32_t tmem_slot;
     int abort_flag;
 };
@@ -65,6 +69,24 @@ __device__ __forceinline__ float tanh_approx(float x) {
     float t;
     asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(x));
     return t;
+}
+
+// Two fp32 values in one 64-bit register for the packed instructions (one issue slot, two results).
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -88,10 +110,10 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
 
     if (tid == 0) {
         mbar_init(&B->w_full, 1);
-        mbar_init(&B->x_full, 1);
-        mbar_init(&B->x_empty, 1 + EPI_WARPS);      // the MMAs and the epilogue warps' statistics pass both read the x tile
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&B->in_full[i], LOAD_WARPS); mbar_init(&B->in_empty[i], 1);
+            mbar_init(&B->x_full[i], 1);
+            mbar_init(&B->x_empty[i], 1 + EPI_WARPS);      // the MMAs and the epilogue warps' statistics pass both read the x tile
+            mbar_init(&B->in_full[i], PASSES); mbar_init(&B->in_empty[i], 1);
             mbar_init(&B->acc_full[i], 1); mbar_init(&B->acc_empty[i], EPI_WARPS);
         }
         B->abort_flag = 0;
@@ -172,51 +194,59 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
             bet[j] = reinterpret_cast<const float4*>(p.ln_in_beta)[j * 8 + sub];
         }
     };
-    // x tile of the CTA's tile number `it`; the buffer is free once the MMAs of the tile before are done
-    auto load_x = [&](int r, int pos0, uint32_t it) {
-        if (!mbar_wait(&B->x_empty, (it & 1) ^ 1, abort_flag)) return false;
-        mbar_arrive_expect_tx(&B->x_full, 2 * XT_BOX);
-        tma_load_4d(smem + OFF_XT, &map_x, &B->x_full, pos0, r, 0, 0);
-        tma_load_4d(smem + OFF_XT + XT_BOX, &map_x, &B->x_full, pos0 + 64, r, 0, 0);
-        return true;
-    };
-
     if (warp < LOAD_WARPS) {
         // ---------------------------- loaders ----------------------------
         float4 gam[4], bet[4];
         load_affine(gam, bet);
-        uint32_t it = 1;                    // the epilogue warps normalise the CTA's first tile
+        // Passes of 16 rows go round robin over the loader warps: pass u is rows 16 (u % 8) of tile 1 + u / 8 of this CTA
+        // (the epilogue warps normalise its first).
+        auto tile_of = [&](uint32_t u) { return (int)(blockIdx.x + (1 + u / PASSES) * gridDim.x); };
         bool ok = true;
-        for (long long t = blockIdx.x + gridDim.x; t < tiles && ok; t += gridDim.x, ++it) {
-            const int r = (int)(t / tpl), pos0 = (int)(t % tpl) * TM;
-            const uint32_t stage = it & 1, ph = (it >> 1) & 1;
-            ok = mbar_wait(&B->in_empty[stage], ph ^ 1, abort_flag) && mbar_wait(&B->acc_empty[stage], ph ^ 1, abort_flag);
+        for (uint32_t u = warp; ok; u += LOAD_WARPS) {
+            const int t = tile_of(u);
+            if (t >= tiles) break;
+            const int r = t / tpl, pos0 = (t - r * tpl) * TM, row0 = (int)(u % PASSES) * PASS_ROWS;
+            const uint32_t it = 1 + u / PASSES, stage = it & 1, ph = (it >> 1) & 1;
+            ok = mbar_wait(&B->in_empty[stage], ph ^ 1, abort_flag);
             if (!ok) break;
-            uint8_t* a_tile = smem + OFF_AZ + stage * A_TILE_BYTES;
-            {   // ask L2 for this warp's 32 rows of the NEXT tile (one lane per row, four 128-byte lines)
-                const long long tn = t + gridDim.x;
-                const int rn = (int)(tn / tpl), posn = (int)(tn % tpl) * TM + warp * 32 + lane;
+            {   // ask L2 for this warp's next 16 rows (two lanes per row, two 128-byte lines each)
+                const int tn = tile_of(u + LOAD_WARPS), rn = tn / tpl;
+                const int posn = (tn - rn * tpl) * TM + (int)((u + LOAD_WARPS) % PASSES) * PASS_ROWS + (lane & 15);
                 if (tn < tiles && posn < p.n) {
-                    const char* rowp = reinterpret_cast<const char*>(p.z + ((long long)rn * p.n + posn) * KC);
+                    const char* rowp = reinterpret_cast<const char*>(p.z + ((long long)rn * p.n + posn) * KC) + (lane >> 4) * 256;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) asm volatile("prefetch.global.L2 [%0];" ::"l"(rowp + j * 128));
+                    for (int j = 0; j < 2; ++j) asm volatile("prefetch.global.L2 [%0];" ::"l"(rowp + j * 128));
                 }
             }
-#pragma unroll 1
-            for (int pass = 0; pass < 2; ++pass) {
-                const int row0 = warp * 32 + pass * 16;
-                float4 v[4][4];
-                fetch16(r, pos0, row0, v);
-                if (pass == 0 && warp == 0 && lane == 0) ok = load_x(r, pos0, it);
-                normalise16(row0, v, a_tile, gam, bet);
-            }
-            if (warp == 0) ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;     // lane 0 waited for the x buffer
-            if (!ok) break;
+            float4 v[4][4];
+            fetch16(r, pos0, row0, v);
+            normalise16(row0, v, smem + OFF_AZ + stage * A_TILE_BYTES, gam, bet);
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(&B->in_full[stage]);
         }
         if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
+    } else if (warp == X_WARP) {
+        // ---------------------------- TMA of the x tiles ----------------------------
+        if (lane == 0) {
+            uint32_t it = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++it) {
+                const int r = t / tpl, pos0 = (t - r * tpl) * TM;
+                const uint32_t stage = it & 1;
+                ok = mbar_wait(&B->x_empty[stage], ((it >> 1) & 1) ^ 1, abort_flag);
+                if (!ok) break;
+                uint8_t* xt = smem + OFF_XT + stage * 2 * XT_BOX;
+                mbar_arrive_expect_tx(&B->x_full[stage], 2 * XT_BOX);
+                tma_load_4d(xt, &map_x, &B->x_full[stage], pos0, r, 0, 0);
+                tma_load_4d(xt + XT_BOX, &map_x, &B->x_full[stage], pos0 + 64, r, 0, 0);
+            }
+            if (!ok) {
+                atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
+                uint64_t t0 = global_timer_ns();
+                while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+            }
+        }
     } else if (warp == MMA_WARP) {
         // ---------------------------- MMA issuer ----------------------------
         // The whole warp runs the loop and waits; one elected lane issues (see sm100::elect_one).
@@ -233,23 +263,23 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
         bool ok = mbar_wait_warp(&B->w_full, 0, abort_flag);
         for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
             const uint32_t stage = it & 1, ph = (it >> 1) & 1;
-            ok = mbar_wait_warp(&B->in_full[stage], ph, abort_flag) && mbar_wait_warp(&B->x_full, it & 1, abort_flag) &&
+            ok = mbar_wait_warp(&B->in_full[stage], ph, abort_flag) && mbar_wait_warp(&B->x_full[stage], ph, abort_flag) &&
                  mbar_wait_warp(&B->acc_empty[stage], ph ^ 1, abort_flag);
             if (!ok) break;
             tc_fence_after();
             if (elect_one()) {
-                const uint32_t az_addr = smem_u32(smem + OFF_AZ + stage * A_TILE_BYTES);
+                const uint32_t az_addr = smem_u32(smem + OFF_AZ + stage * A_TILE_BYTES), xs_addr = xt_addr + stage * 2 * XT_BOX;
                 const uint32_t d = tmem_base + stage * 256;
 #pragma unroll
                 for (int ks = 0; ks < 8; ++ks)      // D_p = x^T-tile (MN-major, 16 d rows per step) * W_pout'^T
-                    umma_bf16(d, desc_mn_sw128(xt_addr + ks * 2048), make_desc_k_sw128(wp_addr + (ks >> 2) * (128 * 128) + (ks & 3) * 32),
+                    umma_bf16(d, desc_mn_sw128(xs_addr + ks * 2048), make_desc_k_sw128(wp_addr + (ks >> 2) * (128 * 128) + (ks & 3) * 32),
                               idesc_p, ks ? 1u : 0u);
 #pragma unroll
                 for (int ks = 0; ks < 8; ++ks)      // D_g = LN_in(z) tile * W_gout'^T
                     umma_bf16(d + 128, make_desc_k_sw128(az_addr + (ks >> 2) * A_KB_BYTES + (ks & 3) * 32),
                               make_desc_k_sw128(wg_addr + (ks >> 2) * (128 * 128) + (ks & 3) * 32), idesc_g, ks ? 1u : 0u);
                 umma_commit(&B->in_empty[stage]);
-                umma_commit(&B->x_empty);
+                umma_commit(&B->x_empty[stage]);
                 umma_commit(&B->acc_full[stage]);
             }
             __syncwarp();
@@ -258,50 +288,61 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
     } else {
         // ---------------------------- epilogue ----------------------------
         const int quarter = warp & 3, chalf = (warp - EPI_WARP0) >> 2;
-        const int lrow = quarter * 32 + lane;                     // position inside the tile
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         uint8_t* stg = smem + OFF_STG + (warp - EPI_WARP0) * STG_BOX;
         uint32_t it = 0;
         bool ok = true;
         if (blockIdx.x < tiles) {
-            // the first tile's x and LayerNorm, 16 rows a warp.  At 45 tokens, one tile per CTA, four loader warps in two passes each
+            // the first tile's LayerNorm, 16 rows a warp.  At 45 tokens, one tile per CTA, four loader warps in two passes each
             // took 3.7 of the kernel's 7 us.
-            const int r = (int)blockIdx.x / tpl, pos0 = ((int)blockIdx.x % tpl) * TM, row0 = (warp - EPI_WARP0) * 16;
-            if (warp == EPI_WARP0 && lane == 0) ok = load_x(r, pos0, 0);
+            const int r = (int)blockIdx.x / tpl, pos0 = ((int)blockIdx.x % tpl) * TM, row0 = (warp - EPI_WARP0) * PASS_ROWS;
             float4 v[4][4], gam[4], bet[4];
             fetch16(r, pos0, row0, v);
             load_affine(gam, bet);
             normalise16(row0, v, smem + OFF_AZ, gam, bet);
             fence_proxy_async();
-            named_bar_sync(EPI_BAR_ID, EPI_WARPS * 32);
-            if (warp - EPI_WARP0 < LOAD_WARPS && lane == 0) mbar_arrive(&B->in_full[0]);      // the loaders' arrivals of this phase
-            ok = __all_sync(0xffffffffu, ok) != 0;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&B->in_full[0]);
         }
         for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
             const int r = (int)(t / tpl), pos0 = (int)(t % tpl) * TM;
             const uint32_t stage = it & 1, ph = (it >> 1) & 1;
-            // LayerNorm statistics over the 128 channels of the raw x tile for this thread's position (both warps of a
-            // lane quarter compute them; it is cheaper here than on the four loader warps, which bound the kernel)
-            ok = mbar_wait(&B->x_full, it & 1, abort_flag);
+            // LayerNorm statistics over the 128 channels of the raw x tile for this quarter's 32 positions (both warps of a lane
+            // quarter compute them): a lane reads two positions of every other four channels.
+            ok = mbar_wait(&B->x_full[stage], ph, abort_flag);
             if (!ok) break;
             float2 st;
             {
-                const uint8_t* col = smem + OFF_XT + (lrow >> 6) * XT_BOX + (lrow & 7) * 2;
-                const int pchunk = (lrow & 63) >> 3;
-                float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
-#pragma unroll 8
-                for (int d = 0; d < 128; d += 2) {
-                    const float xa = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(col + d * 128 + ((pchunk ^ (d & 7)) << 4)));
-                    const float xb = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(col + (d + 1) * 128 + ((pchunk ^ ((d + 1) & 7)) << 4)));
-                    s0 += xa; q0 = fmaf(xa, xa, q0);
-                    s1 += xb; q1 = fmaf(xb, xb, q1);
+                const int pp = lane & 15, dg = lane >> 4;         // positions 2 pp and 2 pp + 1, channels 8 i + 4 dg + 0 .. 3
+                const uint8_t* col = smem + OFF_XT + stage * 2 * XT_BOX + (quarter >> 1) * XT_BOX + (pp & 3) * 4 + dg * 512;
+                const int pchunk = (quarter & 1) * 4 + (pp >> 2);
+                uint64_t s2[2] = {0, 0}, q2[2] = {0, 0};
+#pragma unroll 4
+                for (int i = 0; i < 16; ++i)
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        const uint32_t w = *reinterpret_cast<const uint32_t*>(col + i * 1024 + b * 128 + ((pchunk ^ (dg * 4 + b)) << 4));
+                        const uint64_t x2 = f2_pack(bf16_lo(w), bf16_hi(w));
+                        s2[b & 1] = f2_add(s2[b & 1], x2);
+                        q2[b & 1] = f2_fma(x2, x2, q2[b & 1]);
+                    }
+                const uint64_t s = f2_add(s2[0], s2[1]), q = f2_add(q2[0], q2[1]);
+                float sv[2], qv[2], mean[2], rstd[2];
+                f2_unpack(s, sv[0], sv[1]);
+                f2_unpack(q, qv[0], qv[1]);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    sv[e] += __shfl_xor_sync(0xffffffffu, sv[e], 16);
+                    qv[e] += __shfl_xor_sync(0xffffffffu, qv[e], 16);
+                    mean[e] = sv[e] * (1.f / KC);
+                    rstd[e] = rsqrtf(fmaxf(qv[e] * (1.f / KC) - mean[e] * mean[e], 0.f) + LN_EPS);
+                    mean[e] = __shfl_sync(0xffffffffu, mean[e], lane >> 1);
+                    rstd[e] = __shfl_sync(0xffffffffu, rstd[e], lane >> 1);
                 }
-                const float mean = (s0 + s1) * (1.f / KC);
-                const float var = fmaxf((q0 + q1) * (1.f / KC) - mean * mean, 0.f);
-                st = make_float2(mean, rsqrtf(var + LN_EPS));
+                st = (lane & 1) ? make_float2(mean[1], rstd[1]) : make_float2(mean[0], rstd[0]);
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&B->x_empty);
+            if (lane == 0) mbar_arrive(&B->x_empty[stage]);
             ok = mbar_wait(&B->acc_full[stage], ph, abort_flag);
             if (!ok) break;
             tc_fence_after();
