@@ -8,6 +8,7 @@
 // may be moved above the wait.
 #pragma once
 
+#include <atomic>
 #include <utility>
 
 #include "common.cuh"
@@ -45,6 +46,35 @@ static inline int device_multiprocessors(int* out) {
         if (dev >= 0 && dev < 64) known[dev] = sms;
     }
     *out = sms;
+    return B200PF_OK;
+}
+
+// How many CTA pairs of a kernel are resident at once on the current device (not every SM can be half of a pair): the grid of a
+// persistent pair kernel.  Asked for once per kernel and device.
+template <class... KArgs>
+static inline int resident_pairs(void (*kern)(KArgs...), int threads, int smem, int* out) {
+    static std::atomic<int> known[64];            // one table per kernel type: a translation unit has one pair kernel of a signature
+    int dev = 0, sms = 0, rc;
+    B200PF_CUDA(cudaGetDevice(&dev));
+    int n = dev >= 0 && dev < 64 ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        if ((rc = device_multiprocessors(&sms)) != B200PF_OK) return rc;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(sms / 2 * 2));
+        cfg.blockDim = dim3((unsigned)threads);
+        cfg.dynamicSmemBytes = (size_t)smem;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 2;
+        attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        B200PF_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
+        B200PF_REQUIRE(n > 0, B200PF_ERR_CUDA, "no CTA pair fits on this device");
+        if (dev >= 0 && dev < 64) known[dev].store(n, std::memory_order_relaxed);
+    }
+    *out = n;
     return B200PF_OK;
 }
 
