@@ -1,9 +1,9 @@
 // softmax(q k^T + bias + mask) v with a gate, at fp32 accuracy: one-pass softmax over 64-key tiles, both products as three
 // m16n8k16 fp16 MMAs on two-part operands (split.cuh), fp32 accumulation.
 //
-// mma.sync and not tcgen05: q, k, v rows are 24 or 32 wide and the probabilities need parts of their own, so a tcgen05 form
-// would have to push both through tensor memory; here they go from the accumulators of the first product straight into the
-// A fragments of the second.  A warp owns 16 queries; per 64-key tile it issues 96 MMAs.  With three bf16 parts and six MMAs per
+// For single lines (the single track) and rows of 24, which fill neither the line groups nor the swizzled rows of the tcgen05 form
+// (split_attn_tc.cu: three lines and more, rows of 32); the probabilities go from the accumulators of the first product straight into
+// the A fragments of the second.  A warp owns 16 queries; per 64-key tile it issues 96 MMAs.  With three bf16 parts and six MMAs per
 // product, and every lane fetching its own bias values, a launch took 462 us at 292 tokens x 4 heads and 528 at 256 x 8; with two
 // parts 390 and 430, with staged bias tiles 310 and 311, with one barrier a tile, interleaved accumulators, scores that stay in the
 // products' scale, packed fp32 arithmetic (1190 -> 779 instructions per warp and tile) and masks fetched a tile ahead 258 and 245.
@@ -319,6 +319,8 @@ int launch_attention(const AttnArgs& args, int hd, cudaStream_t st) {
                    "split attention: null or misaligned operand");
     B200PF_REQUIRE(a.lines > 0 && a.lines < 65536 && a.heads > 0 && a.n_q > 0 && a.n_k > 0, B200PF_ERR_INVALID, "split attention: bad sizes");
     B200PF_REQUIRE(hd == 24 || hd == 32, B200PF_ERR_UNSUPPORTED, "split attention: head width 24 or 32 (got %d)", hd);
+    // 322 -> 199 us for the whole sub-operation at 292 tokens x 4 heads, 77 -> 53 at 130, 33 -> 27 at 65, 27 -> 22 at 48
+    if (attention_tc_fits(a, hd)) return launch_attention_tc(a, st);
     // eight warps share a K / V tile; with fewer than two such CTAs per SM, four warps per CTA spread the queries further
     int sms, rc;
     if ((rc = device_multiprocessors(&sms)) != B200PF_OK) return rc;      // its CTAs share an SM: a CtaLimit does not mean them

@@ -25,6 +25,8 @@ struct AttnArgs {
     int lines, heads, q0, n_q, n_k;     // queries q0 .. q0 + n_q - 1 of every line
 };
 int launch_attention(const AttnArgs& a, int hd, cudaStream_t st);
+bool attention_tc_fits(const AttnArgs& a, int hd);                  // split_attn_tc.cu
+int launch_attention_tc(const AttnArgs& a, cudaStream_t st);
 
 }  // namespace split
 }  // namespace b200pf

@@ -115,7 +115,7 @@ static TriMulWs trimul_ws(void* ws, int n, int c) {
     w.bytes = a.used;
     return w;
 }
-struct TriAttWs { __half *x, *og, *qkv; float *gate, *bias; long long bytes; };
+struct TriAttWs { __half *x, *og, *qkv; float *gate, *bias; int bpitch; long long bytes; };
 static TriAttWs triatt_ws(void* ws, int n, int c, int heads, int hd) {
     Arena a(ws);
     const long long nn = (long long)n * n;
@@ -125,7 +125,8 @@ static TriAttWs triatt_ws(void* ws, int n, int c, int heads, int hd) {
     w.og = w.x;                                        // x is spent once q, k, v, g exist
     w.qkv = a.take<__half>(2 * nn * 3 * ht);
     w.gate = a.take<float>(nn * ht);
-    w.bias = a.take<float>(nn * heads);
+    w.bpitch = round_up(n, 4);                         // bias rows start on 16-byte boundaries
+    w.bias = a.take<float>((long long)n * w.bpitch * heads);
     w.bytes = a.used;
     return w;
 }
@@ -251,7 +252,7 @@ int b200pf_split_tri_att(float* z, const uint8_t* mask, const b200pf_split_triat
     int rc;
     LnArgs ln = {};
     ln.x = z; ln.gamma = w->ln_gamma; ln.beta = w->ln_beta; ln.planes = k.x; ln.part_stride = nn * c; ln.rows = nn;
-    ln.head_w = w->head_w; ln.head_out = k.bias; ln.head_stride = nn; ln.n = n; ln.transposed = ending;
+    ln.head_w = w->head_w; ln.head_out = k.bias; ln.head_stride = (long long)n * k.bpitch; ln.n = n; ln.transposed = ending; ln.head_pitch = k.bpitch;
     if ((rc = launch_ln(ln, c, heads, st)) != B200PF_OK) return rc;
     {
         Gemm g;
@@ -267,7 +268,7 @@ int b200pf_split_tri_att(float* z, const uint8_t* mask, const b200pf_split_triat
     AttnArgs a = {};
     a.qkv = k.qkv; a.part_stride = nn * 3 * ht; a.ld = 3 * ht;
     a.line_rows = ending ? 1 : n; a.pos_rows = ending ? n : 1;       // a line is a row of z, or a column
-    a.gate = k.gate; a.bias = k.bias; a.bias_hs = nn; a.bias_qs = n;
+    a.gate = k.gate; a.bias = k.bias; a.bias_hs = (long long)n * k.bpitch; a.bias_qs = k.bpitch;
     a.mask = mask; a.mask_ls = ending ? 1 : n; a.mask_ks = ending ? n : 1; a.mask_add = -1e9f * 1.4426950408889634f;
     a.out = k.og; a.out_part_stride = nn * ht; a.out_row0 = 0; a.qk_scale = w->q_scale * w->k_scale;
     a.lines = n; a.heads = heads; a.q0 = 0; a.n_q = n; a.n_k = n;
@@ -299,7 +300,7 @@ int b200pf_ln_heads(const float* x, const float* gamma, const float* beta, const
     B200PF_REQUIRE(heads == 4 || heads == 8 || heads == 16, B200PF_ERR_UNSUPPORTED, "ln_heads: 4, 8 or 16 heads (got %d)", heads);
     if (rows == 0) return B200PF_OK;
     LnArgs ln = {};
-    ln.x = x; ln.gamma = gamma; ln.beta = beta; ln.rows = rows; ln.head_w = w; ln.head_out = out; ln.head_stride = head_stride; ln.n = 1;
+    ln.x = x; ln.gamma = gamma; ln.beta = beta; ln.rows = rows; ln.head_w = w; ln.head_out = out; ln.head_stride = head_stride; ln.n = 1; ln.head_pitch = 1;
     return launch_ln(ln, c, heads, (cudaStream_t)stream);
 }
 

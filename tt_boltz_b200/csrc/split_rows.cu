@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(256) ln_split_kernel(LnArgs p) {
                     const int idx = b0 + i, h = idx / R;
                     const long long row = base + idx % R;
                     if (row < p.rows) {
-                        const long long at = p.transposed ? (row % p.n) * p.n + row / p.n : row;
+                        const long long line = row / p.n, pos = row - line * p.n, at = p.transposed ? pos * p.head_pitch + line : line * p.head_pitch + pos;
                         p.head_out[h * p.head_stride + at] = acc[i];
                     }
                 }

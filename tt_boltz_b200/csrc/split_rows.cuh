@@ -12,11 +12,12 @@ struct LnArgs {
     __half* planes;             // [2][rows][C], or null: heads only
     long long part_stride;
     long long rows;
-    // a few dot products per row with the normalised row: out[h][row], or, for a pair tensor of width n, out[h][j][i] of row (i, j)
+    // a few dot products per row with the normalised row: row (i, j) of a pair tensor of width n at out[h][i][j], or transposed at
+    // out[h][j][i], lines of `head_pitch`
     const float* head_w;        // [heads][C], divided by the planes' scale
     float* head_out;
     long long head_stride;
-    int n, transposed;
+    int n, transposed, head_pitch;
 };
 bool ln_supported(int c);
 int launch_ln(const LnArgs& a, int c, int heads, cudaStream_t st);
