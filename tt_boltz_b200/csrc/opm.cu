@@ -12,7 +12,7 @@
 //   opm_mask_bits_kernel: the MSA mask as one bit per sequence, 32 sequences per word and token.
 //   opm_finalize_kernel : pair counts by popcount of the two tokens' words, then y / count + bias added into (or
 //                         written over) the fp32 pair rows.
-#include "mma.cuh"
+#include "cp_async.cuh"
 #include "pdl.cuh"
 
 namespace b200pf {
