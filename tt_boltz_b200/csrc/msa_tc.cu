@@ -19,7 +19,8 @@ using rtc::TM;
 constexpr int CM = 64;                                    // MSA channels: one 128-byte k-block
 constexpr int X_BYTES = TM * 128;                         // normalised tile: [128 rows][64] bf16
 constexpr int BOX = 128 * 128;                            // [128 rows][128 bytes], 128-byte swizzle
-constexpr int LOAD_WARPS = 4, MMA_WARP = 4, TMA_WARP = 5, EPI_WARP0 = 6, EPI_WARPS = 8, THREADS = 14 * 32;
+constexpr int LOAD_WARPS = 6, MMA_WARP = 6, TMA_WARP = 7, EPI_WARP0 = 8, EPI_WARPS = 8, THREADS = 16 * 32;
+constexpr int PASS_ROWS = 32, PASSES = TM / PASS_ROWS;    // a loader warp's unit of work
 
 // 32 rows of 64 channels -> bf16 rows row0 .. row0 + 31 of the tile; called by one warp.  Eight lanes per row, two float4
 // each; eight rows per lane at once, so that a warp has all of its loads in flight.  Rows >= valid are written as zeros.
@@ -98,17 +99,19 @@ __device__ __forceinline__ bool load_loop(const LnRows& p, uint8_t* x0, uint64_t
         gam[j] = reinterpret_cast<const float4*>(p.gamma)[j * 8 + (lane & 7)];
         bet[j] = reinterpret_cast<const float4*>(p.beta)[j * 8 + (lane & 7)];
     }
-    uint32_t it = 0;
-    for (int t = blockIdx.x; t < p.t.tiles; t += gridDim.x, ++it) {
-        const uint32_t stage = it & 1, ph = (it >> 1) & 1;
+    // Passes go round robin over the loader warps: pass u is rows 32 (u % 4) of this CTA's tile u / 4.
+    for (uint32_t u = warp;; u += LOAD_WARPS) {
+        const uint32_t it = u / PASSES, stage = it & 1, ph = (it >> 1) & 1;
+        const int t = (int)(blockIdx.x + it * gridDim.x), row0 = (int)(u % PASSES) * PASS_ROWS;
+        if (t >= p.t.tiles) break;
         if (!mbar_wait(&x_empty[stage], ph ^ 1, abort_flag)) return false;
-        const int tn = t + (int)gridDim.x;
+        const int tn = (int)(blockIdx.x + (u + LOAD_WARPS) / PASSES * gridDim.x);
         if (tn < p.t.tiles) {
             const int ln = tn / p.t.tpl, pn = (tn - ln * p.t.tpl) * TM;
-            prefetch_rows(p.m + ((long long)ln * p.t.span + pn) * CM, warp * 32 + lane, p.t.span - pn);
+            prefetch_rows(p.m + ((long long)ln * p.t.span + pn) * CM, (int)((u + LOAD_WARPS) % PASSES) * PASS_ROWS + lane, p.t.span - pn);
         }
         const int line = t / p.t.tpl, pos0 = (t - line * p.t.tpl) * TM;
-        ln64_rows32(p.m + ((long long)line * p.t.span + pos0) * CM, warp * 32, p.t.span - pos0, gam, bet, x0 + stage * X_BYTES, lane);
+        ln64_rows32(p.m + ((long long)line * p.t.span + pos0) * CM, row0, p.t.span - pos0, gam, bet, x0 + stage * X_BYTES, lane);
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(&x_full[stage]);
@@ -169,7 +172,7 @@ msa_transition_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_
     if (tid == 0) {
         mbar_init(&B->w_full, 1);
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&B->x_full[i], LOAD_WARPS); mbar_init(&B->x_empty[i], 1);
+            mbar_init(&B->x_full[i], PASSES); mbar_init(&B->x_empty[i], 1);
             mbar_init(&B->d1_full[i], 1); mbar_init(&B->h_full[i], EPI_WARPS);
             mbar_init(&B->d2_full[i], 1); mbar_init(&B->d2_empty[i], EPI_WARPS);
         }
@@ -316,7 +319,7 @@ pwa_value_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     if (tid == 0) {
         mbar_init(&B->w_full, 1);
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&B->x_full[i], LOAD_WARPS); mbar_init(&B->x_empty[i], 1);
+            mbar_init(&B->x_full[i], PASSES); mbar_init(&B->x_empty[i], 1);
             mbar_init(&B->d_full[i], 1); mbar_init(&B->d_empty[i], EPI_WARPS);
         }
         B->abort_flag = 0;
@@ -456,7 +459,7 @@ pwa_output_kernel(const __grid_constant__ CUtensorMap map_wg, const __grid_const
     if (tid == 0) {
         mbar_init(&B->w_full, 1);
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&B->x_full[i], LOAD_WARPS); mbar_init(&B->x_empty[i], 1);
+            mbar_init(&B->x_full[i], PASSES); mbar_init(&B->x_empty[i], 1);
             mbar_init(&B->g_full[i], 1); mbar_init(&B->g_empty[i], EPI_WARPS);
             mbar_init(&B->val_full[i], EPI_WARPS);
             mbar_init(&B->d2_full[i], 1); mbar_init(&B->d2_empty[i], EPI_WARPS);
