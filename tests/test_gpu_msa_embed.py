@@ -1,0 +1,53 @@
+"""The MSA embedding in one kernel against one-hot, concatenation and linear in 64 bits, with and without the paired feature: one row, rows
+that do not fill a block, more than a lane takes at once.  The projected single representation comes from the linear kernel as it does in the
+module; on top of it are four rounded additions, each half an ulp of at most the sum of the terms' sizes: 2^-22 of that.  A residue
+outside the classes counts as none and is reported; features of another shape or type are refused."""
+import pytest
+import torch
+
+from tt_boltz_b200 import B200MSAModule, _lib, ops
+
+pytestmark = pytest.mark.gpu
+
+
+def case(s, n, paired):
+    g = torch.Generator().manual_seed(100 * s + n)
+    mod = B200MSAModule(64, 128, 384, 1, use_paired_feature=paired)
+    with torch.no_grad():
+        for p in (mod.s_proj.weight, mod.msa_proj.weight):
+            p.copy_(torch.randn(p.shape, generator=g) * 0.1)
+    feats = {"msa": torch.randint(0, 33, (1, s, n), generator=g), "has_deletion": (torch.rand(1, s, n, generator=g) < 0.2),
+             "deletion_value": torch.rand(1, s, n, generator=g).double(), "msa_paired": torch.randint(0, 2, (1, s, n), generator=g)}
+    return mod.cuda(), torch.randn(1, n, 384, generator=g).cuda(), {k: v.cuda() for k, v in feats.items()}
+
+
+@pytest.mark.parametrize("paired", [True, False])
+@pytest.mark.parametrize("s, n", [(1, 1), (3, 5), (1, 17), (7, 64), (33, 130), (600, 301)])
+def test_embedding(s, n, paired):
+    mod, emb, feats = case(s, n, paired)
+    raw = [torch.nn.functional.one_hot(feats["msa"][0], 33).double()] + [feats[k][0][..., None].float().double() for k in ("has_deletion", "deletion_value")]
+    raw += [feats["msa_paired"][0][..., None].double()] if paired else []
+    w = mod.msa_proj.weight.detach().double()
+    e = ops.f32_linear(emb[0], mod.s_proj.weight.detach()).double()[None]
+    raw = torch.cat(raw, -1)
+    got = mod.embed(emb, feats)
+    assert _lib.device_status() == 0
+    assert bool(((got.double() - (raw @ w.t() + e)).abs() <= 2.0 ** -22 * (raw.abs() @ w.abs().t() + e.abs())).all())
+
+
+def test_what_is_refused():
+    mod, emb, feats = case(4, 9, True)
+    with torch.no_grad():
+        good = mod.embed(emb, feats)
+        feats["msa"][0, 2, 3] = 33
+        got = mod.embed(emb, feats)
+        assert _lib.device_status() == 2
+        same = torch.ones(4, 9, dtype=torch.bool)
+        same[2, 3] = False
+        assert torch.equal(got[same], good[same])
+        for key, value in (("msa", feats["msa"].int()), ("msa_paired", feats["msa_paired"][:, :3]), ("deletion_value", feats["deletion_value"][:, :, :5])):
+            with pytest.raises(RuntimeError):
+                mod.embed(emb, {**feats, key: value})
+        with pytest.raises(RuntimeError):
+            mod.embed(emb[:, :5], feats)
+    assert _lib.device_status() == 0

@@ -390,8 +390,8 @@ class B200MSAModule(nn.Module):
     tt_bio/tenstorrent.py:2524-2621): the MSA features are embedded (``msa_proj`` of the one-hot residues, deletion and
     pairing features, plus ``s_proj`` of the single representation for every sequence) and ``msa_blocks`` MSA layers
     run on resident tensors; ``forward(z, emb, feats, use_kernels=False)`` returns the pair tensor after the last
-    block, which the trunk adds to z (tt_bio/boltz2.py:5230).  The one-hot and the concatenation of the raw features
-    are torch indexing at the boundary; both projections and everything after run on the b200pf kernels."""
+    block, which the trunk adds to z (tt_bio/boltz2.py:5230).  A residue outside the 33 classes counts as none and raises the
+    device status word (``_lib.device_status``)."""
 
     def __init__(self, msa_s: int = C_M, token_z: int = 128, token_s: int = 384, msa_blocks: int = 4, msa_dropout: float = 0.0,
                  z_dropout: float = 0.0, pairwise_head_width: int = 32, pairwise_num_heads: int = 4,
@@ -408,21 +408,22 @@ class B200MSAModule(nn.Module):
     def embed(self, emb: torch.Tensor, feats) -> torch.Tensor:
         """m [S, N, 64] fp32 from the single representation emb [1, N, token_s] and the MSA features (reference.py:1252-1276)."""
         from . import ops
-        msa = torch.nn.functional.one_hot(feats["msa"][0], num_classes=NUM_TOKENS).to(torch.float32)
-        parts = [msa, feats["has_deletion"][0].unsqueeze(-1).float(), feats["deletion_value"][0].unsqueeze(-1).float()]
-        if self.use_paired_feature:
-            parts.append(feats["msa_paired"][0].unsqueeze(-1).float())
-        raw = torch.cat(parts, dim=-1)                                      # [S, N, 35 or 36]
-        if raw.shape[-1] % 4:                                               # the linear kernel wants 16-byte rows
-            raw = torch.nn.functional.pad(raw, (0, 4 - raw.shape[-1] % 4))
-        w = self.msa_proj.weight.detach().to(device=raw.device, dtype=torch.float32)
-        if w.shape[1] != raw.shape[-1]:
-            w = torch.nn.functional.pad(w, (0, raw.shape[-1] - w.shape[1]))
-        s_len, n = raw.shape[0], raw.shape[1]
-        m = ops.f32_linear(raw.contiguous(), w.contiguous()).view(s_len, n, C_M)
-        e = ops.f32_linear(emb[0].to(torch.float32).contiguous(),
-                           self.s_proj.weight.detach().to(device=raw.device, dtype=torch.float32).contiguous())
-        call("b200pf_msa_add_token_rows", ptr(m), ptr(e), s_len, n, stream())
+        msa = feats["msa"][0]
+        if msa.dtype != torch.int64:
+            raise RuntimeError(f"the MSA's residues must be int64, got {msa.dtype}")
+        names = ("has_deletion", "deletion_value") + (("msa_paired",) if self.use_paired_feature else ())
+        parts = [feats[k][0].float().contiguous() for k in names]
+        if msa.dim() != 2 or any(t.shape != msa.shape for t in parts):
+            raise RuntimeError(f"the MSA's features must have its residues' shape {tuple(msa.shape)}, got {[tuple(t.shape) for t in parts]}")
+        s_len, n = msa.shape
+        f32 = dict(device=msa.device, dtype=torch.float32)
+        e = ops.f32_linear(emb[0].to(torch.float32).contiguous(), self.s_proj.weight.detach().to(**f32).contiguous())
+        if e.shape[0] != n:
+            raise RuntimeError(f"emb has {e.shape[0]} tokens, the MSA {n}")
+        m = torch.empty(s_len, n, C_M, **f32)
+        msa, w = msa.contiguous(), self.msa_proj.weight.detach().to(**f32).contiguous()
+        call("b200pf_msa_embed", ptr(msa), ptr(parts[0]), ptr(parts[1]), ptr(parts[2]) if self.use_paired_feature else None, ptr(w), ptr(e), ptr(m),
+             s_len, n, stream())
         return m
 
     def forward(self, z: torch.Tensor, emb: torch.Tensor, feats, use_kernels: bool = False) -> torch.Tensor:
