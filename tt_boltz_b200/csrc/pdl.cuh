@@ -49,11 +49,33 @@ static inline int device_multiprocessors(int* out) {
     return B200PF_OK;
 }
 
+// The same on CTA pairs (clusters of two), for kernels that don't name their cluster's size themselves.
+template <class... KArgs, class... Args>
+static inline int launch_pdl_pairs(void (*kern)(KArgs...), unsigned pairs, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * pairs);
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    B200PF_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+    count_launch();
+    return B200PF_OK;
+}
+
 // How many CTA pairs of a kernel are resident at once on the current device (not every SM can be half of a pair): the grid of a
 // persistent pair kernel.  Asked for once per kernel and device.
-template <class... KArgs>
-static inline int resident_pairs(void (*kern)(KArgs...), int threads, int smem, int* out) {
-    static std::atomic<int> known[64];            // one table per kernel type: a translation unit has one pair kernel of a signature
+template <auto KERN>
+static inline int resident_pairs(int threads, int smem, int* out) {
+    static std::atomic<int> known[64];
     int dev = 0, sms = 0, rc;
     B200PF_CUDA(cudaGetDevice(&dev));
     int n = dev >= 0 && dev < 64 ? known[dev].load(std::memory_order_relaxed) : 0;
@@ -70,7 +92,7 @@ static inline int resident_pairs(void (*kern)(KArgs...), int threads, int smem, 
         attr.val.clusterDim.z = 1;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        B200PF_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
+        B200PF_CUDA(cudaOccupancyMaxActiveClusters(&n, KERN, &cfg));
         B200PF_REQUIRE(n > 0, B200PF_ERR_CUDA, "no CTA pair fits on this device");
         if (dev >= 0 && dev < 64) known[dev].store(n, std::memory_order_relaxed);
     }

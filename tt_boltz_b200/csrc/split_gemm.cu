@@ -2,8 +2,8 @@
 // part planes (split.cuh) and fp32 accumulation in tensor memory.
 //
 // One k-block of 64 brings every part of both operands into shared memory once and multiplies them three (fp16 parts) or
-// six (bf16 parts) times, so the kernel asks L2 for a half / a third of the bytes per MMA of a plain bf16 GEMM and is bound
-// by the tensor pipe for large K, by its epilogue for K = 64, and by latency for the single track's few hundred rows.
+// six (bf16 parts) times, so the kernel asks L2 for a half / a third of the bytes per MMA of a plain bf16 GEMM.  Those bytes bound it
+// for large K, less so on CTA pairs (launch_one), its epilogue for K = 64, and latency for the single track's few hundred rows.
 // Persistent, warp-specialised: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 epilogue (two warps per TMEM lane quarter,
 // each half of the columns).  Two accumulator sets let the epilogue of a tile run under the next tile's MMAs.  Every result
 // leaves through a swizzled staging slot per warp and a TMA store (or reduce-add), which also clips ragged edges.
@@ -32,13 +32,13 @@ constexpr int n_products(int pl) { return pl == 2 ? 3 : 6; }
 __host__ __device__ constexpr int product_a(int pl, int q) { return pl == 2 ? (q == 0 ? 1 : 0) : (q == 0 ? 2 : q == 1 || q == 3 ? 1 : 0); }
 __host__ __device__ constexpr int product_b(int pl, int q) { return pl == 2 ? (q == 1 ? 1 : 0) : (q == 2 ? 2 : q == 1 || q == 4 ? 1 : 0); }
 
-template <int PL> __host__ __device__ constexpr uint32_t make_idesc(int n) {
-    // fp32 accumulator; fp16 (0) or bf16 (1) operands, both K-major; M = 128
-    return (1u << 4) | (PL == 3 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+template <int PL> __host__ __device__ constexpr uint32_t make_idesc(int m, int n) {
+    // fp32 accumulator; fp16 (0) or bf16 (1) operands, both K-major
+    return (1u << 4) | (PL == 3 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
-constexpr int stage_bytes(int pl, int bn, int na) { return pl * (na * 128 + bn) * 128; }
-constexpr int stages_of(int pl, int bn, int na) {
-    int s = (SMEM_MAX - SMEM_FIXED) / stage_bytes(pl, bn, na);
+constexpr int stage_bytes(int pl, int bn, int na, bool pair) { return pl * (na * 128 + (pair ? bn / 2 : bn)) * 128; }
+constexpr int stages_of(int pl, int bn, int na, bool pair) {
+    int s = (SMEM_MAX - SMEM_FIXED) / stage_bytes(pl, bn, na, pair);
     return s > 4 ? 4 : s;
 }
 
@@ -63,7 +63,9 @@ struct Sigmoid {
     }
 };
 
-template <int PL, int BN, int NA, int NK, int EPI>
+// PAIR: two CTAs of a cluster share the columns of a tile of 256 rows, 128 each: each loads its rows of A and half of B's, the even one issues
+// the MMAs (cta_group::2), each drains its own rows.
+template <int PL, int BN, int NA, int NK, int EPI, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
 split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CUtensorMap map_a1,
                   const __grid_constant__ CUtensorMap map_b0, const __grid_constant__ CUtensorMap map_b1,
@@ -75,40 +77,48 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
     // sums have no ulps to lose.
     constexpr bool SMALL = PL == 3 || EPI == EPI_CONTRACT;
     constexpr int NACC = SMALL ? 2 : NA * NK, ACC_COLS = NACC * BN, TMEM_COLS = 2 * ACC_COLS;
-    constexpr int STAGES = stages_of(PL, BN, NA), A_PART = 128 * 128;
+    constexpr int STAGES = stages_of(PL, BN, NA, PAIR), A_PART = 128 * 128;
     static_assert(STAGES >= 2 && TMEM_COLS <= 512, "tile too large");
-    constexpr int STAGE = stage_bytes(PL, BN, NA);
+    constexpr int STAGE = stage_bytes(PL, BN, NA, PAIR);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* stg_base = smem + STAGES * STAGE;
     uint64_t* bars = reinterpret_cast<uint64_t*>(stg_base + EPI_WARPS * STG_BYTES);
-    uint64_t* full = bars;
+    uint64_t* full = bars;                                 // of a pair the even CTA's: both CTAs' loads
     uint64_t* empty = bars + STAGES;
     uint64_t* acc_full = bars + 2 * STAGES;
-    uint64_t* acc_empty = acc_full + 2;
+    uint64_t* acc_empty = acc_full + 2;                    // of a pair the even CTA's: both CTAs' epilogue warps
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int bn = p.bn;                                   // columns of a tile: a multiple of 32, at most BN
-    const int mt = (p.m_rows + 127) / 128, nt = (p.n_rows + bn - 1) / bn;
+    const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+    const int worker = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, workers = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
+    constexpr int TILE_M = PAIR ? 256 : 128;
+    const int mt = (p.m_rows + TILE_M - 1) / TILE_M, nt = (p.n_rows + bn - 1) / bn;
     const long long tiles = (long long)p.batches * mt * nt;
-    const uint32_t b_part = (uint32_t)bn * 128;
+    const int b_rows = PAIR ? bn / 2 : bn;                 // of a tile's B rows this CTA's
+    const uint32_t b_part = (uint32_t)b_rows * 128;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], EPI_WARPS); }
+        for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], PAIR ? 2 : 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], PAIR ? 2 * EPI_WARPS : EPI_WARPS); }
         *abort_flag = 0;
         fence_barrier_init();
         fence_proxy_async();
     }
-    if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
+    if (warp == 1) {
+        if (PAIR) { tmem_alloc_pair(tmem_slot, TMEM_COLS); tmem_relinquish_pair(); }
+        else { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
+    }
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&map_a0); tma_prefetch_desc(&map_b0); tma_prefetch_desc(&map_o0);
         if (NK == 2) { tma_prefetch_desc(&map_a1); tma_prefetch_desc(&map_b1); }
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync();                              // the other CTA's barriers and tensor memory are ready
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     grid_dependency_wait();
@@ -122,11 +132,12 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
     };
 
     if (warp == 0 && lane == 0) {
+        const uint32_t full0 = PAIR ? map_to_cta(&full[0], 0) : 0u;
         uint32_t stage = 0, phase = 0;
         bool ok = true;
-        for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+        for (long long t = worker; t < tiles && ok; t += workers) {
             const int bt = (int)(t / (mt * nt)), rem = (int)(t % (mt * nt));
-            const int m0 = (rem / nt) * 128, n0 = (rem % nt) * bn;
+            const int m0 = (rem / nt) * TILE_M + (int)rank * 128, n0 = (rem % nt) * bn + (int)rank * b_rows;
             const int ba = p.a_batched ? bt : 0, bb = p.b_batched ? bt : 0;
 #pragma unroll
             for (int ph = 0; ph < NK; ++ph) {
@@ -139,13 +150,18 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
                     if (!ok) break;
                     uint8_t* sa = smem + stage * STAGE;
                     uint8_t* sb = sa + NA * PL * A_PART;
-                    mbar_arrive_expect_tx(&full[stage], (uint32_t)(PL * (NA * A_PART)) + PL * b_part);
+                    const uint32_t bytes = (uint32_t)(PL * (NA * A_PART)) + PL * b_part;
+                    if (!PAIR || rank == 0) mbar_arrive_expect_tx(&full[stage], bytes);
+                    else mbar_arrive_expect_tx_cluster(full0 + stage * 8, bytes);
+                    auto load = [&](uint8_t* dst, const CUtensorMap* map, int c1, int c2, int c3) {
+                        if (PAIR) tma_load_4d_pair(dst, map, full0 + stage * 8, kb * 64, c1, c2, c3);
+                        else tma_load_4d(dst, map, &full[stage], kb * 64, c1, c2, c3);
+                    };
 #pragma unroll
                     for (int pl = 0; pl < PL; ++pl) {
 #pragma unroll
-                        for (int na = 0; na < NA; ++na)
-                            tma_load_4d(sa + (na * PL + pl) * A_PART, ma, &full[stage], kb * 64, m0 + na * p.a_second_row, ba, pl);
-                        tma_load_4d(sb + pl * b_part, mb, &full[stage], kb * 64, n0, bb, pl);
+                        for (int na = 0; na < NA; ++na) load(sa + (na * PL + pl) * A_PART, ma, m0 + na * p.a_second_row, ba, pl);
+                        load(sb + pl * b_part, mb, n0, bb, pl);
                     }
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
@@ -156,12 +172,16 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
             uint64_t t0 = global_timer_ns();
             while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
         }
-    } else if (warp == 1) {
-        const uint32_t idesc = make_idesc<PL>(bn);
+    } else if (warp == 1 && rank == 0) {
+        const uint32_t idesc = make_idesc<PL>(TILE_M, bn);
+        auto commit = [&](uint64_t* bar) {
+            if (PAIR) { umma_commit_pair(smem_u32(bar)); umma_commit_pair(map_to_cta(bar, 1)); }
+            else umma_commit(bar);
+        };
         const uint64_t d0 = make_desc_k_sw128(smem_u32(smem));
         uint32_t stage = 0, phase = 0, it = 0;
         bool ok = true;
-        for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
+        for (long long t = worker; t < tiles && ok; t += workers, ++it) {
             const int bt = (int)(t / (mt * nt));
             const uint32_t ab = it & 1;
             ok = mbar_wait_warp(&acc_empty[ab], ((it >> 1) & 1) ^ 1, abort_flag);
@@ -187,11 +207,15 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
                                 const uint64_t xa = da + (na * PL + product_a(PL, q)) * (A_PART >> 4), xb = db + product_b(PL, q) * (b_part >> 4);
 #pragma unroll
                                 for (int kk = 0; kk < 4; ++kk)
-                                    if (kk < ksteps) umma_bf16(d, xa + kk * 2, xb + kk * 2, idesc, (kb > kb0 || kk > 0 || (q > 0 && !(SMALL && lead))) ? 1u : 0u);
+                                    if (kk < ksteps) {
+                                        const uint32_t add = (kb > kb0 || kk > 0 || (q > 0 && !(SMALL && lead))) ? 1u : 0u;
+                                        if (PAIR) umma_bf16_pair(d, xa + kk * 2, xb + kk * 2, idesc, add);
+                                        else umma_bf16(d, xa + kk * 2, xb + kk * 2, idesc, add);
+                                    }
                             }
                         }
-                        umma_commit(&empty[stage]);
-                        if (ph == NK - 1 && kb + 1 == kb1) umma_commit(&acc_full[ab]);
+                        commit(&empty[stage]);
+                        if (ph == NK - 1 && kb + 1 == kb1) commit(&acc_full[ab]);
                     }
                     __syncwarp();
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -240,9 +264,9 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
         };
         const Sigmoid sig(EPI == EPI_GATE_ADD ? p.alpha[1] : EPI == EPI_QKVG ? 1.f : p.alpha[0]);
         const float ao = p.alpha[0] * p.out_scale;                          // powers of two
-        for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
+        for (long long t = worker; t < tiles && ok; t += workers, ++it) {
             const int bt = (int)(t / (mt * nt)), rem = (int)(t % (mt * nt));
-            const int m0 = (rem / nt) * 128 + quarter * 32, n0 = (rem % nt) * bn;
+            const int m0 = (rem / nt) * TILE_M + (int)rank * 128 + quarter * 32, n0 = (rem % nt) * bn;
             const uint32_t ab = it & 1;
             uint32_t bits = 0;                                              // mask of the warp's next 32 columns, asked for ahead of the wait
             auto mask_bits = [&](int col) {
@@ -320,14 +344,22 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[ab]);
+            if (lane == 0) {
+                if (PAIR) mbar_arrive_remote(map_to_cta(&acc_empty[ab], 0));
+                else mbar_arrive(&acc_empty[ab]);
+            }
         }
         if (lane == 0) bulk_wait0();
         if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
+    if (PAIR) cluster_sync();                              // nobody signals or reads the other CTA after this
+    if (warp == 1) {
+        tc_fence_after();
+        if (PAIR) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+        else tmem_dealloc(tmem_base, TMEM_COLS);
+    }
 }
 
 static int operand_map(CUtensorMap* m, const Operand& o, int parts, int box_rows, const char* what) {
@@ -353,22 +385,22 @@ static int output_map(CUtensorMap* m, const Output& o) {
     return tmap_encode(m, dt, o.ptr, 4, dims, str, box, o.parts == 1 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, "split output");
 }
 
-template <int PL, int BN, int NA, int NK, int EPI>
-static int launch_one(const Gemm& g, int bn, int sms, cudaStream_t st) {
+template <int PL, int BN, int NA, int NK, int EPI, bool PAIR>
+static int launch_tiles(const Gemm& g, int bn, int sms, cudaStream_t st) {
     unsigned int* status = device_status_word();
     B200PF_REQUIRE(status, B200PF_ERR_CUDA, "split_gemm: no device status word");
     CUtensorMap a[2], b[2], o[2];
     int rc;
     for (int i = 0; i < NK; ++i) {
         if ((rc = operand_map(&a[i], g.a[i], PL, 128, "A")) != B200PF_OK) return rc;
-        if ((rc = operand_map(&b[i], g.b[i], PL, bn, "B")) != B200PF_OK) return rc;
+        if ((rc = operand_map(&b[i], g.b[i], PL, PAIR ? bn / 2 : bn, "B")) != B200PF_OK) return rc;
     }
     if (NK == 1) { a[1] = a[0]; b[1] = b[0]; }
     if ((rc = output_map(&o[0], g.out[0])) != B200PF_OK) return rc;
     if (EPI == EPI_QKVG) { if ((rc = output_map(&o[1], g.out[1])) != B200PF_OK) return rc; }
     else o[1] = o[0];
-    constexpr int smem = stages_of(PL, BN, NA) * stage_bytes(PL, BN, NA) + SMEM_FIXED;
-    auto kern = split_gemm_kernel<PL, BN, NA, NK, EPI>;
+    constexpr int smem = stages_of(PL, BN, NA, PAIR) * stage_bytes(PL, BN, NA, PAIR) + SMEM_FIXED;
+    constexpr auto kern = split_gemm_kernel<PL, BN, NA, NK, EPI, PAIR>;
     B200PF_SMEM_ATTR_ONCE(kern, smem);
     Dev d;
     d.m_rows = g.m_rows; d.n_rows = g.n_rows; d.bn = bn;
@@ -380,8 +412,31 @@ static int launch_one(const Gemm& g, int bn, int sms, cudaStream_t st) {
     d.bias = g.bias; d.mask = g.mask; d.mask_bs = g.mask_bs; d.mask_cs = g.mask_cs;
     for (int i = 0; i < 3; ++i) d.qkv_scale[i] = g.qkv_scale[i];
     d.n_split = g.n_split;
-    const long long tiles = (long long)d.batches * ((g.m_rows + 127) / 128) * ((g.n_rows + bn - 1) / bn);
+    constexpr int TILE_M = PAIR ? 256 : 128;
+    const long long tiles = (long long)d.batches * ((g.m_rows + TILE_M - 1) / TILE_M) * ((g.n_rows + bn - 1) / bn);
+    if (PAIR) {
+        int pairs;
+        if ((rc = resident_pairs<kern>(THREADS, smem, &pairs)) != B200PF_OK) return rc;
+        if (pairs > sms / 2) pairs = sms / 2;
+        return launch_pdl_pairs(kern, (unsigned)(tiles < pairs ? tiles : pairs), dim3(THREADS), smem, st, a[0], a[1], b[0], b[1], o[0], o[1], d, status);
+    }
     return launch_pdl(kern, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(THREADS), smem, st, a[0], a[1], b[0], b[1], o[0], o[1], d, status);
+}
+
+// CTA pairs where there is a tile for every CTA, more than one k-block (which would gain nothing) and pairing leaves few rows empty (an odd
+// number of 128-row tiles wastes one): a k-block
+// then brings 64 KB for 96 (256 columns), 48 for 64 (128) or 80 for 96 (two A tiles) into each SM per 256 x `bn` outputs, and some 9 TB/s out of
+// L2 are what bounds these GEMMs otherwise.  At 331 tokens x 256 channels: transition 274 -> 220 us (tensor pipe 92 %) and 153 -> 140, output
+// gate 94 -> 86, operand planes 176 -> 175 (their epilogue, 35 us, and L2); contraction at 256 tokens 49 -> 43; odd ones (331) stay.  Two 256-wide blocks
+// run 1.04 (110 tokens) to 1.10 times (200) as fast, four attention-free ones 1.03 to 1.14, 64 channels 1.00 to 1.01.  K-blocks of 32, with more stages, are
+// slower (220 -> 250, 98 -> 109); for the planes, stores of 64 columns change nothing.  Three parts have more products per byte.
+template <int PL, int BN, int NA, int NK, int EPI>
+static int launch_one(const Gemm& g, int bn, int sms, cudaStream_t st) {
+    if constexpr (PL == 2) {
+        const long long mt = (g.m_rows + 127) / 128, tiles = (long long)(g.k_splits > 1 ? g.k_splits : g.batches) * mt * ((g.n_rows + bn - 1) / bn);
+        if (g.k[0] > 64 && tiles >= sms && (mt % 2 == 0 || mt >= 9)) return launch_tiles<PL, BN, NA, NK, EPI, true>(g, bn, sms, st);
+    }
+    return launch_tiles<PL, BN, NA, NK, EPI, false>(g, bn, sms, st);
 }
 
 // Tile width for `n` columns: the widest tile (at most `most`, a multiple of `step`) whose waves of CTAs, times the bytes a tile

@@ -584,7 +584,7 @@ extern "C" int b200pf_transition_z_tc(float* z, const float* ln_gamma, const flo
     if (one_each)
         return launch_pdl(transition_one_kernel, dim3((unsigned)tiles), dim3(one::THREADS), one::SMEM_BYTES, (cudaStream_t)stream, m12, m3, mz, a, status);
     int pairs;
-    if ((rc = resident_pairs(transition_pair_kernel, pair::THREADS, pair::SMEM_BYTES, &pairs)) != B200PF_OK) return rc;
+    if ((rc = resident_pairs<transition_pair_kernel>(pair::THREADS, pair::SMEM_BYTES, &pairs)) != B200PF_OK) return rc;
     if (pairs > sms / 2) pairs = sms > 1 ? sms / 2 : 1;
     const long long couples = (tiles + 1) / 2;
     return launch_pdl(transition_pair_kernel, dim3(2u * (unsigned)(couples < pairs ? couples : pairs)), dim3(pair::THREADS), pair::SMEM_BYTES, (cudaStream_t)stream,
