@@ -44,11 +44,12 @@ __device__ __forceinline__ long long x_row_offset(const GemmShape& s, int d, int
     return (long long)grp * s.x_group_stride + (long long)d * s.x_plane_stride + (long long)(row - grp * s.x_row_group) * s.x_pitch;
 }
 
-// One epilogue warp's 32 rows (from `row0`) x 256 columns of a finished accumulator.  Plain planes leave through a swizzled staging tile and
-// TMA stores of [32 rows][64 columns].  As 16-byte stores of a thread per row, 4096 partial sectors a tile, they took 11 k clocks a tile
+// One epilogue warp's 32 rows (from `row0`) x COLS columns of a finished accumulator.  Plain planes leave through SLOTS swizzled staging tiles in
+// turn and TMA stores of [32 rows][64 columns].  As 16-byte stores of a thread per row, 4096 partial sectors a tile, they took 11 k clocks a tile
 // against 3.6 k to 8.2 k of MMAs: 11.7 -> 9.7 us at 203 tokens, 43 -> 35 at 400, 112 -> 94 at 600, 238 -> 224 at 1024 (what is left is
 // the operands, some 9 TB/s out of L2).  Columns in groups (the outer product's blocks of contiguous 2 KB) and row groups that 32 does
 // not divide stay with the direct stores.
+template <int COLS, int SLOTS>
 __device__ __forceinline__ void store_tile(const CUtensorMap* map_x, __nv_bfloat16* x, const GemmShape& s, uint32_t taddr, uint8_t* stg, uint32_t& slot, int d, int row0,
                                            int n0, int lane) {
     using namespace sm100;
@@ -56,17 +57,17 @@ __device__ __forceinline__ void store_tile(const CUtensorMap* map_x, __nv_bfloat
     if (s.x_tma) {
         const int grp = row0 / s.x_row_group, row_in = row0 - grp * s.x_row_group;
 #pragma unroll 1
-        for (int c = 0; c < BN / 64; ++c) {
+        for (int c = 0; c < COLS / 64; ++c) {
             const int col = n0 + c * 64;
             if (col >= s.x_cols || row0 >= s.m_rows) break;          // warp-uniform
             uint32_t r[2][32];
             tmem_ld_32x32(taddr + c * 64, r[0]);
             tmem_ld_32x32(taddr + c * 64 + 32, r[1]);
             tmem_ld_wait();
-            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");      // the store before last has read this tile
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(SLOTS - 1) : "memory");      // the store that filled this tile has read it
             __syncwarp();
             uint8_t* tile = stg + slot * STG_BYTES;
-            slot ^= 1;
+            slot ^= SLOTS - 1;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 uint32_t w[4];
@@ -88,7 +89,7 @@ __device__ __forceinline__ void store_tile(const CUtensorMap* map_x, __nv_bfloat
     }
     __nv_bfloat16* xrow = x + x_row_offset(s, d, row < s.m_rows ? row : 0);
 #pragma unroll 1
-    for (int c = 0; c < BN / 32; ++c) {
+    for (int c = 0; c < COLS / 32; ++c) {
         const int col = n0 + c * 32;
         if (col >= s.x_cols) break;                                  // warp-uniform
         __nv_bfloat16* xdst = s.x_col_group > 0 ? xrow + (long long)(col / s.x_col_group) * s.x_colgroup_stride + (col % s.x_col_group) : xrow + col;
@@ -223,7 +224,7 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             ok = mbar_wait(&acc_full[ab], aphase, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            store_tile(&map_x, x, s, tmem_base + ((uint32_t)(quarter * 32) << 16) + ab * BN, stg + quarter * 2 * STG_BYTES, slot, d, m0 + quarter * 32, n0, lane);
+            store_tile<BN, 2>(&map_x, x, s, tmem_base + ((uint32_t)(quarter * 32) << 16) + ab * BN, stg + quarter * 2 * STG_BYTES, slot, d, m0 + quarter * 32, n0, lane);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[ab]);
@@ -240,20 +241,24 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 // Two CTAs of a cluster (the two SMs of a TPC) share one 256 x 256 output tile: each stages its 128 rows of A and
 // its 128 rows of B (32 KB per k-block instead of the 48 KB a lone CTA needs for 128 x 256: the lone kernel is bound
 // by the 96 bytes per clock it has to pull from L2), the even CTA issues tcgen05.mma.cta_group::2 over both halves,
-// and each CTA drains its own 128 accumulator rows.  Loads land in the loading CTA's own shared memory (never a
+// and each CTA drains its own 128 accumulator rows, with eight epilogue warps: four were as long as the MMAs of a tile or longer up to some
+// 512 tokens (25.8 -> 21.4 us at 300, 35.2 -> 30.1 at 400, 41.6 -> 37.9 at 512, 9.5 -> 8.8 at 203; 92.1 -> 90.6 at 600 and the same at 1024,
+// where the operands bound it).  A staging tile a warp leaves six stages; two with five stages 248 -> 262 at 1024.  The one-CTA kernel, for
+// at most 128 rows, keeps four warps with two tiles each (eight with one: 5.4 -> 5.7 at 117).  Loads land in the loading CTA's own shared memory (never a
 // multicast); their bytes are counted on the even CTA's barrier.  Every role of both CTAs always reaches the two
 // cluster barriers, also after a wait ran out.
 constexpr int P_STAGES = 6, P_STAGE_BYTES = 2 * (128 * BK * 2);
-constexpr int PAIR_SMEM = P_STAGES * P_STAGE_BYTES + STG_TOTAL + 1024 + 256;
+constexpr int P_EPI_WARPS = 8, P_SLOTS = 1, P_STG_TOTAL = P_EPI_WARPS * P_SLOTS * STG_BYTES, PAIR_THREADS = (2 + P_EPI_WARPS) * 32;
+constexpr int PAIR_SMEM = P_STAGES * P_STAGE_BYTES + P_STG_TOTAL + 1024 + 256;
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 trimul_contract_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_x,
                             __nv_bfloat16* __restrict__ x, GemmShape s, unsigned int* status) {
     using namespace sm100;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* stg = smem + P_STAGES * P_STAGE_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(stg + STG_TOTAL);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(stg + P_STG_TOTAL);
     uint64_t* full = bars;                      // [P_STAGES]  used in the even CTA: both CTAs' loads
     uint64_t* empty = bars + P_STAGES;          // [P_STAGES]  one per CTA
     uint64_t* acc_full = bars + 2 * P_STAGES;   // [2]         one per CTA
@@ -270,7 +275,7 @@ trimul_contract_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __g
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < P_STAGES; ++i) { mbar_init(&full[i], 2); mbar_init(&empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 2 * P_EPI_WARPS); }
         *abort_flag = 0;
         fence_barrier_init();
         fence_proxy_async();
@@ -353,7 +358,7 @@ trimul_contract_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __g
         if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
     } else if (warp >= 2) {
         // ---------------- epilogue: this CTA's 128 rows of the tile ----------------
-        const int quarter = warp & 3;
+        const int quarter = warp & 3, half = (warp - 2) >> 2;       // 128 columns each
         uint32_t slot = 0;                            // staging tile of the next store
         bool ok = true;
         long long it = 0;
@@ -365,10 +370,11 @@ trimul_contract_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __g
             ok = mbar_wait(&acc_full[ab], aphase, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            store_tile(&map_x, x, s, tmem_base + ((uint32_t)(quarter * 32) << 16) + ab * BN, stg + quarter * 2 * STG_BYTES, slot, d, m0 + quarter * 32, n0, lane);
+            store_tile<BN / 2, P_SLOTS>(&map_x, x, s, tmem_base + ((uint32_t)(quarter * 32) << 16) + ab * BN + half * (BN / 2), stg + (warp - 2) * P_SLOTS * STG_BYTES, slot, d,
+                                        m0 + quarter * 32, n0 + half * (BN / 2), lane);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(&acc_empty[ab], 0));
+            if (lane == 0) mbar_arrive_remote(map_to_cta(&acc_empty[ab], 0));
         }
         if (lane == 0) bulk_wait0();
         if (!ok && lane == 0) atomicOr(status, DEV_STATUS_MBAR_TIMEOUT);
@@ -459,7 +465,7 @@ static int launch_contract_tc(const b200pf_planes* a, const b200pf_planes* b, b2
         if (dev >= 0 && dev < 64 && resident_pairs[dev] == 0) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)(sms / 2 * 2));
-            cfg.blockDim = dim3(GEMM_THREADS);
+            cfg.blockDim = dim3(PAIR_THREADS);
             cfg.dynamicSmemBytes = PAIR_SMEM;
             cudaLaunchAttribute attr;
             attr.id = cudaLaunchAttributeClusterDimension;
@@ -475,7 +481,7 @@ static int launch_contract_tc(const b200pf_planes* a, const b200pf_planes* b, b2
         }
         long long pairs = (dev >= 0 && dev < 64) ? resident_pairs[dev] : sms / 2;
         unsigned grid = 2u * (unsigned)(tiles < pairs ? tiles : pairs);
-        return launch_pdl(trimul_contract_pair_kernel, dim3(grid), dim3(GEMM_THREADS), PAIR_SMEM, st, map_a, map_b, map_x, (__nv_bfloat16*)x, s, status);
+        return launch_pdl(trimul_contract_pair_kernel, dim3(grid), dim3(PAIR_THREADS), PAIR_SMEM, st, map_a, map_b, map_x, (__nv_bfloat16*)x, s, status);
     }
     long long tiles = (long long)s.channels * ((s.m_rows + BM - 1) / BM) * ((s.n_rows + BN - 1) / BN);
     unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
