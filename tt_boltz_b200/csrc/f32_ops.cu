@@ -419,6 +419,10 @@ ln_proj_heads_kernel(const float* __restrict__ z, const float* __restrict__ gamm
 // 16 j + 4 t .. + 3 (j = 0 .. 7) of rows g and g + 8, so the four lanes of a row read 64 contiguous bytes
 // per load instruction.  K step ks uses the lane's values 2 ks and 2 ks + 1, i.e. channels
 // 16 (ks / 2) + 4 t + 2 (ks % 2) (+1): the k <-> channel map the weights are laid out with in shared memory.
+// Reading z bounds it from some 500 tokens on: 98 us at 1024 for its 604 MB, 6.2 TB/s.  What it took to get there from 114 us
+// (400 tokens 23.1 -> 18.8, 203: 9.4 -> 8.1): the registers of a step's channels take the next rows' as the products free them, the
+// first rows are on their way while the weights are laid out, the statistics are packed, and the row's 1 / sigma goes onto its 16
+// results instead of its 128 channels.
 // Round to tf32 (nearest, ties away from zero: what cvt.rna.tf32.f32 returns for every finite value that does not
 // overflow) with two integer instructions on the bit pattern.  The cvt instruction itself runs at a few lanes per
 // clock: with two of them per operand element the 3xTF32 kernels below were bound by the conversions, at a
@@ -429,20 +433,46 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], uint32_t a0, uint32_t a1
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+    return reinterpret_cast<float2&>(r);
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
+    return reinterpret_cast<float2&>(r);
+}
+
+__global__ void __launch_bounds__(256, 2)
 ln_proj_heads16_mma_kernel(const float* z, const float* gamma, const float* beta, const float* w, float* out, long long out_hs, long long rows) {
     constexpr int C = 128, HEADS = 16;
-    __shared__ uint2 w_hi[16][2][32], w_lo[16][2][32];       // [k step][n tile][lane] -> (b0, b1)
+    __shared__ uint4 w_parts[16][2][32];       // [k step][n tile][lane] -> (b0, b1) of the high parts, (b0, b1) of the low parts
     __shared__ float cs[HEADS];
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const long long step = (long long)gridDim.x * (blockDim.x >> 5) * 16;
+    long long base = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 16;
+    float2 x[2][16];
+    auto fetch = [&](long long from, int q) {      // channels 16 q + 4 t .. + 3 of the lane's two rows
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const long long row = from + g + 8 * r;
+            const float4 v = row < rows ? reinterpret_cast<const float4*>(z + row * C)[4 * q + t] : make_float4(0.f, 0.f, 0.f, 0.f);
+            x[r][2 * q] = make_float2(v.x, v.y);
+            x[r][2 * q + 1] = make_float2(v.z, v.w);
+        }
+    };
     grid_dependency_wait();
     grid_launch_dependents();
-    for (int i = threadIdx.x; i < 16 * 2 * 32; i += blockDim.x) {
-        const int ln = i & 31, nt = (i >> 5) & 1, ks = i >> 6;
-        const int g = ln >> 2, t = ln & 3, h = nt * 8 + g, c0 = 16 * (ks >> 1) + 4 * t + 2 * (ks & 1);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) fetch(base, q);    // in flight while the weights are laid out
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+        const int i = it * 256 + threadIdx.x, ln = i & 31, nt = (i >> 5) & 1, ks = i >> 6;
+        const int wg = ln >> 2, wt = ln & 3, h = nt * 8 + wg, c0 = 16 * (ks >> 1) + 4 * wt + 2 * (ks & 1);
         const float v0 = w[h * C + c0] * gamma[c0], v1 = w[h * C + c0 + 1] * gamma[c0 + 1];
         const uint32_t h0 = to_tf32(v0), h1 = to_tf32(v1);
-        w_hi[ks][nt][ln] = make_uint2(h0, h1);
-        w_lo[ks][nt][ln] = make_uint2(to_tf32(v0 - __uint_as_float(h0)), to_tf32(v1 - __uint_as_float(h1)));
+        w_parts[ks][nt][ln] = make_uint4(h0, h1, to_tf32(v0 - __uint_as_float(h0)), to_tf32(v1 - __uint_as_float(h1)));
     }
     {   // LayerNorm offset carried through the weights, cs[h] = sum_c w[h][c] beta[c]: 16 threads per head (one
         // thread per head walked 128 dependent steps while the rest of the CTA waited at the barrier)
@@ -455,28 +485,15 @@ ln_proj_heads16_mma_kernel(const float* z, const float* gamma, const float* beta
         if (sub == 0) cs[h] = sacc;
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long base = warp * 16; base < rows; base += nwarps * 16) {
-        float x[2][32];
+    for (; base < rows; base += step) {
+        float sm[2], rstd[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const long long row = base + g + 8 * r;
-            const float4* src = reinterpret_cast<const float4*>(z + (row < rows ? row : 0) * C) + t;
+            float2 a = x[r][0], b = x[r][1];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const float4 v = row < rows ? src[4 * q] : make_float4(0.f, 0.f, 0.f, 0.f);
-                x[r][4 * q] = v.x; x[r][4 * q + 1] = v.y; x[r][4 * q + 2] = v.z; x[r][4 * q + 3] = v.w;
-            }
-        }
-        float sm[2], ss[2];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            float a = 0.f;
-#pragma unroll
-            for (int e = 0; e < 32; ++e) a += x[r][e];
-            sm[r] = a;
+            for (int e = 2; e < 16; e += 2) { a = add2(a, x[r][e]); b = add2(b, x[r][e + 1]); }
+            a = add2(a, b);
+            sm[r] = a.x + a.y;
         }
 #pragma unroll
         for (int st = 1; st < 4; st <<= 1)
@@ -485,29 +502,41 @@ ln_proj_heads16_mma_kernel(const float* z, const float* gamma, const float* beta
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const float mean = sm[r] * (1.f / C);
-            float a = 0.f;
+            const float2 neg = make_float2(-mean, -mean);
+            float2 a = make_float2(0.f, 0.f), b = a;
 #pragma unroll
-            for (int e = 0; e < 32; ++e) { x[r][e] -= mean; a = fmaf(x[r][e], x[r][e], a); }
-            ss[r] = a;
+            for (int e = 0; e < 16; e += 2) {
+                x[r][e] = add2(x[r][e], neg);
+                x[r][e + 1] = add2(x[r][e + 1], neg);
+                a = fma2(x[r][e], x[r][e], a);
+                b = fma2(x[r][e + 1], x[r][e + 1], b);
+            }
+            a = add2(a, b);
+            sm[r] = a.x + a.y;
         }
 #pragma unroll
         for (int st = 1; st < 4; st <<= 1)
 #pragma unroll
-            for (int r = 0; r < 2; ++r) ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], st);
-        const float rstd0 = rsqrtf(ss[0] * (1.f / C) + LN_EPS), rstd1 = rsqrtf(ss[1] * (1.f / C) + LN_EPS);
+            for (int r = 0; r < 2; ++r) sm[r] += __shfl_xor_sync(0xffffffffu, sm[r], st);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) rstd[r] = rsqrtf(sm[r] * (1.f / C) + LN_EPS);
         float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        const long long next = base + step;
 #pragma unroll
         for (int ks = 0; ks < 16; ++ks) {
-            const float v0 = x[0][2 * ks] * rstd0, v1 = x[1][2 * ks] * rstd1, v2 = x[0][2 * ks + 1] * rstd0, v3 = x[1][2 * ks + 1] * rstd1;
-            const uint32_t a0 = to_tf32(v0), a1 = to_tf32(v1), a2 = to_tf32(v2), a3 = to_tf32(v3);
-            const uint32_t l0 = to_tf32(v0 - __uint_as_float(a0)), l1 = to_tf32(v1 - __uint_as_float(a1));
-            const uint32_t l2 = to_tf32(v2 - __uint_as_float(a2)), l3 = to_tf32(v3 - __uint_as_float(a3));
+            const uint32_t a0 = to_tf32(x[0][ks].x), a1 = to_tf32(x[1][ks].x), a2 = to_tf32(x[0][ks].y), a3 = to_tf32(x[1][ks].y);
+            const float2 r0 = add2(x[0][ks], make_float2(-__uint_as_float(a0), -__uint_as_float(a2)));
+            const float2 r1 = add2(x[1][ks], make_float2(-__uint_as_float(a1), -__uint_as_float(a3)));
+            // the instruction drops the bits below tf32's by itself: half a unit of its last place is all that rounding takes
+            const uint32_t l0 = __float_as_uint(r0.x) + 0x1000u, l1 = __float_as_uint(r1.x) + 0x1000u;
+            const uint32_t l2 = __float_as_uint(r0.y) + 0x1000u, l3 = __float_as_uint(r1.y) + 0x1000u;
+            if (ks & 1) fetch(next, ks >> 1);          // the next rows, into the registers that are free by now
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-                const uint2 bh = w_hi[ks][nt][lane], bl = w_lo[ks][nt][lane];
-                mma_tf32(acc[nt], l0, l1, l2, l3, bh.x, bh.y);
-                mma_tf32(acc[nt], a0, a1, a2, a3, bl.x, bl.y);
-                mma_tf32(acc[nt], a0, a1, a2, a3, bh.x, bh.y);
+                const uint4 b = w_parts[ks][nt][lane];
+                mma_tf32(acc[nt], l0, l1, l2, l3, b.x, b.y);
+                mma_tf32(acc[nt], a0, a1, a2, a3, b.z, b.w);
+                mma_tf32(acc[nt], a0, a1, a2, a3, b.x, b.y);
             }
         }
         // c0: (row g, head 2t), c1: (row g, head 2t + 1), c2 / c3: the same for row g + 8
@@ -517,7 +546,7 @@ ln_proj_heads16_mma_kernel(const float* z, const float* gamma, const float* beta
             for (int e = 0; e < 4; ++e) {
                 const long long row = base + g + 8 * (e >> 1);
                 const int h = nt * 8 + 2 * t + (e & 1);
-                if (row < rows) out[h * out_hs + row] = acc[nt][e] + cs[h];
+                if (row < rows) out[h * out_hs + row] = fmaf(acc[nt][e], rstd[e >> 1], cs[h]);
             }
     }
 }
