@@ -70,14 +70,24 @@ __device__ __forceinline__ float prob(float x) {
     return y;
 }
 
-template <int HD, int NW>
-__global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnArgs p) {
+// Shared memory of a key group: its K / V, bias and mask tiles
+constexpr int group_bytes(int nw) { return 2 * (KV_STAGE + bias_stage(nw) + KT * 4); }
+
+// A CTA is KS groups of NW warps: every group has the CTA's NW * 16 queries and each KS-th key tile, with two stages and a barrier of its own.
+template <int HD, int NW, int KS>
+__global__ void __launch_bounds__(KS * NW * 32, KS > 1 ? 1 : 16 / NW) split_attention_kernel(AttnArgs p) {
     constexpr int CH = HD / 8, NE = HD / 8, NT = NW * 32;
     static_assert(HD == 24 || HD == 32, "head width");
-    extern __shared__ __align__(128) uint8_t at_smem[];
-    uint8_t* bias_s = at_smem + 2 * KV_STAGE;                                    // [2][NW * 16 queries][BP]
-    float* mterm = reinterpret_cast<float*>(bias_s + 2 * bias_stage(NW));        // [2][KT]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    extern __shared__ __align__(128) uint8_t at_smem_all[];
+    const int kg = KS > 1 ? (int)threadIdx.x / NT : 0;                           // this warp's key group
+    uint8_t* at_smem = at_smem_all + kg * group_bytes(NW);
+    uint8_t* bias_s = at_smem + 2 * KV_STAGE;                                   // [2][NW * 16 queries][BP]
+    float* mterm = reinterpret_cast<float*>(bias_s + 2 * bias_stage(NW));       // [2][KT]
+    const int tid = (int)threadIdx.x - kg * NT, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    auto group_sync = [&] {
+        if (KS == 1) __syncthreads();
+        else asm volatile("bar.sync %0, %1;" ::"r"(kg + 1), "n"(NT) : "memory");
+    };
     const int h = blockIdx.y, line = blockIdx.z;
     const int qw = blockIdx.x * (NW * 16) + warp * 16;                           // this warp's first query, relative to q0
     const bool active = qw < p.n_q;
@@ -99,11 +109,11 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
         if (kk >= p.n_k) return -INFINITY;
         return p.mask && p.mask[line * p.mask_ls + kk * p.mask_ks] == 0 ? p.mask_add : 0.f;
     };
-    float m_next = tid < KT ? mask_term(tid) : 0.f;          // this thread's key of the next tile to be loaded, fetched a tile ahead
-    auto load_tile = [&](int tile) {
+    float m_next = tid < KT ? mask_term(kg * KT + tid) : 0.f;          // this thread's key of the next tile to be loaded, fetched a tile ahead
+    auto load_tile = [&](int tile, int stage) {
         const int k0 = tile * KT;
         {   // K and V parts: four chunk slots per row (HD = 24 leaves the fourth out), NT / 4 rows at a time
-            const uint32_t st = smem_u32(at_smem + (tile & 1) * KV_STAGE);
+            const uint32_t st = smem_u32(at_smem + stage * KV_STAGE);
             const int c = tid & 3;
             if (HD == 32 || c < CH) {
 #pragma unroll
@@ -119,7 +129,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
                 }
             }
         }
-        const uint32_t bst = smem_u32(bias_s + (tile & 1) * bias_stage(NW));
+        const uint32_t bst = smem_u32(bias_s + stage * bias_stage(NW));
         if (p.bias_vec) {
             const int c = (tid % (KT / 4)) * 4, rt = tid / (KT / 4);
             const bool in = k0 + c < p.n_k;
@@ -137,11 +147,11 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(bst + (r * BP + c) * 4),
                              "l"(src + min(qb + r, p.n_q - 1) * p.bias_qs), "r"(in ? 4 : 0) : "memory");
         }
-        if (tid < KT) mterm[(tile & 1) * KT + tid] = m_next;
+        if (tid < KT) mterm[stage * KT + tid] = m_next;
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (tid < KT) m_next = mask_term(k0 + KT + tid);
+        if (tid < KT) m_next = mask_term(k0 + KS * KT + tid);
     };
-    load_tile(0);
+    load_tile(kg, 0);
 
     const int r0 = min(qw + g, p.n_q - 1), r1 = min(qw + g + 8, p.n_q - 1);      // rows past the end repeat the last one
     uint32_t q[2][2][4];
@@ -169,23 +179,23 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
     const uint32_t k_lane = (uint32_t)((lane & 7) * 64), k_sw = (uint32_t)(((lane >> 3) ^ ((lane >> 1) & 3)) << 4);     // row lane & 7, chunk lane / 8
 
 #pragma unroll 1
-    for (int tile = 0; tile < ntiles; ++tile) {
-        // one barrier per tile: behind it this tile has arrived, and every warp is through the tile before, whose stage the
-        // next one overwrites
+    for (int tile = kg, stage = 0; tile < ntiles; tile += KS, stage ^= 1) {
+        // one barrier per tile: behind it this tile has arrived, and every warp of the group is through the tile before, whose
+        // stage the next one overwrites
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        if (tile + 1 < ntiles) load_tile(tile + 1);
+        group_sync();
+        if (tile + KS < ntiles) load_tile(tile + KS, stage ^ 1);
         if (active) {
             float s[8][4];
-            const float* bt = reinterpret_cast<const float*>(bias_s + (tile & 1) * bias_stage(NW)) + (warp * 16 + g) * BP + 2 * t;
+            const float* bt = reinterpret_cast<const float*>(bias_s + stage * bias_stage(NW)) + (warp * 16 + g) * BP + 2 * t;
 #pragma unroll
             for (int ni = 0; ni < 8; ++ni) {
                 const float2 b0 = *reinterpret_cast<const float2*>(bt + 8 * ni), b1 = *reinterpret_cast<const float2*>(bt + 8 * BP + 8 * ni);
                 f2_get(f2_mul(f2(b0.x, b0.y), qk2), s[ni][0], s[ni][1]);
                 f2_get(f2_mul(f2(b1.x, b1.y), qk2), s[ni][2], s[ni][3]);
             }
-            const uint32_t kst = smem_u32(at_smem + (tile & 1) * KV_STAGE), vst = kst + 2 * KV_PART;
-            const float* mt = mterm + (tile & 1) * KT;
+            const uint32_t kst = smem_u32(at_smem + stage * KV_STAGE), vst = kst + 2 * KV_PART;
+            const float* mt = mterm + stage * KT;
             const float2 mine = *reinterpret_cast<const float2*>(mt + 2 * lane);
             const bool masked = __any_sync(0xffffffffu, mine.x != 0.f || mine.y != 0.f);
 #pragma unroll
@@ -275,13 +285,41 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
             }
         }
     }
+    float sum[2], x, y;
+    f2_get(l0, x, y);
+    sum[0] = x + y;
+    f2_get(l1, x, y);
+    sum[1] = x + y;
+    if constexpr (KS > 1) {
+        // the groups' sums and outputs meet in the first one, each brought from its own maximum to the largest
+        constexpr int NV = 4 + 4 * NE;
+        group_sync();                                            // every warp of the group is through its last tile
+        float* mine = reinterpret_cast<float*>(at_smem) + tid;
+        if (kg > 0) {
+            mine[0] = c0; mine[NT] = c1; mine[2 * NT] = sum[0]; mine[3 * NT] = sum[1];
+#pragma unroll
+            for (int e = 0; e < 4 * NE; ++e) mine[(4 + e) * NT] = o[e >> 2][e & 3];
+        }
+        __syncthreads();
+        if (kg > 0) return;
+        static_assert(NV * NT * 4 <= KV_STAGE, "a group's results lie over its first tile");
+#pragma unroll 1
+        for (int k = 1; k < KS; ++k) {
+            const float* other = reinterpret_cast<const float*>(at_smem_all + k * group_bytes(NW)) + tid;
+            const float d0 = fminf(c0, other[0]), d1 = fminf(c1, other[NT]);         // c0 and c1 are minus the maxima
+            const float a0 = exp2f(d0 - c0), a1 = exp2f(d1 - c1), b0 = exp2f(d0 - other[0]), b1 = exp2f(d1 - other[NT]);
+            c0 = d0; c1 = d1;
+            sum[0] = fmaf(sum[0], a0, other[2 * NT] * b0);
+            sum[1] = fmaf(sum[1], a1, other[3 * NT] * b1);
+#pragma unroll
+            for (int e = 0; e < 4 * NE; ++e) o[e >> 2][e & 3] = fmaf(o[e >> 2][e & 3], e & 2 ? a1 : a0, other[(4 + e) * NT] * (e & 2 ? b1 : b0));
+        }
+    }
     if (!active) return;
     float inv[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-        float x, y;
-        f2_get(r ? l1 : l0, x, y);
-        x += y;
+        float x = sum[r];
         x += __shfl_xor_sync(0xffffffffu, x, 1);
         x += __shfl_xor_sync(0xffffffffu, x, 2);
         inv[r] = 1.f / (x * P_SCALE);
@@ -304,11 +342,22 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) split_attention_kernel(AttnA
     }
 }
 
-template <int HD, int NW> static int attn_go(const AttnArgs& a, cudaStream_t st) {
-    constexpr int smem = 2 * KV_STAGE + 2 * bias_stage(NW) + 2 * KT * 4;         // NW = 8: 107,008, two CTAs per SM
-    auto kern = split_attention_kernel<HD, NW>;
+template <int HD, int NW, int KS> static int attn_go(const AttnArgs& a, cudaStream_t st) {
+    constexpr int smem = KS * group_bytes(NW);         // NW = 8: 107,008, two CTAs per SM; three groups of four 210,432
+    auto kern = split_attention_kernel<HD, NW, KS>;
     B200PF_SMEM_ATTR_ONCE(kern, smem);
-    return launch_pdl(kern, dim3((unsigned)((a.n_q + NW * 16 - 1) / (NW * 16)), (unsigned)a.heads, (unsigned)a.lines), dim3(NW * 32), smem, st, a);
+    return launch_pdl(kern, dim3((unsigned)((a.n_q + NW * 16 - 1) / (NW * 16)), (unsigned)a.heads, (unsigned)a.lines), dim3(KS * NW * 32), smem, st, a);
+}
+// A line by itself gives a scheduler one warp, whose chains nothing overlaps, up to some 1000 queries; with three key groups per CTA it has
+// three (an SM's shared memory holds their tiles): 33.6 -> 19.8 us at 509 tokens x 16 heads, 26.7 -> 17.1 at 400, 22.2 -> 14.5 at 300, 17.6 ->
+// 13.0 at 203, 60.8 -> 52 at 1024; beside the pair track, whose kernels wait for the SMs that it holds, a block takes 1303 -> 1289, 518 -> 509 at 300
+// and 261 -> 258.5 at 203.  Two groups: 20.7, 17.4, 14.4 and 12.9; four with a stage each: 19.6, 17.7, 15.8 and 13.6.  Two tiles of
+// keys aren't worth it (130 -> 133 a block at 117).  The choice looks at the keys only: a range of the queries has the bits of all of them.
+template <int HD> static int attn_pick(const AttnArgs& a, int sms, cudaStream_t st) {
+    if (a.lines == 1 && a.n_k > 2 * KT && a.n_k <= 1024) return attn_go<HD, 4, 3>(a, st);
+    // eight warps share a K / V tile; with fewer than two such CTAs per SM, four warps per CTA spread the queries further
+    if ((long long)a.lines * a.heads * ((a.n_q + 127) / 128) >= 2LL * sms) return attn_go<HD, 8, 1>(a, st);
+    return attn_go<HD, 4, 1>(a, st);
 }
 
 int launch_attention(const AttnArgs& args, int hd, cudaStream_t st) {
@@ -321,12 +370,9 @@ int launch_attention(const AttnArgs& args, int hd, cudaStream_t st) {
     B200PF_REQUIRE(hd == 24 || hd == 32, B200PF_ERR_UNSUPPORTED, "split attention: head width 24 or 32 (got %d)", hd);
     // 322 -> 199 us for the whole sub-operation at 292 tokens x 4 heads, 77 -> 53 at 130, 33 -> 27 at 65, 27 -> 22 at 48
     if (attention_tc_fits(a, hd)) return launch_attention_tc(a, st);
-    // eight warps share a K / V tile; with fewer than two such CTAs per SM, four warps per CTA spread the queries further
     int sms, rc;
     if ((rc = device_multiprocessors(&sms)) != B200PF_OK) return rc;      // its CTAs share an SM: a CtaLimit does not mean them
-    const bool wide = (long long)a.lines * a.heads * ((a.n_q + 127) / 128) >= 2LL * sms;
-    if (hd == 24) return wide ? attn_go<24, 8>(a, st) : attn_go<24, 4>(a, st);
-    return wide ? attn_go<32, 8>(a, st) : attn_go<32, 4>(a, st);
+    return hd == 24 ? attn_pick<24>(a, sms, st) : attn_pick<32>(a, sms, st);
 }
 
 }  // namespace split
