@@ -308,6 +308,10 @@ __device__ __forceinline__ uint64_t make_desc_scale_block(uint32_t smem_addr) {
 __device__ __forceinline__ void tmem_cp_scale_block(uint32_t taddr, uint64_t sdesc) {
     asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
 }
+// The same in both CTAs of a pair, each from its own shared memory; issued by ONE thread of the even CTA.
+__device__ __forceinline__ void tmem_cp_scale_block_pair(uint32_t taddr, uint64_t sdesc) {
+    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
+}
 // Instruction descriptor: e4m3 x e4m3 -> fp32 with e8m0 scales, both operands K-major; sf_a / sf_b
 // pick which of the 4 scale bytes of a tensor-memory column belongs to this K = 32 step.
 __host__ __device__ constexpr uint32_t make_idesc_mxf8(int m, int n, uint32_t sf_a, uint32_t sf_b) {
@@ -320,6 +324,16 @@ __device__ __forceinline__ void umma_mxf8(uint32_t tmem_d, uint64_t desc_a, uint
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb) : "memory");
+}
+
+// Over the pair (M = 256): each CTA's tensor memory holds the scales of its own 128 rows of A and those of all rows of B.
+__device__ __forceinline__ void umma_mxf8_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                               uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb) : "memory");
 }
 
