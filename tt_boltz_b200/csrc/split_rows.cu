@@ -6,12 +6,12 @@
 namespace b200pf {
 namespace split {
 
-// Reduces V values per lane over the 32 lanes of a warp; lane l ends up with the totals of max(1, V / 32) values from index
-// reduced_base<V>(l) on (V a power of two; for V < 32 neighbouring lanes hold the same value).
-template <int V> __device__ __forceinline__ void lane_reduce(float (&v)[V], int lane) {
+// Reduces V values per lane over groups of L lanes; a lane ends up with the totals of max(1, V / L) values from index
+// reduced_base<V, L>(lane) on (powers of two; for V < L neighbouring lanes hold the same value).
+template <int V, int L> __device__ __forceinline__ void lane_reduce(float (&v)[V], int lane) {
     int cnt = V;
 #pragma unroll
-    for (int bit = 16; bit >= 1; bit >>= 1) {
+    for (int bit = L / 2; bit >= 1; bit >>= 1) {
         if (cnt > 1) {
             const int half = cnt / 2;
             const bool upper = (lane & bit) != 0;
@@ -27,137 +27,162 @@ template <int V> __device__ __forceinline__ void lane_reduce(float (&v)[V], int 
         }
     }
 }
-template <int V> __device__ __forceinline__ int reduced_base(int lane) {
+template <int V, int L> __device__ __forceinline__ int reduced_base(int lane) {
     int base = 0, half = V / 2;
 #pragma unroll
-    for (int bit = 16; bit >= 1; bit >>= 1)
+    for (int bit = L / 2; bit >= 1; bit >>= 1)
         if (half >= 1) { base += (lane & bit) ? half : 0; half /= 2; }
     return base;
 }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+    return reinterpret_cast<float2&>(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+    return reinterpret_cast<float2&>(r);
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
+    return reinterpret_cast<float2&>(r);
+}
 
+// A row's channels lie over L lanes, V consecutive ones each and J times, so that a warp works on 32 / L rows at a step and on R steps' rows at
+// a time.  With every row over the whole warp, ten shuffles a row and a 64-bit division per head sum bound the 64-wide rows: 10.4 -> 8.1 us
+// at 292 tokens (85,264 rows), with four heads 15.0 -> 12.2; 256 wide with 16 heads, packed sums and a grid that is resident at once
+// 55 -> 47 us for 65,536 rows.  256 and more channels keep four a lane: eight took 21.5 us for 19.5 there.
 template <int C, int NH, int R>
-__global__ void __launch_bounds__(256) ln_split_kernel(LnArgs p) {
-    constexpr int V = C >= 128 ? 4 : 2, J = C / (32 * V);            // V consecutive channels per lane and step
-    static_assert(J * 32 * V == C, "width must be 64 or a multiple of 128");
-    extern __shared__ __align__(16) float head_s[];                  // [NH][C]
-    const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(256, NH > 0 ? 2 : 1) ln_split_kernel(LnArgs p) {
+    constexpr int V = C >= 256 ? 4 : 8, L = C >= 256 ? 32 : C / V, J = C / (L * V), Q = V / 4, RW = 32 / L;
+    static_assert(J * L * V == C, "width must be 64, 128, 256 or 384");
+    extern __shared__ __align__(16) float head_s[];                  // [NH][J][Q][L] four channels each
+    const int lane = threadIdx.x & 31, sub = lane % L, rsub = lane / L;
     grid_dependency_wait();
     grid_launch_dependents();
+    const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), nwarps = (long long)gridDim.x * (blockDim.x >> 5);
     if (NH > 0) {
-        for (int i = threadIdx.x; i < NH * C; i += blockDim.x) head_s[i] = *(p.head_w + i);
+        for (int i = threadIdx.x; i < NH * C; i += blockDim.x) {
+            const int c = i % C, h = i / C, j = c / (L * V), l = c % (L * V) / V, q = c % V / 4;
+            head_s[(((h * J + j) * Q + q) * L + l) * 4 + c % 4] = *(p.head_w + i);
+        }
         __syncthreads();
     }
-    float gam[J][V], bet[J][V];
+    float2 gam[J][V / 2], bet[J][V / 2];
 #pragma unroll
     for (int j = 0; j < J; ++j)
 #pragma unroll
-        for (int e = 0; e < V; ++e) { gam[j][e] = *(p.gamma + (j * 32 + lane) * V + e); bet[j][e] = *(p.beta + (j * 32 + lane) * V + e); }
-    const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long base = warp * R; base < p.rows; base += nwarps * R) {
-        float x[R][J][V];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const long long row = base + r < p.rows ? base + r : p.rows - 1;
-            const float* src = p.x + row * C + lane * V;
-#pragma unroll
-            for (int j = 0; j < J; ++j) {
-                if (V == 4) {
-                    const float4 t = *reinterpret_cast<const float4*>(src + j * 128);
-                    x[r][j][0] = t.x; x[r][j][1] = t.y; x[r][j][2 % V] = t.z; x[r][j][3 % V] = t.w;
-                } else {
-                    const float2 t = *reinterpret_cast<const float2*>(src + j * 64);
-                    x[r][j][0] = t.x; x[r][j][1] = t.y;
-                }
-            }
+        for (int e = 0; e < V / 2; ++e) {
+            const int c = (j * L + sub) * V + 2 * e;
+            gam[j][e] = make_float2(*(p.gamma + c), *(p.gamma + c + 1));
+            bet[j][e] = make_float2(*(p.beta + c), *(p.beta + c + 1));
         }
-        float s[R], ss[R];
+    for (long long base = warp * (R * RW); base < p.rows; base += nwarps * (R * RW)) {
+        float2 x[R][J][V / 2];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            float a = 0.f;
+            const long long mine = base + r * RW + rsub, row = mine < p.rows ? mine : p.rows - 1;
 #pragma unroll
             for (int j = 0; j < J; ++j)
 #pragma unroll
-                for (int e = 0; e < V; ++e) a += x[r][j][e];
-            s[r] = a;
+                for (int q = 0; q < Q; ++q) {
+                    const float4 t = *reinterpret_cast<const float4*>(p.x + row * C + (j * L + sub) * V + 4 * q);
+                    x[r][j][2 * q] = make_float2(t.x, t.y);
+                    x[r][j][2 * q + 1] = make_float2(t.z, t.w);
+                }
+        }
+        float s[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            float2 a = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < J; ++j)
+#pragma unroll
+                for (int e = 0; e < V / 2; ++e) a = add2(a, x[r][j][e]);
+            s[r] = a.x + a.y;
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+        for (int o = L / 2; o > 0; o >>= 1)
 #pragma unroll
             for (int r = 0; r < R; ++r) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const float mean = s[r] * (1.f / C);
-            float a = 0.f;
+            const float2 neg = make_float2(-mean, -mean);
+            float2 a = make_float2(0.f, 0.f);
 #pragma unroll
             for (int j = 0; j < J; ++j)
 #pragma unroll
-                for (int e = 0; e < V; ++e) { x[r][j][e] -= mean; a = fmaf(x[r][j][e], x[r][j][e], a); }
-            ss[r] = a;
+                for (int e = 0; e < V / 2; ++e) { x[r][j][e] = add2(x[r][j][e], neg); a = fma2(x[r][j][e], x[r][j][e], a); }
+            s[r] = a.x + a.y;
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+        for (int o = L / 2; o > 0; o >>= 1)
 #pragma unroll
-            for (int r = 0; r < R; ++r) ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], o);
+            for (int r = 0; r < R; ++r) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const float rstd = rsqrtf(ss[r] * (1.f / C) + LN_EPS);
+            const float rstd = rsqrtf(s[r] * (1.f / C) + LN_EPS);
+            const float2 r2 = make_float2(rstd, rstd);
+            const long long row = base + r * RW + rsub;
 #pragma unroll
             for (int j = 0; j < J; ++j)
 #pragma unroll
-                for (int e = 0; e < V; ++e) x[r][j][e] = fmaf(x[r][j][e] * rstd, gam[j][e], bet[j][e]);
-            if (p.planes && base + r < p.rows) {
-                __half* dst = p.planes + (base + r) * C + lane * V;
+                for (int e = 0; e < V / 2; ++e) x[r][j][e] = fma2(mul2(x[r][j][e], r2), gam[j][e], bet[j][e]);
+            if (p.planes && row < p.rows) {
+                __half* dst = p.planes + row * C + sub * V;
 #pragma unroll
                 for (int j = 0; j < J; ++j) {
-                    uint32_t h0, l0;
-                    split_f16x2(x[r][j][0], x[r][j][1], h0, l0);
-                    if (V == 4) {
-                        uint32_t h1, l1;
-                        split_f16x2(x[r][j][2 % V], x[r][j][3 % V], h1, l1);
-                        *reinterpret_cast<uint2*>(dst + j * 128) = make_uint2(h0, h1);
-                        *reinterpret_cast<uint2*>(dst + p.part_stride + j * 128) = make_uint2(l0, l1);
+                    uint32_t h[V / 2], l[V / 2];
+#pragma unroll
+                    for (int e = 0; e < V / 2; ++e) split_f16x2(x[r][j][e].x, x[r][j][e].y, h[e], l[e]);
+                    if constexpr (V == 8) {
+                        *reinterpret_cast<uint4*>(dst + j * L * V) = make_uint4(h[0], h[1], h[2], h[3]);
+                        *reinterpret_cast<uint4*>(dst + p.part_stride + j * L * V) = make_uint4(l[0], l[1], l[2], l[3]);
                     } else {
-                        *reinterpret_cast<uint32_t*>(dst + j * 64) = h0;
-                        *reinterpret_cast<uint32_t*>(dst + p.part_stride + j * 64) = l0;
+                        *reinterpret_cast<uint2*>(dst + j * L * V) = make_uint2(h[0], h[1]);
+                        *reinterpret_cast<uint2*>(dst + p.part_stride + j * L * V) = make_uint2(l[0], l[1]);
                     }
                 }
             }
         }
-        if (NH > 0) {
-            constexpr int NV = NH > 0 ? R * NH : 1;
+        if constexpr (NH > 0) {
+            constexpr int NV = R * NH;                               // a lane's partial sums, [head][step]
             float acc[NV];
 #pragma unroll
             for (int h = 0; h < NH; ++h) {
+                float2 a[R];
 #pragma unroll
-                for (int r = 0; r < R; ++r) acc[h * R + r] = 0.f;
+                for (int r = 0; r < R; ++r) a[r] = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int j = 0; j < J; ++j) {
-                    const float* w = head_s + h * C + (j * 32 + lane) * V;
-                    float wv[V];
-                    if (V == 4) {
-                        const float4 t = *reinterpret_cast<const float4*>(w);
-                        wv[0] = t.x; wv[1] = t.y; wv[2 % V] = t.z; wv[3 % V] = t.w;
-                    } else {
-                        const float2 t = *reinterpret_cast<const float2*>(w);
-                        wv[0] = t.x; wv[1] = t.y;
+                for (int j = 0; j < J; ++j)
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) {
+                        const float4 w = reinterpret_cast<const float4*>(head_s)[((h * J + j) * Q + q) * L + sub];
+#pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            a[r] = fma2(x[r][j][2 * q], make_float2(w.x, w.y), a[r]);
+                            a[r] = fma2(x[r][j][2 * q + 1], make_float2(w.z, w.w), a[r]);
+                        }
                     }
 #pragma unroll
-                    for (int r = 0; r < R; ++r)
-#pragma unroll
-                        for (int e = 0; e < V; ++e) acc[h * R + r] = fmaf(x[r][j][e], wv[e], acc[h * R + r]);
-                }
+                for (int r = 0; r < R; ++r) acc[h * R + r] = a[r].x + a[r].y;
             }
-            lane_reduce<NV>(acc, lane);
-            const int b0 = reduced_base<NV>(lane);
-            constexpr int PER = NV >= 32 ? NV / 32 : 1, DUP = NV >= 32 ? 1 : 32 / NV;
-            if (lane % DUP == 0) {
+            lane_reduce<NV, L>(acc, lane);
+            const int b0 = reduced_base<NV, L>(lane);
+            constexpr int PER = NV >= L ? NV / L : 1, DUP = NV >= L ? 1 : L / NV;
+            if (sub % DUP == 0) {
 #pragma unroll
                 for (int i = 0; i < PER; ++i) {
                     const int idx = b0 + i, h = idx / R;
-                    const long long row = base + idx % R;
+                    const long long row = base + idx % R * RW + rsub;
                     if (row < p.rows) {
-                        const long long line = row / p.n, pos = row - line * p.n, at = p.transposed ? pos * p.head_pitch + line : line * p.head_pitch + pos;
-                        p.head_out[h * p.head_stride + at] = acc[i];
+                        long long line, pos;
+                        if (p.rows <= 0x7fffffffLL) { line = (unsigned)row / (unsigned)p.n; pos = (unsigned)row - (unsigned)line * (unsigned)p.n; }
+                        else { line = row / p.n; pos = row - line * p.n; }
+                        p.head_out[h * p.head_stride + (p.transposed ? pos * p.head_pitch + line : line * p.head_pitch + pos)] = acc[i];
                     }
                 }
             }
@@ -168,13 +193,13 @@ __global__ void __launch_bounds__(256) ln_split_kernel(LnArgs p) {
 bool ln_supported(int c) { return c == 64 || c == 128 || c == 256 || c == 384; }
 
 template <int C, int NH> static int ln_go(const LnArgs& a, cudaStream_t st) {
-    constexpr int R = NH == 16 ? 4 : NH > 0 ? 4 : (C >= 256 ? 2 : 4);
+    constexpr int R = NH > 0 && C >= 256 ? 4 : 2, RW = C >= 256 ? 1 : 256 / C;
     int sms, rc;
     if ((rc = multiprocessors(&sms)) != B200PF_OK) return rc;
     // few rows: one warp pass per block of fewer warps, so that every SM gets some
-    const int warps = a.rows >= (long long)sms * 8 * R ? 8 : 2;
-    const long long need = (a.rows + (long long)warps * R - 1) / ((long long)warps * R);
-    const long long most = (long long)sms * (NH > 0 ? 4 : 8);
+    const int warps = a.rows >= (long long)sms * 8 * R * RW ? 8 : 2;
+    const long long need = (a.rows + (long long)warps * R * RW - 1) / ((long long)warps * R * RW);
+    const long long most = (long long)sms * (NH > 0 ? 2 : 8);
     return launch_pdl(ln_split_kernel<C, NH, R>, dim3((unsigned)(need < most ? need : most)), dim3(warps * 32), (size_t)NH * C * 4, st, a);
 }
 template <int C> static int ln_heads(const LnArgs& a, int heads, cudaStream_t st) {
