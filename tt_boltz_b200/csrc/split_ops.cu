@@ -106,8 +106,8 @@ struct TriMulWs { __half *x, *tn, *ab; float* t; int pitch, tpitch; long long by
 static TriMulWs trimul_ws(void* ws, int n, int c) {
     Arena a(ws);
     TriMulWs w;
-    w.pitch = round_up(n, 8);
-    w.tpitch = round_up(n, 4);
+    w.pitch = round_up(n, 32);                         // rows of both on 64-byte boundaries: no store or box of one splits a sector
+    w.tpitch = round_up(n, 16);
     w.x = a.take<__half>(2LL * n * n * c);
     w.ab = a.take<__half>(2LL * 2 * c * n * w.pitch);
     w.tn = w.ab;                                       // the operands are spent when the normalised product is written
@@ -125,7 +125,7 @@ static TriAttWs triatt_ws(void* ws, int n, int c, int heads, int hd) {
     w.og = w.x;                                        // x is spent once q, k, v, g exist
     w.qkv = a.take<__half>(2 * nn * 3 * ht);
     w.gate = a.take<float>(nn * ht);
-    w.bpitch = round_up(n, 4);                         // bias rows start on 16-byte boundaries
+    w.bpitch = round_up(n, 16);                        // bias rows start on 64-byte boundaries
     w.bias = a.take<float>((long long)n * w.bpitch * heads);
     w.bytes = a.used;
     return w;

@@ -21,7 +21,7 @@ from typing import Optional
 import torch
 from torch import nn
 
-from . import weights
+from . import ops, weights
 from ._lib import Planes, call, ptr, stream
 
 C_M, C_HID, C_OUT = 64, 32, 128
@@ -89,7 +89,7 @@ class B200OuterProductMean(nn.Module):
         m = m.to(torch.float32).contiguous()
         mask_u8 = _u8(mask)
         dev, st = m.device, stream()
-        pitch = _round_up(s_len, 8)
+        pitch = _round_up(s_len, ops.PLANE_PITCH)
         a_t = torch.empty(n * C_HID * pitch, dtype=torch.bfloat16, device=dev)
         b_t = torch.empty(n * C_HID * pitch, dtype=torch.bfloat16, device=dev)
         call("b200pf_opm_producer", ptr(m), ptr(mask_u8), ptr(w["gamma"]), ptr(w["beta"]), ptr(w["w_ab"]), ptr(a_t), ptr(b_t),
@@ -205,7 +205,7 @@ class B200PairWeightedAveraging(nn.Module):
             raise ValueError("z must be a contiguous fp32 tensor [N, N, 128]")
         w = self._pack(m.device)
         dev, st, heads = m.device, stream(), self.num_heads
-        np_ = pw = _round_up(n, 8)
+        np_ = pw = _round_up(n, ops.PLANE_PITCH)
         logits = torch.empty(16 * n * n, dtype=torch.float32, device=dev)
         call("b200pf_ln_proj_heads", ptr(z), ptr(w["gz"]), ptr(w["bz"]), ptr(w["w_z"]), ptr(logits), n * n, n * n, 128, 16, st)
         wt = torch.empty(heads * n * pw, dtype=torch.bfloat16, device=dev)
@@ -346,7 +346,6 @@ class B200MSALayer(nn.Module):
 def _run_blocks(layers, z: torch.Tensor, m: torch.Tensor, token_mask: torch.Tensor, msa_mask: torch.Tensor) -> None:
     """Every block on the resident z and m; what all blocks share (masks in the kernels' forms, the pair block's workspace) made
     once: the pair mask's two padded forms are six small launches, 25 us a block at 171 tokens."""
-    from . import ops
     from .pairformer import _mask_u8
     with torch.no_grad():
         pair_u8, msa_u8, ws_cache = _u8(token_mask), _u8(msa_mask), {}
