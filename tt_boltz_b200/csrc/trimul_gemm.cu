@@ -46,8 +46,8 @@ __device__ __forceinline__ long long x_row_offset(const GemmShape& s, int d, int
 
 // One epilogue warp's 32 rows (from `row0`) x COLS columns of a finished accumulator.  Plain planes leave through SLOTS swizzled staging tiles in
 // turn and TMA stores of [32 rows][64 columns].  As 16-byte stores of a thread per row, 4096 partial sectors a tile, they took 11 k clocks a tile
-// against 3.6 k to 8.2 k of MMAs: 11.7 -> 9.7 us at 203 tokens, 43 -> 35 at 400, 112 -> 94 at 600, 238 -> 224 at 1024 (what is left is
-// the operands, some 9 TB/s out of L2).  Columns in groups (the outer product's blocks of contiguous 2 KB) and row groups that 32 does
+// against 3.6 k to 8.2 k of MMAs: 11.7 -> 9.7 us at 203 tokens, 43 -> 35 at 400, 112 -> 94 at 600, 238 -> 224 at 1024 (some 9 TB/s of
+// operands come out of L2 then).  Columns in groups (the outer product's blocks of contiguous 2 KB) and row groups that 32 does
 // not divide stay with the direct stores.
 template <int COLS, int SLOTS>
 __device__ __forceinline__ void store_tile(const CUtensorMap* map_x, __nv_bfloat16* x, const GemmShape& s, uint32_t taddr, uint8_t* stg, uint32_t& slot, int d, int row0,
@@ -241,12 +241,13 @@ trimul_contract_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 // Two CTAs of a cluster (the two SMs of a TPC) share one 256 x 256 output tile: each stages its 128 rows of A and
 // its 128 rows of B (32 KB per k-block instead of the 48 KB a lone CTA needs for 128 x 256: the lone kernel is bound
 // by the 96 bytes per clock it has to pull from L2), the even CTA issues tcgen05.mma.cta_group::2 over both halves,
-// and each CTA drains its own 128 accumulator rows, with eight epilogue warps: four were as long as the MMAs of a tile or longer up to some
-// 512 tokens (25.8 -> 21.4 us at 300, 35.2 -> 30.1 at 400, 41.6 -> 37.9 at 512, 9.5 -> 8.8 at 203; 92.1 -> 90.6 at 600 and the same at 1024,
-// where the operands bound it).  A staging tile a warp leaves six stages; two with five stages 248 -> 262 at 1024.  The one-CTA kernel, for
-// at most 128 rows, keeps four warps with two tiles each (eight with one: 5.4 -> 5.7 at 117).  Loads land in the loading CTA's own shared memory (never a
-// multicast); their bytes are counted on the even CTA's barrier.  Every role of both CTAs always reaches the two
-// cluster barriers, also after a wait ran out.
+// and each CTA drains its own 128 accumulator rows, with eight epilogue warps: four were as long as the MMAs of a tile or longer up
+// to some 512 tokens (25.8 -> 21.4 us at 300, 35.2 -> 30.1 at 400, 41.6 -> 37.9 at 512, 9.5 -> 8.8 at 203; 92.1 -> 90.6 at 600 and the
+// same at 1024, 216 us and 0.9 of the tensor rate that the chip sustains).  Tiles of 256 x 512 with one accumulator take a quarter less
+// out of L2 and the same time there (214; 768: 104 -> 109).  A staging tile a warp leaves six stages; two with five stages 248 -> 262
+// at 1024.  The one-CTA kernel, for at most 128 rows, keeps four warps with two tiles each (eight with one: 5.4 -> 5.7 at 117).  Loads
+// land in the loading CTA's own shared memory (never a multicast); their bytes are counted on the even CTA's barrier.  Every role of
+// both CTAs always reaches the two cluster barriers, also after a wait ran out.
 constexpr int P_STAGES = 6, P_STAGE_BYTES = 2 * (128 * BK * 2);
 constexpr int P_EPI_WARPS = 8, P_SLOTS = 1, P_STG_TOTAL = P_EPI_WARPS * P_SLOTS * STG_BYTES, PAIR_THREADS = (2 + P_EPI_WARPS) * 32;
 constexpr int PAIR_SMEM = P_STAGES * P_STAGE_BYTES + P_STG_TOTAL + 1024 + 256;
