@@ -433,16 +433,6 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], uint32_t a0, uint32_t a1
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
-    return reinterpret_cast<float2&>(r);
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
-    return reinterpret_cast<float2&>(r);
-}
 
 __global__ void __launch_bounds__(256, 2)
 ln_proj_heads16_mma_kernel(const float* z, const float* gamma, const float* beta, const float* w, float* out, long long out_hs, long long rows) {

@@ -25,8 +25,8 @@ __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
 // Two values into fp16 part words {hi, lo}.
 __device__ __forceinline__ void split_f16x2(float a, float b, uint32_t& hi, uint32_t& lo) {
     hi = pack_f16x2(a, b);
-    const float2 f = __half22float2(*reinterpret_cast<__half2*>(&hi));
-    lo = pack_f16x2(a - f.x, b - f.y);
+    const float2 left = fma2(__half22float2(*reinterpret_cast<__half2*>(&hi)), make_float2(-1.f, -1.f), make_float2(a, b));
+    lo = pack_f16x2(left.x, left.y);
 }
 // Two values into bf16 part words {h, m, l}.
 __device__ __forceinline__ void split_bf16x3(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {

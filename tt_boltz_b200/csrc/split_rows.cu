@@ -34,21 +34,6 @@ template <int V, int L> __device__ __forceinline__ int reduced_base(int lane) {
         if (half >= 1) { base += (lane & bit) ? half : 0; half /= 2; }
     return base;
 }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
-    return reinterpret_cast<float2&>(r);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
-    return reinterpret_cast<float2&>(r);
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
-    return reinterpret_cast<float2&>(r);
-}
 
 // A row's channels lie over L lanes, V consecutive ones each and J times, so that a warp works on 32 / L rows at a step and on R steps' rows at
 // a time.  With every row over the whole warp, ten shuffles a row and a 64-bit division per head sum bound the 64-wide rows: 10.4 -> 8.1 us
