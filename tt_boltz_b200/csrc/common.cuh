@@ -78,6 +78,18 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
     return reinterpret_cast<float2&>(r);
 }
+// LayerNorm of four channels at a time on them: the sum, the centring with the sum of squares, gain and offset.
+__device__ __forceinline__ float2 low2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 high2(const float4& v) { return make_float2(v.z, v.w); }
+__device__ __forceinline__ void centre4(float4& v, float2 minus_mean, float2& squares) {
+    const float2 a = add2(low2(v), minus_mean), b = add2(high2(v), minus_mean);
+    squares = fma2(b, b, fma2(a, a, squares));
+    v = make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ float4 affine4(const float4& v, float2 rstd, const float4& gain, const float4& offset) {
+    const float2 a = fma2(mul2(low2(v), rstd), low2(gain), low2(offset)), b = fma2(mul2(high2(v), rstd), high2(gain), high2(offset));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

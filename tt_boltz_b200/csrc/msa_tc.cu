@@ -36,7 +36,10 @@ __device__ __forceinline__ void ln64_rows32(const float* src, int row0, int vali
     }
     float s[8], ss[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) s[i] = ((v[i][0].x + v[i][0].y) + (v[i][0].z + v[i][0].w)) + ((v[i][1].x + v[i][1].y) + (v[i][1].z + v[i][1].w));
+    for (int i = 0; i < 8; ++i) {
+        const float2 t = add2(add2(low2(v[i][0]), high2(v[i][0])), add2(low2(v[i][1]), high2(v[i][1])));
+        s[i] = t.x + t.y;
+    }
 #pragma unroll
     for (int step = 1; step < 8; step <<= 1)
 #pragma unroll
@@ -44,13 +47,10 @@ __device__ __forceinline__ void ln64_rows32(const float* src, int row0, int vali
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const float mean = s[i] * (1.f / CM);
-        float a = 0.f;
+        float2 sq = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            v[i][j].x -= mean; v[i][j].y -= mean; v[i][j].z -= mean; v[i][j].w -= mean;
-            a += (v[i][j].x * v[i][j].x + v[i][j].y * v[i][j].y) + (v[i][j].z * v[i][j].z + v[i][j].w * v[i][j].w);
-        }
-        ss[i] = a;
+        for (int j = 0; j < 2; ++j) centre4(v[i][j], make_float2(-mean, -mean), sq);
+        ss[i] = sq.x + sq.y;
     }
 #pragma unroll
     for (int step = 1; step < 8; step <<= 1)
@@ -64,8 +64,9 @@ __device__ __forceinline__ void ln64_rows32(const float* src, int row0, int vali
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             uint2 o;
-            o.x = keep ? pack_bf16x2(fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x), fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y)) : 0u;
-            o.y = keep ? pack_bf16x2(fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z), fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w)) : 0u;
+            const float4 y = affine4(v[i][j], make_float2(rstd, rstd), gam[j], bet[j]);
+            o.x = keep ? pack_bf16x2(y.x, y.y) : 0u;
+            o.y = keep ? pack_bf16x2(y.z, y.w) : 0u;
             *reinterpret_cast<uint2*>(tile + sw128(row, j * 4 + (sub >> 1)) + (sub & 1) * 8) = o;
         }
     }

@@ -29,6 +29,8 @@
 // four with 32 rows each: 269 / 290 -> 232 / 247 us (multiplication, outgoing / incoming) and 352 / 356 -> 326 / 330 (attention, rows /
 // columns) at 1024 tokens, 47.8 -> 43.4 and 61.3 -> 60.2 at 400, the same at 203, where a CTA has three tiles; five are slower
 // everywhere (252 / 273 and 334 / 333), seven no faster (238 / 251 and 324 / 334) and spill in the MXFP8 form.
+// A pass's arithmetic goes two channels to an instruction: 43.7 / 46.4 -> 42.1 / 44.9 and 61.3 / 61.0 -> 58.8 / 59.2 at 400, the attention
+// producer 347 / 360 -> 329 / 328 at 1024, on one box; the gates' alike.
 #include "mxfp8.cuh"
 #include "row512_tc.h"
 #include "rowtc.cuh"
@@ -172,9 +174,10 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
         float s4[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            float s = 0.f;
+            float2 t = add2(low2(v[i][0]), high2(v[i][0]));
 #pragma unroll
-            for (int j = 0; j < 4; ++j) s += (v[i][j].x + v[i][j].y) + (v[i][j].z + v[i][j].w);
+            for (int j = 1; j < 4; ++j) t = add2(t, add2(low2(v[i][j]), high2(v[i][j])));
+            const float s = t.x + t.y;
             s4[i] = s;
         }
 #pragma unroll
@@ -185,12 +188,10 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float mean = s4[i] * (1.f / KC);
-            float ss = 0.f;
+            float2 sq = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                v[i][j].x -= mean; v[i][j].y -= mean; v[i][j].z -= mean; v[i][j].w -= mean;
-                ss += (v[i][j].x * v[i][j].x + v[i][j].y * v[i][j].y) + (v[i][j].z * v[i][j].z + v[i][j].w * v[i][j].w);
-            }
+            for (int j = 0; j < 4; ++j) centre4(v[i][j], make_float2(-mean, -mean), sq);
+            const float ss = sq.x + sq.y;
             ss4[i] = ss;
         }
 #pragma unroll
@@ -203,13 +204,11 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
             const float rstd = rsqrtf(ss4[i] * (1.f / KC) + LN_EPS);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                v[i][j].x = fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x) * kz[i];
-                v[i][j].y = fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y) * kz[i];
-                v[i][j].z = fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z) * kz[i];
-                v[i][j].w = fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w) * kz[i];
+                const float4 y = affine4(v[i][j], make_float2(rstd, rstd), gam[j], bet[j]);
+                const float2 k2 = make_float2(kz[i], kz[i]), a = mul2(low2(y), k2), b = mul2(high2(y), k2);
                 uint2 o;
-                o.x = pack_bf16x2(v[i][j].x, v[i][j].y);
-                o.y = pack_bf16x2(v[i][j].z, v[i][j].w);
+                o.x = pack_bf16x2(a.x, a.y);
+                o.y = pack_bf16x2(b.x, b.y);
                 const int chunk = (j & 1) * 4 + (sub >> 1);
                 *reinterpret_cast<uint2*>(a_tile + (j >> 1) * A_KB_BYTES + sw128(row, chunk) + (sub & 1) * 8) = o;
             }
@@ -353,15 +352,14 @@ row512_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ 
             uint32_t* w = reinterpret_cast<uint32_t*>(o);
 #pragma unroll
             for (int e = 0; e < 32; ++e) {
-                float v0 = __uint_as_float(r[e >> 4][(2 * e) & 31]), v1 = __uint_as_float(r[e >> 4][(2 * e + 1) & 31]);
+                float2 v = make_float2(__uint_as_float(r[e >> 4][(2 * e) & 31]), __uint_as_float(r[e >> 4][(2 * e + 1) & 31]));
                 if (tanh_mode == 1) {
-                    v0 = fmaf(v0, tanh_approx(__uint_as_float(gq[e >> 4][(2 * e) & 31])), v0);
-                    v1 = fmaf(v1, tanh_approx(__uint_as_float(gq[e >> 4][(2 * e + 1) & 31])), v1);
+                    const uint32_t* g = &gq[e >> 4][(2 * e) & 31];
+                    v = fma2(v, make_float2(tanh_approx(__uint_as_float(g[0])), tanh_approx(__uint_as_float(g[1]))), v);
                 } else if (tanh_mode == 2) {
-                    v0 = fmaf(0.5f, tanh_approx(v0), 0.5f);
-                    v1 = fmaf(0.5f, tanh_approx(v1), 0.5f);
+                    v = fma2(make_float2(0.5f, 0.5f), make_float2(tanh_approx(v.x), tanh_approx(v.y)), make_float2(0.5f, 0.5f));
                 }
-                w[e] = pack_bf16x2(v0, v1);
+                w[e] = pack_bf16x2(v.x, v.y);
             }
         };
         // This warp's 32 staging rows x 128 bytes; `inside`: the box is not wholly beyond the tensor's edge.

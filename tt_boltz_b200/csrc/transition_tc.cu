@@ -71,19 +71,18 @@ __device__ __forceinline__ void normalise16(const Args& p, long long base, int r
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int row = row0 + i * 4 + rq;
-        float s = 0.f;
+        float2 t = add2(low2(v[i][0]), high2(v[i][0]));
 #pragma unroll
-        for (int j = 0; j < 4; ++j) s += (v[i][j].x + v[i][j].y) + (v[i][j].z + v[i][j].w);
+        for (int j = 1; j < 4; ++j) t = add2(t, add2(low2(v[i][j]), high2(v[i][j])));
+        float s = t.x + t.y;
         s += __shfl_xor_sync(0xffffffffu, s, 1);
         s += __shfl_xor_sync(0xffffffffu, s, 2);
         s += __shfl_xor_sync(0xffffffffu, s, 4);
         const float mean = s * (1.f / KC);
-        float ss = 0.f;
+        float2 sq = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            v[i][j].x -= mean; v[i][j].y -= mean; v[i][j].z -= mean; v[i][j].w -= mean;
-            ss += (v[i][j].x * v[i][j].x + v[i][j].y * v[i][j].y) + (v[i][j].z * v[i][j].z + v[i][j].w * v[i][j].w);
-        }
+        for (int j = 0; j < 4; ++j) centre4(v[i][j], make_float2(-mean, -mean), sq);
+        float ss = sq.x + sq.y;
         ss += __shfl_xor_sync(0xffffffffu, ss, 1);
         ss += __shfl_xor_sync(0xffffffffu, ss, 2);
         ss += __shfl_xor_sync(0xffffffffu, ss, 4);
@@ -91,8 +90,9 @@ __device__ __forceinline__ void normalise16(const Args& p, long long base, int r
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             uint2 o;
-            o.x = pack_bf16x2(fmaf(v[i][j].x * rstd, w.gam[j].x, w.bet[j].x), fmaf(v[i][j].y * rstd, w.gam[j].y, w.bet[j].y));
-            o.y = pack_bf16x2(fmaf(v[i][j].z * rstd, w.gam[j].z, w.bet[j].z), fmaf(v[i][j].w * rstd, w.gam[j].w, w.bet[j].w));
+            const float4 y = affine4(v[i][j], make_float2(rstd, rstd), w.gam[j], w.bet[j]);
+            o.x = pack_bf16x2(y.x, y.y);
+            o.y = pack_bf16x2(y.z, y.w);
             const int chunk = (j & 1) * 4 + (sub >> 1);
             *reinterpret_cast<uint2*>(a_tile + (j >> 1) * A_KB_BYTES + sw128(row, chunk) + (sub & 1) * 8) = o;
         }
@@ -108,10 +108,9 @@ __device__ __forceinline__ void hidden32(uint32_t t_f1, uint32_t t_f2, uint32_t 
     tmem_ld_wait();
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
-        float a0 = __uint_as_float(f1[2 * e]), a1 = __uint_as_float(f1[2 * e + 1]);
-        float h0 = fmaf(a0, tanh_approx(a0), a0) * __uint_as_float(f2[2 * e]);
-        float h1 = fmaf(a1, tanh_approx(a1), a1) * __uint_as_float(f2[2 * e + 1]);
-        hw[e] = pack_bf16x2(h0, h1);
+        const float2 a = make_float2(__uint_as_float(f1[2 * e]), __uint_as_float(f1[2 * e + 1]));
+        const float2 h = mul2(fma2(a, make_float2(tanh_approx(a.x), tanh_approx(a.y)), a), make_float2(__uint_as_float(f2[2 * e]), __uint_as_float(f2[2 * e + 1])));
+        hw[e] = pack_bf16x2(h.x, h.y);
     }
     tmem_st_32x16(t_h, hw);
 }

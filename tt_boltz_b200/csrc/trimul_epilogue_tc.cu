@@ -149,9 +149,10 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
         float s4[4], ss4[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            float s = 0.f;
+            float2 t = add2(low2(v[i][0]), high2(v[i][0]));
 #pragma unroll
-            for (int j = 0; j < 4; ++j) s += (v[i][j].x + v[i][j].y) + (v[i][j].z + v[i][j].w);
+            for (int j = 1; j < 4; ++j) t = add2(t, add2(low2(v[i][j]), high2(v[i][j])));
+            const float s = t.x + t.y;
             s4[i] = s;
         }
 #pragma unroll
@@ -161,12 +162,10 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float mean = s4[i] * (1.f / KC);
-            float ss = 0.f;
+            float2 sq = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                v[i][j].x -= mean; v[i][j].y -= mean; v[i][j].z -= mean; v[i][j].w -= mean;
-                ss += (v[i][j].x * v[i][j].x + v[i][j].y * v[i][j].y) + (v[i][j].z * v[i][j].z + v[i][j].w * v[i][j].w);
-            }
+            for (int j = 0; j < 4; ++j) centre4(v[i][j], make_float2(-mean, -mean), sq);
+            const float ss = sq.x + sq.y;
             ss4[i] = ss;
         }
 #pragma unroll
@@ -180,8 +179,9 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 uint2 o;
-                o.x = pack_bf16x2(fmaf(v[i][j].x * rstd, gam[j].x, bet[j].x), fmaf(v[i][j].y * rstd, gam[j].y, bet[j].y));
-                o.y = pack_bf16x2(fmaf(v[i][j].z * rstd, gam[j].z, bet[j].z), fmaf(v[i][j].w * rstd, gam[j].w, bet[j].w));
+                const float4 y = affine4(v[i][j], make_float2(rstd, rstd), gam[j], bet[j]);
+                o.x = pack_bf16x2(y.x, y.y);
+                o.y = pack_bf16x2(y.z, y.w);
                 const int chunk = (j & 1) * 4 + (sub >> 1);
                 *reinterpret_cast<uint2*>(a_tile + (j >> 1) * A_KB_BYTES + sw128(row, chunk) + (sub & 1) * 8) = o;
             }
@@ -357,9 +357,12 @@ trimul_epilogue_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
                 float4 o[8];
                 float* of = reinterpret_cast<float*>(o);
 #pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                    float ph2 = fmaf(st.y, fmaf(-st.x, wsum_s[c0 + e], __uint_as_float(pr[e])), wb_s[c0 + e]);
-                    of[e] = fmaf(ph2, tanh_approx(__uint_as_float(gr[e])), ph2);
+                for (int e = 0; e < 32; e += 2) {
+                    const float2 ws = *reinterpret_cast<const float2*>(wsum_s + c0 + e), wb = *reinterpret_cast<const float2*>(wb_s + c0 + e);
+                    const float2 centred = fma2(make_float2(-st.x, -st.x), ws, make_float2(__uint_as_float(pr[e]), __uint_as_float(pr[e + 1])));
+                    const float2 ph2 = fma2(make_float2(st.y, st.y), centred, wb);
+                    const float2 u = fma2(ph2, make_float2(tanh_approx(__uint_as_float(gr[e])), tanh_approx(__uint_as_float(gr[e + 1]))), ph2);
+                    of[e] = u.x; of[e + 1] = u.y;
                 }
                 if (lane == 0) bulk_wait_read0();                  // this warp's previous reduction has read the staging tile
                 __syncwarp();
