@@ -125,13 +125,15 @@ __device__ __forceinline__ bool load_loop(const LnRows& p, uint8_t* x0, uint64_t
 // -43 counts as 2^-62, where that of +43 is 1.
 __device__ __forceinline__ void sigmoid_of(float x0, float x1, float& s0, float& s1) {
     float e0, e1, r;
-    asm("min.NaN.f32 %0, %1, %2;" : "=f"(e0) : "f"(-1.44269504f * x0), "f"(62.f));
-    asm("min.NaN.f32 %0, %1, %2;" : "=f"(e1) : "f"(-1.44269504f * x1), "f"(62.f));
+    const float2 t = mul2(make_float2(x0, x1), make_float2(-1.44269504f, -1.44269504f));
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(e0) : "f"(t.x), "f"(62.f));
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(e1) : "f"(t.y), "f"(62.f));
     asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e0));
     asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e1));
-    const float d0 = 1.f + e0, d1 = 1.f + e1;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d0 * d1));
-    s0 = r * d1; s1 = r * d0;
+    const float2 d = add2(make_float2(e0, e1), make_float2(1.f, 1.f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d.x * d.y));
+    const float2 s = mul2(make_float2(r, r), make_float2(d.y, d.x));
+    s0 = s.x; s1 = s.y;
 }
 
 // A warp's [32 rows][32 fp32] block of an update into m by TMA reduce-add, through a staging tile of its own (STG_WARP bytes): no warp
@@ -277,7 +279,8 @@ msa_transition_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_
                     const float a0 = __uint_as_float(f1[2 * e]), a1 = __uint_as_float(f1[2 * e + 1]);
                     float s0, s1;
                     sigmoid_of(a0, a1, s0, s1);
-                    hw[e] = pack_bf16x2(a0 * s0 * __uint_as_float(f2[2 * e]), a1 * s1 * __uint_as_float(f2[2 * e + 1]));
+                    const float2 u = mul2(mul2(make_float2(a0, a1), make_float2(s0, s1)), make_float2(__uint_as_float(f2[2 * e]), __uint_as_float(f2[2 * e + 1])));
+                    hw[e] = pack_bf16x2(u.x, u.y);
                 }
                 tmem_st_32x16(tmem + lane_off + COL_H + buf * 32 + half * 16, hw);
                 tmem_st_wait();
@@ -610,7 +613,8 @@ pwa_output_kernel(const __grid_constant__ CUtensorMap map_wg, const __grid_const
                         for (int q = 0; q < 4; ++q) {
                             float s0, s1;
                             sigmoid_of(__uint_as_float(g[j * 8 + q * 2]), __uint_as_float(g[j * 8 + q * 2 + 1]), s0, s1);
-                            r[q] = pack_bf16x2(bf16_lo(w[q]) * s0, bf16_hi(w[q]) * s1);
+                            const float2 u = mul2(make_float2(bf16_lo(w[q]), bf16_hi(w[q])), make_float2(s0, s1));
+                            r[q] = pack_bf16x2(u.x, u.y);
                         }
                         *at = make_uint4(r[0], r[1], r[2], r[3]);
                     }

@@ -304,7 +304,12 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
                     float v[32];
                     if (EPI == EPI_STORE || EPI == EPI_CONTRACT || EPI == EPI_ADD || EPI == EPI_QKVG) {
 #pragma unroll
-                        for (int e = 0; e < 32; ++e) v[e] = (SMALL ? __uint_as_float(x[e]) + __uint_as_float(y[e]) : __uint_as_float(x[e])) * p.alpha[0];
+                        for (int e = 0; e < 32; e += 2) {
+                            float2 u = make_float2(__uint_as_float(x[e]), __uint_as_float(x[e + 1]));
+                            if (SMALL) u = add2(u, make_float2(__uint_as_float(y[e]), __uint_as_float(y[e + 1])));
+                            u = mul2(u, make_float2(p.alpha[0], p.alpha[0]));
+                            v[e] = u.x; v[e + 1] = u.y;
+                        }
                         if (p.bias) {
 #pragma unroll
                             for (int e = 0; e < 32; ++e) v[e] += col + e < p.n_rows ? *(p.bias + col + e) : 0.f;
@@ -316,7 +321,10 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_const
                             const float sc = p.qkv_scale[col < third ? 0 : col < 2 * third ? 1 : 2];
                             uint32_t w[2][16];
 #pragma unroll
-                            for (int e = 0; e < 16; ++e) split_f16x2(v[2 * e] * sc, v[2 * e + 1] * sc, w[0][e], w[1][e]);
+                            for (int e = 0; e < 16; ++e) {
+                                const float2 u = mul2(make_float2(v[2 * e], v[2 * e + 1]), make_float2(sc, sc));
+                                split_f16x2(u.x, u.y, w[0][e], w[1][e]);
+                            }
                             put_part(w[0], &map_o0, col, m0, bt, 0);
                             put_part(w[1], &map_o0, col, m0, bt, 1);
                         } else {

@@ -211,10 +211,10 @@ int launch_ln(const LnArgs& a, int c, int heads, cudaStream_t st) {
 // t[d][i][j] -> planes[(i, j)][d]: a block takes 32 positions of one row through shared memory ([D][33]: both the row-wise
 // fill and the column-wise reads are conflict free) and its warps normalise four positions each.
 template <int D>
-__global__ void __launch_bounds__(256) ln_channels_kernel(const float* t, long long plane_stride, int pitch, const float* gamma,
+__global__ void __launch_bounds__(256, D <= 256 ? 4 : 2) ln_channels_kernel(const float* t, long long plane_stride, int pitch, const float* gamma,
                                                           const float* beta, __half* planes, long long part_stride, int n) {
     extern __shared__ float ts[];
-    constexpr int E = D / 32;
+    constexpr int E = D / 64;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     grid_dependency_wait();
     grid_launch_dependents();
@@ -231,15 +231,25 @@ __global__ void __launch_bounds__(256) ln_channels_kernel(const float* t, long l
     }
     __syncthreads();
     // lane: channels 2 lane + 64 e, 2 lane + 1 + 64 e
-    float g[E], b[E];
+    float2 g[E], b[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) { const int c = 2 * lane + 64 * (e >> 1) + (e & 1); g[e] = *(gamma + c); b[e] = *(beta + c); }
-    float x[4][E], s[4], ss[4];
+    for (int e = 0; e < E; ++e) {
+        const int c = 2 * lane + 64 * e;
+        g[e] = make_float2(*(gamma + c), *(gamma + c + 1));
+        b[e] = make_float2(*(beta + c), *(beta + c + 1));
+    }
+    float2 x[4][E];
+    float s[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-        s[r] = 0.f;
+        float2 a = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int e = 0; e < E; ++e) { x[r][e] = ts[(2 * lane + 64 * (e >> 1) + (e & 1)) * 33 + warp * 4 + r]; s[r] += x[r][e]; }
+        for (int e = 0; e < E; ++e) {
+            const float* at = ts + (2 * lane + 64 * e) * 33 + warp * 4 + r;
+            x[r][e] = make_float2(at[0], at[33]);
+            a = add2(a, x[r][e]);
+        }
+        s[r] = a.x + a.y;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -248,26 +258,28 @@ __global__ void __launch_bounds__(256) ln_channels_kernel(const float* t, long l
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const float mean = s[r] * (1.f / D);
-        ss[r] = 0.f;
+        float2 a = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int e = 0; e < E; ++e) { x[r][e] -= mean; ss[r] = fmaf(x[r][e], x[r][e], ss[r]); }
+        for (int e = 0; e < E; ++e) { x[r][e] = add2(x[r][e], make_float2(-mean, -mean)); a = fma2(x[r][e], x[r][e], a); }
+        s[r] = a.x + a.y;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int r = 0; r < 4; ++r) ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], o);
+        for (int r = 0; r < 4; ++r) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int j = j0 + warp * 4 + r;
         if (j >= n) break;
-        const float rstd = rsqrtf(ss[r] * (1.f / D) + LN_EPS);
+        const float rstd = rsqrtf(s[r] * (1.f / D) + LN_EPS);
         __half* dst = planes + ((long long)i * n + j) * D + 2 * lane;
 #pragma unroll
-        for (int e = 0; e < E; e += 2) {
+        for (int e = 0; e < E; ++e) {
+            const float2 u = fma2(mul2(x[r][e], make_float2(rstd, rstd)), g[e], b[e]);
             uint32_t h, l;
-            split_f16x2(fmaf(x[r][e] * rstd, g[e], b[e]), fmaf(x[r][e + 1] * rstd, g[e + 1], b[e + 1]), h, l);
-            *reinterpret_cast<uint32_t*>(dst + 32 * e) = h;
-            *reinterpret_cast<uint32_t*>(dst + part_stride + 32 * e) = l;
+            split_f16x2(u.x, u.y, h, l);
+            *reinterpret_cast<uint32_t*>(dst + 64 * e) = h;
+            *reinterpret_cast<uint32_t*>(dst + part_stride + 64 * e) = l;
         }
     }
 }
