@@ -30,7 +30,7 @@
 // columns) at 1024 tokens, 47.8 -> 43.4 and 61.3 -> 60.2 at 400, the same at 203, where a CTA has three tiles; five are slower
 // everywhere (252 / 273 and 334 / 333), seven no faster (238 / 251 and 324 / 334) and spill in the MXFP8 form.
 // A pass's arithmetic goes two channels to an instruction: 43.7 / 46.4 -> 42.1 / 44.9 and 61.3 / 61.0 -> 58.8 / 59.2 at 400, the attention
-// producer 347 / 360 -> 329 / 328 at 1024, on one box; the gates' alike.
+// producer 347 / 360 -> 329 / 328 at 1024; the gates alike.
 #include "mxfp8.cuh"
 #include "row512_tc.h"
 #include "rowtc.cuh"
