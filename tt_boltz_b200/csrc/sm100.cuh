@@ -286,6 +286,11 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// Untiled bulk copy shared -> global (both addresses and the size multiples of 16 bytes), counted in the thread's bulk group.
+__device__ __forceinline__ void bulk_store_1d(void* dst, const void* smem_src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(smem_src)), "r"(bytes) : "memory");
+}
+
 // ---- block-scaled fp8 (MXFP8: e4m3 values, one e8m0 scale per 32 elements along K) --------------
 // Untiled bulk copy global -> shared (both addresses and the size multiples of 16 bytes).
 __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {

@@ -36,7 +36,7 @@ struct GemmShape {
     int x_cols;          // columns written (whole 8-column vectors below this bound)
     int x_col_group;     // > 0: output columns in groups of this many (a multiple of 32), x_colgroup_stride elements apart
     long long x_colgroup_stride;
-    int x_tma;           // the output leaves through map_x (see store_tile)
+    int x_tma;           // the output leaves through map_x (1), or as blocks of 32 x 32 (2; see store_tile)
 };
 // Output element (d, row, col) lives at (row / x_row_group) * x_group_stride + d * x_plane_stride + (row % x_row_group) * x_pitch + col.
 __device__ __forceinline__ long long x_row_offset(const GemmShape& s, int d, int row) {
@@ -47,14 +47,15 @@ __device__ __forceinline__ long long x_row_offset(const GemmShape& s, int d, int
 // One epilogue warp's 32 rows (from `row0`) x COLS columns of a finished accumulator.  Plain planes leave through SLOTS swizzled staging tiles in
 // turn and TMA stores of [32 rows][64 columns].  As 16-byte stores of a thread per row, 4096 partial sectors a tile, they took 11 k clocks a tile
 // against 3.6 k to 8.2 k of MMAs: 11.7 -> 9.7 us at 203 tokens, 43 -> 35 at 400, 112 -> 94 at 600, 238 -> 224 at 1024 (some 9 TB/s of
-// operands come out of L2 then).  Columns in groups (the outer product's blocks of contiguous 2 KB) and row groups that 32 does
-// not divide stay with the direct stores.
+// operands come out of L2 then).  The outer product's blocks of contiguous 2 KB go through the same tiles and bulk copies: 26.4 -> 20.9 us at
+// 122 sequences x 171 tokens, 50.9 -> 37.3 at 122 x 256, 50.1 -> 45.4 at 1024 x 171, 664 -> 533 at 1024 x 600.  Other columns
+// in groups and row groups that 32 does not divide stay with the direct stores.
 template <int COLS, int SLOTS>
 __device__ __forceinline__ void store_tile(const CUtensorMap* map_x, __nv_bfloat16* x, const GemmShape& s, uint32_t taddr, uint8_t* stg, uint32_t& slot, int d, int row0,
                                            int n0, int lane) {
     using namespace sm100;
     const int row = row0 + lane;
-    if (s.x_tma) {
+    if (s.x_tma == 1) {
         const int grp = row0 / s.x_row_group, row_in = row0 - grp * s.x_row_group;
 #pragma unroll 1
         for (int c = 0; c < COLS / 64; ++c) {
@@ -82,6 +83,39 @@ __device__ __forceinline__ void store_tile(const CUtensorMap* map_x, __nv_bfloat
             __syncwarp();
             if (lane == 0) {
                 tma_store_4d(map_x, tile, col, row_in, d, grp);
+                bulk_commit();
+            }
+        }
+        return;
+    }
+    if (s.x_tma == 2) {         // a warp's 32 rows are one group, 32 columns of them one contiguous block: two a staging tile, a bulk copy each
+#pragma unroll 1
+        for (int c = 0; c < COLS / 64; ++c) {
+            const int col = n0 + c * 64;
+            if (col >= s.x_cols || row0 >= s.m_rows) break;          // warp-uniform
+            uint32_t r[2][32];
+            tmem_ld_32x32(taddr + c * 64, r[0]);
+            tmem_ld_32x32(taddr + c * 64 + 32, r[1]);
+            tmem_ld_wait();
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(SLOTS - 1) : "memory");      // the copies that read this tile are through
+            __syncwarp();
+            uint8_t* tile = stg + slot * STG_BYTES;
+            slot ^= SLOTS - 1;
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(__uint_as_float(r[b][j * 8 + q * 2]), __uint_as_float(r[b][j * 8 + q * 2 + 1]));
+                    *reinterpret_cast<uint4*>(tile + b * 2048 + lane * 64 + j * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+                __nv_bfloat16* dst = x + x_row_offset(s, d, row0) + (long long)(col / 32) * s.x_colgroup_stride;
+                bulk_store_1d(dst, tile, 2048);
+                if (col + 32 < s.x_cols) bulk_store_1d(dst + s.x_colgroup_stride, tile + 2048, 2048);
                 bulk_commit();
             }
         }
@@ -436,8 +470,9 @@ static int launch_contract_tc(const b200pf_planes* a, const b200pf_planes* b, b2
     GemmShape s = shape;
     const int groups = s.m_rows > s.x_row_group ? s.m_rows / s.x_row_group : 1;
     s.x_tma = s.x_col_group == 0 && (groups == 1 ? s.m_rows <= s.x_row_group : s.m_rows % s.x_row_group == 0 && s.x_row_group % 32 == 0);
+    if (s.x_col_group == 32 && s.x_pitch == 32 && s.x_row_group == 32 && s.m_rows % 32 == 0 && s.n_rows % 32 == 0) s.x_tma = 2;
     map_x = map_a;
-    if (s.x_tma) {
+    if (s.x_tma == 1) {
         const int rows = s.m_rows < s.x_row_group ? s.m_rows : s.x_row_group;
         const long long plane = s.channels > 1 ? s.x_plane_stride : (long long)rows * s.x_pitch;      // stride of an extent of 1: anything valid
         cuuint64_t dims[4] = {(cuuint64_t)s.x_cols, (cuuint64_t)rows, (cuuint64_t)s.channels, (cuuint64_t)groups};
