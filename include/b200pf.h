@@ -382,9 +382,12 @@ int b200pf_pwa_output(float* m, const float* ln_gamma, const float* ln_beta, con
                       const b200pf_bf16* o, int s_len, int n, int np, void* stream);
 /* The MSA embedding (MSAModule.forward, tt_bio/reference.py:1252-1276): m[s][i][:] = w [one_hot(msa[s][i]) | has_deletion | deletion_value |
  * paired] + e[i][:].  w [64][36], or [64][35] with paired null; e [n][64] the projected single representation.  A residue outside 0 .. 32
- * counts as none and raises the device status word. */
+ * makes its row NaN and raises the device status word; _checked writes 1 to *bad instead (device memory, or pinned host memory mapped into
+ * the device; read it behind the launch's completion) where bad is not null. */
 int b200pf_msa_embed(const long long* msa, const float* has_deletion, const float* deletion_value, const float* paired, const float* w,
                      const float* e, float* m, int s_len, int n, void* stream);
+int b200pf_msa_embed_checked(const long long* msa, const float* has_deletion, const float* deletion_value, const float* paired, const float* w,
+                             const float* e, float* m, int s_len, int n, unsigned int* bad, void* stream);
 
 /* All-to-all of equal blocks over peer mappings (multi-GPU path, no counterpart in the reference, whose
  * cards do not exchange data: tt_bio/distributed.py fans whole jobs out).  Block t of `send` (world blocks

@@ -1,7 +1,7 @@
 """The MSA embedding in one kernel against one-hot, concatenation and linear in 64 bits, with and without the paired feature: one row, rows
 that do not fill a block, more than a lane takes at once.  The projected single representation comes from the linear kernel as it does in the
-module; on top of it are four rounded additions, each half an ulp of at most the sum of the terms' sizes: 2^-22 of that.  A residue
-outside the classes counts as none and is reported; features of another shape or type are refused."""
+module; on top of it are four rounded additions, each half an ulp of at most the sum of the terms' sizes: 2^-22 of that.  A residue outside the classes makes its
+row NaN and is reported, and a call of the module with one raises; features of another shape or type are refused."""
 import pytest
 import torch
 
@@ -51,3 +51,35 @@ def test_what_is_refused():
         with pytest.raises(RuntimeError):
             mod.embed(emb[:, :5], feats)
     assert _lib.device_status() == 0
+
+
+def module_case(residue):
+    mod, emb, feats = case(5, 9, True)
+    with torch.no_grad():
+        for p in mod.layers.parameters():
+            p.normal_(0.0, 0.05) if p.dim() == 2 else p.fill_(1.0)
+    feats.update({"msa_mask": torch.ones(1, 5, 9, device="cuda"), "token_pad_mask": torch.ones(1, 9, device="cuda")})
+    bad = {**feats, "msa": feats["msa"].clone()}
+    bad["msa"][0, 4, 8] = residue
+    return mod, (torch.randn(1, 9, 9, 128, device="cuda"), emb), feats, bad
+
+
+@pytest.mark.parametrize("residue", [-1, 33, 1 << 40])
+def test_a_call_with_a_bad_residue_raises(residue):
+    mod, args, feats, bad = module_case(residue)
+    good = mod(*args, feats)
+    with pytest.raises(RuntimeError, match="residues"):
+        mod(*args, bad)
+    assert torch.equal(mod(*args, feats), good)                      # nothing is left behind
+    assert bool(torch.isfinite(good).all()) and _lib.device_status() == 0
+
+
+def test_a_captured_call_with_a_bad_residue_is_no_number():
+    mod, args, feats, bad = module_case(33)
+    mod(*args, feats)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        z = mod(*args, bad)
+    graph.replay()
+    assert _lib.device_status() == 2
+    assert bool(torch.isnan(z).all())

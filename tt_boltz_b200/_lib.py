@@ -134,6 +134,7 @@ SIGNATURES = {
     "b200pf_msa_swiglu": [_vp, _vp, _ll, _vp],
     "b200pf_msa_add_rows": [_vp, _vp, _i, _i, _i, _vp],
     "b200pf_msa_embed": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp],
+    "b200pf_msa_embed_checked": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp, _vp],
     "b200pf_msa_transition": [_vp, _vp, _vp, _vp, _vp, _ll, _vp],
     "b200pf_pwa_value": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp],
     "b200pf_pwa_output": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp],

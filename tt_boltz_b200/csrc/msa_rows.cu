@@ -5,6 +5,8 @@
 // Every GEMM operand is bf16 and K-major; the token axis is padded to a multiple of 8 (`np`) so that rows of
 // every operand start 16-byte aligned, with zero rows for the padding tokens (the pair-weighted averaging pads to
 // 32: its projected rows are written in groups of np columns).
+#include <math_constants.h>
+
 #include "pdl.cuh"
 
 namespace b200pf {
@@ -148,17 +150,19 @@ add_rows_kernel(float* __restrict__ m, const __nv_bfloat16* __restrict__ t, int 
 // per feature, W transposed in shared memory.  A warp takes 32 rows at a time: a lane fetches one row's residue and features, then sixteen
 // lanes write a row, four channels each.  Bound by the 256 bytes a row that it writes: 37 us at 1024 x 600 (65 with every lane fetching the
 // features of the rows it writes), where one-hot, conversion, concatenation, linear and addition took some 380 in eight launches.
+// A residue outside the classes has no column: its row is NaN, so that no result passes for one of a sound alignment, and it is reported, in
+// the word that the caller gave or, without one, in the device status word.
 constexpr int RES = 33;
 __global__ void __launch_bounds__(256)
 msa_embed_kernel(const long long* msa, const float* has_del, const float* del_value, const float* paired, const float* w, const float* e, float* m,
-                 uint32_t rows, uint32_t n, unsigned int* status) {
-    __shared__ float4 wt[(RES + 4) * 16];                             // the last row: zeros, what a residue outside the classes counts as
+                 uint32_t rows, uint32_t n, unsigned int* status, volatile unsigned int* bad) {
+    __shared__ float4 wt[(RES + 4) * 16];                             // the last row: NaN, for a residue outside the classes
     const int k_in = RES + 2 + (paired ? 1 : 0), lane = threadIdx.x & 31, c4 = lane & 15;
     grid_dependency_wait();
     grid_launch_dependents();
     for (int i = threadIdx.x; i < (RES + 4) * CM; i += blockDim.x) {
         const int k = i / CM, c = i % CM;
-        reinterpret_cast<float*>(wt)[i] = k < k_in ? w[c * k_in + k] : 0.f;
+        reinterpret_cast<float*>(wt)[i] = k < k_in ? w[c * k_in + k] : k == RES + 3 ? CUDART_NAN_F : 0.f;
     }
     __syncthreads();
     float4 q[3];
@@ -171,7 +175,10 @@ msa_embed_kernel(const long long* msa, const float* has_del, const float* del_va
         const float f0 = has_del[mine], f1 = del_value[mine], f2 = paired ? paired[mine] : 0.f;
         const uint32_t token = mine % n;
         const bool known = r >= 0 && r < RES;
-        if (!known) atomicOr(status, DEV_STATUS_BAD_INDEX);
+        if (!known) {
+            if (bad) *bad = 1u;
+            else atomicOr(status, DEV_STATUS_BAD_INDEX);
+        }
         const int residue = known ? (int)r : RES + 3;
 #pragma unroll 8
         for (int i = 0; i < 32; i += 2) {
@@ -249,8 +256,8 @@ extern "C" int b200pf_msa_add_rows(float* m, const b200pf_bf16* t, int s_len, in
     return B200PF_OK;
 }
 
-extern "C" int b200pf_msa_embed(const long long* msa, const float* has_deletion, const float* deletion_value, const float* paired, const float* w,
-                                const float* e, float* m, int s_len, int n, void* stream) {
+extern "C" int b200pf_msa_embed_checked(const long long* msa, const float* has_deletion, const float* deletion_value, const float* paired, const float* w,
+                                        const float* e, float* m, int s_len, int n, unsigned int* bad, void* stream) {
     B200PF_REQUIRE(msa && has_deletion && deletion_value && w && e && m && aligned16(e) && aligned16(m) && s_len > 0 && n > 0, B200PF_ERR_INVALID,
                    "msa_embed: bad arguments");
     unsigned int* status = device_status_word();
@@ -258,5 +265,10 @@ extern "C" int b200pf_msa_embed(const long long* msa, const float* has_deletion,
     const long long rows = (long long)s_len * n;
     B200PF_REQUIRE(rows < (1LL << 30), B200PF_ERR_UNSUPPORTED, "msa_embed: too many rows");       // 2^30 rows of m are 256 GiB
     return launch_pdl(msa::msa_embed_kernel, dim3(msa::grid_for(rows, 256)), dim3(256), 0, (cudaStream_t)stream, msa, has_deletion,
-                      deletion_value, paired, w, e, m, (uint32_t)rows, (uint32_t)n, status);
+                      deletion_value, paired, w, e, m, (uint32_t)rows, (uint32_t)n, status, bad);
+}
+
+extern "C" int b200pf_msa_embed(const long long* msa, const float* has_deletion, const float* deletion_value, const float* paired, const float* w,
+                                const float* e, float* m, int s_len, int n, void* stream) {
+    return b200pf_msa_embed_checked(msa, has_deletion, deletion_value, paired, w, e, m, s_len, n, nullptr, stream);
 }

@@ -389,8 +389,9 @@ class B200MSAModule(nn.Module):
     tt_bio/tenstorrent.py:2524-2621): the MSA features are embedded (``msa_proj`` of the one-hot residues, deletion and
     pairing features, plus ``s_proj`` of the single representation for every sequence) and ``msa_blocks`` MSA layers
     run on resident tensors; ``forward(z, emb, feats, use_kernels=False)`` returns the pair tensor after the last
-    block, which the trunk adds to z (tt_bio/boltz2.py:5230).  A residue outside the 33 classes counts as none and raises the
-    device status word (``_lib.device_status``)."""
+    block, which the trunk adds to z (tt_bio/boltz2.py:5230).  A residue outside the 33 classes is an error: ``forward``
+    raises.  Where nothing can be read back, in ``embed`` by itself and in a captured call, the residue's row is NaN and the device
+    status word is raised (``_lib.device_status``)."""
 
     def __init__(self, msa_s: int = C_M, token_z: int = 128, token_s: int = 384, msa_blocks: int = 4, msa_dropout: float = 0.0,
                  z_dropout: float = 0.0, pairwise_head_width: int = 32, pairwise_num_heads: int = 4,
@@ -404,8 +405,9 @@ class B200MSAModule(nn.Module):
         self.layers = nn.ModuleList(B200MSALayer(msa_s, token_z, msa_dropout, z_dropout, pairwise_head_width,
                                                  pairwise_num_heads, precision) for _ in range(msa_blocks))
 
-    def embed(self, emb: torch.Tensor, feats) -> torch.Tensor:
-        """m [S, N, 64] fp32 from the single representation emb [1, N, token_s] and the MSA features (reference.py:1252-1276)."""
+    def embed(self, emb: torch.Tensor, feats, bad: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """m [S, N, 64] fp32 from the single representation emb [1, N, token_s] and the MSA features (reference.py:1252-1276); ``bad``, one
+        pinned int32, becomes 1 if a residue lies outside the classes."""
         from . import ops
         msa = feats["msa"][0]
         if msa.dtype != torch.int64:
@@ -421,8 +423,8 @@ class B200MSAModule(nn.Module):
             raise RuntimeError(f"emb has {e.shape[0]} tokens, the MSA {n}")
         m = torch.empty(s_len, n, C_M, **f32)
         msa, w = msa.contiguous(), self.msa_proj.weight.detach().to(**f32).contiguous()
-        call("b200pf_msa_embed", ptr(msa), ptr(parts[0]), ptr(parts[1]), ptr(parts[2]) if self.use_paired_feature else None, ptr(w), ptr(e), ptr(m),
-             s_len, n, stream())
+        call("b200pf_msa_embed_checked", ptr(msa), ptr(parts[0]), ptr(parts[1]), ptr(parts[2]) if self.use_paired_feature else None, ptr(w), ptr(e),
+             ptr(m), s_len, n, None if bad is None else bad.data_ptr(), stream())
         return m
 
     def forward(self, z: torch.Tensor, emb: torch.Tensor, feats, use_kernels: bool = False) -> torch.Tensor:
@@ -438,7 +440,20 @@ class B200MSAModule(nn.Module):
                 msa_mask = msa_mask[idx]
             tok = feats["token_pad_mask"][0].float()
             token_mask = tok[:, None] * tok[None, :]
-            m = self.embed(emb, feats)
-            zw = z[0].to(torch.float32).clone(memory_format=torch.contiguous_format)
-            _run_blocks(self.layers, zw, m, token_mask, msa_mask)
+            # The residues are checked where they are embedded.  The answer is waited for behind the launches of all blocks, which run
+            # meanwhile: the GPU has their work in hand when the caller goes on.
+            capturing = torch.cuda.is_current_stream_capturing()
+            bad = None if capturing else torch.zeros(1, dtype=torch.int32, pin_memory=True)
+            embedded = None if capturing else torch.cuda.Event()
+            m = self.embed(emb, feats, bad)
+            if not capturing:
+                embedded.record()
+            try:
+                zw = z[0].to(torch.float32).clone(memory_format=torch.contiguous_format)
+                _run_blocks(self.layers, zw, m, token_mask, msa_mask)
+            finally:
+                if not capturing:
+                    embedded.synchronize()                                  # nothing writes to ``bad`` any more
+            if not capturing and bad.item():
+                raise RuntimeError(f"the MSA holds residues outside 0 .. {NUM_TOKENS - 1}")
         return zw[None]
