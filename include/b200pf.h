@@ -380,6 +380,9 @@ int b200pf_pwa_value(const float* m, const float* ln_gamma, const float* ln_beta
 /* m[s][tok] += proj_o (sigmoid(proj_g LN m[s][tok]) * o[:][s][:][tok]); w_g = proj_g [256][64], w_o = proj_o [64][256]. */
 int b200pf_pwa_output(float* m, const float* ln_gamma, const float* ln_beta, const b200pf_bf16* w_g, const b200pf_bf16* w_o,
                       const b200pf_bf16* o, int s_len, int n, int np, void* stream);
+/* m[s][i][:] += e[i][:] (fp32 rows of 64): the projected single representation added to every sequence's embedding
+ * (MSAModule.forward, tt_bio/reference.py:1275-1276), for programs that embed the residues themselves. */
+int b200pf_msa_add_token_rows(float* m, const float* e, int s_len, int n, void* stream);
 /* The MSA embedding (MSAModule.forward, tt_bio/reference.py:1252-1276): m[s][i][:] = w [one_hot(msa[s][i]) | has_deletion | deletion_value |
  * paired] + e[i][:].  w [64][36], or [64][35] with paired null; e [n][64] the projected single representation.  A residue outside 0 .. 32
  * makes its row NaN and raises the device status word; _checked writes 1 to *bad instead (device memory, or pinned host memory mapped into

@@ -50,6 +50,7 @@ def test_msa_entry_points_validate_before_any_cuda_call():
         ("b200pf_pwa_gate_transpose", (None, None, None, 8, 8, None), "null or misaligned"),
         ("b200pf_msa_swiglu", (None, None, 8, None), "bad arguments"),
         ("b200pf_msa_add_rows", (None, None, 8, 8, 8, None), "bad arguments"),
+        ("b200pf_msa_add_token_rows", (None, None, 8, 8, None), "bad arguments"),
     ]
     for name, args, text in cases:
         rc = getattr(lib, name)(*args)

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from tt_boltz_b200 import B200MSAModule, _lib, ops
+from tt_boltz_b200._lib import call, ptr, stream
 
 pytestmark = pytest.mark.gpu
 
@@ -83,3 +84,13 @@ def test_a_captured_call_with_a_bad_residue_is_no_number():
     graph.replay()
     assert _lib.device_status() == 2
     assert bool(torch.isnan(z).all())
+
+
+@pytest.mark.parametrize("s, n", [(1, 1), (3, 5), (33, 130), (600, 301)])
+def test_token_rows(s, n):
+    """One rounded addition a value: torch's."""
+    torch.manual_seed(n)
+    m, e = torch.randn(s + 1, n, 64, device="cuda"), torch.randn(n, 64, device="cuda")
+    want = torch.cat([m[:s] + e, m[s:]])
+    call("b200pf_msa_add_token_rows", ptr(m), ptr(e), s, n, stream())
+    assert torch.equal(m, want)
