@@ -416,6 +416,8 @@ class B200MSAModule(nn.Module):
         parts = [feats[k][0].float().contiguous() for k in names]
         if msa.dim() != 2 or any(t.shape != msa.shape for t in parts):
             raise RuntimeError(f"the MSA's features must have its residues' shape {tuple(msa.shape)}, got {[tuple(t.shape) for t in parts]}")
+        if any(t.device != msa.device for t in (*parts, emb)):
+            raise RuntimeError(f"the MSA's residues are on {msa.device}, its features and emb on {sorted({str(t.device) for t in (*parts, emb)})}")
         s_len, n = msa.shape
         f32 = dict(device=msa.device, dtype=torch.float32)
         e = ops.f32_linear(emb[0].to(torch.float32).contiguous(), self.s_proj.weight.detach().to(**f32).contiguous())
