@@ -15,11 +15,39 @@ pytestmark = pytest.mark.gpu
 HEADS, HD = 16, 24
 
 
+def reference(sd, s, bias, mask):
+    n = s.shape[0]
+    x = torch.nn.functional.layer_norm(s.double(), (HEADS * HD,), sd["pre_norm_s.weight"].double(), sd["pre_norm_s.bias"].double(), 1e-5)
+    proj = lambda name, b=None: (x @ sd[f"attention.{name}.weight"].double().T + (0 if b is None else sd[b].double())).view(n, HEADS, HD).transpose(0, 1)
+    q, k, v, gate = proj("proj_q", "attention.proj_q.bias"), proj("proj_k"), proj("proj_v"), torch.sigmoid(proj("proj_g"))
+    logits = q @ k.transpose(1, 2) / HD ** 0.5 + bias.double().view(HEADS, n, n) / 1.4426950408889634 + (mask.double() - 1) * 1e6
+    return ((logits.softmax(-1) @ v) * gate).transpose(0, 1).reshape(n, HEADS * HD), ((q.abs() @ k.abs().transpose(1, 2)) / HD ** 0.5).square().mean().sqrt()
+
+
+def layer0(seed):
+    return {k[len("layers.0."):]: v for k, v in synthetic.make_weights(1, seed=seed, std=0.1, affine_jitter=0.2, with_s=True).items() if k.startswith("layers.0.")}
+
+
+@pytest.mark.parametrize("n, out", [(200, (64, 128)), (200, (0, 64)), (200, (1, 200)), (200, (0, 192)), (129, (0, 128)), (509, (64, 320)), (1025, (64, 1024))])
+def test_keys_excluded_by_the_bias(n, out):
+    """A bias of -inf at whole tiles of keys, a whole key group's among them, and at all keys but one: the others' softmax."""
+    dev, sd = torch.device("cuda:0"), layer0(n)
+    track = ops.pack_single_track(sd, "", HEADS, dev)
+    g = torch.Generator().manual_seed(n)
+    s, bias, mask = torch.randn(n, HEADS * HD, generator=g), torch.randn(HEADS, n, n, generator=g), torch.ones(n, dtype=torch.uint8)
+    bias[:, :, out[0]:out[1]] = -float("inf")
+    got = track.attention(s.to(dev), bias.view(HEADS, n * n).to(dev), mask.to(dev), 0, n, ops.Scratch(dev)).double().sum(0).cpu() / track.pack.struct.o_scale
+    assert _lib.device_status() == 0
+    want, size = reference(sd, s, bias, mask)
+    err = (got - want).norm() / want.norm()
+    assert err < 2.0 ** -19 + 2.0 ** -20 * size, (err, size)
+
+
 @pytest.mark.parametrize("n, dead", [(129, None), (192, (64, 128)), (193, None), (257, (0, 192)), (320, None), (509, (64, 509)), (512, (0, 511)),
                                      (1023, None), (1024, (128, 1000)), (1025, None)])
 def test_against_64_bits(n, dead):
     dev = torch.device("cuda:0")
-    sd = {k[len("layers.0."):]: v for k, v in synthetic.make_weights(1, seed=n, std=0.1, affine_jitter=0.2, with_s=True).items() if k.startswith("layers.0.")}
+    sd = layer0(n)
     track = ops.pack_single_track(sd, "", HEADS, dev)
     g = torch.Generator().manual_seed(n)
     s = torch.randn(n, HEADS * HD, generator=g)
@@ -35,14 +63,8 @@ def test_against_64_bits(n, dead):
         assert torch.equal(part, out[:, r0:r1])
     torch.cuda.synchronize()
     assert _lib.device_status() == 0
-    # the reference, with a probe of the output's scale: the planes hold the gated output times a power of two
-    x = torch.nn.functional.layer_norm(s.double(), (HEADS * HD,), sd["pre_norm_s.weight"].double(), sd["pre_norm_s.bias"].double(), 1e-5)
-    proj = lambda name, b=None: (x @ sd[f"attention.{name}.weight"].double().T + (0 if b is None else sd[b].double())).view(n, HEADS, HD).transpose(0, 1)
-    q, k, v, gate = proj("proj_q", "attention.proj_q.bias"), proj("proj_k"), proj("proj_v"), torch.sigmoid(proj("proj_g"))
-    logits = q @ k.transpose(1, 2) / HD ** 0.5 + bias.double().view(HEADS, n, n) / 1.4426950408889634 + (mask.double() - 1) * 1e6
-    want = ((logits.softmax(-1) @ v) * gate).transpose(0, 1).reshape(n, HEADS * HD)
+    want, size = reference(sd, s, bias, mask)
     got = (out[0].double() + out[1].double()).cpu()
     scale = 2.0 ** torch.round(torch.log2(got.norm() / want.norm()))
     err = (got / scale - want).norm() / want.norm()
-    size = ((q.abs() @ k.abs().transpose(1, 2)) / HD ** 0.5).square().mean().sqrt()
     assert err < 2.0 ** -19 + 2.0 ** -20 * size, (err, size)

@@ -70,6 +70,9 @@ __device__ __forceinline__ float prob(float x) {
     return y;
 }
 
+// The reference of a row that has met no key with a finite score: above that of any other, and so far that two to the difference is 0.
+constexpr float NO_KEYS = 3e38f;
+
 // Shared memory of a key group: its K / V, bias and mask tiles
 constexpr int group_bytes(int nw) { return 2 * (KV_STAGE + bias_stage(nw) + KT * 4); }
 
@@ -231,9 +234,10 @@ __global__ void __launch_bounds__(KS * NW * 32, KS > 1 ? 1 : 16 / NW) split_atte
             }
             mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
             mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-            // every tile holds a key inside n_k, whose score is finite: the new maxima are finite
+            // The maximum of keys that the bias excludes (-inf) is -inf; a finite reference gives each of them, and whatever they are
+            // joined with later, a zero.  A key group may have no other keys than such ones.
             mq0 = mx0; mq1 = mx1;
-            const float d0 = -mx0 * qk_inv, d1 = -mx1 * qk_inv;
+            const float d0 = fminf(-mx0 * qk_inv, NO_KEYS), d1 = fminf(-mx1 * qk_inv, NO_KEYS);
             const float a0 = exp2f(d0 - c0), a1 = exp2f(d1 - c1);                // 0 on the first tile
             c0 = d0; c1 = d1;
             const uint64_t c02 = f2(d0, d0), c12 = f2(d1, d1), a02 = f2(a0, a0), a12 = f2(a1, a1);
