@@ -6,7 +6,7 @@
 // swizzle), one warp issues the MMAs against weights that stay in shared memory, eight epilogue warps read tensor memory, and
 // m is updated by TMA reduce-add, so neither a projection nor a hidden layer goes through memory.
 // What bounds them is memory and, for the transition and the output, the special-function results per gate value: at 1024 sequences x 600
-// tokens the transition takes 130 us, the value kernel 106 us, the output kernel 127 us.  As LayerNorm, GEMM,
+// tokens the transition takes 142 us, the value kernel 106 us, the output kernel 138 us.  As LayerNorm, GEMM,
 // activation, transposition and add kernels of their own the same work took about 500 and 680 us and moved 4 to 5 times as much.
 #include "rowtc.cuh"
 
@@ -120,20 +120,20 @@ __device__ __forceinline__ bool load_loop(const LnRows& p, uint8_t* x0, uint64_t
     return true;
 }
 
-// 1 / (1 + e^-x) of two values by one reciprocal, three special-function results for four: the transition 143 -> 130 us and the output 149 ->
-// 127 at 1024 x 600, the transition 46.6 -> 42.9 at 1024 x 171.  The denominators stay at 2^62 + 1, so that their product is finite: a gate below
-// -43 counts as 2^-62, where that of +43 is 1.
-__device__ __forceinline__ void sigmoid_of(float x0, float x1, float& s0, float& s1) {
-    float e0, e1, r;
-    const float2 t = mul2(make_float2(x0, x1), make_float2(-1.44269504f, -1.44269504f));
-    asm("min.NaN.f32 %0, %1, %2;" : "=f"(e0) : "f"(t.x), "f"(62.f));
-    asm("min.NaN.f32 %0, %1, %2;" : "=f"(e1) : "f"(t.y), "f"(62.f));
-    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e0));
-    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e1));
-    const float2 d = add2(make_float2(e0, e1), make_float2(1.f, 1.f));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d.x * d.y));
-    const float2 s = mul2(make_float2(r, r), make_float2(d.y, d.x));
-    s0 = s.x; s1 = s.y;
+// 1 / (1 + e^-x) of two values, each by itself (the packed instructions round either half alone; 0 where the exponential overflows).  One
+// reciprocal of the denominators' product is three special-function results for four and takes the transition from 142 to 130 us and the
+// output from 138 to 125 at 1024 x 600, but two more roundings a gate (rms error 0.99 for 0.79 units of 2^-24 at arguments around one), and in
+// the output, where the two are neighbouring tokens, either's bits hang on the other, and a NaN of one is both's.  With a correction of
+// the two by their own residuals (0.76) the transition takes 143.
+__device__ __forceinline__ float2 sigmoids(float2 x) {
+    const float2 t = mul2(x, make_float2(-1.44269504f, -1.44269504f));
+    float2 e, s;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(t.x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(t.y));
+    const float2 d = add2(e, make_float2(1.f, 1.f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s.x) : "f"(d.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s.y) : "f"(d.y));
+    return s;
 }
 
 // A warp's [32 rows][32 fp32] block of an update into m by TMA reduce-add, through a staging tile of its own (STG_WARP bytes): no warp
@@ -277,9 +277,7 @@ msa_transition_kernel(const __grid_constant__ CUtensorMap map_w12, const __grid_
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
                     const float a0 = __uint_as_float(f1[2 * e]), a1 = __uint_as_float(f1[2 * e + 1]);
-                    float s0, s1;
-                    sigmoid_of(a0, a1, s0, s1);
-                    const float2 u = mul2(mul2(make_float2(a0, a1), make_float2(s0, s1)), make_float2(__uint_as_float(f2[2 * e]), __uint_as_float(f2[2 * e + 1])));
+                    const float2 u = mul2(mul2(make_float2(a0, a1), sigmoids(make_float2(a0, a1))), make_float2(__uint_as_float(f2[2 * e]), __uint_as_float(f2[2 * e + 1])));
                     hw[e] = pack_bf16x2(u.x, u.y);
                 }
                 tmem_st_32x16(tmem + lane_off + COL_H + buf * 32 + half * 16, hw);
@@ -611,9 +609,8 @@ pwa_output_kernel(const __grid_constant__ CUtensorMap map_wg, const __grid_const
                         uint32_t r[4];
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
-                            float s0, s1;
-                            sigmoid_of(__uint_as_float(g[j * 8 + q * 2]), __uint_as_float(g[j * 8 + q * 2 + 1]), s0, s1);
-                            const float2 u = mul2(make_float2(bf16_lo(w[q]), bf16_hi(w[q])), make_float2(s0, s1));
+                            const float2 gate = sigmoids(make_float2(__uint_as_float(g[j * 8 + q * 2]), __uint_as_float(g[j * 8 + q * 2 + 1])));
+                            const float2 u = mul2(make_float2(bf16_lo(w[q]), bf16_hi(w[q])), gate);
                             r[q] = pack_bf16x2(u.x, u.y);
                         }
                         *at = make_uint4(r[0], r[1], r[2], r[3]);
