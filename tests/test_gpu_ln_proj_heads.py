@@ -11,8 +11,9 @@ from tt_boltz_b200.ops import ptr, stream
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows", [1, 15, 17, 127, 129, 148 * 2 * 128 + 5, 148 * 2 * 128 * 3 - 1])
-def test_against_64_bits(rows):
+@pytest.mark.parametrize("passes, rest", [(0, 1), (0, 15), (0, 17), (0, 127), (0, 129), (1, 5), (3, -1)])
+def test_against_64_bits(passes, rest):
+    rows = passes * torch.cuda.get_device_properties(0).multi_processor_count * 2 * 128 + rest      # two blocks of 128 rows a multiprocessor
     torch.manual_seed(rows)
     dev = "cuda:0"
     z = torch.randn(rows, 128, device=dev) * 3 + torch.randn(rows, 1, device=dev)
