@@ -356,7 +356,9 @@ template <int HD, int NW, int KS> static int attn_go(const AttnArgs& a, cudaStre
 // three (an SM's shared memory holds their tiles): 33.6 -> 19.8 us at 509 tokens x 16 heads, 26.7 -> 17.1 at 400, 22.2 -> 14.5 at 300, 17.6 ->
 // 13.0 at 203, 60.8 -> 52 at 1024; beside the pair track, whose kernels wait for the SMs that it holds, a block takes 1303 -> 1289, 518 -> 509 at 300
 // and 261 -> 258.5 at 203.  Two groups: 20.7, 17.4, 14.4 and 12.9; four with a stage each: 19.6, 17.7, 15.8 and 13.6.  Two tiles of
-// keys aren't worth it (130 -> 133 a block at 117).  The choice looks at the keys only: a range of the queries has the bits of all of them.
+// keys aren't worth it (130 -> 133 a block at 117).  1024 keys stay below where 16 heads need a third round of such CTAs, one per SM: 77 -> 67
+// at 1025 and 73 -> 65 at 1100, where two rounds still do, would gain too, but 1300, 1500 and 2048 lose (85 -> 97, 96 -> 110, 149 -> 170).
+// The choice looks at the keys only: a range of the queries has the bits of all of them.
 template <int HD> static int attn_pick(const AttnArgs& a, int sms, cudaStream_t st) {
     if (a.lines == 1 && a.n_k > 2 * KT && a.n_k <= 1024) return attn_go<HD, 4, 3>(a, st);
     // eight warps share a K / V tile; with fewer than two such CTAs per SM, four warps per CTA spread the queries further

@@ -454,8 +454,8 @@ static int launch_tiles(const Gemm& g, int bn, int sms, cudaStream_t st) {
 }
 
 // CTA pairs where there is a tile for every CTA, more than one k-block (which would gain nothing) and pairing leaves few rows empty (an odd
-// number of 128-row tiles wastes one): a k-block
-// then brings 64 KB for 96 (256 columns), 48 for 64 (128) or 80 for 96 (two A tiles) into each SM per 256 x `bn` outputs, and some 9 TB/s out of
+// number of 128-row tiles wastes one; with the contraction's at 3, 331 tokens x 256 channels, the triangle multiplication takes 432 -> 448 us,
+// at 9, 1100 x 64 and x 128, 1361 -> 1287 and 2836 -> 2664; between them, 5 and 7, pairs would gain 2 to 3 %): a k-block then brings 64 KB for 96 (256 columns), 48 for 64 (128) or 80 for 96 (two A tiles) into each SM per 256 x `bn` outputs, and some 9 TB/s out of
 // L2 are what bounds these GEMMs otherwise.  At 331 tokens x 256 channels: transition 274 -> 220 us (tensor pipe 92 %) and 153 -> 140, output
 // gate 94 -> 86, operand planes 176 -> 175 (their epilogue, 35 us, and L2); contraction at 256 tokens 49 -> 43; odd ones (331) stay.  Two 256-wide blocks
 // run 1.04 (110 tokens) to 1.10 times (200) as fast, four attention-free ones 1.03 to 1.14, 64 channels 1.00 to 1.01.  K-blocks of 32, with more stages, are
