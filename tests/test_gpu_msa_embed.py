@@ -2,6 +2,8 @@
 that do not fill a block, more than a lane takes at once.  The projected single representation comes from the linear kernel as it does in the
 module; on top of it are four rounded additions, each half an ulp of at most the sum of the terms' sizes: 2^-22 of that.  A residue outside the classes makes its
 row NaN and is reported, and a call of the module with one raises; features of another shape or type are refused."""
+import threading
+
 import pytest
 import torch
 
@@ -94,3 +96,30 @@ def test_token_rows(s, n):
     want = torch.cat([m[:s] + e, m[s:]])
     call("b200pf_msa_add_token_rows", ptr(m), ptr(e), s, n, stream())
     assert torch.equal(m, want)
+
+
+def test_a_call_beside_another_threads_capture():
+    """The wait for the embedding's answer is no obstacle to a capture that another thread has under way, nor that to it."""
+    mod, args, feats, _ = module_case(0)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        want = [mod(*args, feats) for _ in range(3)][-1]
+    torch.cuda.synchronize()
+    got, x = [], torch.ones(8, device="cuda")
+
+    def work():
+        try:
+            with torch.cuda.stream(side):
+                got.append(mod(*args, feats))
+        except RuntimeError as e:
+            got.append(e)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="global"):
+        y = x + 1
+        thread = threading.Thread(target=work)
+        thread.start()
+        thread.join()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert isinstance(got[0], torch.Tensor), got[0]
+    assert torch.equal(got[0], want) and bool((y == 2).all())

@@ -22,7 +22,7 @@ import torch
 from torch import nn
 
 from . import ops, weights
-from ._lib import Planes, call, ptr, stream
+from ._lib import Planes, call, ptr, relaxed_capture, stream
 
 C_M, C_HID, C_OUT = 64, 32, 128
 OUTER_BLOCK_BYTES = 1 << 30         # outer products of one block of tokens (2 KB per pair)
@@ -443,19 +443,23 @@ class B200MSAModule(nn.Module):
             tok = feats["token_pad_mask"][0].float()
             token_mask = tok[:, None] * tok[None, :]
             # The residues are checked where they are embedded.  The answer is waited for behind the launches of all blocks, which run
-            # meanwhile: the GPU has their work in hand when the caller goes on.
-            capturing = torch.cuda.is_current_stream_capturing()
-            bad = None if capturing else torch.zeros(1, dtype=torch.int32, pin_memory=True)
-            embedded = None if capturing else torch.cuda.Event()
+            # meanwhile: the GPU has their work in hand when the caller goes on.  Pinned memory and the wait would break a capture that
+            # another thread has under way, if this thread's own mode forbade them.
+            check = not torch.cuda.is_current_stream_capturing()
+            bad = embedded = None
+            if check:
+                with relaxed_capture():
+                    bad, embedded = torch.zeros(1, dtype=torch.int32, pin_memory=True), torch.cuda.Event()
             m = self.embed(emb, feats, bad)
-            if not capturing:
+            if check:
                 embedded.record()
             try:
                 zw = z[0].to(torch.float32).clone(memory_format=torch.contiguous_format)
                 _run_blocks(self.layers, zw, m, token_mask, msa_mask)
             finally:
-                if not capturing:
-                    embedded.synchronize()                                  # nothing writes to ``bad`` any more
-            if not capturing and bad.item():
+                if check:
+                    with relaxed_capture():
+                        embedded.synchronize()                              # nothing writes to ``bad`` any more
+            if check and bad.item():
                 raise RuntimeError(f"the MSA holds residues outside 0 .. {NUM_TOKENS - 1}")
         return zw[None]
